@@ -32,15 +32,31 @@
 
 /* 2/pi; rintf(x * TECTO_TWO_OVER_PI) is the quadrant of the reduction */
 #define TECTO_TWO_OVER_PI 0.6366197466850281f
+/* pi/2 = C1 + C2 + C3 + C4, C1..C3 with 8 significant bits each */
+#define TECTO_PIO2_C1 1.5703125f
+#define TECTO_PIO2_C2 4.825592041015625e-4f
+#define TECTO_PIO2_C3 1.2665987014770508e-6f
+#define TECTO_PIO2_C4 9.92093629470503e-10f
+/* Taylor coefficients 1/n! with alternating signs */
+#define TECTO_SIN_S3 (-1.6666666666666666e-1f)
+#define TECTO_SIN_S5 8.3333333333333332e-3f
+#define TECTO_SIN_S7 (-1.9841269841269841e-4f)
+#define TECTO_SIN_S9 2.7557319223985893e-6f
+#define TECTO_SIN_S11 (-2.5052108385441720e-8f)
+#define TECTO_COS_K2 (-0.5f)
+#define TECTO_COS_K4 4.1666666666666664e-2f
+#define TECTO_COS_K6 (-1.3888888888888889e-3f)
+#define TECTO_COS_K8 2.4801587301587302e-5f
+#define TECTO_COS_K10 (-2.7557319223985888e-7f)
 
 /* The sine series of the reduced argument r (Taylor coefficients 1/n! with alternating signs). */
 TECTO_HD float tecto_sin_series(float r)
 {
-    const float S3 = -1.6666666666666666e-1f;
-    const float S5 = 8.3333333333333332e-3f;
-    const float S7 = -1.9841269841269841e-4f;
-    const float S9 = 2.7557319223985893e-6f;
-    const float S11 = -2.5052108385441720e-8f;
+    const float S3 = TECTO_SIN_S3;
+    const float S5 = TECTO_SIN_S5;
+    const float S7 = TECTO_SIN_S7;
+    const float S9 = TECTO_SIN_S9;
+    const float S11 = TECTO_SIN_S11;
     const float r2 = r * r;
     float ps = fmaf(r2, S11, S9);
     ps = fmaf(r2, ps, S7);
@@ -56,17 +72,17 @@ TECTO_HD float tecto_sin_series(float r)
 TECTO_HD void tecto_sincos_core(float x, int *q, float *s, float *c)
 {
     /* pi/2 = C1 + C2 + C3 + C4, C1..C3 with 8 significant bits each */
-    const float C1 = 1.5703125f;
-    const float C2 = 4.825592041015625e-4f;
-    const float C3 = 1.2665987014770508e-6f;
-    const float C4 = 9.92093629470503e-10f;
+    const float C1 = TECTO_PIO2_C1;
+    const float C2 = TECTO_PIO2_C2;
+    const float C3 = TECTO_PIO2_C3;
+    const float C4 = TECTO_PIO2_C4;
     const float TWO_OVER_PI = TECTO_TWO_OVER_PI;
     /* Taylor coefficients 1/n! with alternating signs */
-    const float K2 = -0.5f;
-    const float K4 = 4.1666666666666664e-2f;
-    const float K6 = -1.3888888888888889e-3f;
-    const float K8 = 2.4801587301587302e-5f;
-    const float K10 = -2.7557319223985888e-7f;
+    const float K2 = TECTO_COS_K2;
+    const float K4 = TECTO_COS_K4;
+    const float K6 = TECTO_COS_K6;
+    const float K8 = TECTO_COS_K8;
+    const float K10 = TECTO_COS_K10;
 
     const float kf = rintf(x * TWO_OVER_PI);
     float r = fmaf(-kf, C1, x);

@@ -1,0 +1,574 @@
+// k_hydro_march.cu - the hydraulic sub-iteration as a persistent march down column strips, two cells
+// per thread.
+// Reference: rain/flux/flow/sediment/transport/evaporate,
+// src/cuda_compute/plate_tectonics_kernel.cu:2430-2593; driver plate_tectonic_sim.cu:331-373.
+//
+// The same sub-iteration as k_hydro (k_erosion.cu), with no row of the vertical halo computed twice.
+// A block of 256 threads owns a column strip of a world (up to kMarchInner = 120 interior columns, 128
+// with the halo of 4 on each side) and marches down its rows, 4 rows per chunk; a thread owns two
+// adjacent cells of one row (64 pairs a row, a warp is half a row).  With r its first row, a chunk
+// computes
+//   the flux of rows r+7 .. r+10,
+//   the flow, the sediment exchange and the evaporation of rows r+2 .. r+5,
+//   the transport of rows r-4 .. r-1,
+// each from what earlier chunks left in shared memory, so the three are independent of each other (one
+// block barrier per chunk, and the latencies of one hidden by the others).  The height, water and rain
+// of rows r+12 .. r+15 are loaded into registers at the chunk's start and go to shared memory at its
+// end; the old flux and the sediment of the next chunk are loaded where the current ones were used up.
+// Two cells a thread and packed arithmetic take 523 warp-instructions per 64 cells where one cell a
+// thread took 1036; two blocks of up to 128 registers per SM (three blocks of 80 wait on the shared-memory
+// pipe: 990 against 762 us).  One sub-iteration, before and after, us: 2048^2 93.9 -> 72, 4096^2
+// 303 -> 232, 8192^2 1120 -> 858 (4.8 TB/s of DRAM traffic), the 49.7 M cell batch 966 -> 762; with the
+// global accesses taken out 58 / 635 / 566 at 2048^2 / 8192^2 / the batch, so it is bound by issue and
+// shared-memory latency with DRAM close behind.
+// Rows live in rings of 16 rows indexed by the march's own row number (a chunk touches at most 15
+// consecutive rows of a ring).  A piece of a strip starts with three chunks of warm-up; every chunk
+// runs all three stages, and only the stores are limited to the piece's rows.  All strip-rows of the
+// batch are laid end to end and each block takes one contiguous range of them.
+//
+// The per-cell arithmetic is k_hydro's, operation for operation, two cells at a time in packed
+// instructions (pair.cuh).  The packed path holds for operands inside the ranges of the engine's own
+// quotients and roots.  A thread with an operand outside them flags its chunk, and when the piece is
+// done the block runs the rows that the flagged chunks reach once more in the scalar IEEE form, whose
+// results are the same bits wherever the packed form holds (inputs and outputs are different buffers,
+// so a second run of a row starts from the same inputs).
+//
+// Addressing.  A thread keeps one running value P = row * 512 + column * 4 (unsigned, wrapping); the
+// byte offset of a ring cell is P & (ring bytes - 1) plus the ring's base and a constant column step.
+// Lanes read their pair's neighbours without clamping: the edge lanes of a phase compute values that no
+// later phase reads, and the guards around the rings keep every read inside the block's shared memory.
+#include "erosion.cuh"
+#include "pair.cuh"
+
+namespace tecto {
+
+namespace {
+
+// The packed path's constants, both halves equal, in the kernel's parameters: the packed instructions
+// take them from the constant bank, where immediates would occupy register pairs through the march.
+struct PairConst {
+    f2 dt, G, nL, rL, dtA, Kc, Ks, Kd, evap;
+    f2 Z, M, one, mone, half, tiny;  // Z: (-0, -0), see mul2_z; M: 1.5 x 2^23; tiny: 1e-6
+    f2 top, C1, C2, C3, C4;          // 2 / pi and the split of pi / 2
+    f2 S3, S5, S7, S9, S11, K2, K4, K6, K8, K10;
+};
+
+struct PairParams {
+    StripParams sp;
+    PairConst c;
+    int ieee;  // the scalar form throughout: a pipe length outside [2^-32, 2^32] or dt < 0
+};
+
+constexpr int kPairThreads = 256;
+constexpr int kPairRows = 4;       // rows per chunk
+constexpr uint32_t kNz90 = 0x24ffffffu, kNz100 = 0x1affffffu;  // nz_bits of 2^-90 and 2^-100
+constexpr uint32_t kRing = 16;     // rows of a ring
+constexpr uint32_t kRBytes = kRing * kMRow, kRMask = kRBytes - 1;
+constexpr uint32_t kOH = kMGuard;          // height
+constexpr uint32_t kOW = kOH + kRBytes;    // water + rain
+constexpr uint32_t kOS = kOW + kRBytes;    // eroded sediment
+constexpr uint32_t kOX = kOS + kRBytes;    // flux left, +y, right, -y
+constexpr uint32_t kOY = kOX + kRBytes;
+constexpr uint32_t kOZ = kOY + kRBytes;
+constexpr uint32_t kOF = kOZ + kRBytes;
+constexpr uint32_t kOVX = kOF + kRBytes;   // velocity
+constexpr uint32_t kOVY = kOVX + kRBytes;
+constexpr uint32_t kHydroMarchSmem = kOVY + kRBytes + kMGuard;
+static_assert(kPairThreads / 64 == kPairRows && kHydroMarchSmem % 16 == 0, "march: one pair per thread and phase");
+
+// ---- scalar IEEE form ---------------------------------------------------------------------------
+
+__device__ __forceinline__ float4 flux_ieee(const HydroParams &p, float4 f, float h, float w, float hl, float wl,
+                                            float hu, float wu, float hr, float wr, float hd, float wd)
+{
+    const float dt = p.dt, dtA = dt * p.A, G = p.G, L = p.L;
+    const float hw = h + w;
+    const float o0 = fmaxf(0.0f, f.x + dtA * ((G * ((hw - hl) - wl)) / L));
+    const float o1 = fmaxf(0.0f, f.y + dtA * ((G * ((hw - hu) - wu)) / L));
+    const float o2 = fmaxf(0.0f, f.z + dtA * ((G * ((hw - hr) - wr)) / L));
+    const float o3 = fmaxf(0.0f, f.w + dtA * ((G * ((hw - hd) - wd)) / L));
+    const float total = (((o0 + o1) + o2) + o3) + 1e-6f;
+    float K = fminf(1.0f, w / (total * dt + 1e-6f));
+    K = fmaxf(K, 0.01f);
+    return make_float4(o0 * K, o1 * K, o2 * K, o3 * K);
+}
+
+// ---- packed forms ------------------------------------------------------------------------------
+
+// sin(x) of both halves for 0.03 <= x < 2^21: tecto_sinf's reduction and series.  The rounding to the
+// nearest integer is the addition of 1.5 x 2^23 (ties to even, as rintf), whose low bits are the
+// quadrant.
+__device__ __forceinline__ f2 sin2(f2 x, const PairConst &c)
+{
+    const f2 t = add2(mul2_z(x, c.top, c.Z), c.M);
+    const f2 nk = sub2(c.M, t);  // -k
+    f2 r = fma2(nk, c.C1, x);
+    r = fma2(nk, c.C2, r);
+    r = fma2(nk, c.C3, r);
+    r = fma2(nk, c.C4, r);
+    const f2 r2 = mul2(r, r);
+    f2 ps = fma2(r2, c.S11, c.S9);
+    ps = fma2(r2, ps, c.S7);
+    ps = fma2(r2, ps, c.S5);
+    ps = fma2(r2, ps, c.S3);
+    const f2 sn = fma2(mul2(r, r2), ps, r);
+    f2 pc = fma2(r2, c.K10, c.K8);
+    pc = fma2(r2, pc, c.K6);
+    pc = fma2(r2, pc, c.K4);
+    pc = fma2(r2, pc, c.K2);
+    const f2 cs = fma2(r2, pc, c.one);
+    const uint32_t q0 = __float_as_uint(lo(t)), q1 = __float_as_uint(hi(t));
+    const float v0 = (q0 & 1u) ? lo(cs) : lo(sn), v1 = (q1 & 1u) ? hi(cs) : hi(sn);
+    return pk(__uint_as_float(__float_as_uint(v0) ^ ((q0 & 2u) << 30)),
+              __uint_as_float(__float_as_uint(v1) ^ ((q1 & 2u) << 30)));
+}
+
+// base + i elements, in one multiply-add
+template <typename T>
+__device__ __forceinline__ unsigned long long gaddr64(const T *base, uint32_t i)
+{
+    unsigned long long a;
+    asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(a) : "r"(i), "n"((int)sizeof(T)), "l"(base));
+    return a;
+}
+// Loads that stay where they are written (the march's prefetches): two cells of one row; VEC, adjacent
+// and 8-byte aligned (even world width), else `step` apart; and one cell's flux.
+template <bool VEC>
+__device__ __forceinline__ f2 gld2(const float *base, uint32_t i, uint32_t step)
+{
+    if (VEC) {
+        f2 v;
+        asm volatile("ld.global.nc.b64 %0, [%1];" : "=l"(v) : "l"(gaddr64(base, i)));
+        return v;
+    }
+    float x, y;
+    asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(x) : "l"(gaddr64(base, i)));
+    asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(y) : "l"(gaddr64(base, i + step)));
+    return pk(x, y);
+}
+// the fluxes of two cells: VEC, one 32-byte access (a whole sector: two 16-byte halves of it, loaded or
+// stored one after the other, cost twice the L1 and L2 requests)
+template <bool VEC>
+__device__ __forceinline__ void gld_flux(const float4 *base, uint32_t i, uint32_t step, float4 &a, float4 &b)
+{
+    if (VEC) {
+        asm volatile("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                     : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+                     : "l"(gaddr64(base, i)));
+        return;
+    }
+    asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w)
+                 : "l"(gaddr64(base, i)));
+    asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+                 : "l"(gaddr64(base, i + step)));
+}
+// Predicated stores: two cells of one row where s0, s1 (VEC: s0 for both), and one cell's flux.
+template <bool VEC>
+__device__ __forceinline__ void gst2(float *base, uint32_t i, f2 v, bool s0, bool s1)
+{
+    const unsigned long long a = gaddr64(base, i);
+    if (VEC) {
+        if (s0) asm volatile("st.global.b64 [%0], %1;" ::"l"(a), "l"(v) : "memory");
+    } else {
+        if (s0) asm volatile("st.global.f32 [%0], %1;" ::"l"(a), "f"(lo(v)) : "memory");
+        if (s1) asm volatile("st.global.f32 [%0+4], %1;" ::"l"(a), "f"(hi(v)) : "memory");
+    }
+}
+
+template <bool VEC>
+__device__ __forceinline__ void gst_flux(float4 *base, uint32_t i, f2 x, f2 y, f2 z, f2 w, bool s0, bool s1)
+{
+    const unsigned long long a = gaddr64(base, i);
+    if (VEC) {
+        if (s0)
+            asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(a), "f"(lo(x)), "f"(lo(y)),
+                         "f"(lo(z)), "f"(lo(w)), "f"(hi(x)), "f"(hi(y)), "f"(hi(z)), "f"(hi(w))
+                         : "memory");
+        return;
+    }
+    if (s0)
+        asm volatile("st.global.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(a), "f"(lo(x)), "f"(lo(y)), "f"(lo(z)), "f"(lo(w))
+                     : "memory");
+    if (s1)
+        asm volatile("st.global.v4.f32 [%0+16], {%1, %2, %3, %4};" ::"l"(a), "f"(hi(x)), "f"(hi(y)), "f"(hi(z)),
+                     "f"(hi(w))
+                     : "memory");
+}
+
+// Rows [r0, r1) of the strip with interior columns [x0, x0 + iw) of world q.  VEC: the world's width is
+// even.  IEEE: the scalar form, for any operands; else the packed form, which needs p.fastL, dt >= 0 and
+// H >= 4, and leaves in flagged[0], flagged[1] the first and last chunk with an operand outside its
+// ranges.
+template <bool VEC, bool IEEE>
+__device__ __forceinline__ void march_piece(const HydroParams &p, const PairConst &c, const HydroWorld &q, char *S,
+                                            int x0, int iw, int r0, int r1, int *flagged)
+{
+    const int W = q.W, H = q.H;
+    const uint32_t Wu = (uint32_t)W, N = Wu * (uint32_t)H, W4 = 4u * Wu;
+    const f2 Z = c.Z;
+    const int col = 2 * ((int)threadIdx.x & 63), rr = (int)threadIdx.x >> 6;
+    const uint32_t gcol = (uint32_t)wrapc(x0 - 4 + col, W);
+    const uint32_t gstep = VEC ? 1u : (uint32_t)wrapc(x0 - 3 + col, W) - gcol;
+    const int gxi = x0 + col - 4;  // global column of the pair's first cell, interior columns
+    // columns each stage covers: loads [0, iw+8), flux [1, iw+7), flow [2, iw+6), interior [4, iw+4).
+    // A warp with no such column only keeps the barriers; the others run all 32 lanes.
+    const bool in0 = col >= 4 && col < iw + 4, in1 = col >= 4 && col + 1 < iw + 4;
+    const bool live_f = col < iw + 7, live_w = col >= 2 && col < iw + 6;
+    const bool active = __any_sync(0xffffffffu, (col & ~63) < iw + 8);
+    const int K = (r1 - r0 + kPairRows - 1) / kPairRows;
+    const uint32_t nrows = (uint32_t)(r1 - r0);
+    // g + 4 rows, and g - 1 row, wrapped (g < N; the packed forms run where 4 rows are at most N)
+    auto adv = [&](uint32_t g) -> uint32_t {
+        if (IEEE) return (uint32_t)(((unsigned long long)g + 4ull * Wu) % N);
+        const uint32_t v = g + W4;  // < 2N <= 2^31
+        return min(v, v - N);
+    };
+    // Per chunk k (first row rk = r0 + 4k) this thread's base row is t = rk + rr and its items are rows
+    // t + c: flux c = 7, flow c = 2, transport c = -4, and the loads c = 12 (height, water and rain),
+    // c = 11 (old flux) and c = 6 (sediment).
+    constexpr int kFirst = -3;
+    uint32_t P = (uint32_t)(r0 + kFirst * kPairRows + rr) * kMRow + (uint32_t)col * 4u;  // ring value of row t
+    int tr = rr + kFirst * kPairRows;                                                    // t - r0
+    uint32_t B = (uint32_t)(r0 + kFirst * kPairRows + rr) * Wu + (uint32_t)gxi;          // global offset of row t
+    float fy = (float)(r0 + (kFirst - 1) * kPairRows + rr);                              // row t - 4
+    const f2 fgx = pk((float)gxi, (float)(gxi + 1));
+    // ring value of the sediment tap of a floored position (fx, fy) is fy * 512 + (fx - x0 + 4) * 4;
+    // the floors come as the bits of 1.5 x 2^23 + floor
+    const uint32_t tap_c = 0u - (0x4B400000u << 9) - ((0x4B400000u + (uint32_t)(x0 - 4)) << 2);
+    uint32_t g = (uint32_t)wrapc(r0 - 4 + rr, H) * Wu + gcol;    // height row t + 8, then t + 12 ahead
+    uint32_t gs = (uint32_t)wrapc(r0 - 14 + rr, H) * Wu + gcol;  // sediment row t - 2, then t + 2 ahead
+    uint32_t gf = (uint32_t)wrapc(r0 - 5 + rr, H) * Wu + gcol;   // flux row t + 7
+    if (active) {
+        const uint32_t a = (P + 8 * kMRow) & kRMask;
+        st2(S, a + kOH, gld2<VEC>(q.h_in, g, gstep));
+        st2(S, a + kOW, add2(gld2<VEC>(q.w_in, g, gstep), gld2<VEC>(q.rain, g, gstep)));
+        g = adv(g);
+        gs = adv(gs);
+    }
+    f2 lh = 0, lw = 0, lr = 0, ns = 0;
+    float4 fa, fb;  // old flux of this thread's two cells
+    // the loads of the next chunk: its old flux (row t + 7), its sediment (t + 2), and the height, water
+    // and rain that it puts into the rings at its end (t + 12)
+    auto prefetch = [&]() {
+        lh = gld2<VEC>(q.h_in, g, gstep);
+        lw = gld2<VEC>(q.w_in, g, gstep);
+        lr = gld2<VEC>(q.rain, g, gstep);
+        ns = gld2<VEC>(q.s_in, gs, gstep);
+        gld_flux<VEC>(q.f_in, gf, gstep, fa, fb);
+        g = adv(g);
+        gs = adv(gs);
+        gf = adv(gf);
+    };
+    if (active) prefetch();
+    __syncthreads();
+
+#pragma unroll 1
+    for (int k = kFirst; k <= K; ++k) {
+        bool bad = false;  // an operand of this thread outside the packed path's ranges
+        if (active) {
+            // ---- flow, sediment exchange, evaporation ----
+            {
+                const uint32_t a0 = (P + 2 * kMRow) & kRMask, au = (P + 3 * kMRow) & kRMask, ad = (P + kMRow) & kRMask;
+                const uint32_t f0 = a0, fu = au, fd = ad;
+                const f2 sd = ns;
+                f2 hn, wn, s_new, ux, uy;
+                if constexpr (IEEE) {
+                    FlowOut v[2];
+#pragma unroll
+                    for (uint32_t c4 = 0; c4 < 8; c4 += 4) {
+                        const float4 fC = make_float4(mld(S, f0 + c4 + kOX), mld(S, f0 + c4 + kOY), mld(S, f0 + c4 + kOZ),
+                                                      mld(S, f0 + c4 + kOF));
+                        v[c4 >> 2] = flow_cell_general(
+                            p, fC, mld(S, f0 + c4 + kOZ - 4), mld(S, fu + c4 + kOF), mld(S, f0 + c4 + kOX + 4),
+                            mld(S, fd + c4 + kOY), mld(S, fd + c4 + kOF), mld(S, a0 + c4 + kOW), mld(S, a0 + c4 + kOH),
+                            c4 ? hi(sd) : lo(sd), mld(S, a0 + c4 + kOH - 4), mld(S, a0 + c4 + kOH + 4),
+                            mld(S, au + c4 + kOH), mld(S, ad + c4 + kOH));
+                    }
+                    hn = pk(v[0].hn, v[1].hn);
+                    wn = pk(v[0].wn, v[1].wn);
+                    s_new = pk(v[0].s1, v[1].s1);
+                    ux = pk(v[0].ux, v[1].ux);
+                    uy = pk(v[0].uy, v[1].uy);
+                } else {
+                    const f2 cx = ld2(S, f0 + kOX), cy = ld2(S, f0 + kOY), cz = ld2(S, f0 + kOZ), cw = ld2(S, f0 + kOF);
+                    const float lz = mld(S, f0 + kOZ - 4), rx = mld(S, f0 + kOX + 8);
+                    const f2 uw = ld2(S, fu + kOF), dy = ld2(S, fd + kOY), dw = ld2(S, fd + kOF);
+                    const f2 w = ld2(S, a0 + kOW), hc = ld2(S, a0 + kOH);
+                    // flow (:2487-2533); a flux is never -0, so the reference's sum from zero starts at its first term
+                    const f2 in = add2(pk((lz + lo(uw)) + hi(cx), (lo(cz) + hi(uw)) + rx), dy);
+                    const f2 out = add2(add2(add2(cx, cy), cz), cw);
+                    wn = max2(add2(w, mul2_z(c.dt, sub2(in, out), Z)), 0.0f);
+                    const f2 nx = add2(pk(lz - lo(cx), lo(cz) - hi(cx)), cz);
+                    const f2 nfx = mul2(pk(lo(nx) - hi(cx), hi(nx) - rx), c.half);
+                    const f2 nfy = mul2(sub2(add2(sub2(uw, cy), cy), dw), c.half);
+                    const f2 hh = max2(wn, 0.01f);
+                    const f2 nhh = mul2(hh, c.mone);
+                    const f2 rh = rcp2(hh, nhh, c.one);
+                    ux = div2(nfx, nhh, rh);
+                    uy = div2(nfy, nhh, rh);
+                    f2 m2 = add2(mul2_z(ux, ux, Z), mul2_z(uy, uy, Z));
+                    f2 mag = sqrt2(m2, c.half, c.mone);
+                    const bool over = !(lo(m2) <= 0x1p64f) || !(hi(m2) <= 0x1p64f);
+                    const float m0 = lo(mag), m1 = hi(mag);
+                    if (__any_sync(0xffffffffu, m0 > 50.0f || m1 > 50.0f)) {  // the velocity clamp (:2524-2528)
+                        const f2 mc = pk(m0 > 50.0f ? m0 : 50.0f, m1 > 50.0f ? m1 : 50.0f);
+                        const f2 nm = mul2(mc, c.mone);
+                        const f2 sc = div2(dup2(50.0f), nm, rcp2(mc, nm, c.one));  // 1 where there is no clamp
+                        ux = mul2(ux, sc);
+                        uy = mul2(uy, sc);
+                        const f2 mm = add2(mul2_z(ux, ux, Z), mul2_z(uy, uy, Z));
+                        const f2 mr = sqrt2(mm, c.half, c.mone);
+                        mag = pk(m0 > 50.0f ? lo(mr) : m0, m1 > 50.0f ? hi(mr) : m1);
+                    }
+                    // sediment (:2535-2570); the slope reads the pre-erosion height (:351-358)
+                    const f2 dzx = mul2(pk(hi(hc) - mld(S, a0 + kOH - 4), mld(S, a0 + kOH + 8) - lo(hc)), c.half);
+                    const f2 dzy = mul2(sub2(ld2(S, au + kOH), ld2(S, ad + kOH)), c.half);
+                    const f2 s2 = add2(mul2_z(dzx, dzx, Z), mul2_z(dzy, dzy, Z));
+                    const f2 sx = max2(sqrt2(s2, c.half, c.mone), 0.03f);
+                    const f2 C = min2(mul2(mul2(c.Kc, sin2(sx, c)), mag), 5.0f);
+                    const f2 ce = mul2(mul2(c.Ks, sub2(C, sd)), c.dt);
+                    const f2 cd = mul2(mul2(c.Kd, sub2(sd, C)), c.dt);
+                    // what leaves the bed: eroded where the capacity exceeds the sediment, else minus the deposit
+                    const f2 de = pk(lo(C) > lo(sd) ? fminf(lo(ce), lo(hc)) : -fminf(lo(cd), lo(sd)),
+                                     hi(C) > hi(sd) ? fminf(hi(ce), hi(hc)) : -fminf(hi(cd), hi(sd)));
+                    hn = sub2(hc, de);
+                    s_new = add2(sd, de);
+                    // quotients: dividends a zero or at least 2^-90 (one above 2^64 fails the test on m2), depth at
+                // most 2^32; roots: arguments a zero or at least 2^-100; sine argument below 2^21
+                const bool big = !(max3_nan(lo(s2), hi(s2), 0.0f) <= 0x1p42f) || !(fmaxf(lo(hh), hi(hh)) <= 0x1p32f);
+                const float mq = fminf(min3(lo(nfx), hi(nfx), lo(nfy)), fabsf(hi(nfy)));
+                const float ms = fminf(min3(lo(m2), hi(m2), lo(s2)), fabsf(hi(s2)));
+                const bool mine = live_w && (uint32_t)(tr + 4) < nrows + 4u;
+                if (mine && (over || big || mq < 0x1p-90f || ms < 0x1p-100f)) {
+                    const uint32_t zq = min(min(nz_bits(lo(nfx)), nz_bits(hi(nfx))), min(nz_bits(lo(nfy)), nz_bits(hi(nfy))));
+                    const uint32_t zs = min(min(nz_bits(lo(m2)), nz_bits(hi(m2))), min(nz_bits(lo(s2)), nz_bits(hi(s2))));
+                    bad = over || big || zq < kNz90 || zs < kNz100;
+                }
+                }
+                st2(S, a0 + kOS, s_new);
+                st2(S, a0 + kOVX, ux);
+                st2(S, a0 + kOVY, uy);
+                // evaporate (:2587-2593)
+                const f2 wo = max2(sub2(wn, mul2_z(mul2(min2(wn, 20.0f), c.evap), c.dt, Z)), 0.0f);
+                const bool row = (uint32_t)(tr + 2) < nrows, s0 = row && in0, s1 = row && in1;
+                gst2<VEC>(q.h_out, B + 2u * Wu, hn, s0, s1);
+                gst2<VEC>(q.w_out, B + 2u * Wu, wo, s0, s1);
+            }
+            // ---- transport (:2572-2585): bilinear taps within two cells ----
+            {
+                const uint32_t pv = (P - 4 * kMRow) & kRMask;
+                const f2 px = sub2(fgx, mul2_z(ld2(S, pv + kOVX), c.dt, Z));
+                const f2 py = sub2(dup2(fy), mul2_z(ld2(S, pv + kOVY), c.dt, Z));
+                const f2 tx = add2_rm(px, c.M), ty = add2_rm(py, c.M);
+                const f2 wx = sub2(px, sub2(tx, c.M)), wy = sub2(py, sub2(ty, c.M));
+                const f2 vx = sub2(c.one, wx), vy = sub2(c.one, wy);
+                // a tap offset is in [-2, 1] by the velocity clamp; the mask keeps any other inside the ring
+                const uint32_t o0 = tap_c + (__float_as_uint(lo(ty)) << 9) + (__float_as_uint(lo(tx)) << 2);
+                const uint32_t o1 = tap_c + (__float_as_uint(hi(ty)) << 9) + (__float_as_uint(hi(tx)) << 2);
+                const uint32_t u0 = (o0 & kRMask) + kOS, d0 = ((o0 + kMRow) & kRMask) + kOS;
+                const uint32_t u1 = (o1 & kRMask) + kOS, d1 = ((o1 + kMRow) & kRMask) + kOS;
+                const f2 I0 = add2(mul2_z(vx, pk(mld(S, u0), mld(S, u1)), Z), mul2_z(wx, pk(mld(S, u0 + 4), mld(S, u1 + 4)), Z));
+                const f2 I1 = add2(mul2_z(vx, pk(mld(S, d0), mld(S, d1)), Z), mul2_z(wx, pk(mld(S, d0 + 4), mld(S, d1 + 4)), Z));
+                const f2 sn = add2(mul2_z(vy, I0, Z), mul2_z(wy, I1, Z));
+                const bool row = (uint32_t)(tr - 4) < nrows;
+                gst2<VEC>(q.s_out, B - W4, sn, row && in0, row && in1);
+            }
+            // ---- flux (:2439-2485) ----
+            {
+                const uint32_t a0 = (P + 7 * kMRow) & kRMask, au = (P + 8 * kMRow) & kRMask, ad = (P + 6 * kMRow) & kRMask;
+                f2 ox, oy, oz, ow;
+                if constexpr (IEEE) {
+                    float4 v[2];
+#pragma unroll
+                    for (uint32_t c4 = 0; c4 < 8; c4 += 4)
+                        v[c4 >> 2] = flux_ieee(p, c4 ? fb : fa, mld(S, a0 + c4 + kOH), mld(S, a0 + c4 + kOW),
+                                               mld(S, a0 + c4 + kOH - 4), mld(S, a0 + c4 + kOW - 4),
+                                               mld(S, au + c4 + kOH), mld(S, au + c4 + kOW), mld(S, a0 + c4 + kOH + 4),
+                                               mld(S, a0 + c4 + kOW + 4), mld(S, ad + c4 + kOH), mld(S, ad + c4 + kOW));
+                    ox = pk(v[0].x, v[1].x);
+                    oy = pk(v[0].y, v[1].y);
+                    oz = pk(v[0].z, v[1].z);
+                    ow = pk(v[0].w, v[1].w);
+                } else {
+                    const f2 h = ld2(S, a0 + kOH), w = ld2(S, a0 + kOW);
+                    const f2 hw = add2(h, w);
+                    // (left of cell 0, right of cell 1), (right of cell 0, left of cell 1), +y, -y
+                    f2 gA = sub2(sub2(hw, pk(mld(S, a0 + kOH - 4), mld(S, a0 + kOH + 8))),
+                                 pk(mld(S, a0 + kOW - 4), mld(S, a0 + kOW + 8)));
+                    f2 gB = pk((lo(hw) - hi(h)) - hi(w), (hi(hw) - lo(h)) - lo(w));
+                    f2 gU = sub2(sub2(hw, ld2(S, au + kOH)), ld2(S, au + kOW));
+                    f2 gD = sub2(sub2(hw, ld2(S, ad + kOH)), ld2(S, ad + kOW));
+                    const f2 G = c.G;
+                    gA = mul2(G, gA);
+                    gB = mul2(G, gB);
+                    gU = mul2(G, gU);
+                    gD = mul2(G, gD);
+                    const f2 nL = c.nL, rL = c.rL, dtA = c.dtA;
+                    const f2 tA = mul2_z(dtA, div2(gA, nL, rL), Z), tB = mul2_z(dtA, div2(gB, nL, rL), Z);
+                    const f2 tU = mul2_z(dtA, div2(gU, nL, rL), Z), tD = mul2_z(dtA, div2(gD, nL, rL), Z);
+                    // the sign of a zero quotient does not survive the sums and clamps below
+                    ox = pk(fmaxf(0.0f, fa.x + lo(tA)), fmaxf(0.0f, fb.x + hi(tB)));
+                    oy = pk(fmaxf(0.0f, fa.y + lo(tU)), fmaxf(0.0f, fb.y + hi(tU)));
+                    oz = pk(fmaxf(0.0f, fa.z + lo(tB)), fmaxf(0.0f, fb.z + hi(tA)));
+                    ow = pk(fmaxf(0.0f, fa.w + lo(tD)), fmaxf(0.0f, fb.w + hi(tD)));
+                    const f2 total = add2(add2(add2(add2(ox, oy), oz), ow), c.tiny);
+                    const f2 den = add2(mul2_z(total, c.dt, Z), c.tiny);
+                    const f2 nden = mul2(den, c.mone);
+                    const f2 qK = div2(w, nden, rcp2(den, nden, c.one));
+                    const f2 Kf = max2(min2(qK, 1.0f), 0.01f);
+                    // every dividend a zero or in [2^-90, 2^64), the denominators (>= 1e-6) at most 2^32; a water
+                    // below 2^-90 has a quotient far below 0.01, whatever its last bits.  A dividend below 2^-90
+                    // is looked at again: it may be a zero.
+                    const float mx = max3_nan(max3_nan(max3_nan(max3_nan(lo(gA), hi(gA), lo(gB)), hi(gB), lo(gU)), hi(gU),
+                                                       lo(gD)), hi(gD), max3_nan(lo(w), hi(w), 0.0f));
+                    const float mn = min3(min3(min3(lo(gA), hi(gA), lo(gB)), hi(gB), lo(gU)), min3(hi(gU), lo(gD), hi(gD)), 1.0f);
+                    const bool mine = live_f && (uint32_t)(tr + 10) < nrows + 6u;
+                    if (mine && (!(mx < 0x1p64f) || mn < 0x1p-90f || !(fmaxf(lo(den), hi(den)) <= 0x1p32f))) {
+                        const uint32_t z = min(
+                            min(min(nz_bits(lo(gA)), nz_bits(hi(gA))), min(nz_bits(lo(gB)), nz_bits(hi(gB)))),
+                            min(min(nz_bits(lo(gU)), nz_bits(hi(gU))), min(nz_bits(lo(gD)), nz_bits(hi(gD)))));
+                        bad = bad || !(mx < 0x1p64f) || z < kNz90 || !(fmaxf(lo(den), hi(den)) <= 0x1p32f);
+                    }
+                    ox = mul2(ox, Kf);
+                    oy = mul2(oy, Kf);
+                    oz = mul2(oz, Kf);
+                    ow = mul2(ow, Kf);
+                }
+                st2(S, a0 + kOX, ox);
+                st2(S, a0 + kOY, oy);
+                st2(S, a0 + kOZ, oz);
+                st2(S, a0 + kOF, ow);
+                const bool row = (uint32_t)(tr + 7) < nrows, s0 = row && in0, s1 = row && in1;
+                gst_flux<VEC>(q.f_out, B + 7u * Wu, ox, oy, oz, ow, s0, s1);
+            }
+            // ---- the loaded rows ----
+            const uint32_t a = (P + 12 * kMRow) & kRMask;
+            st2(S, a + kOH, lh);
+            st2(S, a + kOW, add2(lw, lr));
+            prefetch();
+        }
+        if (!IEEE && bad) {
+            atomicMin(flagged, k);
+            atomicMax(flagged + 1, k);
+        }
+        __syncthreads();
+        P += kPairRows * kMRow;
+        tr += kPairRows;
+        B += W4;
+        fy = fy + (float)kPairRows;
+    }
+}
+
+__device__ __noinline__ void march_ieee(const PairParams &pp, const HydroWorld &q, char *S, int x0, int iw, int r0,
+                                        int r1)
+{
+    march_piece<false, true>(pp.sp.p, pp.c, q, S, x0, iw, r0, r1, nullptr);
+}
+
+__global__ __launch_bounds__(kPairThreads, 2) void k_hydro_march(const __grid_constant__ PairParams pp)
+{
+    const StripParams &sp = pp.sp;
+    extern __shared__ float4 march_smem[];
+    char *S = reinterpret_cast<char *>(march_smem);
+    __shared__ HydroWorld s_q;
+    __shared__ int s_flag[2];
+    // the edge lanes read ring cells before anything writes them: start from zeros
+    for (uint32_t i = threadIdx.x; i < kHydroMarchSmem / 16; i += kPairThreads)
+        march_smem[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    const unsigned long long nb = gridDim.x;
+    // this block's strip-rows [a0, b0)
+    const unsigned long long a0 = sp.rows * (unsigned long long)blockIdx.x / nb;
+    const unsigned long long b0 = sp.rows * (unsigned long long)(blockIdx.x + 1) / nb;
+    int lo_s = 0, hi_s = sp.nstrips - 1;
+    while (lo_s < hi_s) {
+        const int mid = (lo_s + hi_s + 1) >> 1;
+        if ((unsigned long long)sp.strips[mid].w <= a0) lo_s = mid;
+        else hi_s = mid - 1;
+    }
+    unsigned long long a = a0;
+    for (int s = lo_s; a < b0 && s < sp.nstrips; ++s) {
+        const uint4 d = sp.strips[s];
+        __syncthreads();  // the previous piece is done with s_q and the rings
+        if (threadIdx.x == 0) {
+            s_q = hydro_world(sp.p, sp.p.worlds[d.x]);
+            s_flag[0] = 0x7fffffff;
+            s_flag[1] = -0x7fffffff;
+        }
+        __syncthreads();
+        const unsigned long long first = d.w, last = first + (unsigned long long)s_q.H;
+        if (a >= last) continue;
+        const int r0 = (int)(a - first), r1 = (int)((b0 < last ? b0 : last) - first);
+        const int x0 = (int)d.y, iw = (int)d.z;
+        if (pp.ieee || s_q.H < kPairRows) {
+            march_ieee(pp, s_q, S, x0, iw, r0, r1);
+        } else {
+            if (s_q.W & 1) march_piece<false, false>(sp.p, pp.c, s_q, S, x0, iw, r0, r1, s_flag);
+            else march_piece<true, false>(sp.p, pp.c, s_q, S, x0, iw, r0, r1, s_flag);
+            // the piece's last barrier has passed since the last flag
+            const int k0 = s_flag[0], k1 = s_flag[1];
+            if (k1 >= k0) {
+                // a cell of chunk k (flux rows r+7 .. r+10, flow rows r+2 .. r+5) reaches outputs three rows away
+                __syncthreads();
+                march_ieee(pp, s_q, S, x0, iw, max(r0, r0 + kPairRows * k0),
+                           min(r1, r0 + kPairRows * k1 + 14));
+            }
+        }
+        a = first + (unsigned long long)r1;
+    }
+}
+
+constexpr int kHydroMarchMinRows = 16;
+
+}  // namespace
+
+int hydro_march_attributes()
+{
+    TECTO_CUDA(cudaFuncSetAttribute(k_hydro_march, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kHydroMarchSmem));
+    return TECTO_OK;
+}
+
+void launch_hydro_march(const Batch &b, StripParams sp, cudaStream_t st)
+{
+    sp.nwarps = march_blocks(b, (const void *)k_hydro_march, kPairThreads, kHydroMarchSmem, kHydroMarchMinRows);
+    const HydroParams &p = sp.p;
+    auto d = [](float v) { return pk_host(v); };
+    PairParams pp{};
+    pp.sp = sp;
+    pp.ieee = p.fastL == 0 || !(p.dt >= 0.0f);
+    PairConst &c = pp.c;
+    c.dt = d(p.dt);
+    c.G = d(p.G);
+    c.nL = d(-p.L);
+    c.rL = d(p.rL);
+    c.dtA = d(p.dt * p.A);
+    c.Kc = d(p.Kc);
+    c.Ks = d(p.Ks);
+    c.Kd = d(p.Kd);
+    c.evap = d(p.evap);
+    c.Z = d(-0.0f);
+    c.M = d(12582912.0f);
+    c.one = d(1.0f);
+    c.mone = d(-1.0f);
+    c.half = d(0.5f);
+    c.tiny = d(1e-6f);
+    c.top = d(TECTO_TWO_OVER_PI);
+    c.C1 = d(TECTO_PIO2_C1);
+    c.C2 = d(TECTO_PIO2_C2);
+    c.C3 = d(TECTO_PIO2_C3);
+    c.C4 = d(TECTO_PIO2_C4);
+    c.S3 = d(TECTO_SIN_S3);
+    c.S5 = d(TECTO_SIN_S5);
+    c.S7 = d(TECTO_SIN_S7);
+    c.S9 = d(TECTO_SIN_S9);
+    c.S11 = d(TECTO_SIN_S11);
+    c.K2 = d(TECTO_COS_K2);
+    c.K4 = d(TECTO_COS_K4);
+    c.K6 = d(TECTO_COS_K6);
+    c.K8 = d(TECTO_COS_K8);
+    c.K10 = d(TECTO_COS_K10);
+    k_hydro_march<<<(unsigned)sp.nwarps, kPairThreads, kHydroMarchSmem, st>>>(pp);
+}
+
+}  // namespace tecto

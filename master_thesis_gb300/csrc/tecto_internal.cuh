@@ -343,6 +343,7 @@ constexpr int kHydroVariantCount = 9;
 constexpr int kDefaultHydroVariant = 4;          // 64 x 32 cells, 1024 threads
 constexpr int kHydroStripVariant = 8;            // marching column strips in registers (fused path only)
 constexpr int kHydroMarchVariant = 9;            // marching row chunks in shared memory (fused path only)
+constexpr size_t kMarchMinCells = 1572864;       // cells from which a batch marches by default
 constexpr int kStripInner = 56;                  // interior columns of one register strip (64 with the halo)
 constexpr int kMarchInner = 120;                 // interior columns of one shared-memory strip (128 with it)
 // the strip table of a batch: every member's columns cut into strips of kStripInner columns for

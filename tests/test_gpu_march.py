@@ -1,0 +1,61 @@
+"""The packed marching kernel (hydraulicTile 9) outside the ranges of its packed arithmetic.
+
+Inside them the variant tests compare it with the oracle; here the operands leave them (quotients of tiny
+or huge operands, the velocity clamp, a negative step, a pipe length that the fast quotients do not take),
+so that rows run a second time in the scalar form.  Every field equals the oracle's bit for bit: the
+same IEEE operations in the same order.
+"""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+import master_thesis_gb300 as T
+import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def fields(kind, W, H):
+    rng = np.random.default_rng(W * 131 + H)
+    f32 = np.float32
+    h = rng.normal(0.2, 0.1, (H, W)).astype(f32)
+    water = np.abs(rng.normal(0, 0.2, (H, W))).astype(f32)
+    sed = np.abs(rng.normal(0, 0.05, (H, W))).astype(f32)
+    flux = np.abs(rng.normal(0, 0.02, (H, W, 4))).astype(f32)
+    at = rng.random((H, W)) < 0.02
+    if kind == "tiny":  # level ground, differences and fluxes far below 2^-90, some subnormal
+        h[:] = 0
+        water = (water * 1e-36).astype(f32)
+        flux = (flux * f32(1e-35)).astype(f32)
+        water[at] = 0
+    elif kind == "huge":
+        h[at] = f32(3e24)
+        water[rng.random((H, W)) < 0.02] = f32(8e20)
+    elif kind == "clamp":  # shallow water between strong fluxes: velocities above 50 cells a second
+        water = (water * f32(0.01)).astype(f32)
+        flux[at] *= f32(400)
+    elif kind == "flat":  # zero slopes, zero fluxes, zero quotients of both signs
+        h[:] = f32(0.25)
+        flux[:] = 0
+        water[~at] = 0
+    return h, water, sed, flux
+
+
+@pytest.mark.parametrize("W,H", [(124, 37), (61, 23), (250, 9), (122, 4)])
+@pytest.mark.parametrize("kind", ["tiny", "huge", "clamp", "flat", "backward", "short_pipe"])
+def test_operands_outside_the_packed_ranges(kind, W, H):
+    s = T.baseline_settings()
+    s.step.hydraulicTile = 9
+    dt = -0.02 if kind == "backward" else 0.02
+    if kind == "short_pipe":
+        s.kernel.hydrationPipeLength = 1e-12
+    h, water, sed, flux = fields(kind, W, H)
+    with T.World(s, W, H, seed=1000) as w:
+        for f, a in ((T.FIELD_HEIGHT, h), (T.FIELD_WATER, water), (T.FIELD_SEDIMENT, sed), (T.FIELD_FLUX, flux)):
+            w.upload(f, a)
+        w.hydraulic(3, dt)
+        want = O.hydraulic(h, water, sed, flux, 3, dt, 1000, s)
+        for name, f, v in zip(("height", "water", "sediment", "flux"),
+                              (T.FIELD_HEIGHT, T.FIELD_WATER, T.FIELD_SEDIMENT, T.FIELD_FLUX), want):
+            np.testing.assert_array_equal(w.download(f), v.reshape(w.download(f).shape), err_msg=f"{kind} {name}")
