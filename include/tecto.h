@@ -140,11 +140,11 @@ typedef struct tecto_step_settings {
                                  strips of 120 cells marched down 4 rows at a time by a block of 256
                                  threads, two cells a thread, rows kept in shared memory (8 and 9: the
                                  split path, 50 dt >= 1.5, runs variant 4) */
-    int thermalTile;          /* 0 = autotuner's choice, else 4; 1: 64x32 tiles / 1024 threads, up to 5
+    int thermalTile;          /* 0 = autotuner's choice, else 5 from 2^20 cells and 4 below; 1: 64x32 tiles / 1024 threads, up to 5
                                  iterations per launch; 2: 64x16 / 512, 2 blocks per SM, up to 4;
                                  3: 64x16 / 768, 2 blocks per SM, up to 3; 4: 64x16 / 512, 3 blocks
-                                 per SM, up to 2; 5: column strips of up to 124 cells marched down
-                                 8 rows at a time by a block of 512 threads, one iteration per launch */
+                                 per SM, up to 2; 5: column strips of up to 60 cells marched down by
+                                 one warp each, two cells a lane, one iteration per launch */
     int plateDynamics;        /* TECTO_PLATE_DYNAMICS_*: 0 fixed plate velocities (the benchmark), 1 the
                                  reference's applyPlateMovementChanges after every step */
     int platePolicy;          /* TECTO_PLATE_RELABEL | TECTO_PLATE_MERGE bits, 0 = neither */
@@ -430,7 +430,7 @@ int tecto_batch_phase_thermal(tecto_batch *batch, int iterations, tecto_stream_t
  * (total cells and mean world cells, half-octave classes); batches whose settings leave
  * hydraulicTile / thermalTile / sortRadixBits at 0 use the choice cached for their class, else for
  * the nearest tuned class on their device, else the defaults (hydraulic variant 9 from 1.5 M cells
- * and 4 below, thermal variant 4, 8-bit digits). */
+ * and 4 below, thermal variant 5 from 2^20 cells and 4 below, 8-bit digits). */
 typedef struct tecto_tuning {
     int hydraulicTile;       /* chosen variant, 1..9 */
     int sortRadixBits;       /* chosen digit width, 8..11 */

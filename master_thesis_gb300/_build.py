@@ -31,6 +31,7 @@ SOURCES = [
     "k_resolve.cu",
     "k_erosion.cu",
     "k_hydro_march.cu",
+    "k_thermal_march.cu",
     "k_ccl.cu",
     "tecto_export.cu",
     "tecto_init.cu",

@@ -531,7 +531,7 @@ int hydro_march_attributes()
 
 void launch_hydro_march(const Batch &b, StripParams sp, cudaStream_t st)
 {
-    sp.nwarps = march_blocks(b, (const void *)k_hydro_march, kPairThreads, kHydroMarchSmem, kHydroMarchMinRows);
+    sp.nwarps = march_blocks(b, sp.rows, (const void *)k_hydro_march, kPairThreads, kHydroMarchSmem, kHydroMarchMinRows);
     const HydroParams &p = sp.p;
     auto d = [](float v) { return pk_host(v); };
     PairParams pp{};

@@ -34,12 +34,10 @@ void build_tiles(const Batch &b, int kind, std::vector<uint2> &out)
     }
 }
 
-}  // namespace
-
-void build_strips(const Batch &b, std::vector<uint4> &out, unsigned long long *rows)
+// every member's columns cut into strips of `inner`
+std::vector<uint4> build_strips(const Batch &b, int inner, unsigned long long *rows)
 {
-    out.clear();
-    const int inner = b.hydro_variant == kHydroStripVariant ? kStripInner : kMarchInner;
+    std::vector<uint4> out;
     unsigned long long r = 0;
     for (size_t wi = 0; wi < b.members.size(); ++wi) {
         const tecto_world *w = b.members[wi];
@@ -50,9 +48,8 @@ void build_strips(const Batch &b, std::vector<uint4> &out, unsigned long long *r
         }
     }
     *rows = r;
+    return out;
 }
-
-namespace {
 
 // Copy the state of group `g` (0 height, 1 water/sediment/flux, 2 plate ids) of world w into
 // ping-pong half `to`.
@@ -166,13 +163,16 @@ void batch_release(Batch &b)
 
 // Tile variant and digit width: explicit settings first, then the autotuner's choice for this
 // batch (or its cached choice for the shape class), then the defaults.
+// The default thermal variant: one iteration with tiles (variant 4, two iterations a launch) against the
+// march (5), us: 512^2 5.3 / 6.5, 1024^2 11.6 / 11.0, 2048^2 37.4 / 23.0, 8192^2 570 / 230.
 // The default hydraulic variant follows the batch's cells: one sub-iteration with tiles (variant 4)
 // against the march (9), us: 256^2 12.7 / 14.1, 1024^2 31.2 / 31.1, 1200x1000 31.8 / 33.2, 1101x1301
 // 41.2 / 41.5, 1500x1100 45.4 / 37.5, 2048^2 103 / 72, 8192^2 1446 / 858, a 49.7 M cell batch 1269 / 762.
 static void choose_tuning(const Batch &b, int *variant, int *rb, int *tvariant)
 {
     *tvariant = thermal_variant_for(b.settings);
-    if (*tvariant == 0) *tvariant = b.tuned_thermal ? b.tuned_thermal : kDefaultThermalVariant;
+    if (*tvariant == 0) *tvariant = b.tuned_thermal;
+    if (*tvariant == 0) *tvariant = b.total >= kThermalMarchMinCells ? kThermalMarchVariant : kDefaultThermalVariant;
     *variant = hydro_variant_for(b.settings);
     if (*variant == 0) *variant = b.tuned_hydro;
     if (*variant == 0) *variant = b.total >= kMarchMinCells ? kHydroMarchVariant : kDefaultHydroVariant;
@@ -232,10 +232,13 @@ int batch_prepare(Batch &b, cudaStream_t st)
         b.ntiles[k] = (int)tiles[k].size();
         need += a256(tiles[k].size() * sizeof(uint2));
     }
-    std::vector<uint4> strips;
-    build_strips(b, strips, &b.strip_rows);
-    b.nstrips = (int)strips.size();
-    need += a256(strips.size() * sizeof(uint4));
+    std::vector<uint4> strips[ST_COUNT];
+    for (int k = 0; k < ST_COUNT; ++k) {
+        const int inner = k == ST_THERMAL ? kThermalInner : variant == kHydroStripVariant ? kStripInner : kMarchInner;
+        strips[k] = build_strips(b, inner, &b.strips[k].rows);
+        b.strips[k].n = (int)strips[k].size();
+        need += a256(strips[k].size() * sizeof(uint4));
+    }
     if (need > b.table_bytes) {
         if (b.table_arena) cudaFree(b.table_arena);
         b.table_arena = nullptr;
@@ -252,15 +255,18 @@ int batch_prepare(Batch &b, cudaStream_t st)
         b.d_tiles[k] = (uint2 *)p;
         p += a256(tiles[k].size() * sizeof(uint2));
     }
-    b.d_strips = (uint4 *)p;
-    p += a256(strips.size() * sizeof(uint4));
+    for (int k = 0; k < ST_COUNT; ++k) {
+        b.strips[k].d = (uint4 *)p;
+        p += a256(strips[k].size() * sizeof(uint4));
+    }
     TECTO_CUDA(cudaMemcpyAsync(b.d_worlds, table.data(), n * sizeof(WorldDev), cudaMemcpyHostToDevice, st));
     TECTO_CUDA(cudaMemcpyAsync(b.d_vbase, vbase.data(), (n + 1) * 4, cudaMemcpyHostToDevice, st));
     for (int k = 0; k < TK_COUNT; ++k)
         TECTO_CUDA(cudaMemcpyAsync(b.d_tiles[k], tiles[k].data(), tiles[k].size() * sizeof(uint2),
                                    cudaMemcpyHostToDevice, st));
-    TECTO_CUDA(cudaMemcpyAsync(b.d_strips, strips.data(), strips.size() * sizeof(uint4), cudaMemcpyHostToDevice,
-                               st));
+    for (int k = 0; k < ST_COUNT; ++k)
+        TECTO_CUDA(cudaMemcpyAsync(b.strips[k].d, strips[k].data(), strips[k].size() * sizeof(uint4),
+                                   cudaMemcpyHostToDevice, st));
     // batch-level buffers: key/value ping-pong for `capacity` cells, the control block, then the
     // sort scratch of the current size and digit width
     const int kb = key_bits_for(total);

@@ -162,6 +162,15 @@ enum TileKind { TK_RESOLVE = 0, TK_THERMAL, TK_HYDRO, TK_CCL, TK_STATS, TK_COUNT
 // CCL tiles: one warp per row of kCclTileX cells, kCclTileY rows per block
 constexpr int kCclTileX = 32, kCclTileY = 32;
 
+// Column strips of a marching kernel over a batch: {world, first column, interior width, first
+// strip-row}, strip-rows counted over all strips.
+enum StripKind { ST_HYDRO = 0, ST_THERMAL, ST_COUNT };
+struct StripTable {
+    uint4 *d = nullptr;
+    int n = 0;
+    unsigned long long rows = 0;
+};
+
 // One batch: members, their device table, work lists and the batch-level buffers.
 struct Batch {
     std::vector<tecto_world *> members;
@@ -183,11 +192,7 @@ struct Batch {
     uint32_t *d_vbase = nullptr;             // [n + 1] ascending virtual bases, last = total
     uint2 *d_tiles[TK_COUNT] = {};           // (world, ty << 16 | tx)
     int ntiles[TK_COUNT] = {};
-    // column strips of the marching hydraulic kernel (hydraulic variant kHydroStripVariant):
-    // {world, first column, interior width, first strip-row}, strip-rows counted over all strips
-    uint4 *d_strips = nullptr;
-    int nstrips = 0;
-    unsigned long long strip_rows = 0;
+    StripTable strips[ST_COUNT];             // column strips of the marching kernels
     void *table_arena = nullptr;
     size_t table_bytes = 0;
     // batch-level buffers, sized for `capacity` cells
@@ -343,15 +348,14 @@ constexpr int kHydroVariantCount = 9;
 constexpr int kDefaultHydroVariant = 4;          // 64 x 32 cells, 1024 threads
 constexpr int kHydroStripVariant = 8;            // marching column strips in registers (fused path only)
 constexpr int kHydroMarchVariant = 9;            // marching row chunks in shared memory (fused path only)
-constexpr size_t kMarchMinCells = 1572864;       // cells from which a batch marches by default
+constexpr size_t kMarchMinCells = 1572864;       // cells from which the hydraulic march is the default
 constexpr int kStripInner = 56;                  // interior columns of one register strip (64 with the halo)
 constexpr int kMarchInner = 120;                 // interior columns of one shared-memory strip (128 with it)
-// the strip table of a batch: every member's columns cut into strips of kStripInner columns for
-// kHydroStripVariant, of kMarchInner otherwise (the marching hydraulic and thermal kernels)
-void build_strips(const Batch &b, std::vector<uint4> &out, unsigned long long *rows);
+constexpr int kThermalInner = 60;                // interior columns of one thermal strip (64 with the halo)
 constexpr int kThermalVariantCount = 5;
 constexpr int kDefaultThermalVariant = 4;        // 64 x 16 cells, 512 threads, 2 iterations per launch
-constexpr int kThermalMarchVariant = 5;          // marching row chunks down column strips, one iteration per launch
+constexpr size_t kThermalMarchMinCells = 1 << 20;  // cells from which the thermal march is the default
+constexpr int kThermalMarchVariant = 5;          // warps marching down column strips, one iteration per launch
 int thermal_variant_for(const tecto_settings &s);  // 0 when the settings leave the choice open
 
 // Autotuner cache (tecto_tune.cu): best hydraulic tile variant and sort digit width for a batch

@@ -1,9 +1,10 @@
-"""The packed marching kernel (hydraulicTile 9) outside the ranges of its packed arithmetic.
+"""The packed marching kernels (hydraulicTile 9, thermalTile 5) at the edges of their packed arithmetic.
 
 Inside them the variant tests compare it with the oracle; here the operands leave them (quotients of tiny
 or huge operands, the velocity clamp, a negative step, a pipe length that the fast quotients do not take),
 so that rows run a second time in the scalar form.  Every field equals the oracle's bit for bit: the
-same IEEE operations in the same order.
+same IEEE operations in the same order.  The thermal march has three forms by its parameters, and runs a
+piece again where a slope sum is above 2^32.
 """
 from __future__ import annotations
 
@@ -59,3 +60,27 @@ def test_operands_outside_the_packed_ranges(kind, W, H):
         for name, f, v in zip(("height", "water", "sediment", "flux"),
                               (T.FIELD_HEIGHT, T.FIELD_WATER, T.FIELD_SEDIMENT, T.FIELD_FLUX), want):
             np.testing.assert_array_equal(w.download(f), v.reshape(w.download(f).shape), err_msg=f"{kind} {name}")
+
+
+# (threshold angle, amplitude, strength): the packed form with the amplitude folded in, the packed form,
+# the scalar form for a threshold below 2^-32
+@pytest.mark.parametrize("thr,A,S", [(0.01, 0.5, 1.0), (0.01, 2.0**-9, 1.0), (0.01, 0.3, 1.0), (0.01, 0.5, 0.7),
+                                     (1e-12, 0.5, 1.0)])
+@pytest.mark.parametrize("W,H", [(64, 7), (60, 1), (61, 50), (122, 2), (187, 33)])
+@pytest.mark.parametrize("kind", ["rough", "flat", "huge"])
+def test_thermal_march_forms(kind, W, H, thr, A, S):
+    s = T.baseline_settings()
+    s.step.thermalTile = 5
+    s.kernel.thermalThresholdAngle, s.kernel.thermalCellSize = thr, 1.0
+    s.kernel.thermalErosionAmplitude, s.kernel.thermalErosionStrength = A, S
+    rng = np.random.default_rng(W * 17 + H)
+    h = rng.normal(0, 0.1, (H, W)).astype(np.float32)
+    if kind == "flat":  # zeros of both signs, a few peaks
+        h = np.where(rng.random((H, W)) < 0.1, h, np.where(rng.random((H, W)) < 0.5, 0.0, -0.0)).astype(np.float32)
+    elif kind == "huge":
+        h[rng.random((H, W)) < 0.01] = 3e10
+    with T.World(s, W, H, seed=1000) as w:
+        w.upload(T.FIELD_HEIGHT, h)
+        w.thermal(3)
+        got, want = w.download(T.FIELD_HEIGHT), O.thermal(h, 3, s).reshape(H, W)
+    np.testing.assert_array_equal(got.view(np.uint32), want.view(np.uint32))
