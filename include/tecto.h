@@ -133,13 +133,12 @@ typedef struct tecto_step_settings {
     int upliftRadius;         /* taps on each side (<= 8) */
     int cclConnectivity;      /* TECTO_CCL_* */
     int sortRadixBits;        /* collision sort digit width 8..11; 0 = autotuner's choice, else 8 */
-    int hydraulicTile;        /* 0 = autotuner's choice, else 9 from 1.5 M cells and 4 below; 1: 64x16/256 threads, 2: 64x32/256,
-                                 3: 64x32/512, 4: 64x32/1024, 5: 64x64/1024, 6: 64x16/512 (3 blocks
-                                 per SM), 7: 64x16/384 (4 blocks per SM), 8: column strips of 56
-                                 cells marched down by one warp each, no block barriers, 9: column
-                                 strips of 120 cells marched down 4 rows at a time by a block of 256
-                                 threads, two cells a thread, rows kept in shared memory (8 and 9: the
-                                 split path, 50 dt >= 1.5, runs variant 4) */
+    int hydraulicTile;        /* 0 = autotuner's choice, else by the batch's cells: 1 up to 2^17, 3 up to
+                                 2^20, 4 up to 2.5 M, then 9.  Tiles of cells / warps, two cells a lane:
+                                 1: 56x8/16, 2: 56x8/8, 3: 56x16/8, 4: 56x24/8, 5: 56x32/10, 6: 56x16/6,
+                                 7: 56x4/12; 9 (and 8): column strips of 120 cells marched down 4 rows at
+                                 a time by a block of 256 threads, two cells a thread, rows kept in shared
+                                 memory (the split path, 50 dt >= 1.5, runs variant 4) */
     int thermalTile;          /* 0 = autotuner's choice, else 5 from 2^20 cells and 4 below; 1: 64x32 tiles / 1024 threads, up to 5
                                  iterations per launch; 2: 64x16 / 512, 2 blocks per SM, up to 4;
                                  3: 64x16 / 768, 2 blocks per SM, up to 3; 4: 64x16 / 512, 3 blocks
@@ -429,8 +428,8 @@ int tecto_batch_phase_thermal(tecto_batch *batch, int iterations, tecto_stream_t
  * The caller's worlds are not touched.  The choice is cached per device and batch shape class
  * (total cells and mean world cells, half-octave classes); batches whose settings leave
  * hydraulicTile / thermalTile / sortRadixBits at 0 use the choice cached for their class, else for
- * the nearest tuned class on their device, else the defaults (hydraulic variant 9 from 1.5 M cells
- * and 4 below, thermal variant 5 from 2^20 cells and 4 below, 8-bit digits). */
+ * the nearest tuned class on their device, else the defaults (by the batch's
+ * cells, see hydraulicTile and thermalTile; 8-bit digits). */
 typedef struct tecto_tuning {
     int hydraulicTile;       /* chosen variant, 1..9 */
     int sortRadixBits;       /* chosen digit width, 8..11 */

@@ -30,6 +30,7 @@ SOURCES = [
     "k_policy.cu",
     "k_resolve.cu",
     "k_erosion.cu",
+    "k_hydro_tile.cu",
     "k_hydro_march.cu",
     "k_thermal_march.cu",
     "k_ccl.cu",

@@ -37,21 +37,11 @@
 // byte offset of a ring cell is P & (ring bytes - 1) plus the ring's base and a constant column step.
 // Lanes read their pair's neighbours without clamping: the edge lanes of a phase compute values that no
 // later phase reads, and the guards around the rings keep every read inside the block's shared memory.
-#include "erosion.cuh"
-#include "pair.cuh"
+#include "hydro_pair.cuh"
 
 namespace tecto {
 
 namespace {
-
-// The packed path's constants, both halves equal, in the kernel's parameters: the packed instructions
-// take them from the constant bank, where immediates would occupy register pairs through the march.
-struct PairConst {
-    f2 dt, G, nL, rL, dtA, Kc, Ks, Kd, evap;
-    f2 Z, M, one, mone, half, tiny;  // Z: (-0, -0), see mul2_z; M: 1.5 x 2^23; tiny: 1e-6
-    f2 top, C1, C2, C3, C4;          // 2 / pi and the split of pi / 2
-    f2 S3, S5, S7, S9, S11, K2, K4, K6, K8, K10;
-};
 
 struct PairParams {
     StripParams sp;
@@ -61,7 +51,6 @@ struct PairParams {
 
 constexpr int kPairThreads = 256;
 constexpr int kPairRows = 4;       // rows per chunk
-constexpr uint32_t kNz90 = 0x24ffffffu, kNz100 = 0x1affffffu;  // nz_bits of 2^-90 and 2^-100
 constexpr uint32_t kRing = 16;     // rows of a ring
 constexpr uint32_t kRBytes = kRing * kMRow, kRMask = kRBytes - 1;
 constexpr uint32_t kOH = kMGuard;          // height
@@ -76,61 +65,6 @@ constexpr uint32_t kOVY = kOVX + kRBytes;
 constexpr uint32_t kHydroMarchSmem = kOVY + kRBytes + kMGuard;
 static_assert(kPairThreads / 64 == kPairRows && kHydroMarchSmem % 16 == 0, "march: one pair per thread and phase");
 
-// ---- scalar IEEE form ---------------------------------------------------------------------------
-
-__device__ __forceinline__ float4 flux_ieee(const HydroParams &p, float4 f, float h, float w, float hl, float wl,
-                                            float hu, float wu, float hr, float wr, float hd, float wd)
-{
-    const float dt = p.dt, dtA = dt * p.A, G = p.G, L = p.L;
-    const float hw = h + w;
-    const float o0 = fmaxf(0.0f, f.x + dtA * ((G * ((hw - hl) - wl)) / L));
-    const float o1 = fmaxf(0.0f, f.y + dtA * ((G * ((hw - hu) - wu)) / L));
-    const float o2 = fmaxf(0.0f, f.z + dtA * ((G * ((hw - hr) - wr)) / L));
-    const float o3 = fmaxf(0.0f, f.w + dtA * ((G * ((hw - hd) - wd)) / L));
-    const float total = (((o0 + o1) + o2) + o3) + 1e-6f;
-    float K = fminf(1.0f, w / (total * dt + 1e-6f));
-    K = fmaxf(K, 0.01f);
-    return make_float4(o0 * K, o1 * K, o2 * K, o3 * K);
-}
-
-// ---- packed forms ------------------------------------------------------------------------------
-
-// sin(x) of both halves for 0.03 <= x < 2^21: tecto_sinf's reduction and series.  The rounding to the
-// nearest integer is the addition of 1.5 x 2^23 (ties to even, as rintf), whose low bits are the
-// quadrant.
-__device__ __forceinline__ f2 sin2(f2 x, const PairConst &c)
-{
-    const f2 t = add2(mul2_z(x, c.top, c.Z), c.M);
-    const f2 nk = sub2(c.M, t);  // -k
-    f2 r = fma2(nk, c.C1, x);
-    r = fma2(nk, c.C2, r);
-    r = fma2(nk, c.C3, r);
-    r = fma2(nk, c.C4, r);
-    const f2 r2 = mul2(r, r);
-    f2 ps = fma2(r2, c.S11, c.S9);
-    ps = fma2(r2, ps, c.S7);
-    ps = fma2(r2, ps, c.S5);
-    ps = fma2(r2, ps, c.S3);
-    const f2 sn = fma2(mul2(r, r2), ps, r);
-    f2 pc = fma2(r2, c.K10, c.K8);
-    pc = fma2(r2, pc, c.K6);
-    pc = fma2(r2, pc, c.K4);
-    pc = fma2(r2, pc, c.K2);
-    const f2 cs = fma2(r2, pc, c.one);
-    const uint32_t q0 = __float_as_uint(lo(t)), q1 = __float_as_uint(hi(t));
-    const float v0 = (q0 & 1u) ? lo(cs) : lo(sn), v1 = (q1 & 1u) ? hi(cs) : hi(sn);
-    return pk(__uint_as_float(__float_as_uint(v0) ^ ((q0 & 2u) << 30)),
-              __uint_as_float(__float_as_uint(v1) ^ ((q1 & 2u) << 30)));
-}
-
-// base + i elements, in one multiply-add
-template <typename T>
-__device__ __forceinline__ unsigned long long gaddr64(const T *base, uint32_t i)
-{
-    unsigned long long a;
-    asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(a) : "r"(i), "n"((int)sizeof(T)), "l"(base));
-    return a;
-}
 // Loads that stay where they are written (the march's prefetches): two cells of one row; VEC, adjacent
 // and 8-byte aligned (even world width), else `step` apart; and one cell's flux.
 template <bool VEC>
@@ -164,39 +98,6 @@ __device__ __forceinline__ void gld_flux(const float4 *base, uint32_t i, uint32_
                  : "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
                  : "l"(gaddr64(base, i + step)));
 }
-// Predicated stores: two cells of one row where s0, s1 (VEC: s0 for both), and one cell's flux.
-template <bool VEC>
-__device__ __forceinline__ void gst2(float *base, uint32_t i, f2 v, bool s0, bool s1)
-{
-    const unsigned long long a = gaddr64(base, i);
-    if (VEC) {
-        if (s0) asm volatile("st.global.b64 [%0], %1;" ::"l"(a), "l"(v) : "memory");
-    } else {
-        if (s0) asm volatile("st.global.f32 [%0], %1;" ::"l"(a), "f"(lo(v)) : "memory");
-        if (s1) asm volatile("st.global.f32 [%0+4], %1;" ::"l"(a), "f"(hi(v)) : "memory");
-    }
-}
-
-template <bool VEC>
-__device__ __forceinline__ void gst_flux(float4 *base, uint32_t i, f2 x, f2 y, f2 z, f2 w, bool s0, bool s1)
-{
-    const unsigned long long a = gaddr64(base, i);
-    if (VEC) {
-        if (s0)
-            asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(a), "f"(lo(x)), "f"(lo(y)),
-                         "f"(lo(z)), "f"(lo(w)), "f"(hi(x)), "f"(hi(y)), "f"(hi(z)), "f"(hi(w))
-                         : "memory");
-        return;
-    }
-    if (s0)
-        asm volatile("st.global.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(a), "f"(lo(x)), "f"(lo(y)), "f"(lo(z)), "f"(lo(w))
-                     : "memory");
-    if (s1)
-        asm volatile("st.global.v4.f32 [%0+16], {%1, %2, %3, %4};" ::"l"(a), "f"(hi(x)), "f"(hi(y)), "f"(hi(z)),
-                     "f"(hi(w))
-                     : "memory");
-}
-
 // Rows [r0, r1) of the strip with interior columns [x0, x0 + iw) of world q.  VEC: the world's width is
 // even.  IEEE: the scalar form, for any operands; else the packed form, which needs p.fastL, dt >= 0 and
 // H >= 4, and leaves in flagged[0], flagged[1] the first and last chunk with an operand outside its
@@ -268,6 +169,25 @@ __device__ __forceinline__ void march_piece(const HydroParams &p, const PairCons
     for (int k = kFirst; k <= K; ++k) {
         bool bad = false;  // an operand of this thread outside the packed path's ranges
         if (active) {
+            // ---- transport (:2572-2585): bilinear taps within two cells ----
+            {
+                const uint32_t pv = (P - 4 * kMRow) & kRMask;
+                const f2 px = sub2(fgx, mul2_z(ld2(S, pv + kOVX), c.dt, Z));
+                const f2 py = sub2(dup2(fy), mul2_z(ld2(S, pv + kOVY), c.dt, Z));
+                const f2 tx = add2_rm(px, c.M), ty = add2_rm(py, c.M);
+                const f2 wx = sub2(px, sub2(tx, c.M)), wy = sub2(py, sub2(ty, c.M));
+                const f2 vx = sub2(c.one, wx), vy = sub2(c.one, wy);
+                // a tap offset is in [-2, 1] by the velocity clamp; the mask keeps any other inside the ring
+                const uint32_t o0 = tap_c + (__float_as_uint(lo(ty)) << 9) + (__float_as_uint(lo(tx)) << 2);
+                const uint32_t o1 = tap_c + (__float_as_uint(hi(ty)) << 9) + (__float_as_uint(hi(tx)) << 2);
+                const uint32_t u0 = (o0 & kRMask) + kOS, d0 = ((o0 + kMRow) & kRMask) + kOS;
+                const uint32_t u1 = (o1 & kRMask) + kOS, d1 = ((o1 + kMRow) & kRMask) + kOS;
+                const f2 I0 = add2(mul2_z(vx, pk(mld(S, u0), mld(S, u1)), Z), mul2_z(wx, pk(mld(S, u0 + 4), mld(S, u1 + 4)), Z));
+                const f2 I1 = add2(mul2_z(vx, pk(mld(S, d0), mld(S, d1)), Z), mul2_z(wx, pk(mld(S, d0 + 4), mld(S, d1 + 4)), Z));
+                const f2 sn = add2(mul2_z(vy, I0, Z), mul2_z(wy, I1, Z));
+                const bool row = (uint32_t)(tr - 4) < nrows;
+                gst2<VEC>(q.s_out, B - W4, sn, row && in0, row && in1);
+            }
             // ---- flow, sediment exchange, evaporation ----
             {
                 const uint32_t a0 = (P + 2 * kMRow) & kRMask, au = (P + 3 * kMRow) & kRMask, ad = (P + kMRow) & kRMask;
@@ -292,88 +212,23 @@ __device__ __forceinline__ void march_piece(const HydroParams &p, const PairCons
                     ux = pk(v[0].ux, v[1].ux);
                     uy = pk(v[0].uy, v[1].uy);
                 } else {
-                    const f2 cx = ld2(S, f0 + kOX), cy = ld2(S, f0 + kOY), cz = ld2(S, f0 + kOZ), cw = ld2(S, f0 + kOF);
-                    const float lz = mld(S, f0 + kOZ - 4), rx = mld(S, f0 + kOX + 8);
-                    const f2 uw = ld2(S, fu + kOF), dy = ld2(S, fd + kOY), dw = ld2(S, fd + kOF);
-                    const f2 w = ld2(S, a0 + kOW), hc = ld2(S, a0 + kOH);
-                    // flow (:2487-2533); a flux is never -0, so the reference's sum from zero starts at its first term
-                    const f2 in = add2(pk((lz + lo(uw)) + hi(cx), (lo(cz) + hi(uw)) + rx), dy);
-                    const f2 out = add2(add2(add2(cx, cy), cz), cw);
-                    wn = max2(add2(w, mul2_z(c.dt, sub2(in, out), Z)), 0.0f);
-                    const f2 nx = add2(pk(lz - lo(cx), lo(cz) - hi(cx)), cz);
-                    const f2 nfx = mul2(pk(lo(nx) - hi(cx), hi(nx) - rx), c.half);
-                    const f2 nfy = mul2(sub2(add2(sub2(uw, cy), cy), dw), c.half);
-                    const f2 hh = max2(wn, 0.01f);
-                    const f2 nhh = mul2(hh, c.mone);
-                    const f2 rh = rcp2(hh, nhh, c.one);
-                    ux = div2(nfx, nhh, rh);
-                    uy = div2(nfy, nhh, rh);
-                    f2 m2 = add2(mul2_z(ux, ux, Z), mul2_z(uy, uy, Z));
-                    f2 mag = sqrt2(m2, c.half, c.mone);
-                    const bool over = !(lo(m2) <= 0x1p64f) || !(hi(m2) <= 0x1p64f);
-                    const float m0 = lo(mag), m1 = hi(mag);
-                    if (__any_sync(0xffffffffu, m0 > 50.0f || m1 > 50.0f)) {  // the velocity clamp (:2524-2528)
-                        const f2 mc = pk(m0 > 50.0f ? m0 : 50.0f, m1 > 50.0f ? m1 : 50.0f);
-                        const f2 nm = mul2(mc, c.mone);
-                        const f2 sc = div2(dup2(50.0f), nm, rcp2(mc, nm, c.one));  // 1 where there is no clamp
-                        ux = mul2(ux, sc);
-                        uy = mul2(uy, sc);
-                        const f2 mm = add2(mul2_z(ux, ux, Z), mul2_z(uy, uy, Z));
-                        const f2 mr = sqrt2(mm, c.half, c.mone);
-                        mag = pk(m0 > 50.0f ? lo(mr) : m0, m1 > 50.0f ? hi(mr) : m1);
-                    }
-                    // sediment (:2535-2570); the slope reads the pre-erosion height (:351-358)
-                    const f2 dzx = mul2(pk(hi(hc) - mld(S, a0 + kOH - 4), mld(S, a0 + kOH + 8) - lo(hc)), c.half);
-                    const f2 dzy = mul2(sub2(ld2(S, au + kOH), ld2(S, ad + kOH)), c.half);
-                    const f2 s2 = add2(mul2_z(dzx, dzx, Z), mul2_z(dzy, dzy, Z));
-                    const f2 sx = max2(sqrt2(s2, c.half, c.mone), 0.03f);
-                    const f2 C = min2(mul2(mul2(c.Kc, sin2(sx, c)), mag), 5.0f);
-                    const f2 ce = mul2(mul2(c.Ks, sub2(C, sd)), c.dt);
-                    const f2 cd = mul2(mul2(c.Kd, sub2(sd, C)), c.dt);
-                    // what leaves the bed: eroded where the capacity exceeds the sediment, else minus the deposit
-                    const f2 de = pk(lo(C) > lo(sd) ? fminf(lo(ce), lo(hc)) : -fminf(lo(cd), lo(sd)),
-                                     hi(C) > hi(sd) ? fminf(hi(ce), hi(hc)) : -fminf(hi(cd), hi(sd)));
-                    hn = sub2(hc, de);
-                    s_new = add2(sd, de);
-                    // quotients: dividends a zero or at least 2^-90 (one above 2^64 fails the test on m2), depth at
-                // most 2^32; roots: arguments a zero or at least 2^-100; sine argument below 2^21
-                const bool big = !(max3_nan(lo(s2), hi(s2), 0.0f) <= 0x1p42f) || !(fmaxf(lo(hh), hi(hh)) <= 0x1p32f);
-                const float mq = fminf(min3(lo(nfx), hi(nfx), lo(nfy)), fabsf(hi(nfy)));
-                const float ms = fminf(min3(lo(m2), hi(m2), lo(s2)), fabsf(hi(s2)));
-                const bool mine = live_w && (uint32_t)(tr + 4) < nrows + 4u;
-                if (mine && (over || big || mq < 0x1p-90f || ms < 0x1p-100f)) {
-                    const uint32_t zq = min(min(nz_bits(lo(nfx)), nz_bits(hi(nfx))), min(nz_bits(lo(nfy)), nz_bits(hi(nfy))));
-                    const uint32_t zs = min(min(nz_bits(lo(m2)), nz_bits(hi(m2))), min(nz_bits(lo(s2)), nz_bits(hi(s2))));
-                    bad = over || big || zq < kNz90 || zs < kNz100;
-                }
+                    Flow2 o;
+                    const Flux2 fc{ld2(S, f0 + kOX), ld2(S, f0 + kOY), ld2(S, f0 + kOZ), ld2(S, f0 + kOF)};
+                    const bool mine = live_w && (uint32_t)(tr + 4) < nrows + 4u;
+                    bad = flow_pair(c, fc, mld(S, f0 + kOZ - 4), mld(S, f0 + kOX + 8), ld2(S, fu + kOF),
+                                    ld2(S, fd + kOY), ld2(S, fd + kOF), ld2(S, a0 + kOW), ld2(S, a0 + kOH),
+                                    mld(S, a0 + kOH - 4), mld(S, a0 + kOH + 8), ld2(S, au + kOH), ld2(S, ad + kOH), sd,
+                                    mine, o) || bad;
+                    hn = o.hn, wn = o.wn, s_new = o.s1, ux = o.ux, uy = o.uy;
                 }
                 st2(S, a0 + kOS, s_new);
                 st2(S, a0 + kOVX, ux);
                 st2(S, a0 + kOVY, uy);
                 // evaporate (:2587-2593)
-                const f2 wo = max2(sub2(wn, mul2_z(mul2(min2(wn, 20.0f), c.evap), c.dt, Z)), 0.0f);
+                const f2 wo = evaporate2(c, wn);
                 const bool row = (uint32_t)(tr + 2) < nrows, s0 = row && in0, s1 = row && in1;
                 gst2<VEC>(q.h_out, B + 2u * Wu, hn, s0, s1);
                 gst2<VEC>(q.w_out, B + 2u * Wu, wo, s0, s1);
-            }
-            // ---- transport (:2572-2585): bilinear taps within two cells ----
-            {
-                const uint32_t pv = (P - 4 * kMRow) & kRMask;
-                const f2 px = sub2(fgx, mul2_z(ld2(S, pv + kOVX), c.dt, Z));
-                const f2 py = sub2(dup2(fy), mul2_z(ld2(S, pv + kOVY), c.dt, Z));
-                const f2 tx = add2_rm(px, c.M), ty = add2_rm(py, c.M);
-                const f2 wx = sub2(px, sub2(tx, c.M)), wy = sub2(py, sub2(ty, c.M));
-                const f2 vx = sub2(c.one, wx), vy = sub2(c.one, wy);
-                // a tap offset is in [-2, 1] by the velocity clamp; the mask keeps any other inside the ring
-                const uint32_t o0 = tap_c + (__float_as_uint(lo(ty)) << 9) + (__float_as_uint(lo(tx)) << 2);
-                const uint32_t o1 = tap_c + (__float_as_uint(hi(ty)) << 9) + (__float_as_uint(hi(tx)) << 2);
-                const uint32_t u0 = (o0 & kRMask) + kOS, d0 = ((o0 + kMRow) & kRMask) + kOS;
-                const uint32_t u1 = (o1 & kRMask) + kOS, d1 = ((o1 + kMRow) & kRMask) + kOS;
-                const f2 I0 = add2(mul2_z(vx, pk(mld(S, u0), mld(S, u1)), Z), mul2_z(wx, pk(mld(S, u0 + 4), mld(S, u1 + 4)), Z));
-                const f2 I1 = add2(mul2_z(vx, pk(mld(S, d0), mld(S, d1)), Z), mul2_z(wx, pk(mld(S, d0 + 4), mld(S, d1 + 4)), Z));
-                const f2 sn = add2(mul2_z(vy, I0, Z), mul2_z(wy, I1, Z));
-                const bool row = (uint32_t)(tr - 4) < nrows;
-                gst2<VEC>(q.s_out, B - W4, sn, row && in0, row && in1);
             }
             // ---- flux (:2439-2485) ----
             {
@@ -393,48 +248,12 @@ __device__ __forceinline__ void march_piece(const HydroParams &p, const PairCons
                     ow = pk(v[0].w, v[1].w);
                 } else {
                     const f2 h = ld2(S, a0 + kOH), w = ld2(S, a0 + kOW);
-                    const f2 hw = add2(h, w);
-                    // (left of cell 0, right of cell 1), (right of cell 0, left of cell 1), +y, -y
-                    f2 gA = sub2(sub2(hw, pk(mld(S, a0 + kOH - 4), mld(S, a0 + kOH + 8))),
-                                 pk(mld(S, a0 + kOW - 4), mld(S, a0 + kOW + 8)));
-                    f2 gB = pk((lo(hw) - hi(h)) - hi(w), (hi(hw) - lo(h)) - lo(w));
-                    f2 gU = sub2(sub2(hw, ld2(S, au + kOH)), ld2(S, au + kOW));
-                    f2 gD = sub2(sub2(hw, ld2(S, ad + kOH)), ld2(S, ad + kOW));
-                    const f2 G = c.G;
-                    gA = mul2(G, gA);
-                    gB = mul2(G, gB);
-                    gU = mul2(G, gU);
-                    gD = mul2(G, gD);
-                    const f2 nL = c.nL, rL = c.rL, dtA = c.dtA;
-                    const f2 tA = mul2_z(dtA, div2(gA, nL, rL), Z), tB = mul2_z(dtA, div2(gB, nL, rL), Z);
-                    const f2 tU = mul2_z(dtA, div2(gU, nL, rL), Z), tD = mul2_z(dtA, div2(gD, nL, rL), Z);
-                    // the sign of a zero quotient does not survive the sums and clamps below
-                    ox = pk(fmaxf(0.0f, fa.x + lo(tA)), fmaxf(0.0f, fb.x + hi(tB)));
-                    oy = pk(fmaxf(0.0f, fa.y + lo(tU)), fmaxf(0.0f, fb.y + hi(tU)));
-                    oz = pk(fmaxf(0.0f, fa.z + lo(tB)), fmaxf(0.0f, fb.z + hi(tA)));
-                    ow = pk(fmaxf(0.0f, fa.w + lo(tD)), fmaxf(0.0f, fb.w + hi(tD)));
-                    const f2 total = add2(add2(add2(add2(ox, oy), oz), ow), c.tiny);
-                    const f2 den = add2(mul2_z(total, c.dt, Z), c.tiny);
-                    const f2 nden = mul2(den, c.mone);
-                    const f2 qK = div2(w, nden, rcp2(den, nden, c.one));
-                    const f2 Kf = max2(min2(qK, 1.0f), 0.01f);
-                    // every dividend a zero or in [2^-90, 2^64), the denominators (>= 1e-6) at most 2^32; a water
-                    // below 2^-90 has a quotient far below 0.01, whatever its last bits.  A dividend below 2^-90
-                    // is looked at again: it may be a zero.
-                    const float mx = max3_nan(max3_nan(max3_nan(max3_nan(lo(gA), hi(gA), lo(gB)), hi(gB), lo(gU)), hi(gU),
-                                                       lo(gD)), hi(gD), max3_nan(lo(w), hi(w), 0.0f));
-                    const float mn = min3(min3(min3(lo(gA), hi(gA), lo(gB)), hi(gB), lo(gU)), min3(hi(gU), lo(gD), hi(gD)), 1.0f);
+                    Flux2 o;
                     const bool mine = live_f && (uint32_t)(tr + 10) < nrows + 6u;
-                    if (mine && (!(mx < 0x1p64f) || mn < 0x1p-90f || !(fmaxf(lo(den), hi(den)) <= 0x1p32f))) {
-                        const uint32_t z = min(
-                            min(min(nz_bits(lo(gA)), nz_bits(hi(gA))), min(nz_bits(lo(gB)), nz_bits(hi(gB)))),
-                            min(min(nz_bits(lo(gU)), nz_bits(hi(gU))), min(nz_bits(lo(gD)), nz_bits(hi(gD)))));
-                        bad = bad || !(mx < 0x1p64f) || z < kNz90 || !(fmaxf(lo(den), hi(den)) <= 0x1p32f);
-                    }
-                    ox = mul2(ox, Kf);
-                    oy = mul2(oy, Kf);
-                    oz = mul2(oz, Kf);
-                    ow = mul2(ow, Kf);
+                    bad = flux_pair(c, h, w, mld(S, a0 + kOH - 4), mld(S, a0 + kOH + 8), mld(S, a0 + kOW - 4),
+                                    mld(S, a0 + kOW + 8), ld2(S, au + kOH), ld2(S, au + kOW), ld2(S, ad + kOH),
+                                    ld2(S, ad + kOW), fa, fb, mine, o) || bad;
+                    ox = o.x, oy = o.y, oz = o.z, ow = o.w;
                 }
                 st2(S, a0 + kOX, ox);
                 st2(S, a0 + kOY, oy);
@@ -532,42 +351,10 @@ int hydro_march_attributes()
 void launch_hydro_march(const Batch &b, StripParams sp, cudaStream_t st)
 {
     sp.nwarps = march_blocks(b, sp.rows, (const void *)k_hydro_march, kPairThreads, kHydroMarchSmem, kHydroMarchMinRows);
-    const HydroParams &p = sp.p;
-    auto d = [](float v) { return pk_host(v); };
     PairParams pp{};
     pp.sp = sp;
-    pp.ieee = p.fastL == 0 || !(p.dt >= 0.0f);
-    PairConst &c = pp.c;
-    c.dt = d(p.dt);
-    c.G = d(p.G);
-    c.nL = d(-p.L);
-    c.rL = d(p.rL);
-    c.dtA = d(p.dt * p.A);
-    c.Kc = d(p.Kc);
-    c.Ks = d(p.Ks);
-    c.Kd = d(p.Kd);
-    c.evap = d(p.evap);
-    c.Z = d(-0.0f);
-    c.M = d(12582912.0f);
-    c.one = d(1.0f);
-    c.mone = d(-1.0f);
-    c.half = d(0.5f);
-    c.tiny = d(1e-6f);
-    c.top = d(TECTO_TWO_OVER_PI);
-    c.C1 = d(TECTO_PIO2_C1);
-    c.C2 = d(TECTO_PIO2_C2);
-    c.C3 = d(TECTO_PIO2_C3);
-    c.C4 = d(TECTO_PIO2_C4);
-    c.S3 = d(TECTO_SIN_S3);
-    c.S5 = d(TECTO_SIN_S5);
-    c.S7 = d(TECTO_SIN_S7);
-    c.S9 = d(TECTO_SIN_S9);
-    c.S11 = d(TECTO_SIN_S11);
-    c.K2 = d(TECTO_COS_K2);
-    c.K4 = d(TECTO_COS_K4);
-    c.K6 = d(TECTO_COS_K6);
-    c.K8 = d(TECTO_COS_K8);
-    c.K10 = d(TECTO_COS_K10);
+    pp.ieee = sp.p.fastL == 0 || !(sp.p.dt >= 0.0f);
+    pp.c = pair_const(sp.p);
     k_hydro_march<<<(unsigned)sp.nwarps, kPairThreads, kHydroMarchSmem, st>>>(pp);
 }
 

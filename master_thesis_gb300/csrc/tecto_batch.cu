@@ -165,9 +165,19 @@ void batch_release(Batch &b)
 // batch (or its cached choice for the shape class), then the defaults.
 // The default thermal variant: one iteration with tiles (variant 4, two iterations a launch) against the
 // march (5), us: 512^2 5.3 / 6.5, 1024^2 11.6 / 11.0, 2048^2 37.4 / 23.0, 8192^2 570 / 230.
-// The default hydraulic variant follows the batch's cells: one sub-iteration with tiles (variant 4)
-// against the march (9), us: 256^2 12.7 / 14.1, 1024^2 31.2 / 31.1, 1200x1000 31.8 / 33.2, 1101x1301
-// 41.2 / 41.5, 1500x1100 45.4 / 37.5, 2048^2 103 / 72, 8192^2 1446 / 858, a 49.7 M cell batch 1269 / 762.
+// The default hydraulic variant follows the batch's cells, as whole steps measured it, us:
+//                64^2  256^2  512^2  1001x613  1024^2  1500x1100  2048^2  12 worlds (0.6 M)  40 worlds (1.0 M)
+//   1 (56x8)      146    197    353       608     906       1424    3379        621              1130
+//   3 (56x16)     178    200    319       502     688       1036    2388        504               872
+//   4 (56x24)     205    221    305       527     705       1001    2250        527               863
+//   9 (march)     283    305    411       674     791       1038    2068        674              1041
+// Small batches want many short tiles, large ones little halo.
+static int default_hydro_variant(size_t cells)
+{
+    if (cells >= kMarchMinCells) return kHydroMarchVariant;
+    return cells <= (size_t)1 << 17 ? 1 : cells <= (size_t)1 << 20 ? 3 : 4;
+}
+
 static void choose_tuning(const Batch &b, int *variant, int *rb, int *tvariant)
 {
     *tvariant = thermal_variant_for(b.settings);
@@ -175,7 +185,7 @@ static void choose_tuning(const Batch &b, int *variant, int *rb, int *tvariant)
     if (*tvariant == 0) *tvariant = b.total >= kThermalMarchMinCells ? kThermalMarchVariant : kDefaultThermalVariant;
     *variant = hydro_variant_for(b.settings);
     if (*variant == 0) *variant = b.tuned_hydro;
-    if (*variant == 0) *variant = b.total >= kMarchMinCells ? kHydroMarchVariant : kDefaultHydroVariant;
+    if (*variant == 0) *variant = default_hydro_variant(b.total);
     *rb = b.settings.step.sortRadixBits;
     if (!valid_radix_bits(*rb)) *rb = valid_radix_bits(b.tuned_rb) ? b.tuned_rb : kDefaultRadixBits;
 }
@@ -234,7 +244,7 @@ int batch_prepare(Batch &b, cudaStream_t st)
     }
     std::vector<uint4> strips[ST_COUNT];
     for (int k = 0; k < ST_COUNT; ++k) {
-        const int inner = k == ST_THERMAL ? kThermalInner : variant == kHydroStripVariant ? kStripInner : kMarchInner;
+        const int inner = k == ST_THERMAL ? kThermalInner : kMarchInner;
         strips[k] = build_strips(b, inner, &b.strips[k].rows);
         b.strips[k].n = (int)strips[k].size();
         need += a256(strips[k].size() * sizeof(uint4));

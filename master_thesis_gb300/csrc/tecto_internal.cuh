@@ -345,11 +345,10 @@ int ensure_kernel_attributes();
 int hydro_variant_for(const tecto_settings &s);  // 0 when the settings leave the choice open
 constexpr int kDefaultRadixBits = 8;
 constexpr int kHydroVariantCount = 9;
-constexpr int kDefaultHydroVariant = 4;          // 64 x 32 cells, 1024 threads
-constexpr int kHydroStripVariant = 8;            // marching column strips in registers (fused path only)
+constexpr int kDefaultHydroVariant = 4;          // 56 x 24 cells: where the autotuner starts from
+constexpr int kHydroStripVariant = 8;            // from here on: the march (8 is kept as another number for it)
 constexpr int kHydroMarchVariant = 9;            // marching row chunks in shared memory (fused path only)
-constexpr size_t kMarchMinCells = 1572864;       // cells from which the hydraulic march is the default
-constexpr int kStripInner = 56;                  // interior columns of one register strip (64 with the halo)
+constexpr size_t kMarchMinCells = 2500000;       // cells from which the hydraulic march is the default
 constexpr int kMarchInner = 120;                 // interior columns of one shared-memory strip (128 with it)
 constexpr int kThermalInner = 60;                // interior columns of one thermal strip (64 with the halo)
 constexpr int kThermalVariantCount = 5;
