@@ -123,6 +123,7 @@ __global__ __launch_bounds__(256, 8) void k_ccl_local(const WorldDev *worlds, co
                                                    int mode, int period)
 {
     static_assert(CX == 32 && CY % 8 == 0, "one warp per tile row, eight warps");
+    kernel_wait();
     __shared__ int par[CX * CY];
     int x0, y0;
     const WorldDev *wd = ccl_tile(worlds, tiles, period, &x0, &y0);
@@ -217,6 +218,7 @@ __global__ __launch_bounds__(256, 8) void k_ccl_local(const WorldDev *worlds, co
 __global__ __launch_bounds__(128) void k_ccl_border(const WorldDev *worlds, const uint2 *tiles, int cur_id,
                                                     int mode, int period)
 {
+    kernel_wait();
     int x0, y0;
     const WorldDev *wd = ccl_tile(worlds, tiles, period, &x0, &y0);
     if (!wd) return;
@@ -245,6 +247,7 @@ __global__ __launch_bounds__(128) void k_ccl_border(const WorldDev *worlds, cons
 
 __global__ void k_ccl_flatten(const WorldDev *worlds, const uint2 *tiles, int period)
 {
+    kernel_wait();
     int x0, y0;
     const WorldDev *wd = ccl_tile(worlds, tiles, period, &x0, &y0);
     if (!wd) return;
@@ -271,9 +274,9 @@ int launch_ccl(Batch &b, int connectivity, bool due_only, cudaStream_t st)
     const int period = due_only ? (b.settings.sim.iterationsForCCL > 0 ? b.settings.sim.iterationsForCCL : 1) : 0;
     const unsigned grid = (unsigned)b.ntiles[TK_CCL];
     const uint2 *tiles = b.d_tiles[TK_CCL];
-    k_ccl_local<<<grid, 256, 0, st>>>(b.d_worlds, tiles, b.cur_id, connectivity, period);
-    k_ccl_border<<<grid, 128, 0, st>>>(b.d_worlds, tiles, b.cur_id, connectivity, period);
-    k_ccl_flatten<<<grid, 256, 0, st>>>(b.d_worlds, tiles, period);
+    launch_chained(k_ccl_local, grid, 256, 0, st, b.d_worlds, tiles, b.cur_id, connectivity, period);
+    launch_chained(k_ccl_border, grid, 128, 0, st, b.d_worlds, tiles, b.cur_id, connectivity, period);
+    launch_chained(k_ccl_flatten, grid, 256, 0, st, b.d_worlds, tiles, period);
     TECTO_CUDA(cudaGetLastError());
     b.launches += 3;
     return TECTO_OK;

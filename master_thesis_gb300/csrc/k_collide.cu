@@ -1,5 +1,7 @@
 // k_collide.cu - plate displacement, collision words from the sorted arrivals, collision-type
 // evidence and the plate-pair type bitmap.  Reference: src/cuda_compute/plate_tectonics_kernel.cu.
+#include <algorithm>
+
 #include "tecto_internal.cuh"
 
 namespace tecto {
@@ -8,13 +10,20 @@ namespace {
 
 // Per-plate integer displacement (getPixelMovements, :248-257) and the sub-cell centre update
 // of applyPlateMovementChanges (:1871-1878), one block per world; the record before the update is
-// kept in plates_prev for the kernels of the same step.  Also resets the world's per-step
-// accretion list.  With plate dynamics it first turns the sums k_plate_stats left into each
+// kept in plates_prev for the kernels of the same step.  The blocks after those of the worlds clear the
+// sort's scratch (clear_words 16-byte words).  With plate dynamics it first turns the sums k_plate_stats left into each
 // plate's mass, size and geometric centre (mergeAndCountSizeMass, calculatePlateCenters
 // :2191-2226: the angular means back to cells through atan2), and clears them.  The reference
 // computes no centre before its first iteration ends, so iteration 0 keeps the stored one.
-__global__ void k_plates(const WorldDev *worlds, int dynamics)
+__global__ void k_plates(const WorldDev *worlds, int nworlds, int dynamics, uint4 *clear, size_t clear_words)
 {
+    kernel_wait();
+    if ((int)blockIdx.x >= nworlds) {
+        const size_t step = (size_t)(gridDim.x - nworlds) * blockDim.x;
+        for (size_t i = (size_t)(blockIdx.x - nworlds) * blockDim.x + threadIdx.x; i < clear_words; i += step)
+            clear[i] = make_uint4(0u, 0u, 0u, 0u);
+        return;
+    }
     const WorldDev &wd = worlds[blockIdx.x];
     const int k = threadIdx.x;
     if (dynamics && k < kPlates) {
@@ -56,7 +65,6 @@ __global__ void k_plates(const WorldDev *worlds, int dynamics)
     } else if (k == kPlates) {
         wd.off[k] = make_int2(0, 0);
     }
-    if (k == 0) wd.ctl->acc_count = 0;
 }
 
 // writeCollision's classification (:794-836): returns category 0..4 or -1 to skip.  The early
@@ -89,6 +97,7 @@ __global__ __launch_bounds__(256) void k_words(const uint32_t *keys, const uint3
                                                const WorldDev *worlds, const uint32_t *vbase, int nworlds,
                                                int cur_id, int cur_h, float thr, int cooldown)
 {
+    kernel_wait();
     __shared__ uint32_t s_vbase[kMaxBatchWorlds + 1];
     for (int i = threadIdx.x; i <= nworlds; i += blockDim.x) s_vbase[i] = vbase[i];
     __syncthreads();
@@ -160,12 +169,15 @@ __global__ __launch_bounds__(256) void k_words(const uint32_t *keys, const uint3
     }
 }
 
-// createCollisionTypeMatrix (:890-972) for every world of the batch; also clears the evidence.
+// createCollisionTypeMatrix (:890-972) for every world of the batch; also clears the evidence and resets
+// the world's accretion list (k_sort_hist has cleared the cells of the step before's).
 __global__ void k_type_matrix(const WorldDev *worlds, int cooldown, int minSize)
 {
+    kernel_wait();
     const uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= (uint32_t)kPairs) return;
     const WorldDev &wd = worlds[blockIdx.y];
+    if (idx == 0) wd.ctl->acc_count = 0;
     PairCounts *counts = wd.counts;
     uint8_t *bm = wd.type_bitmap;
     const PairCounts pc = counts[idx];
@@ -202,12 +214,15 @@ int launch_plates(Batch &b, cudaStream_t st)
         set_error("plateDynamics must be TECTO_PLATE_DYNAMICS_OFF or TECTO_PLATE_DYNAMICS_REFERENCE");
         return TECTO_ERR_UNSUPPORTED;
     }
-    int rc = launch_clear_marks(b, st);  // must run before k_plates resets the list count
-    if (rc != TECTO_OK) return rc;
+    int rc;
     // plate dynamics and the plate policy read the per-plate mass, size and centre of the step
     const int stats = dyn != TECTO_PLATE_DYNAMICS_OFF || b.settings.step.platePolicy != 0;
     if (stats && (rc = launch_plate_stats(b, st)) != TECTO_OK) return rc;
-    k_plates<<<(unsigned)b.members.size(), 256, 0, st>>>(b.d_worlds, stats);
+    // the clear is spread over up to two blocks per SM, 16 KB each at least
+    const size_t bytes = sort_clear_bytes(b.sort, b.total);
+    const unsigned nw = (unsigned)b.members.size(), nclear = (unsigned)std::min<size_t>((bytes + 16383) / 16384, 304);
+    launch_chained(k_plates, nw + nclear, 256, 0, st, b.d_worlds, (int)nw, stats, reinterpret_cast<uint4 *>(b.sort.hist),
+                   bytes / 16);
     TECTO_CUDA(cudaGetLastError());
     b.launches += 1;
     return TECTO_OK;
@@ -230,7 +245,7 @@ int launch_sort_keys(Batch &b, cudaStream_t st)
     const int rc = run_sort(a, b.sort, st, &half);
     if (rc != TECTO_OK) return rc;
     b.sort_final = half;
-    b.launches += 2 + (uint64_t)b.sort.passes;
+    b.launches += 1 + (uint64_t)b.sort.passes;
     return TECTO_OK;
 }
 
@@ -238,9 +253,9 @@ int launch_words(Batch &b, cudaStream_t st)
 {
     const uint32_t n = (uint32_t)b.total;
     const tecto_kernel_settings &ks = b.settings.kernel;
-    k_words<<<(n + 255) / 256, 256, 0, st>>>(b.keys[b.sort_final], b.vals[b.sort_final], n, b.d_worlds,
-                                             b.d_vbase, (int)b.members.size(), b.cur_id, b.cur_h,
-                                             ks.continentalCrustThreshold, ks.collisionTypeUpdateCooldown);
+    launch_chained(k_words, (n + 255) / 256, 256, 0, st, b.keys[b.sort_final], b.vals[b.sort_final], n, b.d_worlds,
+                   b.d_vbase, (int)b.members.size(), b.cur_id, b.cur_h, ks.continentalCrustThreshold,
+                   ks.collisionTypeUpdateCooldown);
     TECTO_CUDA(cudaGetLastError());
     b.launches += 1;
     return TECTO_OK;
@@ -250,7 +265,7 @@ int launch_type_matrix(Batch &b, cudaStream_t st)
 {
     const tecto_kernel_settings &ks = b.settings.kernel;
     const dim3 grid((kPairs + 255) / 256, (unsigned)b.members.size());
-    k_type_matrix<<<grid, 256, 0, st>>>(b.d_worlds, ks.collisionTypeUpdateCooldown, ks.minCollisionSize);
+    launch_chained(k_type_matrix, grid, 256, 0, st, b.d_worlds, ks.collisionTypeUpdateCooldown, ks.minCollisionSize);
     TECTO_CUDA(cudaGetLastError());
     b.launches += 1;
     return TECTO_OK;

@@ -288,6 +288,7 @@ __device__ __noinline__ void march_ieee(const PairParams &pp, const HydroWorld &
 
 __global__ __launch_bounds__(kPairThreads, 2) void k_hydro_march(const __grid_constant__ PairParams pp)
 {
+    kernel_release();
     const StripParams &sp = pp.sp;
     extern __shared__ float4 march_smem[];
     char *S = reinterpret_cast<char *>(march_smem);
@@ -306,6 +307,7 @@ __global__ __launch_bounds__(kPairThreads, 2) void k_hydro_march(const __grid_co
         if ((unsigned long long)sp.strips[mid].w <= a0) lo_s = mid;
         else hi_s = mid - 1;
     }
+    kernel_wait();
     unsigned long long a = a0;
     for (int s = lo_s; a < b0 && s < sp.nstrips; ++s) {
         const uint4 d = sp.strips[s];
@@ -355,7 +357,7 @@ void launch_hydro_march(const Batch &b, StripParams sp, cudaStream_t st)
     pp.sp = sp;
     pp.ieee = sp.p.fastL == 0 || !(sp.p.dt >= 0.0f);
     pp.c = pair_const(sp.p);
-    k_hydro_march<<<(unsigned)sp.nwarps, kPairThreads, kHydroMarchSmem, st>>>(pp);
+    launch_chained(k_hydro_march, (unsigned)sp.nwarps, kPairThreads, kHydroMarchSmem, st, pp);
 }
 
 }  // namespace tecto

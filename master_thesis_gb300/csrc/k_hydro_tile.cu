@@ -217,6 +217,7 @@ __device__ __forceinline__ void tile_body(const TileParams &tp, const HydroWorld
         flow_rows_ieee<TY, NW, FUSED>(tp.p, q, S, x0, y0);
         __syncthreads();
     }
+    kernel_release();
     if (!FUSED) return;
 
     // transport (:2572-2585, bilinear with wrap, cuda_helper.cuh:48-65) on rows 4 .. TY + 3.  The byte offset
@@ -259,6 +260,7 @@ __global__ __launch_bounds__(NW * 32, MINB) void k_hydro(const __grid_constant__
         s_xy[1] = ty * TY;
     }
     __syncthreads();
+    kernel_wait();
     if (s_q.W & 1) tile_body<TY, NW, FUSED, false>(tp, s_q, S, s_xy[0], s_xy[1]);
     else tile_body<TY, NW, FUSED, true>(tp, s_q, S, s_xy[0], s_xy[1]);
 }
@@ -267,6 +269,7 @@ __global__ __launch_bounds__(NW * 32, MINB) void k_hydro(const __grid_constant__
 // hydraulic work list (tiles of 64 x ty cells).
 __global__ void k_rain(const WorldDev *worlds, const uint2 *tiles, int ty_cells, float dt, float rainfall)
 {
+    kernel_wait();
     int wi, tx, ty;
     tile_of(tiles[blockIdx.x], &wi, &tx, &ty);
     const WorldDev &wd = worlds[wi];
@@ -283,6 +286,7 @@ __global__ void k_rain(const WorldDev *worlds, const uint2 *tiles, int ty_cells,
 __global__ __launch_bounds__(256) void k_transport(const WorldDev *worlds, const uint2 *tiles, int ty_cells,
                                                    int cur_wsf, float dt)
 {
+    kernel_wait();
     int wi, tx, ty;
     tile_of(tiles[blockIdx.x], &wi, &tx, &ty);
     const WorldDev &wd = worlds[wi];
@@ -340,14 +344,14 @@ void hydro_tile_extent(int variant, int *tx, int *ty)
 
 void launch_rain(const Batch &b, float dt, float rainfall, cudaStream_t st)
 {
-    k_rain<<<(unsigned)b.ntiles[TK_HYDRO], 256, 0, st>>>(b.d_worlds, b.d_tiles[TK_HYDRO], variant_of(b.hydro_variant).ty, dt,
-                                                          rainfall);
+    launch_chained(k_rain, (unsigned)b.ntiles[TK_HYDRO], 256, 0, st, b.d_worlds, b.d_tiles[TK_HYDRO],
+                   variant_of(b.hydro_variant).ty, dt, rainfall);
 }
 
 void launch_transport(const Batch &b, float dt, cudaStream_t st)
 {
-    k_transport<<<(unsigned)b.ntiles[TK_HYDRO], 256, 0, st>>>(b.d_worlds, b.d_tiles[TK_HYDRO],
-                                                               variant_of(b.hydro_variant).ty, b.cur_wsf, dt);
+    launch_chained(k_transport, (unsigned)b.ntiles[TK_HYDRO], 256, 0, st, b.d_worlds, b.d_tiles[TK_HYDRO],
+                   variant_of(b.hydro_variant).ty, b.cur_wsf, dt);
 }
 
 void launch_hydro_tile(const Batch &b, const HydroParams &p, bool fused, cudaStream_t st)
@@ -358,8 +362,7 @@ void launch_hydro_tile(const Batch &b, const HydroParams &p, bool fused, cudaStr
     tp.c = pair_const(p);
     tp.ieee = p.fastL == 0 || !(p.dt >= 0.0f);
     const unsigned grid = (unsigned)b.ntiles[TK_HYDRO];
-    if (fused) v.fused<<<grid, v.nt, v.smem, st>>>(tp);
-    else v.split<<<grid, v.nt, v.smem, st>>>(tp);
+    launch_chained(fused ? v.fused : v.split, grid, v.nt, v.smem, st, tp);
 }
 
 }  // namespace tecto

@@ -200,6 +200,7 @@ __device__ __forceinline__ float resolve_cell(const ResolveParams &p, const Reso
 template <int R, bool DYN>
 __global__ __launch_bounds__(256, 6) void k_resolve(ResolveParams p)
 {
+    kernel_wait();
     constexpr int SX = RX + 2 * R, SY = RY + 2 * R;
     __shared__ uint32_t s_word[SY * SX];
     __shared__ float s_tmp[(R > 0) ? SY * RX : 1];
@@ -281,24 +282,31 @@ __global__ __launch_bounds__(256, 6) void k_resolve(ResolveParams p)
     }
 }
 
-// flipDivergedBitmap (:772-780) for every world; clears the per-step bits for the next step
-__global__ void k_flip(const WorldDev *worlds)
+// flipDivergedBitmap (:772-780) for one world; clears the per-step bits for the next step
+__device__ __forceinline__ void flip_word(const WorldDev &wd, int i)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < kDivWords) {
-        const WorldDev &wd = worlds[blockIdx.y];
         wd.div_bitmap[i] ^= wd.has_div[i];
         wd.has_div[i] = 0u;
     }
 }
 
-// applyAccretion (:747-770) over the cells that received a mark this step; clears the marks.
-// Grid: (blocks, worlds).
-__global__ void k_finish(const WorldDev *worlds, int cur_h, int cur_id, float thr)
+__global__ void k_flip(const WorldDev *worlds)
 {
+    kernel_wait();
+    flip_word(worlds[blockIdx.y], blockIdx.x * blockDim.x + threadIdx.x);
+}
+
+// applyAccretion (:747-770) over the cells that received a mark this step; clears the marks.  With flip the
+// divergence bitmap, with bump the iteration counter (nothing after it in the step reads it).
+// Grid: (blocks, worlds), at least kDivWords threads per world.
+__global__ void k_finish(const WorldDev *worlds, int cur_h, int cur_id, float thr, int flip, int bump)
+{
+    kernel_wait();
     const WorldDev &wd = worlds[blockIdx.y];
     const uint32_t count = wd.ctl->acc_count;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    for (uint32_t i = t; i < count; i += gridDim.x * blockDim.x) {
         const uint32_t c = wd.acc_list[i];
         const unsigned long long m = wd.acc[c];
         wd.acc[c] = 0ull;
@@ -307,21 +315,15 @@ __global__ void k_finish(const WorldDev *worlds, int cur_h, int cur_id, float th
         const uint8_t accId = (uint8_t)(255u - value);
         if (accId != 255 && wd.h[cur_h][c] >= thr) wd.id[cur_id][c] = accId;
     }
+    if (flip) flip_word(wd, (int)t);
+    if (bump && t == 0) wd.ctl->iteration += 1u;
 }
 
 __global__ void k_bump_iteration(const WorldDev *worlds, int nworlds)
 {
+    kernel_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < nworlds) worlds[i].ctl->iteration += 1u;
-}
-
-// Clears the previous step's decoded marks before this step's resolve.  Grid: (blocks, worlds).
-__global__ void k_clear_acc_u8(const WorldDev *worlds)
-{
-    const WorldDev &wd = worlds[blockIdx.y];
-    const uint32_t count = wd.ctl->acc_count;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x)
-        wd.acc_u8[wd.acc_list[i]] = 0;
 }
 
 }  // namespace
@@ -337,7 +339,7 @@ void gaussian_weights(float sigma, int radius, float *out)
     for (int k = 0; k <= 2 * radius; ++k) out[k] = (float)(tmp[k] / sum);
 }
 
-int launch_resolve(Batch &b, cudaStream_t st)
+int launch_resolve(Batch &b, bool flip, cudaStream_t st)
 {
     const tecto_settings &s = b.settings;
     ResolveParams p{};
@@ -370,55 +372,30 @@ int launch_resolve(Batch &b, cudaStream_t st)
         }
         gaussian_weights(s.step.upliftSigma, R, p.wts);
     }
-    const unsigned grid = (unsigned)b.ntiles[TK_RESOLVE];
-    if (s.step.plateDynamics == TECTO_PLATE_DYNAMICS_REFERENCE) {
-        switch (R) {
-            case 0: k_resolve<0, true><<<grid, 256, 0, st>>>(p); break;
-            case 1: k_resolve<1, true><<<grid, 256, 0, st>>>(p); break;
-            case 2: k_resolve<2, true><<<grid, 256, 0, st>>>(p); break;
-            case 3: k_resolve<3, true><<<grid, 256, 0, st>>>(p); break;
-            case 4: k_resolve<4, true><<<grid, 256, 0, st>>>(p); break;
-            case 5: k_resolve<5, true><<<grid, 256, 0, st>>>(p); break;
-            case 6: k_resolve<6, true><<<grid, 256, 0, st>>>(p); break;
-            case 7: k_resolve<7, true><<<grid, 256, 0, st>>>(p); break;
-            default: k_resolve<8, true><<<grid, 256, 0, st>>>(p); break;
-        }
-    } else switch (R) {
-        case 0: k_resolve<0, false><<<grid, 256, 0, st>>>(p); break;
-        case 1: k_resolve<1, false><<<grid, 256, 0, st>>>(p); break;
-        case 2: k_resolve<2, false><<<grid, 256, 0, st>>>(p); break;
-        case 3: k_resolve<3, false><<<grid, 256, 0, st>>>(p); break;
-        case 4: k_resolve<4, false><<<grid, 256, 0, st>>>(p); break;
-        case 5: k_resolve<5, false><<<grid, 256, 0, st>>>(p); break;
-        case 6: k_resolve<6, false><<<grid, 256, 0, st>>>(p); break;
-        case 7: k_resolve<7, false><<<grid, 256, 0, st>>>(p); break;
-        default: k_resolve<8, false><<<grid, 256, 0, st>>>(p); break;
-    }
-    k_flip<<<dim3((kDivWords + 255) / 256, (unsigned)b.members.size()), 256, 0, st>>>(b.d_worlds);
+    static constexpr void (*kern[2][kMaxBlurRadius + 1])(ResolveParams) = {
+        {k_resolve<0, false>, k_resolve<1, false>, k_resolve<2, false>, k_resolve<3, false>, k_resolve<4, false>,
+         k_resolve<5, false>, k_resolve<6, false>, k_resolve<7, false>, k_resolve<8, false>},
+        {k_resolve<0, true>, k_resolve<1, true>, k_resolve<2, true>, k_resolve<3, true>, k_resolve<4, true>,
+         k_resolve<5, true>, k_resolve<6, true>, k_resolve<7, true>, k_resolve<8, true>}};
+    const int dyn = s.step.plateDynamics == TECTO_PLATE_DYNAMICS_REFERENCE ? 1 : 0;
+    launch_chained(kern[dyn][R], (unsigned)b.ntiles[TK_RESOLVE], 256, 0, st, p);
+    if (flip) launch_chained(k_flip, dim3((kDivWords + 255) / 256, (unsigned)b.members.size()), 256, 0, st, b.d_worlds);
     TECTO_CUDA(cudaGetLastError());
-    b.launches += 2;
+    b.launches += flip ? 2 : 1;
     b.cur_h ^= 1;
     b.cur_id ^= 1;
     return TECTO_OK;
 }
 
-int launch_finish(Batch &b, cudaStream_t st)
+int launch_finish(Batch &b, bool flip, bool bump, cudaStream_t st)
 {
     if (b.settings.step.plateDynamics == TECTO_PLATE_DYNAMICS_REFERENCE) {
         const int rc = launch_plate_motion(b, st);  // executeIteration: before applyAccretion
         if (rc != TECTO_OK) return rc;
     }
-    k_finish<<<dim3(4, (unsigned)b.members.size()), 256, 0, st>>>(b.d_worlds, b.cur_h, b.cur_id,
-                                                                   b.settings.kernel.continentalCrustThreshold);
-    TECTO_CUDA(cudaGetLastError());
-    b.launches += 1;
-    return TECTO_OK;
-}
-
-// Runs before launch_plates resets the list count: clears the previous step's decoded marks.
-int launch_clear_marks(Batch &b, cudaStream_t st)
-{
-    k_clear_acc_u8<<<dim3(4, (unsigned)b.members.size()), 256, 0, st>>>(b.d_worlds);
+    static_assert(4 * 256 >= kDivWords, "k_finish: one thread per divergence word");
+    launch_chained(k_finish, dim3(4, (unsigned)b.members.size()), 256, 0, st, b.d_worlds, b.cur_h, b.cur_id,
+                   b.settings.kernel.continentalCrustThreshold, (int)flip, (int)bump);
     TECTO_CUDA(cudaGetLastError());
     b.launches += 1;
     return TECTO_OK;
@@ -427,7 +404,7 @@ int launch_clear_marks(Batch &b, cudaStream_t st)
 int launch_bump_iteration(Batch &b, cudaStream_t st)
 {
     const int n = (int)b.members.size();
-    k_bump_iteration<<<(n + 255) / 256, 256, 0, st>>>(b.d_worlds, n);
+    launch_chained(k_bump_iteration, (n + 255) / 256, 256, 0, st, b.d_worlds, n);
     TECTO_CUDA(cudaGetLastError());
     b.launches += 1;
     return TECTO_OK;

@@ -27,6 +27,7 @@ constexpr int kLookAhead = 8;  // predecessor tiles read per look-back round
 // From this many tiles (16 M keys) a pass runs three blocks per SM: measured faster at 67 M keys
 // (8192^2) and slower at 4 M (2048^2)
 constexpr size_t kSortWideTiles = 4096;
+constexpr int kDoneCounter = 8;  // word of SortScratch::counters that counts finished histogram blocks
 
 template <int RB>
 struct Digits {
@@ -82,12 +83,50 @@ __device__ __forceinline__ void st_volatile(uint32_t *p, uint32_t v)
     *(volatile uint32_t *)p = v;
 }
 
-// Digit histograms of all passes in one read of the keys; generated keys are stored to keys_gen.
+// Block-wide exclusive scan of one value per thread (256 threads); returns the exclusive prefix
+// and the block total.  s_w holds kWarps words; the call ends with a barrier.
+__device__ __forceinline__ uint32_t block_scan(uint32_t v, uint32_t *s_w, uint32_t *total)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t inc = v;
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t u = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += u;
+    }
+    if (lane == 31) s_w[warp] = inc;
+    __syncthreads();
+    uint32_t wb = 0, all = 0;
+#pragma unroll
+    for (int k = 0; k < kWarps; ++k) {
+        const uint32_t x = s_w[k];
+        wb += k < warp ? x : 0u;
+        all += x;
+    }
+    __syncthreads();
+    *total = all;
+    return wb + inc - v;
+}
+
+// Digit histograms of all passes in one read of the keys; generated keys are stored to keys_gen.  The block
+// that finishes last turns each pass's counts into exclusive digit starts, in place (thread t owns digits
+// t, t + 256, ...; the chunks of 256 digits are scanned in order).  With generated keys the blocks first
+// clear the decoded accretion marks of the step before (the worlds' lists, split over the blocks).
 template <bool GEN, int RB>
 __global__ __launch_bounds__(256) void k_sort_hist(GenArgs g, const uint32_t *keys_in, size_t n,
-                                                   int passes, uint32_t *hist, uint32_t *keys_gen)
+                                                   int passes, uint32_t *hist, uint32_t *keys_gen, uint32_t *done)
 {
     using D = Digits<RB>;
+    kernel_wait();
+    if (GEN) {
+        const int parts = max(1, (int)gridDim.x / g.nworlds);
+        for (int it = (int)blockIdx.x; it < g.nworlds * parts; it += (int)gridDim.x) {
+            const int wi = it / parts, part = it - wi * parts;
+            const WorldDev &wd = g.worlds[wi];
+            const uint32_t count = wd.ctl->acc_count;
+            for (uint32_t i = (uint32_t)part * 256u + threadIdx.x; i < count; i += (uint32_t)parts * 256u)
+                wd.acc_u8[wd.acc_list[i]] = 0;
+        }
+    }
     __shared__ uint32_t s_hist[D::MAX_PASSES][D::R];
     __shared__ uint32_t s_vbase[GEN ? kMaxBatchWorlds : 1];
     for (int i = threadIdx.x; i < D::MAX_PASSES * D::R; i += blockDim.x) (&s_hist[0][0])[i] = 0;
@@ -121,45 +160,20 @@ __global__ __launch_bounds__(256) void k_sort_hist(GenArgs g, const uint32_t *ke
         const uint32_t v = (&s_hist[0][0])[i];
         if (v) atomicAdd(&hist[i], v);
     }
-}
-
-// Block-wide exclusive scan of one value per thread (256 threads); returns the exclusive prefix
-// and the block total.  s_w holds kWarps words; the call ends with a barrier.
-__device__ __forceinline__ uint32_t block_scan(uint32_t v, uint32_t *s_w, uint32_t *total)
-{
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint32_t inc = v;
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t u = __shfl_up_sync(0xffffffffu, inc, o);
-        if (lane >= o) inc += u;
-    }
-    if (lane == 31) s_w[warp] = inc;
-    __syncthreads();
-    uint32_t wb = 0, all = 0;
-#pragma unroll
-    for (int k = 0; k < kWarps; ++k) {
-        const uint32_t x = s_w[k];
-        wb += k < warp ? x : 0u;
-        all += x;
-    }
-    __syncthreads();
-    *total = all;
-    return wb + inc - v;
-}
-
-// Exclusive scan of each pass's digit counts, in place.  One block of 256 threads; thread t owns
-// digits t, t + 256, ... and the chunks of 256 digits are scanned in order.
-template <int RB>
-__global__ void k_sort_scan(uint32_t *hist, int passes)
-{
-    using D = Digits<RB>;
     __shared__ uint32_t s_w[kWarps];
+    __shared__ bool s_last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicAdd(done, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
     const int t = threadIdx.x;
     for (int p = 0; p < passes; ++p) {
         uint32_t carry = 0;
         for (int c = 0; c < D::DPT; ++c) {
             uint32_t *h = hist + (size_t)p * D::R + c * kSortThreads + t;
-            const uint32_t v = *h;
+            const uint32_t v = ld_volatile(h);
             uint32_t tot = 0;
             const uint32_t ex = block_scan(v, s_w, &tot);
             *h = carry + ex;
@@ -341,6 +355,7 @@ __global__ __launch_bounds__(kSortThreads) void k_sort_pass(
     const uint32_t *keys_in, const uint32_t *vals_in, uint32_t *keys_out, uint32_t *vals_out, size_t n,
     int shift, const uint32_t *digit_start, uint32_t *status, uint32_t *tile_counter, uint32_t *error)
 {
+    kernel_wait();
     sort_pass_body<RB>(keys_in, vals_in, keys_out, vals_out, n, shift, digit_start, status, tile_counter, error);
 }
 
@@ -349,6 +364,7 @@ __global__ __launch_bounds__(kSortThreads, 3) void k_sort_pass_wide(
     const uint32_t *keys_in, const uint32_t *vals_in, uint32_t *keys_out, uint32_t *vals_out, size_t n,
     int shift, const uint32_t *digit_start, uint32_t *status, uint32_t *tile_counter, uint32_t *error)
 {
+    kernel_wait();
     sort_pass_body<RB>(keys_in, vals_in, keys_out, vals_out, n, shift, digit_start, status, tile_counter, error);
 }
 
@@ -372,10 +388,6 @@ int run_sort_rb(const SortArgs &a, const SortScratch &scr, cudaStream_t st, int 
     const int passes = scr.passes;
     const size_t tiles = (a.n + kSortTile - 1) / kSortTile;
     constexpr int R = Digits<RB>::R;
-    // one memset covers hist, status and counters (contiguous in the scratch layout)
-    const size_t clear = align256((size_t)passes * R * 4) + align256((size_t)passes * tiles * R * 4) +
-                         align256(kMaxSortPasses * 4);
-    TECTO_CUDA(cudaMemsetAsync(scr.hist, 0, clear, st));
     const bool gen = a.worlds != nullptr;
     const GenArgs g{a.worlds, a.vbase, a.nworlds, a.cur_id};
     int hist_blocks = (int)((a.n + 255) / 256);
@@ -383,20 +395,21 @@ int run_sort_rb(const SortArgs &a, const SortScratch &scr, cudaStream_t st, int 
     // generated keys go to the second key half, which the first pass reads and does not write
     const uint32_t *kin = a.keys_in, *vin = a.vals_in;
     if (gen) {
-        k_sort_hist<true, RB><<<hist_blocks, 256, 0, st>>>(g, nullptr, a.n, passes, scr.hist, a.keys[1]);
+        launch_chained(k_sort_hist<true, RB>, hist_blocks, 256, 0, st, g, nullptr, a.n, passes, scr.hist, a.keys[1],
+                       scr.counters + kDoneCounter);
         kin = a.keys[1];
         vin = nullptr;
     } else {
-        k_sort_hist<false, RB><<<hist_blocks, 256, 0, st>>>(g, a.keys_in, a.n, passes, scr.hist, nullptr);
+        launch_chained(k_sort_hist<false, RB>, hist_blocks, 256, 0, st, g, a.keys_in, a.n, passes, scr.hist, nullptr,
+                       scr.counters + kDoneCounter);
     }
-    k_sort_scan<RB><<<1, kSortThreads, 0, st>>>(scr.hist, passes);
     int half = 0;
     for (int p = 0; p < passes; ++p) {
         uint32_t *kout = a.keys[half], *vout = a.vals[half];
         uint32_t *status = scr.status + (size_t)p * tiles * R;
         auto pass = tiles >= kSortWideTiles ? k_sort_pass_wide<RB> : k_sort_pass<RB>;
-        pass<<<(unsigned)tiles, kSortThreads, pass_smem<RB>(), st>>>(
-            kin, vin, kout, vout, a.n, RB * p, scr.hist + (size_t)p * R, status, scr.counters + p, scr.error);
+        launch_chained(pass, (unsigned)tiles, kSortThreads, pass_smem<RB>(), st, kin, vin, kout, vout, a.n, RB * p,
+                       scr.hist + (size_t)p * R, status, scr.counters + p, scr.error);
         kin = kout;
         vin = vout;
         half ^= 1;
@@ -455,6 +468,20 @@ void sort_scratch_carve(void *base, size_t n, int key_bits, int rb, SortScratch 
     out->counters = (uint32_t *)p;
     p += align256(kMaxSortPasses * 4);
     out->error = (uint32_t *)p;
+}
+
+// hist, status and counters, contiguous in the scratch layout
+size_t sort_clear_bytes(const SortScratch &scr, size_t n)
+{
+    const size_t R = (size_t)1 << scr.radix_bits, tiles = (n + kSortTile - 1) / kSortTile;
+    return align256((size_t)scr.passes * R * 4) + align256((size_t)scr.passes * tiles * R * 4) +
+           align256(kMaxSortPasses * 4);
+}
+
+int run_sort_clear(const SortScratch &scr, size_t n, cudaStream_t st)
+{
+    TECTO_CUDA(cudaMemsetAsync(scr.hist, 0, sort_clear_bytes(scr, n), st));
+    return TECTO_OK;
 }
 
 int run_sort(const SortArgs &a, const SortScratch &scr, cudaStream_t st, int *result_half)
@@ -538,7 +565,8 @@ extern "C" int tecto_sort_pairs_radix(const uint32_t *keys_in, const uint32_t *v
     a.key_bits = key_bits;
     TECTO_CUDA(cudaMemsetAsync(scr.error, 0, 4, st));
     int half = 0;
-    rc = run_sort(a, scr, st, &half);
+    rc = run_sort_clear(scr, n, st);
+    if (rc == TECTO_OK) rc = run_sort(a, scr, st, &half);
     if (rc != TECTO_OK) return rc;
     TECTO_CUDA(cudaMemcpyAsync(keys_out, a.keys[half], n * 4, cudaMemcpyDeviceToDevice, st));
     TECTO_CUDA(cudaMemcpyAsync(vals_out, a.vals[half], n * 4, cudaMemcpyDeviceToDevice, st));

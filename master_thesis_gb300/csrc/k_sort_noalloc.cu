@@ -96,7 +96,8 @@ extern "C" int tecto_sort_pairs_noalloc(const uint32_t *keys_in, const uint32_t 
     a.key_bits = key_bits;
     TECTO_CUDA(cudaMemsetAsync(scr.error, 0, 4, st));  // the array keeps the previous call's flag
     int result_half = -1;
-    rc = run_sort(a, scr, st, &result_half);
+    rc = run_sort_clear(scr, n, st);
+    if (rc == TECTO_OK) rc = run_sort(a, scr, st, &result_half);
     if (rc != TECTO_OK) return rc;
     if (result_half != last) {
         set_error("tecto_sort_pairs_noalloc: internal pass parity mismatch");

@@ -215,9 +215,9 @@ template <int MODE>
 __global__ __launch_bounds__(kTWarps * 32, 5) void k_thermal_march(const __grid_constant__ TMarchParams tp)
 {
     __shared__ __align__(16) char s_ring[kTWarps][kTWarpSmem];
+    kernel_release();
     const int lane = (int)threadIdx.x & 31, wib = (int)threadIdx.x >> 5;
     const int gw = (int)blockIdx.x * kTWarps + wib;
-    if (gw >= tp.nwarps) return;
     char *S = s_ring[wib] + kTGuard;
     // this warp's strip-rows [a, b)
     unsigned long long a = tp.rows * (unsigned long long)gw / (unsigned long long)tp.nwarps;
@@ -228,6 +228,8 @@ __global__ __launch_bounds__(kTWarps * 32, 5) void k_thermal_march(const __grid_
         if ((unsigned long long)tp.strips[mid].w <= a) lo_s = mid;
         else hi_s = mid - 1;
     }
+    kernel_wait();
+    if (gw >= tp.nwarps) return;
     for (int s = lo_s; a < b && s < tp.nstrips; ++s) {
         const uint4 d = tp.strips[s];
         const WorldDev &wd = tp.p.worlds[d.x];
@@ -256,7 +258,7 @@ void launch_mode(const Batch &b, TMarchParams &tp, cudaStream_t st)
 {
     const int nb = march_blocks(b, tp.rows, (const void *)k_thermal_march<MODE>, kTWarps * 32, 0, kTWarps * kTMinRows);
     tp.nwarps = nb * kTWarps;
-    k_thermal_march<MODE><<<(unsigned)nb, kTWarps * 32, 0, st>>>(tp);
+    launch_chained(k_thermal_march<MODE>, (unsigned)nb, kTWarps * 32, 0, st, tp);
 }
 
 }  // namespace

@@ -729,7 +729,7 @@ int tecto_phase_collide(tecto_world *w, tecto_stream_t stream)
 int tecto_phase_resolve(tecto_world *w, tecto_stream_t stream)
 {
     TECTO_PHASE_PROLOGUE
-    rc = launch_resolve(*b, st);
+    rc = launch_resolve(*b, true, st);
     if (rc == TECTO_OK && b->settings.step.upliftMode == TECTO_UPLIFT_REFERENCE) rc = launch_uplift_ref(*b, st);
     TECTO_PHASE_EPILOGUE
 }
@@ -755,7 +755,7 @@ int tecto_phase_finish(tecto_world *w, tecto_stream_t stream)
     TECTO_PHASE_PROLOGUE
     const int period = w->settings.sim.iterationsForCCL > 0 ? w->settings.sim.iterationsForCCL : 1;
     const bool due = w->iteration % (uint32_t)period == 0;
-    if ((rc = launch_finish(*b, st)) == TECTO_OK &&
+    if ((rc = launch_finish(*b, false, false, st)) == TECTO_OK &&
         (!due || (rc = launch_ccl(*b, w->settings.step.cclConnectivity, false, st)) == TECTO_OK) &&
         (!w->settings.step.platePolicy || (rc = launch_plate_policy(*b, due ? 1 : 0, st)) == TECTO_OK) &&
         (rc = launch_bump_iteration(*b, st)) == TECTO_OK)

@@ -322,14 +322,16 @@ int batch_enqueue_step(Batch &b, cudaStream_t st, int ccl)
     if ((rc = launch_sort_keys(b, st)) != TECTO_OK) return rc;
     if ((rc = launch_words(b, st)) != TECTO_OK) return rc;
     if ((rc = launch_type_matrix(b, st)) != TECTO_OK) return rc;
-    if ((rc = launch_resolve(b, st)) != TECTO_OK) return rc;
+    if ((rc = launch_resolve(b, false, st)) != TECTO_OK) return rc;
     if (s.step.upliftMode == TECTO_UPLIFT_REFERENCE && (rc = launch_uplift_ref(b, st)) != TECTO_OK) return rc;
     if ((rc = launch_thermal(b, s.step.thermalIterations, st)) != TECTO_OK) return rc;
     if ((rc = launch_hydraulic(b, s.step.hydraulicIterations, s.step.hydraulicDt, st)) != TECTO_OK) return rc;
-    if ((rc = launch_finish(b, st)) != TECTO_OK) return rc;
+    // the labelling and the policy read the iteration counter: with either it advances after them
+    const bool bump = !ccl && !s.step.platePolicy;
+    if ((rc = launch_finish(b, true, bump, st)) != TECTO_OK) return rc;
     if (ccl && (rc = launch_ccl(b, s.step.cclConnectivity, ccl == 2, st)) != TECTO_OK) return rc;
     if (s.step.platePolicy && (rc = launch_plate_policy(b, ccl, st)) != TECTO_OK) return rc;
-    return launch_bump_iteration(b, st);
+    return bump ? TECTO_OK : launch_bump_iteration(b, st);
 }
 
 static void sync_members(Batch &b)

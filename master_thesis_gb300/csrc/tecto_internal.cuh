@@ -257,6 +257,41 @@ int cuda_fail(cudaError_t e, const char *what);
         if (e_ != cudaSuccess) return ::tecto::cuda_fail(e_, #call); \
     } while (0)
 
+// ---- launches ---------------------------------------------------------------------------
+//
+// The kernels of a step follow each other within microseconds, so a launch's own latency counts.  They are
+// launched with programmatic stream serialisation: a kernel's blocks may be placed before the kernel ahead
+// of it has completed, and each kernel calls kernel_wait(), which returns when everything before it has
+// completed and is visible.  Every thread of such a kernel calls it before it touches memory that a kernel
+// writes, so completion is transitive along the stream; before it a kernel may read its parameters and the
+// batch's tables (worlds, tiles, strips, virtual bases), which batch_prepare has synchronised.  A launch
+// behind anything else (a copy, a kernel launched the ordinary way) waits for all of it.
+//
+// kernel_release() lets the next kernel's blocks be placed once every block of this one has called it (or
+// ended).  The tile kernels call it before their last phase: placed earlier, the next kernel's blocks fill
+// the SMs that have room at that moment and stay there, two on some and none on others (a 256^2 step of
+// 80 tiles 197 -> 305 us).  The marching kernels fill the machine and call it at once, so that the next
+// one's prologue is done when they end.  A step, us, without and with this: 64^2 143 -> 131, 256^2
+// 191 -> 177, 1001x613 498 -> 483, 1024^2 682 -> 651, 2048^2 1914 -> 1826.
+__device__ __forceinline__ void kernel_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void kernel_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <typename... P, typename... A>
+inline void launch_chained(void (*kern)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t st, A &&...args)
+{
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c{};
+    c.gridDim = grid;
+    c.blockDim = dim3(threads);
+    c.dynamicSmemBytes = smem;
+    c.stream = st;
+    c.attrs = &at;
+    c.numAttrs = 1;
+    cudaLaunchKernelEx(&c, kern, static_cast<P>(args)...);
+}
+
 // ---- device helpers ---------------------------------------------------------------------
 
 // CudaTexture::wrapCoordinate (src/cuda_compute/types/cuda_texture.cuh:67-76)
@@ -322,10 +357,10 @@ int launch_plates(Batch &b, cudaStream_t st);
 int launch_sort_keys(Batch &b, cudaStream_t st);
 int launch_words(Batch &b, cudaStream_t st);
 int launch_type_matrix(Batch &b, cudaStream_t st);
-int launch_resolve(Batch &b, cudaStream_t st);
+int launch_resolve(Batch &b, bool flip, cudaStream_t st);  // flip: flipDivergedBitmap too (else launch_finish does)
 int launch_thermal(Batch &b, int iterations, cudaStream_t st);
 int launch_hydraulic(Batch &b, int iterations, float dt, cudaStream_t st);
-int launch_finish(Batch &b, cudaStream_t st);
+int launch_finish(Batch &b, bool flip, bool bump, cudaStream_t st);  // bump: the iteration counters too
 // plate dynamics (TECTO_PLATE_DYNAMICS_REFERENCE): per-plate sums at the start of a step, and
 // applyPlateMovementChanges at its end
 int launch_plate_stats(Batch &b, cudaStream_t st);
@@ -333,7 +368,6 @@ int launch_plate_motion(Batch &b, cudaStream_t st);
 // plate policy after a step (TECTO_PLATE_RELABEL / TECTO_PLATE_MERGE): ccl 0 no labelling ran, 1 it
 // ran for the world (single world), 2 per world when due (batch)
 int launch_plate_policy(Batch &b, int ccl, cudaStream_t st);
-int launch_clear_marks(Batch &b, cudaStream_t st);
 int launch_bump_iteration(Batch &b, cudaStream_t st);
 // due_only: skip worlds whose step counter is not a multiple of iterationsForCCL
 int launch_ccl(Batch &b, int connectivity, bool due_only, cudaStream_t st);
@@ -382,7 +416,10 @@ bool valid_radix_bits(int rb);
 int sort_passes_for(int key_bits, int rb);
 size_t sort_scratch_bytes(size_t n, int key_bits, int rb);
 void sort_scratch_carve(void *base, size_t n, int key_bits, int rb, SortScratch *out);
+// The caller clears sort_clear_bytes from scr.hist on first (run_sort_clear does it with a memset).
 int run_sort(const SortArgs &a, const SortScratch &scr, cudaStream_t st, int *result_half);
+int run_sort_clear(const SortScratch &scr, size_t n, cudaStream_t st);
+size_t sort_clear_bytes(const SortScratch &scr, size_t n);
 int sort_kernel_attributes();  // once, outside graph capture, before any digit width above 8
 
 int key_bits_for(size_t n);

@@ -141,7 +141,10 @@ int tune_shapes(const tecto_settings &settings, const std::vector<int2> &shapes,
         tb.settings.step.sortRadixBits = rb;
         if ((rc = batch_prepare(tb, st)) != TECTO_OK) break;
         float ms = 0;
-        rc = time_best(st, 3, &ms, [&]() { return launch_sort_keys(tb, st); });
+        rc = time_best(st, 3, &ms, [&]() {
+            const int cr = run_sort_clear(tb.sort, tb.total, st);
+            return cr == TECTO_OK ? launch_sort_keys(tb, st) : cr;
+        });
         res.sort_ms[rb - 8] = ms;
         if (rc == TECTO_OK && ms < best_sms) {
             best_sms = ms;
