@@ -132,7 +132,8 @@ typedef struct tecto_step_settings {
     float upliftSigma;        /* Gaussian sigma in cells */
     int upliftRadius;         /* taps on each side (<= 8) */
     int cclConnectivity;      /* TECTO_CCL_* */
-    int sortRadixBits;        /* collision sort digit width 8..11; 0 = autotuner's choice, else 8 */
+    int sortRadixBits;        /* collision sort digit width 8..11; 0 = autotuner's choice, else 9 where it
+                                 saves a pass over 8 and 8 elsewhere */
     int hydraulicTile;        /* 0 = autotuner's choice, else by the batch's cells: 1 up to 2^17, 3 up to
                                  2^20, 4 up to 2.5 M, then 9.  Tiles of cells / warps, two cells a lane:
                                  1: 56x8/16, 2: 56x8/8, 3: 56x16/8, 4: 56x24/8, 5: 56x32/10, 6: 56x16/6,
@@ -341,7 +342,7 @@ int tecto_sort_pairs_radix(const uint32_t *keys_in, const uint32_t *vals_in, uin
                            uint32_t *vals_out, size_t n, int key_bits, int radix_bits, void *scratch,
                            size_t scratch_bytes, tecto_stream_t stream);
 /* 1 when a sort of n pairs runs its passes in the form for large sorts (from 4096 tiles of 4096
- * keys, i.e. 16 777 216 pairs: three blocks per SM), 0 when it runs the form for smaller sorts.
+ * keys, i.e. 16 777 216 pairs), 0 when it runs the form for smaller sorts; both are one form now.
  * The collision sort of a batch or world uses the same rule on its cell count. */
 int tecto_sort_wide_pass(size_t n);
 
@@ -429,7 +430,7 @@ int tecto_batch_phase_thermal(tecto_batch *batch, int iterations, tecto_stream_t
  * (total cells and mean world cells, half-octave classes); batches whose settings leave
  * hydraulicTile / thermalTile / sortRadixBits at 0 use the choice cached for their class, else for
  * the nearest tuned class on their device, else the defaults (by the batch's
- * cells, see hydraulicTile and thermalTile; 8-bit digits). */
+ * cells, see hydraulicTile, thermalTile and sortRadixBits). */
 typedef struct tecto_tuning {
     int hydraulicTile;       /* chosen variant, 1..9 */
     int sortRadixBits;       /* chosen digit width, 8..11 */

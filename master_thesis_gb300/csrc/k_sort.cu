@@ -24,27 +24,27 @@ namespace {
 
 constexpr int kWarps = kSortThreads / 32;
 constexpr int kLookAhead = 8;  // predecessor tiles read per look-back round
-// From this many tiles (16 M keys) a pass runs three blocks per SM: measured faster at 67 M keys
-// (8192^2) and slower at 4 M (2048^2)
-constexpr size_t kSortWideTiles = 4096;
 constexpr int kDoneCounter = 8;  // word of SortScratch::counters that counts finished histogram blocks
 
 template <int RB>
 struct Digits {
     static constexpr int R = 1 << RB;               // digit values per pass
-    static constexpr int DPT = R / kSortThreads;     // digits owned by each thread of a pass
+    static constexpr int DPT = R / kSortThreads;     // digits owned by each thread of the scan
     static constexpr uint32_t MASK = (uint32_t)R - 1u;
     static constexpr int MAX_PASSES = (32 + RB - 1) / RB;
     static_assert(RB >= 8 && RB <= kMaxRadixBits, "digit width out of range");
 };
 
-// Dynamic shared memory of one pass: per-warp digit counts, per-digit tile start and global
-// base, the staged keys and values.
+// Whether a pass ranks with lane masks: a warp's masks share its part of the staging area (R words in
+// 2 * 32 * kSortItems).
+template <int RB>
+constexpr bool kMaskRank = (1 << RB) <= 2 * 32 * kSortItems;
+
+// Dynamic shared memory of one pass: per-warp digit counts, the digits' offsets, the staged keys and values.
 template <int RB>
 constexpr size_t pass_smem()
 {
-    return ((size_t)kWarps * Digits<RB>::R + 2 * (size_t)Digits<RB>::R + 2 * (size_t)kSortTile) *
-           sizeof(uint32_t);
+    return ((size_t)(kWarps + 1) * Digits<RB>::R + 2 * (size_t)kSortTile) * sizeof(uint32_t);
 }
 
 // Batch-virtual destination of virtual cell i: the owning world's getPixelMovements destination
@@ -56,16 +56,31 @@ struct GenArgs {
     int cur_id;
 };
 
-__device__ __forceinline__ uint32_t gen_key(size_t i, const GenArgs &g, const uint32_t *s_vbase)
+// The keys of the `count` (1 .. 4) cells from virtual cell v on: the world and the row are found once and
+// advanced.
+__device__ __forceinline__ void gen_keys(uint32_t v, int count, const GenArgs &g, const uint32_t *s_vbase, uint32_t *key)
 {
-    const uint32_t v = (uint32_t)i;  // n < 2^30
-    const WorldDev &wd = g.worlds[find_world(s_vbase, g.nworlds, v)];
-    const uint32_t local = v - wd.vbase;
-    const int W = wd.W;
-    const int y = (int)(local / (uint32_t)W);
-    const int x = (int)(local - (uint32_t)y * (uint32_t)W);
-    const int2 o = wd.off[wd.id[g.cur_id][local]];
-    return wd.vbase + cidx(x + o.x, y + o.y, W, wd.H);
+    int wi = find_world(s_vbase, g.nworlds, v);
+    const WorldDev *wd = g.worlds + wi;
+    uint32_t local = v - wd->vbase;
+    int W = wd->W, H = wd->H;
+    int y = (int)(local / (uint32_t)W), x = (int)(local - (uint32_t)y * (uint32_t)W);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        if (q >= count) break;
+        const int2 o = wd->off[wd->id[g.cur_id][local]];
+        key[q] = wd->vbase + cidx(x + o.x, y + o.y, W, H);
+        ++local;
+        if (++x == W) {
+            x = 0;
+            if (++y == H && q + 1 < count) {  // the next world's first cell
+                wd = g.worlds + ++wi;
+                W = wd->W, H = wd->H;
+                y = 0;
+                local = 0;
+            }
+        }
+    }
 }
 
 __device__ __forceinline__ void load_vbase(const GenArgs &g, uint32_t *s_vbase)
@@ -83,8 +98,9 @@ __device__ __forceinline__ void st_volatile(uint32_t *p, uint32_t v)
     *(volatile uint32_t *)p = v;
 }
 
-// Block-wide exclusive scan of one value per thread (256 threads); returns the exclusive prefix
-// and the block total.  s_w holds kWarps words; the call ends with a barrier.
+// Block-wide exclusive scan of one value per thread (W warps); returns the exclusive prefix and the block
+// total.  s_w holds W words; the call ends with a barrier.
+template <int W>
 __device__ __forceinline__ uint32_t block_scan(uint32_t v, uint32_t *s_w, uint32_t *total)
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -97,7 +113,7 @@ __device__ __forceinline__ uint32_t block_scan(uint32_t v, uint32_t *s_w, uint32
     __syncthreads();
     uint32_t wb = 0, all = 0;
 #pragma unroll
-    for (int k = 0; k < kWarps; ++k) {
+    for (int k = 0; k < W; ++k) {
         const uint32_t x = s_w[k];
         wb += k < warp ? x : 0u;
         all += x;
@@ -132,27 +148,44 @@ __global__ __launch_bounds__(256) void k_sort_hist(GenArgs g, const uint32_t *ke
     for (int i = threadIdx.x; i < D::MAX_PASSES * D::R; i += blockDim.x) (&s_hist[0][0])[i] = 0;
     if (GEN) load_vbase(g, s_vbase);
     __syncthreads();
+    // four consecutive keys a thread; every lane runs the same number of rounds for the votes below
     const unsigned lane = threadIdx.x & 31u;
-    const size_t stride = (size_t)gridDim.x * blockDim.x;
-    // every lane runs the same number of rounds so that the warp-wide match stays converged
-    const size_t rounds = (n + stride - 1) / stride;
-    for (size_t r = 0; r < rounds; ++r) {
-        const size_t i = r * stride + (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-        const bool valid = i < n;
-        uint32_t key = 0;
-        if (valid) {
-            if (GEN) {
-                key = gen_key(i, g, s_vbase);
-                keys_gen[i] = key;
+    const size_t stride = (size_t)gridDim.x * 1024u;
+    const bool vec = !GEN && (reinterpret_cast<uintptr_t>(keys_in) & 15u) == 0;  // the caller's alignment
+    for (size_t b0 = (size_t)blockIdx.x * 1024u; b0 < n; b0 += stride) {
+        const size_t i = b0 + 4u * threadIdx.x;
+        const int count = i >= n ? 0 : n - i < 4 ? (int)(n - i) : 4;
+        uint32_t key[4] = {0u, 0u, 0u, 0u};
+        if (GEN) {
+            if (count) gen_keys((uint32_t)i, count, g, s_vbase, key);
+            if (count == 4) *reinterpret_cast<uint4 *>(keys_gen + i) = make_uint4(key[0], key[1], key[2], key[3]);
+            else
+                for (int q = 0; q < count; ++q) keys_gen[i + q] = key[q];
+        } else {
+            if (vec && count == 4) {
+                const uint4 k4 = *reinterpret_cast<const uint4 *>(keys_in + i);
+                key[0] = k4.x, key[1] = k4.y, key[2] = k4.z, key[3] = k4.w;
             } else {
-                key = keys_in[i];
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                    if (q < count) key[q] = keys_in[i + q];
             }
         }
         for (int p = 0; p < passes; ++p) {
-            const uint32_t d = valid ? ((key >> (RB * p)) & D::MASK) : (uint32_t)D::R;
-            const unsigned peers = __match_any_sync(0xffffffffu, d);
-            if (valid && (peers & ((1u << lane) - 1u)) == 0)
-                atomicAdd(&s_hist[p][d], (uint32_t)__popc(peers));
+            uint32_t d[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) d[q] = (key[q] >> (RB * p)) & D::MASK;
+            const bool four = count == 4 && d[0] == d[1] && d[0] == d[2] && d[0] == d[3];
+            const uint32_t d0 = __shfl_sync(0xffffffffu, d[0], 0);
+            if (__all_sync(0xffffffffu, four && d[0] == d0)) {  // the warp's 128 keys share the digit
+                if (lane == 0) atomicAdd(&s_hist[p][d0], 128u);
+            } else if (four) {
+                atomicAdd(&s_hist[p][d[0]], 4u);
+            } else {
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                    if (q < count) atomicAdd(&s_hist[p][d[q]], 1u);
+            }
         }
     }
     __syncthreads();
@@ -175,197 +208,206 @@ __global__ __launch_bounds__(256) void k_sort_hist(GenArgs g, const uint32_t *ke
             uint32_t *h = hist + (size_t)p * D::R + c * kSortThreads + t;
             const uint32_t v = ld_volatile(h);
             uint32_t tot = 0;
-            const uint32_t ex = block_scan(v, s_w, &tot);
+            const uint32_t ex = block_scan<kWarps>(v, s_w, &tot);
             *h = carry + ex;
             carry += tot;
         }
     }
 }
 
-// One onesweep pass.  vals_in == nullptr: the value of position i is i.  Two kernels share the
-// body: k_sort_pass (the compiler takes 128 registers: two blocks per SM) for small sorts, and
-// k_sort_pass_wide (three blocks per SM: 80 registers, a few more bytes of spill) once there are
-// enough tiles to fill the extra residency.
-template <int RB>
-__device__ __forceinline__ void sort_pass_body(
-    const uint32_t *keys_in, const uint32_t *vals_in, uint32_t *keys_out, uint32_t *vals_out, size_t n,
-    int shift, const uint32_t *digit_start, uint32_t *status, uint32_t *tile_counter, uint32_t *error)
+// One tile of a onesweep pass.  vals_in == nullptr: the value of position i is i.
+// FULL: every position of the tile is below n.
+template <int RB, bool FULL>
+__device__ __forceinline__ void sort_tile(const uint32_t *keys_in, const uint32_t *vals_in, uint32_t *keys_out,
+                                          uint32_t *vals_out, uint32_t n, int shift, const uint32_t *digit_start,
+                                          uint32_t *status, uint32_t tile, uint32_t *error, uint32_t *sm, uint32_t *s_w)
 {
     using D = Digits<RB>;
-    constexpr int R = D::R, DPT = D::DPT;
-    extern __shared__ __align__(16) uint32_t sm_sort[];
-    uint32_t *s_cnt = sm_sort;                   // [kWarps][R] per-warp counts, then warp offsets
-    uint32_t *s_start = s_cnt + kWarps * R;      // tile-local exclusive start per digit
-    uint32_t *s_base = s_start + R;              // global output position of the digit's run
-    uint32_t *s_keys = s_base + R;
-    uint32_t *s_vals = s_keys + kSortTile;
-    __shared__ uint32_t s_w[kWarps];
-    __shared__ uint32_t s_tile;
-
+    constexpr int R = D::R, W = kWarps, DPT = D::DPT, NT = kSortThreads;
+    constexpr uint32_t T = kSortTile;
+    uint32_t *s_cnt = sm;               // [W][R] per-warp counts, then the tile position of the warp's first key
+    uint32_t *s_off = s_cnt + W * R;    // output position of a digit's run less its position in the tile
+    uint32_t *s_keys = s_off + R;
+    uint32_t *s_vals = s_keys + T;
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    if (t == 0) s_tile = atomicAdd(tile_counter, 1u);
-    for (int i = t; i < kWarps * R; i += kSortThreads) s_cnt[i] = 0;
-    __syncthreads();
-    const uint32_t tile = s_tile;
-    const size_t base = (size_t)tile * kSortTile;
+    const uint32_t base = tile * T, wbase = base + (uint32_t)warp * (32 * kSortItems) + (uint32_t)lane;
 
-    uint32_t k[kSortItems], v[kSortItems], rank[kSortItems];
-    const size_t wbase = base + (size_t)warp * (32 * kSortItems);
+    uint32_t k[kSortItems], rank[kSortItems];
 #pragma unroll
-    for (int it = 0; it < kSortItems; ++it) {
-        const size_t idx = wbase + (size_t)it * 32 + lane;
-        if (idx < n) {
-            k[it] = keys_in[idx];
-            v[it] = vals_in ? vals_in[idx] : (uint32_t)idx;
-        } else {
-            k[it] = 0;
-            v[it] = 0;
-        }
-    }
+    for (int it = 0; it < kSortItems; ++it) k[it] = FULL || wbase + it * 32 < n ? keys_in[wbase + it * 32] : 0u;
 
     // Warp-level ranking: items are visited in element order (item, lane), so the rank of an
-    // item among equal digits of its warp preserves input order (stability).
+    // item among equal digits of its warp preserves input order (stability).  The lanes with an item's digit
+    // come from a vote where the whole warp has one digit (the upper digits of keys that are nearly in
+    // order), else from a lane mask per digit that the lanes set with shared atomics and the first of them
+    // clears again.  The widest digits, whose masks do not fit the staging area, take a ballot per bit.
     const unsigned lt = (1u << lane) - 1u;
     uint32_t *my_cnt = s_cnt + warp * R;
+    uint32_t *my_mask = s_keys + warp * R;  // the staging area is not in use yet
 #pragma unroll
     for (int it = 0; it < kSortItems; ++it) {
-        const bool valid = wbase + (size_t)it * 32 + lane < n;
+        const bool valid = FULL || wbase + it * 32 < n;
         const uint32_t d = (k[it] >> shift) & D::MASK;
-        unsigned peers = __ballot_sync(0xffffffffu, valid);
-#pragma unroll
-        for (int b = 0; b < RB; ++b) {
-            const bool bit = (d >> b) & 1u;
-            const unsigned bb = __ballot_sync(0xffffffffu, bit);
-            peers &= bit ? bb : ~bb;
+        const uint32_t d0 = __shfl_sync(0xffffffffu, d, 0);
+        if (__all_sync(0xffffffffu, valid && d == d0)) {
+            const uint32_t before = my_cnt[d0];
+            __syncwarp();
+            if (lane == 0) my_cnt[d0] = before + 32u;
+            __syncwarp();
+            rank[it] = before + (uint32_t)lane;
+            continue;
         }
-        uint32_t before = 0;
-        if (valid) before = my_cnt[d];
+        unsigned peers;
+        if constexpr (kMaskRank<RB>) {
+            if (valid) atomicOr(my_mask + d, 1u << lane);
+            __syncwarp();
+            peers = valid ? my_mask[d] : 0u;
+        } else {
+            peers = __ballot_sync(0xffffffffu, valid);
+#pragma unroll
+            for (int b = 0; b < RB; ++b) {
+                const bool bit = (d >> b) & 1u;
+                const unsigned bb = __ballot_sync(0xffffffffu, bit);
+                peers &= bit ? bb : ~bb;
+            }
+        }
+        const uint32_t before = my_cnt[d];
         __syncwarp();
-        if (valid && (peers & lt) == 0) my_cnt[d] = before + (uint32_t)__popc(peers);
+        if (valid && (peers & lt) == 0) {
+            my_cnt[d] = before + (uint32_t)__popc(peers);
+            if constexpr (kMaskRank<RB>) my_mask[d] = 0u;
+        }
         __syncwarp();
         rank[it] = before + (uint32_t)__popc(peers & lt);
     }
     __syncthreads();
 
-    // Per owned digit d = t + 256 c: warp offsets and the tile's count of that digit, published
-    // at once so that later tiles can start their look-back.
+    // Per owned digit: the tile's count of it, published at once so that later tiles can start their
+    // look-back; then its tile-local start (chunks of 256 digits in order) and the position of each warp's
+    // first key of it.
     uint32_t run[DPT];
     uint32_t *my_status = status + (size_t)tile * R;
 #pragma unroll
     for (int c = 0; c < DPT; ++c) {
-        const int d = t + c * kSortThreads;
+        const int d = t + c * NT;
         uint32_t r = 0;
 #pragma unroll
-        for (int w = 0; w < kWarps; ++w) {
+        for (int w = 0; w < W; ++w) r += s_cnt[w * R + d];
+        st_volatile(my_status + d, (tile == 0 ? kFlagPrefix : kFlagAggregate) | r);
+        run[c] = r;
+    }
+    uint32_t carry = 0, start[DPT];
+#pragma unroll
+    for (int c = 0; c < DPT; ++c) {
+        const int d = t + c * NT;
+        uint32_t tot = 0;
+        start[c] = carry + block_scan<W>(run[c], s_w, &tot);
+        carry += tot;
+        uint32_t r = start[c];
+#pragma unroll
+        for (int w = 0; w < W; ++w) {
             const uint32_t x = s_cnt[w * R + d];
             s_cnt[w * R + d] = r;
             r += x;
         }
-        run[c] = r;
-        st_volatile(my_status + d, (tile == 0 ? kFlagPrefix : kFlagAggregate) | r);
     }
-    // Tile-local exclusive start of every digit (chunks of 256 digits in order).
-    uint32_t carry = 0;
+    __syncthreads();
+
+    // Scatter the keys into shared memory in digit order.
 #pragma unroll
-    for (int c = 0; c < DPT; ++c) {
-        uint32_t tot = 0;
-        const uint32_t ex = block_scan(run[c], s_w, &tot);
-        s_start[t + c * kSortThreads] = carry + ex;
-        carry += tot;
+    for (int it = 0; it < kSortItems; ++it) {
+        if (FULL || wbase + it * 32 < n) {
+            rank[it] += my_cnt[(k[it] >> shift) & D::MASK];
+            s_keys[rank[it]] = k[it];
+        }
     }
 
-    // Decoupled look-back for the owned digits, walked side by side.  Each round reads the status
-    // words of up to kLookAhead predecessors at once (independent loads in flight together) and
-    // consumes them newest first until one is not yet published or carries an inclusive prefix.
+    // Decoupled look-back for the owned digits.  Each round reads the status words of up to kLookAhead
+    // predecessors at once (independent loads in flight together) and consumes them newest first until one
+    // is not yet published or carries an inclusive prefix.
     uint32_t prefix[DPT];
 #pragma unroll
     for (int c = 0; c < DPT; ++c) prefix[c] = 0;
     if (tile > 0) {
-        int j[DPT];
-#pragma unroll
-        for (int c = 0; c < DPT; ++c) j[c] = (int)tile - 1;
         uint32_t spins = 0;
-        bool pending = true;
-        while (pending) {
-            pending = false;
-            bool progressed = false;
 #pragma unroll
-            for (int c = 0; c < DPT; ++c) {
-                if (j[c] < 0) continue;
-                const uint32_t *col = status + t + c * kSortThreads;
-                const int j0 = j[c];
+        for (int c = 0; c < DPT; ++c) {
+            const int d = t + c * NT;
+            int j = (int)tile - 1;
+            while (j >= 0) {
+                const uint32_t *col = status + (size_t)j * R + d;
                 uint32_t sv[kLookAhead];
 #pragma unroll
-                for (int q = 0; q < kLookAhead; ++q) sv[q] = j0 - q >= 0 ? ld_volatile(col + (size_t)(j0 - q) * R) : 0u;
+                for (int q = 0; q < kLookAhead; ++q) sv[q] = j >= q ? ld_volatile(col - q * R) : kFlagPrefix;
+                bool go = true;
                 int used = 0;
-                bool done = false;
 #pragma unroll
                 for (int q = 0; q < kLookAhead; ++q) {
-                    if (done || used < q || j0 - q < 0) continue;
-                    const uint32_t st = sv[q];
-                    if ((st & ~kValueMask) == 0) continue;  // not yet published: read it again next round
-                    progressed = true;
-                    prefix[c] += st & kValueMask;
-                    used = q + 1;
-                    done = (st & kFlagPrefix) != 0;
+                    go = go && (sv[q] & ~kValueMask) != 0;  // not yet published: read it again next round
+                    if (go) {
+                        prefix[c] += sv[q] & kValueMask;
+                        used = q + 1;
+                        if (sv[q] & kFlagPrefix) {
+                            used = j + 1;
+                            go = false;
+                        }
+                    }
                 }
-                j[c] = done ? -1 : j0 - used;
-                if (j[c] >= 0) pending = true;
+                j -= used;
+                if (used == 0 && ++spins > kSpinLimit) {  // a predecessor never published
+                    atomicOr(error, kErrLookbackTimeout);
+                    break;
+                }
             }
-            if (pending && !progressed && ++spins > kSpinLimit) {  // a predecessor never published
-                atomicOr(error, kErrLookbackTimeout);
-                break;
-            }
+            st_volatile(my_status + d, kFlagPrefix | ((prefix[c] + run[c]) & kValueMask));
         }
-#pragma unroll
-        for (int c = 0; c < DPT; ++c)
-            st_volatile(my_status + t + c * kSortThreads, kFlagPrefix | ((prefix[c] + run[c]) & kValueMask));
     }
 #pragma unroll
     for (int c = 0; c < DPT; ++c) {
-        const int d = t + c * kSortThreads;
-        s_base[d] = digit_start[d] + prefix[c];
+        const int d = t + c * NT;
+        s_off[d] = digit_start[d] + prefix[c] - start[c];
     }
-    __syncthreads();
-
-    // Scatter into shared memory in digit order.
+    // the values are read only now, so that they occupy no registers while the keys are ranked
 #pragma unroll
-    for (int it = 0; it < kSortItems; ++it) {
-        if (wbase + (size_t)it * 32 + lane < n) {
-            const uint32_t d = (k[it] >> shift) & D::MASK;
-            const uint32_t pos = s_start[d] + my_cnt[d] + rank[it];
-            s_keys[pos] = k[it];
-            s_vals[pos] = v[it];
-        }
-    }
+    for (int it = 0; it < kSortItems; ++it)
+        if (FULL || wbase + it * 32 < n) s_vals[rank[it]] = vals_in ? vals_in[wbase + it * 32] : wbase + it * 32;
     __syncthreads();
-    const size_t rem = n - base;
-    const uint32_t tile_n = rem < (size_t)kSortTile ? (uint32_t)rem : (uint32_t)kSortTile;
-    for (uint32_t jj = t; jj < tile_n; jj += kSortThreads) {
+    const uint32_t tile_n = FULL ? T : n - base;
+#pragma unroll 4
+    for (uint32_t jj = t; jj < tile_n; jj += NT) {
         const uint32_t key = s_keys[jj];
-        const uint32_t d = (key >> shift) & D::MASK;
-        const uint32_t out = s_base[d] + (jj - s_start[d]);
+        const uint32_t out = s_off[(key >> shift) & D::MASK] + jj;
         keys_out[out] = key;
         vals_out[out] = s_vals[jj];
     }
 }
 
+// A sort of 3 M pairs 193 -> 103 us, of 43.6 M 1.91 -> 1.01 ms, against ranking by eight ballots a key with
+// the values held in registers at two and three blocks per SM.
+// Four blocks per SM (64 registers, some of the ranks spilled): a tile waits on its loads and its look-back
+// most of the time.  Tiles of 8192 keys by 512 threads were no faster (8192^2: 3.99 against 3.60 ms for a
+// step's phases other than erosion).
 template <int RB>
-__global__ __launch_bounds__(kSortThreads) void k_sort_pass(
-    const uint32_t *keys_in, const uint32_t *vals_in, uint32_t *keys_out, uint32_t *vals_out, size_t n,
+__global__ __launch_bounds__(kSortThreads, 4) void k_sort_pass(
+    const uint32_t *keys_in, const uint32_t *vals_in, uint32_t *keys_out, uint32_t *vals_out, uint32_t n,
     int shift, const uint32_t *digit_start, uint32_t *status, uint32_t *tile_counter, uint32_t *error)
 {
+    using D = Digits<RB>;
+    extern __shared__ __align__(16) uint32_t sm_sort[];
+    __shared__ uint32_t s_w[kWarps];
+    __shared__ uint32_t s_tile;
     kernel_wait();
-    sort_pass_body<RB>(keys_in, vals_in, keys_out, vals_out, n, shift, digit_start, status, tile_counter, error);
-}
-
-template <int RB>
-__global__ __launch_bounds__(kSortThreads, 3) void k_sort_pass_wide(
-    const uint32_t *keys_in, const uint32_t *vals_in, uint32_t *keys_out, uint32_t *vals_out, size_t n,
-    int shift, const uint32_t *digit_start, uint32_t *status, uint32_t *tile_counter, uint32_t *error)
-{
-    kernel_wait();
-    sort_pass_body<RB>(keys_in, vals_in, keys_out, vals_out, n, shift, digit_start, status, tile_counter, error);
+    if (threadIdx.x == 0) s_tile = atomicAdd(tile_counter, 1u);
+    for (int i = threadIdx.x; i < kWarps * D::R; i += kSortThreads) {
+        sm_sort[i] = 0;
+        if constexpr (kMaskRank<RB>) sm_sort[(kWarps + 1) * D::R + i] = 0;
+    }
+    __syncthreads();
+    const uint32_t tile = s_tile;
+    if ((tile + 1) * kSortTile <= n)
+        sort_tile<RB, true>(keys_in, vals_in, keys_out, vals_out, n, shift, digit_start, status, tile, error, sm_sort, s_w);
+    else
+        sort_tile<RB, false>(keys_in, vals_in, keys_out, vals_out, n, shift, digit_start, status, tile, error, sm_sort, s_w);
 }
 
 size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
@@ -373,10 +415,7 @@ size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 template <int RB>
 int set_sort_attributes()
 {
-    TECTO_CUDA(cudaFuncSetAttribute(k_sort_pass<RB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)pass_smem<RB>()));
-    TECTO_CUDA(cudaFuncSetAttribute(k_sort_pass_wide<RB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)pass_smem<RB>()));
+    TECTO_CUDA(cudaFuncSetAttribute(k_sort_pass<RB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pass_smem<RB>()));
     return TECTO_OK;
 }
 
@@ -390,7 +429,7 @@ int run_sort_rb(const SortArgs &a, const SortScratch &scr, cudaStream_t st, int 
     constexpr int R = Digits<RB>::R;
     const bool gen = a.worlds != nullptr;
     const GenArgs g{a.worlds, a.vbase, a.nworlds, a.cur_id};
-    int hist_blocks = (int)((a.n + 255) / 256);
+    int hist_blocks = (int)((a.n + 1023) / 1024);
     if (hist_blocks > 152 * 8) hist_blocks = 152 * 8;
     // generated keys go to the second key half, which the first pass reads and does not write
     const uint32_t *kin = a.keys_in, *vin = a.vals_in;
@@ -405,11 +444,11 @@ int run_sort_rb(const SortArgs &a, const SortScratch &scr, cudaStream_t st, int 
     }
     int half = 0;
     for (int p = 0; p < passes; ++p) {
-        uint32_t *kout = a.keys[half], *vout = a.vals[half];
+        const bool direct = a.keys_final && p > 0 && p == passes - 1;
+        uint32_t *kout = direct ? a.keys_final : a.keys[half], *vout = direct ? a.vals_final : a.vals[half];
         uint32_t *status = scr.status + (size_t)p * tiles * R;
-        auto pass = tiles >= kSortWideTiles ? k_sort_pass_wide<RB> : k_sort_pass<RB>;
-        launch_chained(pass, (unsigned)tiles, kSortThreads, pass_smem<RB>(), st, kin, vin, kout, vout, a.n, RB * p,
-                       scr.hist + (size_t)p * R, status, scr.counters + p, scr.error);
+        launch_chained(k_sort_pass<RB>, (unsigned)tiles, kSortThreads, pass_smem<RB>(), st, kin, vin, kout, vout,
+                       (uint32_t)a.n, RB * p, scr.hist + (size_t)p * R, status, scr.counters + p, scr.error);
         kin = kout;
         vin = vout;
         half ^= 1;
@@ -528,7 +567,7 @@ extern "C" size_t tecto_sort_scratch_bytes(size_t n, int key_bits)
 
 extern "C" int tecto_sort_wide_pass(size_t n)
 {
-    return (n + tecto::kSortTile - 1) / tecto::kSortTile >= (size_t)tecto::kSortWideTiles ? 1 : 0;
+    return n > ((size_t)1 << 24) - (size_t)tecto::kSortTile ? 1 : 0;
 }
 
 extern "C" int tecto_sort_pairs_radix(const uint32_t *keys_in, const uint32_t *vals_in, uint32_t *keys_out,
@@ -563,13 +602,17 @@ extern "C" int tecto_sort_pairs_radix(const uint32_t *keys_in, const uint32_t *v
     a.vals[1] = (uint32_t *)(p + 3 * arr);
     a.n = n;
     a.key_bits = key_bits;
+    a.keys_final = keys_out;
+    a.vals_final = vals_out;
     TECTO_CUDA(cudaMemsetAsync(scr.error, 0, 4, st));
     int half = 0;
     rc = run_sort_clear(scr, n, st);
     if (rc == TECTO_OK) rc = run_sort(a, scr, st, &half);
     if (rc != TECTO_OK) return rc;
-    TECTO_CUDA(cudaMemcpyAsync(keys_out, a.keys[half], n * 4, cudaMemcpyDeviceToDevice, st));
-    TECTO_CUDA(cudaMemcpyAsync(vals_out, a.vals[half], n * 4, cudaMemcpyDeviceToDevice, st));
+    if (scr.passes == 1) {  // the one pass reads the inputs, which the outputs may overlap
+        TECTO_CUDA(cudaMemcpyAsync(keys_out, a.keys[half], n * 4, cudaMemcpyDeviceToDevice, st));
+        TECTO_CUDA(cudaMemcpyAsync(vals_out, a.vals[half], n * 4, cudaMemcpyDeviceToDevice, st));
+    }
     uint32_t err = 0;
     TECTO_CUDA(cudaMemcpyAsync(&err, scr.error, 4, cudaMemcpyDeviceToHost, st));
     TECTO_CUDA(cudaStreamSynchronize(st));

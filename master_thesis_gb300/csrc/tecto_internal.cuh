@@ -411,6 +411,8 @@ struct SortArgs {
     uint32_t *vals[2];
     size_t n;
     int key_bits;
+    uint32_t *keys_final = nullptr;  // where the last of two or more passes writes, if set
+    uint32_t *vals_final = nullptr;
 };
 bool valid_radix_bits(int rb);
 int sort_passes_for(int key_bits, int rb);
