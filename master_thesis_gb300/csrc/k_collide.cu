@@ -93,79 +93,162 @@ __device__ __forceinline__ int evidence_category(const uint8_t *bm, uint8_t A, u
 // writes zero words into the gap of destinations nobody moved into, and for convergent cells
 // adds the collision-type evidence of the determineCollisionType kernel (:838-888) with
 // warp-aggregated atomics.
+//
+// The bytes (13 a cell) take 100 us for a batch of 49.7 M cells; instructions and the chain of gathers
+// (key, source, plate, height) bound it: 248 us there, 260 us for 67 M cells in one world.  With one position
+// a thread and runs, gaps and evidence worked off in place it took 629 and 508 us (230 warp instructions per
+// 32 positions, now 104), since nearly every warp held some lane with each of them.  So a block takes
+// EACH x 256 positions: the worlds of its first and last key bound every search (most blocks lie in one
+// world), keys and plate ids are staged in shared memory, runs of two and more are collected and worked off
+// densely, and a warp fills a gap with all its lanes.
+template <int EACH>
 __global__ __launch_bounds__(256) void k_words(const uint32_t *keys, const uint32_t *vals, uint32_t n,
                                                const WorldDev *worlds, const uint32_t *vbase, int nworlds,
                                                int cur_id, int cur_h, float thr, int cooldown)
 {
     kernel_wait();
+    constexpr int kSpan = EACH * 256;
+    constexpr uint32_t kNone = 0xffffffffu;   // no key: the batch has fewer cells
     __shared__ uint32_t s_vbase[kMaxBatchWorlds + 1];
-    for (int i = threadIdx.x; i <= nworlds; i += blockDim.x) s_vbase[i] = vbase[i];
+    __shared__ uint32_t s_key[kSpan + 4];  // [1 + p]: position p of the block; one before and three after
+    __shared__ uint8_t s_id[kSpan + 3];    // plate of position p's source
+    __shared__ uint16_t s_run[kSpan / 2];  // first positions of the runs of two and more
+    __shared__ int s_w[2], s_runs;
+    const int t = threadIdx.x;
+    const unsigned lane = t & 31u;
+    const uint32_t j0 = blockIdx.x * (uint32_t)kSpan;
+    const int m = (int)min((uint32_t)kSpan, n - j0);
+    const uint32_t last = keys[j0 + m - 1], before = j0 > 0 ? keys[j0 - 1] : kNone;
+    uint32_t key[EACH], val[EACH];
+#pragma unroll
+    for (int i = 0; i < EACH; ++i) {
+        const int p = i * 256 + t;
+        key[i] = p < m ? keys[j0 + p] : kNone;
+        val[i] = p < m ? vals[j0 + p] : 0u;
+    }
+    if (nworlds > 1)
+        for (int i = t; i <= nworlds; i += 256) s_vbase[i] = vbase[i];
+    if (t < 2) s_w[t] = 0;
+    if (t == 2) s_runs = 0;
     __syncthreads();
-    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    const unsigned lane = threadIdx.x & 31u;
-    const bool valid = j < n;
-    bool leader = false;
-    uint8_t ids[4] = {0, 0, 0, 0};
-    float hs[4] = {0, 0, 0, 0};
-    int cnt = 0;
-    int wi = 0;
-    if (valid) {
-        const uint32_t key = keys[j];
-        const uint32_t prev = j > 0 ? keys[j - 1] : 0xffffffffu;
-        leader = j == 0 || prev != key;
-        if (leader) {
-            // gap of destinations without arrivals (they may belong to earlier worlds)
-            const uint32_t gap0 = j == 0 ? 0u : prev + 1u;
-            for (uint32_t c = gap0; c < key; ++c) {
-                const WorldDev &gw = worlds[find_world(s_vbase, nworlds, c)];
-                gw.word[c - gw.vbase] = 0u;
-            }
-            wi = find_world(s_vbase, nworlds, key);
-            const WorldDev &wd = worlds[wi];
-            uint32_t wv = 0;
-            for (int k = 0; k < 4; ++k) {
-                if (j + k >= n || keys[j + k] != key) break;
-                const uint32_t src = vals[j + k] - wd.vbase;
-                ids[k] = wd.id[cur_id][src];
-                hs[k] = wd.h[cur_h][src];  // determineCollisionHeight: height at the arrival's source
-                wv |= (uint32_t)(255u - ids[k]) << (8 * k);
-                ++cnt;
-            }
-            wd.word[key - wd.vbase] = wv;
+    if (nworlds > 1) {
+        // of the first cell the block writes and of the last (a gap may begin in an earlier world)
+        if (t == 0) s_w[0] = find_world(s_vbase, nworlds, min(before + 1u, key[0]));
+        if (t == 32) s_w[1] = find_world(s_vbase, nworlds, last);
+        __syncthreads();
+    }
+    const int w0 = s_w[0], nw = s_w[1] - w0 + 1;
+    const auto world_of = [&](uint32_t c) -> const WorldDev & {
+        return worlds[nw == 1 ? w0 : w0 + find_world(s_vbase + w0, nw, c)];
+    };
+#pragma unroll
+    for (int i = 0; i < EACH; ++i) {
+        const int p = i * 256 + t;
+        s_key[1 + p] = key[i];
+        if (p < m) {
+            const WorldDev &wd = world_of(key[i]);
+            s_id[p] = wd.id[cur_id][val[i] - wd.vbase];
         }
-        if (j == n - 1) {
-            const uint32_t total = s_vbase[nworlds];  // vbase[n] holds the batch's cell count
-            for (uint32_t c = key + 1u; c < total; ++c) {
-                const WorldDev &gw = worlds[find_world(s_vbase, nworlds, c)];
-                gw.word[c - gw.vbase] = 0u;
+    }
+    if (t < 3) {  // the run at the block's end may go on
+        const uint64_t j = (uint64_t)j0 + kSpan + t;
+        const uint32_t k = j < n ? keys[j] : kNone;
+        s_key[1 + kSpan + t] = k;
+        if (j < n && k == last) {
+            const WorldDev &wd = world_of(k);
+            s_id[kSpan + t] = wd.id[cur_id][vals[j] - wd.vbase];
+        }
+    } else if (t == 3) {
+        s_key[0] = before;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < EACH; ++i) {
+        const int p = i * 256 + t;
+        const uint32_t prev = s_key[p];
+        const bool leader = p < m && prev != key[i];
+        const bool run = leader && s_key[p + 2] == key[i];
+        if (leader && !run) {
+            const WorldDev &wd = world_of(key[i]);
+            wd.word[key[i] - wd.vbase] = 255u - s_id[p];
+        }
+        const unsigned runs = __ballot_sync(0xffffffffu, run);
+        if (runs) {
+            int at = 0;
+            if (lane == 0) at = atomicAdd(&s_runs, __popc(runs));
+            at = __shfl_sync(0xffffffffu, at, 0) + __popc(runs & ((1u << lane) - 1u));
+            if (run) s_run[at] = (uint16_t)p;
+        }
+        // destinations without arrivals before this one (from 0 at the first position: kNone + 1)
+        const uint32_t gap = leader ? key[i] - (prev + 1u) : 0u;
+        for (unsigned g = __ballot_sync(0xffffffffu, gap > 0u); g; g &= g - 1u) {
+            const int from = __ffs(g) - 1;
+            const uint32_t c0 = __shfl_sync(0xffffffffu, prev, from) + 1u, len = __shfl_sync(0xffffffffu, gap, from);
+            for (uint32_t c = lane; c < len; c += 32) {
+                const WorldDev &wd = world_of(c0 + c);
+                wd.word[c0 + c - wd.vbase] = 0u;
             }
         }
     }
-    // pairs in determineCollisionType's order for 2, 3 and 4 arrivals (counts are sums, so the
-    // order only has to cover the same pairs)
-    const int npairs = cnt >= 4 ? 6 : cnt == 3 ? 3 : cnt == 2 ? 1 : 0;
-    const uint8_t PA[6] = {0, 0, 0, 1, 1, 2};
-    const uint8_t PB[6] = {1, 2, 3, 2, 3, 3};
-    const uint8_t PA3[3] = {0, 0, 1};
-    const uint8_t PB3[3] = {1, 2, 2};
-    const uint8_t *bm = npairs ? worlds[wi].type_bitmap : nullptr;
-#pragma unroll
-    for (int slot = 0; slot < 6; ++slot) {
-        uint32_t keyv = 0xffffffffu;
-        uint32_t pair = 0;
-        int cat = -1;
-        if (slot < npairs) {
-            const int a = cnt == 3 ? PA3[slot] : PA[slot];
-            const int b = cnt == 3 ? PB3[slot] : PB[slot];
-            cat = evidence_category(bm, ids[a], ids[b], hs[a], hs[b], thr, cooldown, &pair);
-            // aggregation key: world, pair and category (worlds differ within a warp rarely)
-            if (cat >= 0) keyv = ((uint32_t)wi * (uint32_t)kPairs + pair) * 5u + (uint32_t)cat;
+    if (j0 + m == n) {
+        const uint32_t total = nworlds > 1 ? s_vbase[nworlds] : vbase[nworlds];  // the batch's cell count
+        for (uint32_t c = last + 1u + t; c < total; c += 256) {
+            const WorldDev &wd = worlds[nworlds > 1 ? find_world(s_vbase, nworlds, c) : 0];
+            wd.word[c - wd.vbase] = 0u;
         }
-        const unsigned any = __ballot_sync(0xffffffffu, keyv != 0xffffffffu);
-        if (any == 0) continue;
-        const unsigned peers = __match_any_sync(0xffffffffu, keyv);
-        if (keyv != 0xffffffffu && (peers & ((1u << lane) - 1u)) == 0)
-            atomicAdd(&worlds[wi].counts[pair].c[cat], __popc(peers));
+    }
+    __syncthreads();
+    // Convergent cells.  Evidence: pairs in determineCollisionType's order for 2, 3 and 4 arrivals (counts
+    // are sums, so the order only has to cover the same pairs).
+    const int nruns = s_runs;
+    for (int r = t; r - (int)lane < nruns; r += 256) {
+        uint8_t ids[4] = {0, 0, 0, 0};
+        float hs[4] = {0, 0, 0, 0};
+        int cnt = 0, wi = 0;
+        const uint8_t *bm = nullptr;
+        if (r < nruns) {
+            const int p = s_run[r];
+            const uint32_t k = s_key[1 + p];
+            cnt = 2 + (s_key[p + 3] == k);
+            cnt += s_key[p + 4] == k;
+            const WorldDev &wd = world_of(k);
+            wi = (int)(&wd - worlds);
+            const float *h = wd.h[cur_h];
+            uint32_t wv = 0;
+#pragma unroll
+            for (int a = 0; a < 4; ++a) {
+                if (a >= cnt) break;
+                ids[a] = s_id[p + a];
+                hs[a] = h[vals[j0 + p + a] - wd.vbase];  // determineCollisionHeight: height at the arrival's source
+                wv |= (uint32_t)(255u - ids[a]) << (8 * a);
+            }
+            wd.word[k - wd.vbase] = wv;
+            bm = wd.type_bitmap;
+        }
+        const int npairs = cnt >= 4 ? 6 : cnt == 3 ? 3 : cnt == 2 ? 1 : 0;
+        const uint8_t PA[6] = {0, 0, 0, 1, 1, 2};
+        const uint8_t PB[6] = {1, 2, 3, 2, 3, 3};
+        const uint8_t PA3[3] = {0, 0, 1};
+        const uint8_t PB3[3] = {1, 2, 2};
+#pragma unroll
+        for (int slot = 0; slot < 6; ++slot) {
+            uint32_t keyv = kNone;
+            uint32_t pair = 0;
+            int cat = -1;
+            if (slot < npairs) {
+                const int a = PA[slot], b = PB[slot], a3 = PA3[slot < 3 ? slot : 0], b3 = PB3[slot < 3 ? slot : 0];
+                const bool three = cnt == 3;
+                cat = evidence_category(bm, three ? ids[a3] : ids[a], three ? ids[b3] : ids[b], three ? hs[a3] : hs[a],
+                                        three ? hs[b3] : hs[b], thr, cooldown, &pair);
+                // aggregation key: world, pair and category (worlds differ within a warp rarely)
+                if (cat >= 0) keyv = ((uint32_t)wi * (uint32_t)kPairs + pair) * 5u + (uint32_t)cat;
+            }
+            const unsigned any = __ballot_sync(0xffffffffu, keyv != kNone);
+            if (any == 0) continue;
+            const unsigned peers = __match_any_sync(0xffffffffu, keyv);
+            if (keyv != kNone && (peers & ((1u << lane) - 1u)) == 0)
+                atomicAdd(&worlds[wi].counts[pair].c[cat], __popc(peers));
+        }
     }
 }
 
@@ -253,9 +336,13 @@ int launch_words(Batch &b, cudaStream_t st)
 {
     const uint32_t n = (uint32_t)b.total;
     const tecto_kernel_settings &ks = b.settings.kernel;
-    launch_chained(k_words, (n + 255) / 256, 256, 0, st, b.keys[b.sort_final], b.vals[b.sort_final], n, b.d_worlds,
-                   b.d_vbase, (int)b.members.size(), b.cur_id, b.cur_h, ks.continentalCrustThreshold,
-                   ks.collisionTypeUpdateCooldown);
+    // Four positions a thread halve the time where the chip is full; below that one a thread leaves more
+    // blocks (steps without erosion, one against four a thread: 256^2 44.3 / 46.2 us, 512^2 51.6 / 53.4,
+    // 1001x613 65.7 / 64.5, 1024^2 86.8 / 83.4, 2048^2 224 / 215).
+    const int each = n >= (1u << 19) ? 4 : 1;
+    launch_chained(each == 4 ? k_words<4> : k_words<1>, (n + each * 256u - 1) / (each * 256u), 256, 0, st, b.keys[b.sort_final],
+                   b.vals[b.sort_final], n, b.d_worlds, b.d_vbase, (int)b.members.size(), b.cur_id, b.cur_h,
+                   ks.continentalCrustThreshold, ks.collisionTypeUpdateCooldown);
     TECTO_CUDA(cudaGetLastError());
     b.launches += 1;
     return TECTO_OK;
