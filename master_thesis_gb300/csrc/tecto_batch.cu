@@ -174,16 +174,21 @@ static int default_radix_bits(size_t cells)
 // The default thermal variant: one iteration with tiles (variant 4, two iterations a launch) against the
 // march (5), us: 512^2 5.3 / 6.5, 1024^2 11.6 / 11.0, 2048^2 37.4 / 23.0, 8192^2 570 / 230.
 // The default hydraulic variant follows the batch's cells, as whole steps measured it, us:
-//                64^2  256^2  512^2  1001x613  1024^2  1500x1100  2048^2  12 worlds (0.6 M)  40 worlds (1.0 M)
-//   1 (56x8)      146    197    353       608     906       1424    3379        621              1130
-//   3 (56x16)     178    200    319       502     688       1036    2388        504               872
-//   4 (56x24)     205    221    305       527     705       1001    2250        527               863
-//   9 (march)     283    305    411       674     791       1038    2068        674              1041
-// Small batches want many short tiles, large ones little halo.
-static int default_hydro_variant(size_t cells)
+//                256^2  512^2  1001x613  1024^2  1200x1000  1101x1301  2000x1000  2048^2  12 worlds (0.6 M)
+//   1 (56x8)      167    313     567       838       942       1169       1543      3061        572
+//   3 (56x16)     168    279     461       617       700        838       1099      2078        455
+//   4 (56x24)     187    266     484       632       695        837       1014      1948        475
+//   9 (march)     253    372     529       654       670        792        927      1484        552
+// Small batches want many short tiles, large ones little halo.  The march also wants worlds that fill its
+// strips: worlds 128 to 256 wide, whose strips hold 1.3 and 1.37 times their cells, take 1108 against 1025 us
+// (1.6 M cells) and 1644 against 1571 (2.5 M); 256 to 600 wide, 1.1 times, 925 against 927 (1.6 M).
+static int default_hydro_variant(const Batch &b)
 {
-    if (cells >= kMarchMinCells) return kHydroMarchVariant;
-    return cells <= (size_t)1 << 17 ? 1 : cells <= (size_t)1 << 20 ? 3 : 4;
+    unsigned long long strips = 0;  // cells the march's strips hold
+    for (const tecto_world *w : b.members)
+        strips += (unsigned long long)((w->W + kMarchInner - 1) / kMarchInner) * kMarchInner * (unsigned long long)w->H;
+    if (b.total >= kMarchMinCells && 4 * strips <= 5 * (unsigned long long)b.total) return kHydroMarchVariant;
+    return b.total <= (size_t)1 << 17 ? 1 : b.total <= (size_t)1 << 20 ? 3 : 4;
 }
 
 static void choose_tuning(const Batch &b, int *variant, int *rb, int *tvariant)
@@ -193,7 +198,7 @@ static void choose_tuning(const Batch &b, int *variant, int *rb, int *tvariant)
     if (*tvariant == 0) *tvariant = b.total >= kThermalMarchMinCells ? kThermalMarchVariant : kDefaultThermalVariant;
     *variant = hydro_variant_for(b.settings);
     if (*variant == 0) *variant = b.tuned_hydro;
-    if (*variant == 0) *variant = default_hydro_variant(b.total);
+    if (*variant == 0) *variant = default_hydro_variant(b);
     *rb = b.settings.step.sortRadixBits;
     if (!valid_radix_bits(*rb)) *rb = valid_radix_bits(b.tuned_rb) ? b.tuned_rb : default_radix_bits(b.total);
 }
@@ -252,7 +257,7 @@ int batch_prepare(Batch &b, cudaStream_t st)
     }
     std::vector<uint4> strips[ST_COUNT];
     for (int k = 0; k < ST_COUNT; ++k) {
-        const int inner = k == ST_THERMAL ? kThermalInner : kMarchInner;
+        const int inner = k == ST_THERMAL ? kThermalInner : k == ST_HYDRO_TWO ? kMarchTwoInner : kMarchInner;
         strips[k] = build_strips(b, inner, &b.strips[k].rows);
         b.strips[k].n = (int)strips[k].size();
         need += a256(strips[k].size() * sizeof(uint4));

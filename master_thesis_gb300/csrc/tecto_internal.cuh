@@ -164,7 +164,7 @@ constexpr int kCclTileX = 32, kCclTileY = 32;
 
 // Column strips of a marching kernel over a batch: {world, first column, interior width, first
 // strip-row}, strip-rows counted over all strips.
-enum StripKind { ST_HYDRO = 0, ST_THERMAL, ST_COUNT };
+enum StripKind { ST_HYDRO = 0, ST_HYDRO_TWO, ST_THERMAL, ST_COUNT };
 struct StripTable {
     uint4 *d = nullptr;
     int n = 0;
@@ -382,7 +382,8 @@ constexpr int kHydroVariantCount = 9;
 constexpr int kDefaultHydroVariant = 4;          // 56 x 24 cells: where the autotuner starts from
 constexpr int kHydroStripVariant = 8;            // from here on: the march (8 is kept as another number for it)
 constexpr int kHydroMarchVariant = 9;            // marching row chunks in shared memory (fused path only)
-constexpr size_t kMarchMinCells = 2500000;       // cells from which the hydraulic march is the default
+constexpr size_t kMarchMinCells = 1200000;       // cells from which the hydraulic march is the default
+constexpr int kMarchTwoInner = 112;              // of a strip that takes two sub-iterations at once
 constexpr int kMarchInner = 120;                 // interior columns of one shared-memory strip (128 with it)
 constexpr int kThermalInner = 60;                // interior columns of one thermal strip (64 with the halo)
 constexpr int kThermalVariantCount = 5;

@@ -84,3 +84,24 @@ def test_thermal_march_forms(kind, W, H, thr, A, S):
         w.thermal(3)
         got, want = w.download(T.FIELD_HEIGHT), O.thermal(h, 3, s).reshape(H, W)
     np.testing.assert_array_equal(got.view(np.uint32), want.view(np.uint32))
+
+
+@pytest.mark.parametrize("W,H,iters", [(5, 3, 2), (3, 40, 4), (113, 4, 2), (112, 61, 2), (225, 9, 5), (49, 130, 2),
+                                       (160, 33, 4), (1001, 47, 2)])
+@pytest.mark.parametrize("kind", ["tiny", "clamp", "huge"])
+def test_two_sub_iterations_in_one_march(kind, W, H, iters):
+    """Two sub-iterations share a march where 112-column strips are not many more than 120-column ones:
+    pieces of a few rows, strips of one column and narrower than half a block, worlds that wrap within a
+    halo, odd widths, operands that send rows through the scalar form in the first or the second of two, and
+    an odd number left over.  Bit for bit as the oracle."""
+    s = T.baseline_settings()
+    s.step.hydraulicTile = 9
+    h, water, sed, flux = fields(kind, W, H)
+    with T.World(s, W, H, seed=1000) as w:
+        for f, a in ((T.FIELD_HEIGHT, h), (T.FIELD_WATER, water), (T.FIELD_SEDIMENT, sed), (T.FIELD_FLUX, flux)):
+            w.upload(f, a)
+        w.hydraulic(iters, 0.02)
+        want = O.hydraulic(h, water, sed, flux, iters, 0.02, 1000, s)
+        for name, f, v in zip(("height", "water", "sediment", "flux"),
+                              (T.FIELD_HEIGHT, T.FIELD_WATER, T.FIELD_SEDIMENT, T.FIELD_FLUX), want):
+            np.testing.assert_array_equal(w.download(f).view(np.uint32), v.view(np.uint32), err_msg=name)
