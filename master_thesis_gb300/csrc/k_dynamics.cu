@@ -23,6 +23,7 @@ namespace {
 __global__ __launch_bounds__(256) void k_plate_stats(const WorldDev *worlds, const uint2 *tiles, int cur_h,
                                                      int cur_id)
 {
+    kernel_wait();
     __shared__ unsigned long long s_mass[kPlates];
     __shared__ unsigned long long s_ang[4][kPlates];
     __shared__ int s_size[kPlates], s_samp[kPlates];
@@ -48,10 +49,20 @@ __global__ __launch_bounds__(256) void k_plate_stats(const WorldDev *worlds, con
         const bool xs = x % 10 == 0;
         const float ax = (kTwoPiF * (float)x) / (float)W;
         const float sin_x = tecto_sinf(ax), cos_x = tecto_cosf(ax);
-        for (int y = y0; y < y1; ++y) {
-            const size_t d = (size_t)y * (size_t)W + (size_t)x;
-            const int p = id[d];
-            const float hv = h[d];
+        constexpr int kRows = kStatTileY;  // all loads first
+        int ids[kRows];
+        float hs[kRows];
+#pragma unroll
+        for (int k = 0; k < kRows; ++k) {
+            const size_t d = (size_t)min(y0 + k, y1 - 1) * (size_t)W + (size_t)x;
+            ids[k] = id[d];
+            hs[k] = h[d];
+        }
+#pragma unroll
+        for (int k = 0; k < kRows; ++k) {
+            const int y = y0 + k, p = ids[k];
+            const float hv = hs[k];
+            if (y >= y1) break;
             if (p != run) {
                 if (run >= 0 && run < kPlates) {
                     atomicAdd(s_mass + run, run_m);
@@ -107,6 +118,7 @@ struct MotionParams {
 // velocity and direction.
 __global__ void k_plate_motion(const WorldDev *worlds, MotionParams mp)
 {
+    kernel_wait();
     const WorldDev &wd = worlds[blockIdx.x];
     const int k = threadIdx.x;
     if (k >= kPlates) return;
@@ -164,7 +176,7 @@ __global__ void k_plate_motion(const WorldDev *worlds, MotionParams mp)
 
 int launch_plate_stats(Batch &b, cudaStream_t st)
 {
-    k_plate_stats<<<(unsigned)b.ntiles[TK_STATS], 256, 0, st>>>(b.d_worlds, b.d_tiles[TK_STATS], b.cur_h, b.cur_id);
+    launch_chained(k_plate_stats, (unsigned)b.ntiles[TK_STATS], 256, 0, st, b.d_worlds, b.d_tiles[TK_STATS], b.cur_h, b.cur_id);
     TECTO_CUDA(cudaGetLastError());
     b.launches += 1;
     return TECTO_OK;
@@ -175,7 +187,7 @@ int launch_plate_motion(Batch &b, cudaStream_t st)
     const tecto_kernel_settings &ks = b.settings.kernel;
     const MotionParams mp{ks.curlNoiseMultiplier, ks.environmentalDragCoefficient, ks.velocitySmoothingFactor,
                           ks.directionSmoothingFactor};
-    k_plate_motion<<<(unsigned)b.members.size(), 256, 0, st>>>(b.d_worlds, mp);
+    launch_chained(k_plate_motion, (unsigned)b.members.size(), 256, 0, st, b.d_worlds, mp);
     TECTO_CUDA(cudaGetLastError());
     b.launches += 1;
     return TECTO_OK;

@@ -302,8 +302,10 @@ __global__ __launch_bounds__(256) void k_transport(const WorldDev *worlds, const
         const float px = (float)x - v.x * dt, py = (float)y - v.y * dt;
         const int ix0 = (int)floorf(px), iy0 = (int)floorf(py);
         const float wx = px - (float)ix0, wy = py - (float)iy0;
-        const float I0 = (1.0f - wx) * s1[cidx(ix0, iy0, W, H)] + wx * s1[cidx(ix0 + 1, iy0, W, H)];
-        const float I1 = (1.0f - wx) * s1[cidx(ix0, iy0 + 1, W, H)] + wx * s1[cidx(ix0 + 1, iy0 + 1, W, H)];
+        const int xa = wrap_fast(ix0, W), xb = wrap_fast(ix0 + 1, W);
+        const float *ra = s1 + (uint32_t)(wrap_fast(iy0, H) * W), *rb = s1 + (uint32_t)(wrap_fast(iy0 + 1, H) * W);
+        const float I0 = (1.0f - wx) * ra[xa] + wx * ra[xb];
+        const float I1 = (1.0f - wx) * rb[xa] + wx * rb[xb];
         s_out[i] = (1.0f - wy) * I0 + wy * I1;
     }
 }

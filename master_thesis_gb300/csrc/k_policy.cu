@@ -37,6 +37,7 @@ template <int PHASE>
 __global__ __launch_bounds__(256) void k_rl_cells(const WorldDev *worlds, const uint2 *tiles, int cur_id,
                                                   int period)
 {
+    kernel_wait();
     int wi, tx, ty;
     tile_of(tiles[blockIdx.x], &wi, &tx, &ty);
     const WorldDev &wd = worlds[wi];
@@ -51,8 +52,14 @@ __global__ __launch_bounds__(256) void k_rl_cells(const WorldDev *worlds, const 
     if (PHASE == 1) {
         // cells down a column mostly share a label: count runs in a register, one atomic per run
         uint32_t run = 0xffffffffu, n = 0u;
-        for (int y = y0; y < y1; ++y) {
-            const uint32_t lab = wd.labels[(uint32_t)y * (uint32_t)wd.W + (uint32_t)x];
+        uint32_t labs[kStatTileY];  // all loads first
+#pragma unroll
+        for (int k = 0; k < kStatTileY; ++k)
+            labs[k] = wd.labels[(uint32_t)min(y0 + k, y1 - 1) * (uint32_t)wd.W + (uint32_t)x];
+#pragma unroll
+        for (int k = 0; k < kStatTileY; ++k) {
+            const uint32_t lab = labs[k];
+            if (y0 + k >= y1) break;
             if (lab != run) {
                 if (n) atomicAdd(count + run, n);
                 run = lab;
@@ -95,6 +102,7 @@ constexpr int kSelThreads = 1024;
 __global__ __launch_bounds__(kSelThreads) void k_rl_select(const WorldDev *worlds, int cur_id, int period,
                                                            int minPlateSize)
 {
+    kernel_wait();
     const WorldDev &wd = worlds[blockIdx.x];
     if (!relabel_due(wd, period)) return;
     __shared__ unsigned int hist[256];
@@ -158,31 +166,44 @@ __global__ __launch_bounds__(kSelThreads) void k_rl_select(const WorldDev *world
     __syncthreads();
     if ((uint32_t)t < n) wd.policy->top[rank] = mine;
     __syncthreads();
+    // createLabelIdLookup: free ids are those below min(255, components) whose plate has no cells.  What it
+    // reads is gathered by one thread an entry, the order is one thread's.
+    __shared__ uint32_t s_label[256];
+    __shared__ int s_count[256];
+    __shared__ uint8_t s_plate[256], s_free[256];
+    __shared__ bool s_largest[256];
+    uint32_t *lookup = reinterpret_cast<uint32_t *>(wd.s1);
+    if ((uint32_t)t < n) {
+        const unsigned long long k = wd.policy->top[t];
+        const uint32_t label = (uint32_t)(k & 0xFFFFFFFFull);
+        const uint8_t plate = wd.id[cur_id][label];
+        s_label[t] = label;
+        s_count[t] = (int)(k >> 32);
+        s_plate[t] = plate;
+        s_largest[t] = s_count[t] == wd.policy->max_count[plate];
+        s_free[t] = wd.dyn[t].size == 0;
+    }
+    __syncthreads();
     if (t == 0) {
-        // createLabelIdLookup: free ids are those below min(255, components) whose plate has no cells
-        uint8_t avail[kPlates];
-        int navail = 0, next = 0;
-        for (uint32_t k = 0; k < n; ++k)
-            if (wd.dyn[k].size == 0) avail[navail++] = (uint8_t)k;
-        uint32_t *lookup = reinterpret_cast<uint32_t *>(wd.s1);
-        const uint8_t *id = wd.id[cur_id];
+        int next = -1;
+        const auto free_id = [&]() {  // the next free id, n if there is none
+            do ++next;
+            while (next < (int)n && !s_free[next]);
+            return next;
+        };
         for (uint32_t r = 0; r < n; ++r) {
-            const unsigned long long k = wd.policy->top[r];
-            const uint32_t label = (uint32_t)(k & 0xFFFFFFFFull);
-            const int c = (int)(k >> 32);
-            const uint8_t plate = id[label];
-            if (c == wd.policy->max_count[plate]) {
-                lookup[label] = plate;
-            } else if (c >= minPlateSize && next < navail) {
-                const uint8_t nid = avail[next++];
-                wd.plates[nid] = wd.plates[plate];
-                wd.dyn[nid] = wd.dyn[plate];
-                lookup[label] = nid;
+            const uint8_t plate = s_plate[r];
+            if (s_largest[r]) {
+                lookup[s_label[r]] = plate;
+            } else if (s_count[r] >= minPlateSize && next < (int)n && free_id() < (int)n) {
+                wd.plates[next] = wd.plates[plate];
+                wd.dyn[next] = wd.dyn[plate];
+                lookup[s_label[r]] = (uint32_t)next;
             }
         }
-        for (int p = 0; p < 256; ++p) wd.policy->max_count[p] = 0;
         wd.ctl->comp_count = 0u;
     }
+    for (int p = t; p < 256; p += kSelThreads) wd.policy->max_count[p] = 0;
 }
 
 // assignUnassignedIdsToNeighbor in rounds, one block per world: each listed cell still without an id
@@ -190,6 +211,7 @@ __global__ __launch_bounds__(kSelThreads) void k_rl_select(const WorldDev *world
 // of the round; stops when none is left or a round assigns nothing.
 __global__ __launch_bounds__(1024) void k_rl_fill(const WorldDev *worlds, int cur_id, int period)
 {
+    kernel_wait();
     const WorldDev &wd = worlds[blockIdx.x];
     if (!relabel_due(wd, period)) return;
     __shared__ unsigned int s_assigned, s_left;
@@ -254,6 +276,7 @@ __global__ __launch_bounds__(1024) void k_rl_fill(const WorldDev *worlds, int cu
 // getNeighboringPlates: plate pairs that touch across a +x or +y edge (wrapped), as triangle bits.
 __global__ __launch_bounds__(256) void k_mg_neighbors(const WorldDev *worlds, const uint2 *tiles, int cur_id)
 {
+    kernel_wait();
     int wi, tx, ty;
     tile_of(tiles[blockIdx.x], &wi, &tx, &ty);
     const WorldDev &wd = worlds[wi];
@@ -304,6 +327,7 @@ __device__ __forceinline__ bool merge_test(const WorldDev &wd, int x, int y, con
 // addresses; the neighbour bits are cleared for the next step.
 __global__ __launch_bounds__(1024) void k_mg_decide(const WorldDev *worlds, MergeParams mp)
 {
+    kernel_wait();
     const WorldDev &wd = worlds[blockIdx.x];
     __shared__ unsigned int s_cand[kMaxCand];
     __shared__ unsigned int s_n;
@@ -313,19 +337,22 @@ __global__ __launch_bounds__(1024) void k_mg_decide(const WorldDev *worlds, Merg
     for (int p = t; p < 256; p += blockDim.x) s_merge[p] = 0;
     __syncthreads();
     PolicyState &ps = *wd.policy;
-    for (uint32_t b = t; b < (uint32_t)kPairs; b += blockDim.x) {
-        if (!(ps.neighbors[b / 32u] & (1u << (b % 32u)))) continue;
-        // pair (x, y), x < y, of triangle index b
-        int x = 0;
-        uint32_t base = 0u;
-        while (base + (uint32_t)(kPlates - 1 - x) <= b) {
-            base += (uint32_t)(kPlates - 1 - x);
-            ++x;
+    for (uint32_t w = t; w < (uint32_t)kDivWords; w += blockDim.x) {
+        for (uint32_t bits = ps.neighbors[w]; bits; bits &= bits - 1u) {
+            const uint32_t b = 32u * w + (uint32_t)(__ffs(bits) - 1);
+            // pair (x, y), x < y, of triangle index b: the row from the root of x (2 kPlates - 1 - x) / 2 = b, which
+            // the roots' rounding may miss by one
+            constexpr float kSide = 2.0f * kPlates - 1.0f;
+            int x = (int)((kSide - sqrtf(kSide * kSide - 8.0f * (float)b)) * 0.5f);
+            const auto start = [](int r) { return (uint32_t)(r * (2 * kPlates - 1 - r) / 2); };
+            if (start(x) > b) --x;
+            else if (start(x + 1) <= b) ++x;
+            const uint32_t base = start(x);
+            const int y = x + 1 + (int)(b - base);
+            if (!merge_test(wd, x, y, mp)) continue;
+            const unsigned int slot = atomicAdd(&s_n, 1u);
+            if (slot < (unsigned int)kMaxCand) s_cand[slot] = (unsigned int)y * (unsigned int)kPlates + (unsigned int)x;
         }
-        const int y = x + 1 + (int)(b - base);
-        if (!merge_test(wd, x, y, mp)) continue;
-        const unsigned int slot = atomicAdd(&s_n, 1u);
-        if (slot < (unsigned int)kMaxCand) s_cand[slot] = (unsigned int)y * (unsigned int)kPlates + (unsigned int)x;
     }
     __syncthreads();
     const unsigned int n = min(s_n, (unsigned int)kMaxCand);
@@ -381,6 +408,7 @@ __global__ __launch_bounds__(1024) void k_mg_decide(const WorldDev *worlds, Merg
 // mergeAndCountSizeMass's remap: a child's cells take the parent's id.
 __global__ __launch_bounds__(256) void k_mg_apply(const WorldDev *worlds, const uint2 *tiles, int cur_id)
 {
+    kernel_wait();
     int wi, tx, ty;
     tile_of(tiles[blockIdx.x], &wi, &tx, &ty);
     const WorldDev &wd = worlds[wi];
@@ -414,21 +442,21 @@ int launch_plate_policy(Batch &b, int ccl, cudaStream_t st)
     const unsigned nw = (unsigned)b.members.size();
     if ((pol & TECTO_PLATE_RELABEL) && ccl) {
         const int period = ccl == 2 ? (s.sim.iterationsForCCL > 0 ? s.sim.iterationsForCCL : 1) : 0;
-        k_rl_cells<0><<<grid, 256, 0, st>>>(b.d_worlds, tiles, b.cur_id, period);
-        k_rl_cells<1><<<grid, 256, 0, st>>>(b.d_worlds, tiles, b.cur_id, period);
-        k_rl_cells<2><<<grid, 256, 0, st>>>(b.d_worlds, tiles, b.cur_id, period);
-        k_rl_select<<<nw, kSelThreads, 0, st>>>(b.d_worlds, b.cur_id, period, s.kernel.minPlateSize);
-        k_rl_cells<3><<<grid, 256, 0, st>>>(b.d_worlds, tiles, b.cur_id, period);
-        k_rl_fill<<<nw, 1024, 0, st>>>(b.d_worlds, b.cur_id, period);
+        launch_chained(k_rl_cells<0>, grid, 256, 0, st, b.d_worlds, tiles, b.cur_id, period);
+        launch_chained(k_rl_cells<1>, grid, 256, 0, st, b.d_worlds, tiles, b.cur_id, period);
+        launch_chained(k_rl_cells<2>, grid, 256, 0, st, b.d_worlds, tiles, b.cur_id, period);
+        launch_chained(k_rl_select, nw, kSelThreads, 0, st, b.d_worlds, b.cur_id, period, s.kernel.minPlateSize);
+        launch_chained(k_rl_cells<3>, grid, 256, 0, st, b.d_worlds, tiles, b.cur_id, period);
+        launch_chained(k_rl_fill, nw, 1024, 0, st, b.d_worlds, b.cur_id, period);
         TECTO_CUDA(cudaGetLastError());
         b.launches += 6;
     }
     if (pol & TECTO_PLATE_MERGE) {
         const MergeParams mp{s.kernel.mergeMinVelocity, s.kernel.mergeDotDirectionThreshold,
                              s.kernel.mergeVelocityDiffThreshold, s.kernel.targetMaximumPlateArea};
-        k_mg_neighbors<<<grid, 256, 0, st>>>(b.d_worlds, tiles, b.cur_id);
-        k_mg_decide<<<nw, 1024, 0, st>>>(b.d_worlds, mp);
-        k_mg_apply<<<grid, 256, 0, st>>>(b.d_worlds, tiles, b.cur_id);
+        launch_chained(k_mg_neighbors, grid, 256, 0, st, b.d_worlds, tiles, b.cur_id);
+        launch_chained(k_mg_decide, nw, 1024, 0, st, b.d_worlds, mp);
+        launch_chained(k_mg_apply, grid, 256, 0, st, b.d_worlds, tiles, b.cur_id);
         TECTO_CUDA(cudaGetLastError());
         b.launches += 3;
     }

@@ -62,19 +62,30 @@ __device__ int2 cont_prop(const float *h_old, int W, int H, int2 p, const tecto_
     const int nextX = stepX > 0 ? p.x + 1 : p.x, nextY = stepY > 0 ? p.y + 1 : p.y;
     float tmx = ((float)nextX - posx) / ndx;
     float tmy = ((float)nextY - posy) / ndy;
-    int2 prev = p;
-    for (int i = 0; i < iters; ++i) {
-        if (tmx < tmy) {
-            p.x += stepX;
-            tmx = tmx + tdx;
-        } else {
-            p.y += stepY;
-            tmy = tmy + tdy;
+    // the path does not depend on what it meets: four cells are loaded at a time
+    constexpr int kAhead = 4;
+    for (int i = 0; i < iters; i += kAhead) {
+        int2 q[kAhead];
+        float v[kAhead];
+#pragma unroll
+        for (int j = 0; j < kAhead; ++j) {
+            if (i + j < iters) {
+                if (tmx < tmy) {
+                    p.x += stepX;
+                    tmx = tmx + tdx;
+                } else {
+                    p.y += stepY;
+                    tmy = tmy + tdy;
+                }
+            }
+            q[j] = p;
+            v[j] = h_old[cidx(p.x, p.y, W, H)];
         }
-        if (h_old[cidx(p.x, p.y, W, H)] < thr) return p;
-        prev = p;
+#pragma unroll
+        for (int j = 0; j < kAhead; ++j)
+            if (v[j] < thr) return q[j];
     }
-    return prev;
+    return p;
 }
 
 // One continental collision source: the cell its primary plate reaches and, per arrival slot k,
@@ -97,7 +108,8 @@ __device__ __forceinline__ bool source_of(const UpArgs &a, const WorldDev &wd, u
     s.primary = 255 - (int)((cp >> (8 * pidx)) & 0xFFu);
     if (s.primary >= kPlates) return false;  // the owner's slot always holds a plate
     const int W = wd.W, H = wd.H;
-    const int2 pos = make_int2((int)(local % (uint32_t)W), (int)(local / (uint32_t)W));
+    const uint32_t y = row_of(wd, local);
+    const int2 pos = make_int2((int)(local - y * (uint32_t)W), (int)y);
     const float *h_old = wd.h[a.cur_h ^ 1];
     const float cur = h_old[local];
     s.pp = cont_prop(h_old, W, H, pos, wd.plates_prev[s.primary], cur, a.prop_thr, a.prop_iters);
@@ -135,6 +147,7 @@ __device__ __forceinline__ void emit(const UpArgs &a, const WorldDev &wd, uint32
 // Clears this step's propagation state.
 __global__ void k_up_clear(UpArgs a)
 {
+    kernel_wait();
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < a.total; v += gridDim.x * blockDim.x) {
         a.u.cnt[v] = 0u;
         a.u.succ[v] = 0u;
@@ -149,6 +162,7 @@ __global__ void k_up_clear(UpArgs a)
 template <bool FILL>
 __global__ __launch_bounds__(kUpThreads) void k_up_inserts(UpArgs a)
 {
+    kernel_wait();
     __shared__ uint32_t s_vbase[kMaxBatchWorlds + 1];
     load_vbase(a, s_vbase);
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < a.total; v += gridDim.x * blockDim.x) {
@@ -166,14 +180,48 @@ __global__ __launch_bounds__(kUpThreads) void k_up_inserts(UpArgs a)
     }
 }
 
-// Bucket of target v holding n entries, sorted by key in place (insertion sort; buckets are
-// short).  Returns the entry count that fits the scratch.
+// Bucket of target v holding n entries, sorted by key in place.  Returns the entry count that fits the
+// scratch.  All lanes of the warp (n 0 for none): a short bucket is its own lane's, by insertion; one of
+// more than kOwnSort entries, whose insertions would keep the warp waiting on one lane's memory accesses, is
+// ranked by all lanes (keys are distinct).
+constexpr uint32_t kOwnSort = 8, kRankItems = 8;  // ranked up to 32 x kRankItems
+
 __device__ __forceinline__ uint32_t sorted_bucket(const UpArgs &a, uint32_t v, uint32_t n, size_t *base)
 {
-    const size_t b = a.u.off[v];
+    const size_t b = n ? a.u.off[v] : 0;
     *base = b;
-    if (n == 0u || b >= a.u.ecap) return 0u;
+    if (b >= a.u.ecap) n = 0u;
     if (b + n > a.u.ecap) n = (uint32_t)(a.u.ecap - b);
+    const uint32_t lane = threadIdx.x & 31u;
+    const bool ranked = n > kOwnSort && n <= 32u * kRankItems;
+    for (unsigned m = __ballot_sync(0xffffffffu, ranked); m; m &= m - 1u) {
+        const int from = __ffs(m) - 1;
+        const uint32_t cnt = __shfl_sync(0xffffffffu, n, from);
+        const unsigned long long at = __shfl_sync(0xffffffffu, (unsigned long long)b, from);
+        uint32_t *key = a.u.ent_key + at, *val = a.u.ent_val + at;
+        uint32_t k[kRankItems], x[kRankItems], rank[kRankItems];
+#pragma unroll
+        for (uint32_t i = 0; i < kRankItems; ++i) {
+            const uint32_t j = lane + 32u * i;
+            k[i] = j < cnt ? key[j] : 0u;
+            x[i] = j < cnt ? val[j] : 0u;
+            rank[i] = 0u;
+        }
+        for (uint32_t q = 0; q < cnt; ++q) {
+            const uint32_t kq = key[q];
+#pragma unroll
+            for (uint32_t i = 0; i < kRankItems; ++i) rank[i] += kq < k[i] ? 1u : 0u;
+        }
+        __syncwarp();
+#pragma unroll
+        for (uint32_t i = 0; i < kRankItems; ++i)
+            if (lane + 32u * i < cnt) {
+                key[rank[i]] = k[i];
+                val[rank[i]] = x[i];
+            }
+        __syncwarp();
+    }
+    if (ranked) return n;
     for (uint32_t i = 1; i < n; ++i) {
         const uint32_t k = a.u.ent_key[b + i], val = a.u.ent_val[b + i];
         uint32_t j = i;
@@ -215,10 +263,12 @@ __device__ __forceinline__ bool insert_pair(uint32_t &inv, uint32_t a, uint32_t 
 // Step 2: per target, the inserts in (source, slot) order.
 __global__ __launch_bounds__(kUpThreads) void k_up_apply_inserts(UpArgs a)
 {
-    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < a.total; v += gridDim.x * blockDim.x) {
+    kernel_wait();
+    const uint32_t lane = threadIdx.x & 31u;
+    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v - lane < a.total; v += gridDim.x * blockDim.x) {
         size_t b;
-        const uint32_t raw = a.u.cnt[v];
-        a.u.cnt[v] = 0u;  // the contribution pass counts into the same array
+        const uint32_t raw = v < a.total ? a.u.cnt[v] : 0u;
+        if (raw) a.u.cnt[v] = 0u;  // the contribution pass counts into the same array
         const uint32_t n = sorted_bucket(a, v, raw, &b);
         if (n == 0u) continue;
         uint32_t inv = 0u;
@@ -247,6 +297,7 @@ __device__ __forceinline__ void count_at(int2 pos, int2 *positions, int *counts,
 template <bool FILL>
 __global__ __launch_bounds__(kUpThreads) void k_up_contrib(UpArgs a)
 {
+    kernel_wait();
     __shared__ uint32_t s_vbase[kMaxBatchWorlds + 1];
     load_vbase(a, s_vbase);
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < a.total; v += gridDim.x * blockDim.x) {
@@ -281,9 +332,11 @@ __global__ __launch_bounds__(kUpThreads) void k_up_contrib(UpArgs a)
 // Step 3b: per target, the contributions summed in (source, position) order onto 0.
 __global__ __launch_bounds__(kUpThreads) void k_up_sum(UpArgs a)
 {
-    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < a.total; v += gridDim.x * blockDim.x) {
+    kernel_wait();
+    const uint32_t lane = threadIdx.x & 31u;
+    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v - lane < a.total; v += gridDim.x * blockDim.x) {
         size_t b;
-        const uint32_t n = sorted_bucket(a, v, a.u.cnt[v], &b);
+        const uint32_t n = sorted_bucket(a, v, v < a.total ? a.u.cnt[v] : 0u, &b);
         if (n == 0u) continue;
         float acc = 0.0f;
         for (uint32_t i = 0; i < n; ++i) acc = acc + __uint_as_float(a.u.ent_val[b + i]);
@@ -296,6 +349,7 @@ __global__ __launch_bounds__(kUpThreads) void k_up_sum(UpArgs a)
 // (the reference's buffer persists; its stale values only reach non-seed cells).
 __global__ __launch_bounds__(kUpThreads) void k_up_combine(UpArgs a)
 {
+    kernel_wait();
     __shared__ uint32_t s_vbase[kMaxBatchWorlds + 1];
     load_vbase(a, s_vbase);
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < a.total; v += gridDim.x * blockDim.x) {
@@ -322,7 +376,8 @@ __global__ __launch_bounds__(kUpThreads) void k_up_combine(UpArgs a)
     }
 }
 
-__device__ __forceinline__ int jfa_top(int W, int H)
+// half the smallest power of two that covers the larger side
+__host__ __device__ __forceinline__ int jfa_top(int W, int H)
 {
     const int m = W > H ? W : H;
     int s = 1;
@@ -330,9 +385,9 @@ __device__ __forceinline__ int jfa_top(int W, int H)
     return s >> 1;
 }
 
-__device__ __forceinline__ int jfa_dist2(int cx, int cy, int seed, int W, int H)
+__device__ __forceinline__ int jfa_dist2(const WorldDev &wd, int cx, int cy, int seed, int W, int H)
 {
-    const int sx = seed % W, sy = seed / W;
+    const int sy = (int)row_of(wd, (uint32_t)seed), sx = seed - sy * W;
     int dx = abs(cx - sx), dy = abs(cy - sy);
     dx = min(dx, W - dx);
     dy = min(dy, H - dy);
@@ -340,34 +395,39 @@ __device__ __forceinline__ int jfa_dist2(int cx, int cy, int seed, int W, int H)
 }
 
 // JFAPass (:1512-1570) with step `step`; a world whose own sequence starts below `step` copies.
+// Instructions bound it (8 MB of seeds at 1024^2, in L2): rows by products instead of divisions, the wraps of
+// the three rows and columns once, the nine seeds loaded together.  1024^2: 24.2 -> 12.2 us.
 __global__ __launch_bounds__(kUpThreads) void k_jfa_pass(UpArgs a, const int32_t *in, int32_t *out, int step)
 {
+    kernel_wait();
     __shared__ uint32_t s_vbase[kMaxBatchWorlds + 1];
     load_vbase(a, s_vbase);
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < a.total; v += gridDim.x * blockDim.x) {
         const WorldDev &wd = a.worlds[find_world(s_vbase, a.nworlds, v)];
         const int W = wd.W, H = wd.H;
         int best = in[v];
-        if (step > jfa_top(W, H)) {
+        if (step >= max(W, H)) {  // above jfa_top
             out[v] = best;
             continue;
         }
         const uint32_t local = v - wd.vbase;
-        const int x = (int)(local % (uint32_t)W), y = (int)(local / (uint32_t)W);
+        const int y = (int)row_of(wd, local), x = (int)local - y * W;
         const int32_t *win = in + wd.vbase;
-        int bestDist = 0x7FFFFFFF;
-        if (best >= 0) bestDist = jfa_dist2(x, y, best, W, H);
-        for (int oy = -1; oy <= 1; ++oy)
-            for (int ox = -1; ox <= 1; ++ox) {
-                if (ox == 0 && oy == 0) continue;
-                const int cand = win[cidx(x + ox * step, y + oy * step, W, H)];
-                if (cand < 0) continue;
-                const int dist = jfa_dist2(x, y, cand, W, H);
-                if (dist < bestDist) {
-                    bestDist = dist;
-                    best = cand;
-                }
+        const int col[3] = {wrap_fast(x - step, W), x, wrap_fast(x + step, W)};
+        const int row[3] = {wrap_fast(y - step, H) * W, y * W, wrap_fast(y + step, H) * W};
+        int cand[9];
+#pragma unroll
+        for (int k = 0; k < 9; ++k) cand[k] = k == 4 ? best : win[(uint32_t)(row[k / 3] + col[k % 3])];
+        int bestDist = best >= 0 ? jfa_dist2(wd, x, y, best, W, H) : 0x7FFFFFFF;
+#pragma unroll
+        for (int k = 0; k < 9; ++k) {
+            if (k == 4) continue;
+            const int dist = jfa_dist2(wd, x, y, cand[k], W, H);
+            if (cand[k] >= 0 && dist < bestDist) {
+                bestDist = dist;
+                best = cand[k];
             }
+        }
         out[v] = best;
     }
 }
@@ -386,16 +446,17 @@ __device__ __forceinline__ float continental_profile(float x)
 // JFAComputeDistance (:1572-1600) and applyUplift (:1662-1738) on the resolved heights, in place.
 __global__ __launch_bounds__(kUpThreads) void k_up_apply(UpArgs a, const int32_t *seeds)
 {
+    kernel_wait();
     __shared__ uint32_t s_vbase[kMaxBatchWorlds + 1];
     load_vbase(a, s_vbase);
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < a.total; v += gridDim.x * blockDim.x) {
         const WorldDev &wd = a.worlds[find_world(s_vbase, a.nworlds, v)];
         const int W = wd.W, H = wd.H;
         const uint32_t local = v - wd.vbase;
-        const int x = (int)(local % (uint32_t)W), y = (int)(local / (uint32_t)W);
+        const int y = (int)row_of(wd, local), x = (int)local - y * W;
         const int seed = seeds[v];
         int dist = -1;
-        if (seed >= 0) dist = (int)sqrtf((float)jfa_dist2(x, y, seed, W, H));
+        if (seed >= 0) dist = (int)sqrtf((float)jfa_dist2(wd, x, y, seed, W, H));
         a.u.dist[v] = dist;
         if (dist <= -1) continue;
         const uint32_t o = wd.vbase + (uint32_t)seed;
@@ -410,7 +471,7 @@ __global__ __launch_bounds__(kUpThreads) void k_up_apply(UpArgs a, const int32_t
             const float mult = 1.0f + value * a.under_mult;
             *h = fmaxf(*h * mult, a.min_clamp);
         } else if (type == 0 && prim == plate) {
-            const int ox = seed % W, oy = seed / W;
+            const int oy = (int)row_of(wd, (uint32_t)seed), ox = seed - oy * W;
             const float sx = (float)W, sy = (float)H;
             const float ddx = fmodf((float)(x - ox) + sx * 0.5f, sx) - sx * 0.5f;
             const float ddy = fmodf((float)(y - oy) + sy * 0.5f, sy) - sy * 0.5f;
@@ -439,6 +500,7 @@ __global__ __launch_bounds__(kUpThreads) void k_up_apply(UpArgs a, const int32_t
 
 __global__ __launch_bounds__(1024) void k_scan_local(const uint32_t *cnt, uint32_t *off, uint32_t *blk, uint32_t n)
 {
+    kernel_wait();
     __shared__ uint32_t s_w[32];
     const uint32_t base = blockIdx.x * kScanBlock + threadIdx.x * kScanItems;
     uint32_t x[kScanItems], sum = 0;
@@ -468,6 +530,7 @@ __global__ __launch_bounds__(1024) void k_scan_local(const uint32_t *cnt, uint32
 
 __global__ __launch_bounds__(1024) void k_scan_blocks(uint32_t *blk, uint32_t nblk)
 {
+    kernel_wait();
     __shared__ uint32_t s_w[32];
     const uint32_t per = (nblk + 1023) / 1024;
     const uint32_t b0 = threadIdx.x * per;
@@ -494,6 +557,7 @@ __global__ __launch_bounds__(1024) void k_scan_blocks(uint32_t *blk, uint32_t nb
 
 __global__ void k_scan_add(uint32_t *cnt, uint32_t *off, const uint32_t *blk, uint32_t n)
 {
+    kernel_wait();
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         off[i] += blk[i / kScanBlock];
         cnt[i] = 0u;  // the fill pass counts again as its cursor
@@ -511,9 +575,9 @@ int scan_buckets(Batch &b, cudaStream_t st)
     const uint32_t n = (uint32_t)b.total;
     const uint32_t nblk = (n + kScanBlock - 1) / kScanBlock;
     UpliftRefScratch &u = b.upref;
-    k_scan_local<<<nblk, 1024, 0, st>>>(u.cnt, u.off, u.blk, n);
-    k_scan_blocks<<<1, 1024, 0, st>>>(u.blk, nblk);
-    k_scan_add<<<grid_for(n), kUpThreads, 0, st>>>(u.cnt, u.off, u.blk, n);
+    launch_chained(k_scan_local, nblk, 1024, 0, st, u.cnt, u.off, u.blk, n);
+    launch_chained(k_scan_blocks, 1, 1024, 0, st, u.blk, nblk);
+    launch_chained(k_scan_add, grid_for(n), kUpThreads, 0, st, u.cnt, u.off, u.blk, n);
     b.launches += 3;
     return TECTO_OK;
 }
@@ -597,34 +661,29 @@ int launch_uplift_ref(Batch &b, cudaStream_t st)
     a.over_range = ks.subductionOverRange;
     const unsigned g = grid_for(b.total);
     int rc;
-    k_up_clear<<<g, kUpThreads, 0, st>>>(a);
-    k_up_inserts<false><<<g, kUpThreads, 0, st>>>(a);
+    launch_chained(k_up_clear, g, kUpThreads, 0, st, a);
+    launch_chained(k_up_inserts<false>, g, kUpThreads, 0, st, a);
     b.launches += 2;
     if ((rc = scan_buckets(b, st)) != TECTO_OK) return rc;
-    k_up_inserts<true><<<g, kUpThreads, 0, st>>>(a);
-    k_up_apply_inserts<<<g, kUpThreads, 0, st>>>(a);
-    k_up_contrib<false><<<g, kUpThreads, 0, st>>>(a);
+    launch_chained(k_up_inserts<true>, g, kUpThreads, 0, st, a);
+    launch_chained(k_up_apply_inserts, g, kUpThreads, 0, st, a);
+    launch_chained(k_up_contrib<false>, g, kUpThreads, 0, st, a);
     b.launches += 3;
     if ((rc = scan_buckets(b, st)) != TECTO_OK) return rc;
-    k_up_contrib<true><<<g, kUpThreads, 0, st>>>(a);
-    k_up_sum<<<g, kUpThreads, 0, st>>>(a);
-    k_up_combine<<<g, kUpThreads, 0, st>>>(a);
+    launch_chained(k_up_contrib<true>, g, kUpThreads, 0, st, a);
+    launch_chained(k_up_sum, g, kUpThreads, 0, st, a);
+    launch_chained(k_up_combine, g, kUpThreads, 0, st, a);
     b.launches += 3;
     int top = 0;
-    for (const tecto_world *w : b.members) {
-        const int m = std::max(w->W, w->H);
-        int s = 1;
-        while (s < m) s <<= 1;
-        top = std::max(top, s >> 1);
-    }
+    for (const tecto_world *w : b.members) top = std::max(top, jfa_top(w->W, w->H));
     int cur = 0;
     for (int step = top; step > 0; step >>= 1) {
-        k_jfa_pass<<<g, kUpThreads, 0, st>>>(a, b.upref.jfa[cur], b.upref.jfa[cur ^ 1], step);
+        launch_chained(k_jfa_pass, g, kUpThreads, 0, st, a, b.upref.jfa[cur], b.upref.jfa[cur ^ 1], step);
         cur ^= 1;
         b.launches += 1;
     }
     b.upref_final = cur;
-    k_up_apply<<<g, kUpThreads, 0, st>>>(a, b.upref.jfa[cur]);
+    launch_chained(k_up_apply, g, kUpThreads, 0, st, a, b.upref.jfa[cur]);
     b.launches += 1;
     TECTO_CUDA(cudaGetLastError());
     return TECTO_OK;

@@ -227,6 +227,9 @@ int tecto_world_create(const tecto_settings *settings, int width, int height, ui
     d.H = height;
     d.N = (uint32_t)N;
     d.vbase = 0;
+    d.div_p = 31;
+    while ((1ull << (d.div_p - 31)) < (unsigned long long)width) ++d.div_p;
+    d.div_m = (uint32_t)(((1ull << d.div_p) + (unsigned long long)width - 1) / (unsigned long long)width);
     d.h[0] = (float *)(base + o_h0);
     d.h[1] = (float *)(base + o_h1);
     d.w[0] = (float *)(base + o_w0);

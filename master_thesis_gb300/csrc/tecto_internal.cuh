@@ -109,6 +109,8 @@ struct WorldDev {
     int W, H;
     uint32_t N;
     uint32_t vbase;         // first virtual cell index of this world in its batch
+    uint32_t div_m;         // row_of: n / W is (n * div_m) >> div_p
+    int div_p;
     float *h[2];            // height, ping-pong
     float *w[2];            // water
     float *s[2];            // sediment
@@ -321,6 +323,13 @@ __host__ __device__ __forceinline__ uint32_t cidx(int x, int y, int W, int H)
 __host__ __device__ __forceinline__ uint32_t tri_index(uint32_t i, uint32_t j)
 {
     return i * (2u * kPlates - i - 1u) / 2u + (j - i - 1u);
+}
+
+// Row of cell n (below 2^31) of the world: n / W by a product.  div_m = ceil(2^p / W) with p = 31 + the
+// smallest s with 2^s >= W is below 2^32 and over by less than W / 2^p of itself, less than 1 / n.
+__device__ __forceinline__ uint32_t row_of(const WorldDev &w, uint32_t n)
+{
+    return (uint32_t)(((unsigned long long)n * w.div_m) >> w.div_p);
 }
 
 // The world owning virtual cell v: largest b with vbase[b] <= v (vbase ascending, n entries).
