@@ -134,12 +134,16 @@ typedef struct tecto_step_settings {
     int cclConnectivity;      /* TECTO_CCL_* */
     int sortRadixBits;        /* collision sort digit width 8..11; 0 = autotuner's choice, else 9 where it
                                  saves a pass over 8 and 8 elsewhere */
-    int hydraulicTile;        /* 0 = autotuner's choice, else by the batch's cells: 1 up to 2^17, 3 up to
-                                 2^20, 4 up to 2.5 M, then 9.  Tiles of cells / warps, two cells a lane:
+    int hydraulicTile;        /* 0 = autotuner's choice, else by the batch's cells: 1 up to 2^17, 4 up to
+                                 450 000, 3 up to 2^20, 4 above, and 9 from 500 000 cells on where its strips are full
+                                 (from 500 000 / u^2 where the worlds fill the share u of them).  Tiles of
+                                 cells / warps, two cells a lane:
                                  1: 56x8/16, 2: 56x8/8, 3: 56x16/8, 4: 56x24/8, 5: 56x32/10, 6: 56x16/6,
-                                 7: 56x4/12; 9 (and 8): column strips of 120 cells marched down 4 rows at
-                                 a time by a block of 256 threads, two cells a thread, rows kept in shared
-                                 memory (the split path, 50 dt >= 1.5, runs variant 4) */
+                                 7: 56x4/12; 9 (and 8): column strips marched down 4 rows at a time, two
+                                 cells a thread, rows kept in shared memory: two sub-iterations in one
+                                 march of 116-column strips by blocks of 512 threads, a single one in
+                                 120-column strips by blocks of 256 (the split path, 50 dt >= 1.5, runs
+                                 variant 4) */
     int thermalTile;          /* 0 = autotuner's choice, else 5 from 2^20 cells and 4 below; 1: 64x32 tiles / 1024 threads, up to 5
                                  iterations per launch; 2: 64x16 / 512, 2 blocks per SM, up to 4;
                                  3: 64x16 / 768, 2 blocks per SM, up to 3; 4: 64x16 / 512, 3 blocks
@@ -432,7 +436,7 @@ int tecto_batch_phase_thermal(tecto_batch *batch, int iterations, tecto_stream_t
  * the nearest tuned class on their device, else the defaults (by the batch's
  * cells, see hydraulicTile, thermalTile and sortRadixBits). */
 typedef struct tecto_tuning {
-    int hydraulicTile;       /* chosen variant, 1..9 */
+    int hydraulicTile;       /* chosen variant, 1..8 (8 is the march) */
     int sortRadixBits;       /* chosen digit width, 8..11 */
     int thermalTile;         /* chosen variant, 1..5 */
     float hydraulic_ms[9];   /* one hydraulic sub-iteration with variant 1..9 */

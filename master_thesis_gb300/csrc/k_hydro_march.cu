@@ -70,6 +70,9 @@ constexpr uint32_t kOE = kOVY + kRBytes;
 constexpr uint32_t kSet = 10 * kRBytes;
 constexpr uint32_t kHydroPairSmem = kOE + kRBytes + kSet + kMGuard;
 constexpr int kLag = 10;
+// What a piece costs beside its rows, in rows: its warm-up, of two also the second's lag, and its first loads.
+// Of two, 16 / 26 / 36 / 48: 1024^2 20.9 / 19.1 / 18.9 / 19.1 us, the batch 672 / 655 / 648 / 657.
+constexpr unsigned kWarmAlone = 24, kWarmRows = 36;
 enum Role { kAlone = 0, kFirstOfTwo, kSecondOfTwo };
 static_assert(kPairThreads / 64 == kPairRows && kHydroMarchSmem % 16 == 0, "march: one pair per thread and phase");
 
@@ -117,7 +120,7 @@ __device__ __forceinline__ void march_piece(const HydroParams &p, const PairCons
     const int W = q.W, H = q.H;
     const uint32_t Wu = (uint32_t)W, N = Wu * (uint32_t)H, W4 = 4u * Wu;
     const f2 Z = c.Z;
-    constexpr int HALO = ROLE ? 8 : 4, LAG = ROLE == kSecondOfTwo ? kLag : 0;
+    constexpr int HALO = ROLE ? 6 : 4, LAG = ROLE == kSecondOfTwo ? kLag : 0;
     constexpr uint32_t D = ROLE == kSecondOfTwo ? kSet : 0;
     constexpr uint32_t OH = kOH + D, OW = kOW + D, OS = kOS + D, OX = kOX + D, OY = kOY + D, OZ = kOZ + D, OF = kOF + D,
                        OVX = kOVX + D, OVY = kOVY + D;
@@ -125,12 +128,13 @@ __device__ __forceinline__ void march_piece(const HydroParams &p, const PairCons
     const uint32_t gcol = (uint32_t)wrapc(x0 - HALO + col, W);
     const uint32_t gstep = VEC ? 1u : (uint32_t)wrapc(x0 - HALO + 1 + col, W) - gcol;
     const int gxi = x0 + col - HALO;  // global column of the pair's first cell, interior columns
-    // columns each stage covers: loads [0, iw+8), flux [1, iw+7), flow [2, iw+6), interior [4, iw+4); the first
-    // of two has 8 more, and the second is 4 to their right.
+    // columns each stage covers: loads [0, iw+8), flux [1, iw+7), flow [2, iw+6), interior [4, iw+4).  Of two, the first
+    // loads [0, iw+12): its flux covers [1, iw+11), its flow, whose height and water the second's flux needs,
+    // [2, iw+10), its transport [4, iw+8); the second's flux [3, iw+9), flow [4, iw+8), interior [6, iw+6).
     // A warp with no such column only keeps the barriers; the others run all 32 lanes.
     const bool in0 = col >= HALO && col < iw + HALO, in1 = col >= HALO && col + 1 < iw + HALO;
-    const bool live_f = ROLE == kFirstOfTwo ? col < iw + 15 : col >= HALO - 4 && col < iw + HALO + 3;
-    const bool live_w = ROLE == kFirstOfTwo ? col >= 2 && col < iw + 14 : col >= HALO - 2 && col < iw + HALO + 2;
+    const bool live_f = ROLE == kFirstOfTwo ? col < iw + 11 : col >= HALO - 4 && col < iw + HALO + 3;
+    const bool live_w = ROLE == kFirstOfTwo ? col >= 2 && col < iw + 10 : col >= HALO - 2 && col < iw + HALO + 2;
     const bool active = __any_sync(0xffffffffu, (col & ~63) < iw + 2 * HALO);
     const int K = (r1 - r0 + (ROLE ? kLag : 0) + kPairRows - 1) / kPairRows;
     const uint32_t nrows = (uint32_t)(r1 - r0);
@@ -354,14 +358,14 @@ __global__ __launch_bounds__(kPairThreads, 2) void k_hydro_march(const __grid_co
     // the edge lanes read ring cells before anything writes them: start from zeros
     for (uint32_t i = threadIdx.x; i < kHydroMarchSmem / 16; i += kPairThreads)
         march_smem[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    const unsigned long long nb = gridDim.x;
-    // this block's strip-rows [a0, b0)
-    const unsigned long long a0 = sp.rows * (unsigned long long)blockIdx.x / nb;
-    const unsigned long long b0 = sp.rows * (unsigned long long)(blockIdx.x + 1) / nb;
+    // this block's strip-rows [a0, b0), with kWarmAlone more to each strip (see k_hydro_march_pair)
+    const unsigned long long nb = gridDim.x, all = sp.rows + (unsigned long long)sp.nstrips * kWarmAlone;
+    const unsigned long long a0 = all * (unsigned long long)blockIdx.x / nb;
+    const unsigned long long b0 = all * (unsigned long long)(blockIdx.x + 1) / nb;
     int lo_s = 0, hi_s = sp.nstrips - 1;
     while (lo_s < hi_s) {
         const int mid = (lo_s + hi_s + 1) >> 1;
-        if ((unsigned long long)sp.strips[mid].w <= a0) lo_s = mid;
+        if ((unsigned long long)sp.strips[mid].w + (unsigned long long)mid * kWarmAlone <= a0) lo_s = mid;
         else hi_s = mid - 1;
     }
     kernel_wait();
@@ -375,9 +379,11 @@ __global__ __launch_bounds__(kPairThreads, 2) void k_hydro_march(const __grid_co
             s_flag[1] = -0x7fffffff;
         }
         __syncthreads();
-        const unsigned long long first = d.w, last = first + (unsigned long long)s_q.H;
+        const unsigned long long first = d.w + (unsigned long long)(s + 1) * kWarmAlone,
+                                 last = first + (unsigned long long)s_q.H;
         if (a >= last) continue;
-        const int r0 = (int)(a - first), r1 = (int)((b0 < last ? b0 : last) - first);
+        if (b0 <= first) break;
+        const int r0 = a > first ? (int)(a - first) : 0, r1 = (int)((b0 < last ? b0 : last) - first);
         const int x0 = (int)d.y, iw = (int)d.z;
         if (pp.ieee || s_q.H < kPairRows) {
             march_ieee(pp, s_q, S, x0, iw, r0, r1);
@@ -413,7 +419,7 @@ __device__ __noinline__ void march_two_ieee(const PairParams &pp, const HydroWor
 }
 
 // Two sub-iterations in one march.  The block's first 256 threads run the first on 128 columns, leaving what
-// it would store in shared memory; the other 256 run the second on the 112 columns inside, ten rows behind,
+// it would store in shared memory; the other 256 run the second on the 116 columns inside, ten rows behind,
 // which is as close as the first's height and as far as the rings allow.
 // A sub-iteration moves 34 bytes a cell instead of 60 (DRAM 37% busy), and its instructions are as many as
 // alone (530 a 64 cells, issue 56%, the shared-memory pipe 59%); one sub-iteration, alone and of two, us:
@@ -430,13 +436,15 @@ __global__ __launch_bounds__(2 * kPairThreads, 1) void k_hydro_march_pair(const 
     __shared__ int s_flag[2];
     for (uint32_t i = threadIdx.x; i < kHydroPairSmem / 16; i += 2 * kPairThreads)
         march_smem[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    const unsigned long long nb = gridDim.x;
-    const unsigned long long a0 = sp.rows * (unsigned long long)blockIdx.x / nb;
-    const unsigned long long b0 = sp.rows * (unsigned long long)(blockIdx.x + 1) / nb;
+    // Each strip counts kWarmRows more than it has, before its first: a block that starts another strip pays a
+    // second warm-up, and takes that many rows less.
+    const unsigned long long nb = gridDim.x, all = sp.rows + (unsigned long long)sp.nstrips * kWarmRows;
+    const unsigned long long a0 = all * (unsigned long long)blockIdx.x / nb;
+    const unsigned long long b0 = all * (unsigned long long)(blockIdx.x + 1) / nb;
     int lo_s = 0, hi_s = sp.nstrips - 1;
     while (lo_s < hi_s) {
         const int mid = (lo_s + hi_s + 1) >> 1;
-        if ((unsigned long long)sp.strips[mid].w <= a0) lo_s = mid;
+        if ((unsigned long long)sp.strips[mid].w + (unsigned long long)mid * kWarmRows <= a0) lo_s = mid;
         else hi_s = mid - 1;
     }
     kernel_wait();
@@ -450,9 +458,11 @@ __global__ __launch_bounds__(2 * kPairThreads, 1) void k_hydro_march_pair(const 
             s_flag[1] = -0x7fffffff;
         }
         __syncthreads();
-        const unsigned long long first = d.w, last = first + (unsigned long long)s_q.H;
+        const unsigned long long first = d.w + (unsigned long long)(s + 1) * kWarmRows,
+                                 last = first + (unsigned long long)s_q.H;
         if (a >= last) continue;
-        const int r0 = (int)(a - first), r1 = (int)((b0 < last ? b0 : last) - first);
+        if (b0 <= first) break;
+        const int r0 = a > first ? (int)(a - first) : 0, r1 = (int)((b0 < last ? b0 : last) - first);
         const int x0 = (int)d.y, iw = (int)d.z;
         if (s_q.H < kPairRows) {
             march_two_ieee(pp, s_q, S, x0, iw, r0, r1);

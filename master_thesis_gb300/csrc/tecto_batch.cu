@@ -174,21 +174,23 @@ static int default_radix_bits(size_t cells)
 // The default thermal variant: one iteration with tiles (variant 4, two iterations a launch) against the
 // march (5), us: 512^2 5.3 / 6.5, 1024^2 11.6 / 11.0, 2048^2 37.4 / 23.0, 8192^2 570 / 230.
 // The default hydraulic variant follows the batch's cells, as whole steps measured it, us:
-//                256^2  512^2  1001x613  1024^2  1200x1000  1101x1301  2000x1000  2048^2  12 worlds (0.6 M)
-//   1 (56x8)      167    313     567       838       942       1169       1543      3061        572
-//   3 (56x16)     168    279     461       617       700        838       1099      2078        455
-//   4 (56x24)     187    266     484       632       695        837       1014      1948        475
-//   9 (march)     253    372     529       654       670        792        927      1484        552
-// Small batches want many short tiles, large ones little halo.  The march also wants worlds that fill its
-// strips: worlds 128 to 256 wide, whose strips hold 1.3 and 1.37 times their cells, take 1108 against 1025 us
-// (1.6 M cells) and 1644 against 1571 (2.5 M); 256 to 600 wide, 1.1 times, 925 against 927 (1.6 M).
+//                256^2  512^2  724^2  1001x613  1024^2  1200x1000  2048^2  12 worlds (0.6 M)  60 worlds (1.6 M)
+//   1 (56x8)      167    313           567       838       942       3061        572
+//   3 (56x16)     168    279    367    461       617       700       2078        455              1051
+//   4 (56x24)     187    266    371    484       632       695       1948        475              1025
+//   9 (march)     253    283    390    432       547       583       1471        473               993
+// Small batches want many short tiles.  The march wants rows enough for every SM, and worlds that fill its
+// strips: the 12 worlds 200 to 300 wide and the 60 from 128 to 256 wide use 0.77 of theirs.  The line lies
+// at kMarchMinCells x (1 / use)^2 cells: 524 k x 0.75 at 724^2 and 0.6 M x 0.6 for the 12 are below it, 614 k x 0.86 at
+// 1001x613 and 1.04 M x 0.59 of 40 worlds 128 to 256 wide (752 against 766 us) above.
 static int default_hydro_variant(const Batch &b)
 {
-    unsigned long long strips = 0;  // cells the march's strips hold
-    for (const tecto_world *w : b.members)
-        strips += (unsigned long long)((w->W + kMarchInner - 1) / kMarchInner) * kMarchInner * (unsigned long long)w->H;
-    if (b.total >= kMarchMinCells && 4 * strips <= 5 * (unsigned long long)b.total) return kHydroMarchVariant;
-    return b.total <= (size_t)1 << 17 ? 1 : b.total <= (size_t)1 << 20 ? 3 : 4;
+    double strips = 0.0;  // cells the march's strips hold
+    for (const tecto_world *w : b.members) strips += (double)((w->W + kMarchInner - 1) / kMarchInner * kMarchInner) * w->H;
+    const double cells = (double)b.total, use = strips > 0.0 ? cells / strips : 0.0;
+    const bool split = 50.0f * fabsf(b.settings.step.hydraulicDt) >= 1.5f;  // the march's transport reaches two cells
+    if (!split && cells * use * use >= (double)kMarchMinCells) return kHydroMarchVariant;
+    return b.total <= (size_t)1 << 17 ? 1 : b.total <= 450000 || b.total > (size_t)1 << 20 ? 4 : 3;
 }
 
 static void choose_tuning(const Batch &b, int *variant, int *rb, int *tvariant)

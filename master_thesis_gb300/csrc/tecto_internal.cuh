@@ -391,8 +391,8 @@ constexpr int kHydroVariantCount = 9;
 constexpr int kDefaultHydroVariant = 4;          // 56 x 24 cells: where the autotuner starts from
 constexpr int kHydroStripVariant = 8;            // from here on: the march (8 is kept as another number for it)
 constexpr int kHydroMarchVariant = 9;            // marching row chunks in shared memory (fused path only)
-constexpr size_t kMarchMinCells = 1200000;       // cells from which the hydraulic march is the default
-constexpr int kMarchTwoInner = 112;              // of a strip that takes two sub-iterations at once
+constexpr size_t kMarchMinCells = 500000;        // cells from which the hydraulic march is the default
+constexpr int kMarchTwoInner = 116;              // of a strip that takes two sub-iterations at once
 constexpr int kMarchInner = 120;                 // interior columns of one shared-memory strip (128 with it)
 constexpr int kThermalInner = 60;                // interior columns of one thermal strip (64 with the halo)
 constexpr int kThermalVariantCount = 5;

@@ -103,10 +103,15 @@ int tune_shapes(const tecto_settings &settings, const std::vector<int2> &shapes,
         tb.dirty = true;
         rc = batch_step_graph(tb, 1, st, false);  // plate offsets and a settled state to time on
     }
-    // hydraulic tile variants: one sub-iteration each, best of a few
+    // hydraulic tile variants: two sub-iterations each, best of a few; the march, which has two numbers, once
+    // under its first
     int best_v = kDefaultHydroVariant;
     float best_vms = INFINITY;
     for (int v = 1; v <= kHydroVariantCount && rc == TECTO_OK; ++v) {
+        if (v > kHydroStripVariant) {
+            res.hydraulic_ms[v - 1] = res.hydraulic_ms[kHydroStripVariant - 1];
+            continue;
+        }
         tb.settings.step.hydraulicTile = v;
         if ((rc = batch_prepare(tb, st)) != TECTO_OK) break;
         float ms = 0;

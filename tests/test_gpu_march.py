@@ -87,10 +87,10 @@ def test_thermal_march_forms(kind, W, H, thr, A, S):
 
 
 @pytest.mark.parametrize("W,H,iters", [(5, 3, 2), (3, 40, 4), (113, 4, 2), (112, 61, 2), (225, 9, 5), (49, 130, 2),
-                                       (160, 33, 4), (1001, 47, 2)])
+                                       (160, 33, 4), (1001, 47, 2), (116, 21, 2), (117, 21, 2), (52, 70, 2), (53, 70, 2)])
 @pytest.mark.parametrize("kind", ["tiny", "clamp", "huge"])
 def test_two_sub_iterations_in_one_march(kind, W, H, iters):
-    """Two sub-iterations share a march where 112-column strips are not many more than 120-column ones:
+    """Two sub-iterations share a march where its narrower strips are not many more than 120-column ones:
     pieces of a few rows, strips of one column and narrower than half a block, worlds that wrap within a
     halo, odd widths, operands that send rows through the scalar form in the first or the second of two, and
     an odd number left over.  Bit for bit as the oracle."""
