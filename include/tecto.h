@@ -134,16 +134,16 @@ typedef struct tecto_step_settings {
     int cclConnectivity;      /* TECTO_CCL_* */
     int sortRadixBits;        /* collision sort digit width 8..11; 0 = autotuner's choice, else 9 where it
                                  saves a pass over 8 and 8 elsewhere */
-    int hydraulicTile;        /* 0 = autotuner's choice, else by the batch's cells: 1 up to 2^17, 4 up to
-                                 450 000, 3 up to 2^20, 4 above, and 9 from 500 000 cells on where its strips are full
-                                 (from 500 000 / u^2 where the worlds fill the share u of them).  Tiles of
-                                 cells / warps, two cells a lane:
-                                 1: 56x8/16, 2: 56x8/8, 3: 56x16/8, 4: 56x24/8, 5: 56x32/10, 6: 56x16/6,
-                                 7: 56x4/12; 9 (and 8): column strips marched down 4 rows at a time, two
-                                 cells a thread, rows kept in shared memory: two sub-iterations in one
-                                 march of 116-column strips by blocks of 512 threads, a single one in
-                                 120-column strips by blocks of 256 (the split path, 50 dt >= 1.5, runs
-                                 variant 4) */
+    int hydraulicTile;        /* 0 = autotuner's choice, else by a model of the batch's tiles and strips:
+                                 1 up to 0.1 M cells, 5, 3 and 4 by the waves up to 0.6 M, 9 above where
+                                 worlds fill its strips.  Tiles of cells / warps, two cells a lane, for
+                                 one sub-iteration and for two at once: 1: 56x8/16, 52x9/20; 2: 56x8/8,
+                                 52x12/8; 3: 56x16/8, 52x24/16; 4: 56x24/8, 52x28/12; 5: 56x32/10,
+                                 52x20/12; 6: 56x16/6; 7: 56x4/12; 9 (and 8): column strips marched down
+                                 4 rows at a time, two cells a thread, rows kept in shared memory: two
+                                 sub-iterations in one march of 116-column strips by blocks of 512
+                                 threads, a single one in 120-column strips by blocks of 256 (the split
+                                 path, 50 dt >= 1.5, runs variant 4) */
     int thermalTile;          /* 0 = autotuner's choice, else 5 from 2^20 cells and 4 below; 1: 64x32 tiles / 1024 threads, up to 5
                                  iterations per launch; 2: 64x16 / 512, 2 blocks per SM, up to 4;
                                  3: 64x16 / 768, 2 blocks per SM, up to 3; 4: 64x16 / 512, 3 blocks

@@ -265,6 +265,243 @@ __global__ __launch_bounds__(NW * 32, MINB) void k_hydro(const __grid_constant__
     else tile_body<TY, NW, FUSED, true>(tp, s_q, S, s_xy[0], s_xy[1]);
 }
 
+// ---- two sub-iterations on one tile ------------------------------------------------------------------
+//
+// Where the launches and the latency of the phases are the time (small worlds), a tile of 64 columns takes two
+// sub-iterations at once: a halo of 6 instead of 4, 52 columns inside, and nothing but the second's results
+// leaves the block.  Four phases between barriers: the first's flux; its flow; its transport together with the
+// second's flux; the second's flow; then the second's transport.
+// One sub-iteration as the two of a launch, us: 256^2 5.7 -> 3.5, 512^2 9.6 -> 7.4, 1001x613 17 -> 14.8; the
+// launch and the loads come once for two, against 1.7 to 2.3 times the cells inside (1.5 to 2.1 with a halo of
+// 4).  The shapes differ in rows, warps and tiles an SM holds; default_hydro_variant chooses by the waves.
+constexpr int HTX2 = 52;
+
+// Byte layout as TileMem's, with 12 rows of halo; rain of its own (the second adds it too), and the height
+// and water the second starts from.  The first's transported sediment takes the place of its height.
+template <int TY>
+struct TwoMem {
+    static constexpr int rows = TY + 12;
+    static constexpr uint32_t A = rows * kRow;
+    static constexpr uint32_t H = kGuard, W = H + A, S = W + A, X = S + A, Y = X + A, Z = Y + A, F = Z + A, V = F + A,
+                              R = V + A, H2 = R + A, W2 = H2 + A;
+    static constexpr uint32_t bytes = W2 + A + kGuard;
+};
+
+// The flux of the pair at byte o from heights at h and water at w, fluxes from o + x0 .. on.
+template <bool IEEE>
+__device__ __forceinline__ bool two_flux(const TileParams &tp, const char *S, uint32_t h, uint32_t w, float4 fa,
+                                         float4 fb, bool mine, Flux2 &v)
+{
+    if constexpr (IEEE) {
+        float4 u[2];
+#pragma unroll
+        for (uint32_t c = 0; c < 8; c += 4)
+            u[c >> 2] = flux_ieee(tp.p, c ? fb : fa, mld(S, h + c), mld(S, w + c), mld(S, h + c - 4), mld(S, w + c - 4),
+                                  mld(S, h + c + kRow), mld(S, w + c + kRow), mld(S, h + c + 4), mld(S, w + c + 4),
+                                  mld(S, h + c - kRow), mld(S, w + c - kRow));
+        v = Flux2{pk(u[0].x, u[1].x), pk(u[0].y, u[1].y), pk(u[0].z, u[1].z), pk(u[0].w, u[1].w)};
+        return false;
+    }
+    return flux_pair(tp.c, ld2(S, h), ld2(S, w), mld(S, h - 4), mld(S, h + 8), mld(S, w - 4), mld(S, w + 8),
+                     ld2(S, h + kRow), ld2(S, w + kRow), ld2(S, h - kRow), ld2(S, w - kRow), fa, fb, mine, v);
+}
+
+// The flow of the pair whose fluxes lie at x, y, z, f, with the height at h, water at w and sediment sd.
+template <bool IEEE>
+__device__ __forceinline__ bool two_flow(const TileParams &tp, const char *S, uint32_t x, uint32_t y, uint32_t z,
+                                         uint32_t f, uint32_t h, uint32_t w, f2 sd, bool mine, Flow2 &v)
+{
+    if constexpr (IEEE) {
+        FlowOut u[2];
+#pragma unroll
+        for (uint32_t c = 0; c < 8; c += 4)
+            u[c >> 2] = flow_cell_general(
+                tp.p, make_float4(mld(S, x + c), mld(S, y + c), mld(S, z + c), mld(S, f + c)), mld(S, z + c - 4),
+                mld(S, f + c + kRow), mld(S, x + c + 4), mld(S, y + c - kRow), mld(S, f + c - kRow), mld(S, w + c),
+                mld(S, h + c), c ? hi(sd) : lo(sd), mld(S, h + c - 4), mld(S, h + c + 4), mld(S, h + c + kRow),
+                mld(S, h + c - kRow));
+        v = Flow2{pk(u[0].hn, u[1].hn), pk(u[0].wn, u[1].wn), pk(u[0].s1, u[1].s1), pk(u[0].ux, u[1].ux),
+                  pk(u[0].uy, u[1].uy)};
+        return false;
+    }
+    const Flux2 b{ld2(S, x), ld2(S, y), ld2(S, z), ld2(S, f)};
+    return flow_pair(tp.c, b, mld(S, z - 4), mld(S, x + 8), ld2(S, f + kRow), ld2(S, y - kRow), ld2(S, f - kRow),
+                     ld2(S, w), ld2(S, h), mld(S, h - 4), mld(S, h + 8), ld2(S, h + kRow), ld2(S, h - kRow), sd, mine, v);
+}
+
+// The sediment that reaches the pair with velocity (ux, uy) at the columns gx and the row gy: taps around the
+// bytes t0, t1 that the floored position 0 stands for, in the array of `size` bytes at S.
+__device__ __forceinline__ f2 two_transport(const PairConst &c, const char *S, uint32_t size, f2 ux, f2 uy, f2 gx, float gy,
+                                            uint32_t t0, uint32_t t1)
+{
+    const f2 px = sub2(gx, mul2_z(ux, c.dt, c.Z)), py = sub2(dup2(gy), mul2_z(uy, c.dt, c.Z));
+    const f2 tx = add2_rm(px, c.M), ty = add2_rm(py, c.M);
+    const f2 wx = sub2(px, sub2(tx, c.M)), wy = sub2(py, sub2(ty, c.M));
+    const f2 vx = sub2(c.one, wx), vy = sub2(c.one, wy);
+    // a tap offset is in [-2, 1] by the velocity clamp; the minimum keeps any other inside the array
+    const uint32_t last = size - kRow - 8;
+    const char *u = S + min(t0 + (__float_as_uint(lo(ty)) << 8) + (__float_as_uint(lo(tx)) << 2), last);
+    const char *v = S + min(t1 + (__float_as_uint(hi(ty)) << 8) + (__float_as_uint(hi(tx)) << 2), last);
+    const f2 I0 = add2(mul2_z(vx, pk(mld(u, 0), mld(v, 0)), c.Z), mul2_z(wx, pk(mld(u, 4), mld(v, 4)), c.Z));
+    const f2 I1 = add2(mul2_z(vx, pk(mld(u, kRow), mld(v, kRow)), c.Z), mul2_z(wx, pk(mld(u, kRow + 4), mld(v, kRow + 4)), c.Z));
+    return add2(mul2_z(vy, I0, c.Z), mul2_z(wy, I1, c.Z));
+}
+
+// True where an operand of this thread left the packed ranges (IEEE: never).
+template <int TY, int NW, bool VEC, bool IEEE>
+__device__ __forceinline__ bool two_body(const TileParams &tp, const HydroWorld &q, char *S, int x0, int y0)
+{
+    using M = TwoMem<TY>;
+    const PairConst &c = tp.c;
+    const int W = q.W, H = q.H;
+    const int lane = (int)threadIdx.x & 31, warp = (int)threadIdx.x >> 5, col = 2 * lane;
+    const uint32_t Sa = (uint32_t)__cvta_generic_to_shared(S);
+    const uint32_t c0 = (uint32_t)wrapc(x0 - 6 + col, W), c1 = VEC ? c0 + 1 : (uint32_t)wrapc(x0 - 5 + col, W);
+    const int iw = min(HTX2, W - x0), ih = min(TY, H - y0);
+    const bool in0 = col >= 6 && col < iw + 6, in1 = col >= 6 && col + 1 < iw + 6;
+    const uint32_t L = (uint32_t)lane * 8u;
+    const uint32_t B = (uint32_t)y0 * (uint32_t)W + (uint32_t)(x0 - 6 + col);  // global offset of row y0, this pair
+
+#pragma unroll 2
+    for (int ly = warp; ly < M::rows; ly += NW) {
+        const uint32_t g = (uint32_t)wrapc(y0 - 6 + ly, H) * (uint32_t)W, d = Sa + (uint32_t)ly * kRow + L;
+        cp_pair<VEC>(d + M::H, q.h_in + g, c0, c1);
+        cp_pair<VEC>(d + M::W, q.w_in + g, c0, c1);
+        cp_pair<VEC>(d + M::R, q.rain + g, c0, c1);
+        if (ly >= 2 && ly < M::rows - 2) cp_pair<VEC>(d + M::S, q.s_in + g, c0, c1);
+        if (ly >= 1 && ly < M::rows - 1) {
+            const char *f0 = reinterpret_cast<const char *>(q.f_in + g + c0), *f1 = reinterpret_cast<const char *>(q.f_in + g + c1);
+            cp8(d + M::X, f0);
+            cp8(d + M::Y, f0 + 8);
+            cp8(d + M::Z, f1);
+            cp8(d + M::F, f1 + 8);
+        }
+    }
+    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+    for (int ly = warp; ly < M::rows; ly += NW) {
+        const uint32_t o = (uint32_t)ly * kRow + L;
+        st2(S, o + M::W, add2(ld2(S, o + M::W), ld2(S, o + M::R)));
+    }
+    __syncthreads();
+
+    // the first's flux
+    bool bad = false;
+#pragma unroll 1
+    for (int ly = warp + 1; ly < M::rows - 1; ly += NW) {
+        const uint32_t o = (uint32_t)ly * kRow + L;
+        const f2 a = ld2(S, o + M::X), b = ld2(S, o + M::Y), d = ld2(S, o + M::Z), e = ld2(S, o + M::F);
+        Flux2 v;
+        const bool x = two_flux<IEEE>(tp, S, o + M::H, o + M::W, make_float4(lo(a), hi(a), lo(b), hi(b)),
+                                      make_float4(lo(d), hi(d), lo(e), hi(e)), col < iw + 11, v);
+        bad = bad || x;
+        st2(S, o + M::X, v.x);
+        st2(S, o + M::Y, v.y);
+        st2(S, o + M::Z, v.z);
+        st2(S, o + M::F, v.w);
+    }
+    __syncthreads();
+
+    // the first's flow, sediment exchange and evaporation, and the second's rain
+#pragma unroll 1
+    for (int ly = warp + 2; ly < M::rows - 2; ly += NW) {
+        const uint32_t o = (uint32_t)ly * kRow + L;
+        Flow2 v;
+        const bool x = two_flow<IEEE>(tp, S, o + M::X, o + M::Y, o + M::Z, o + M::F, o + M::H, o + M::W,
+                                      ld2(S, o + M::S), col >= 2 && col < iw + 10, v);
+        bad = bad || x;
+        st2(S, o + M::W, v.ux);
+        st2(S, o + M::V, v.uy);
+        st2(S, o + M::S, v.s1);
+        st2(S, o + M::H2, v.hn);
+        st2(S, o + M::W2, add2(evaporate2(c, v.wn), ld2(S, o + M::R)));
+    }
+    __syncthreads();
+
+    // the first's transport, at the positions of the world's own rows and columns, and the second's flux
+    const f2 gx = pk((float)(int)c0, (float)(int)c1);
+    const uint32_t zero = 0u - (0x4B400000u << 8) - (0x4B400000u << 2);
+#pragma unroll 1
+    for (int ly = warp + 3; ly < M::rows - 3; ly += NW) {
+        const uint32_t o = (uint32_t)ly * kRow + L;
+        if (ly >= 4 && ly < M::rows - 4) {
+            const int gy = wrapc(y0 - 6 + ly, H);
+            const uint32_t t = zero + ((uint32_t)(ly - gy) << 8) + ((uint32_t)col << 2);
+            st2(S, o + M::H, two_transport(c, S + M::S, M::A, ld2(S, o + M::W), ld2(S, o + M::V), gx, (float)gy, t - (c0 << 2),
+                                           t + 4u - (c1 << 2)));
+        }
+        const f2 a = ld2(S, o + M::X), b = ld2(S, o + M::Y), d = ld2(S, o + M::Z), e = ld2(S, o + M::F);
+        Flux2 v;
+        const bool x = two_flux<IEEE>(tp, S, o + M::H2, o + M::W2, make_float4(lo(a), lo(b), lo(d), lo(e)),
+                                      make_float4(hi(a), hi(b), hi(d), hi(e)), col >= 2 && col < iw + 9, v);
+        bad = bad || x;
+        st2(S, o + M::X, v.x);
+        st2(S, o + M::Y, v.y);
+        st2(S, o + M::Z, v.z);
+        st2(S, o + M::F, v.w);
+        const bool row = (unsigned)(ly - 6) < (unsigned)ih;
+        gst_flux<VEC>(q.f_out, B + (uint32_t)(ly - 6) * (uint32_t)W, v.x, v.y, v.z, v.w, row && in0, row && in1);
+    }
+    __syncthreads();
+
+    // the second's flow, sediment exchange and evaporation
+#pragma unroll 1
+    for (int ly = warp + 4; ly < M::rows - 4; ly += NW) {
+        const uint32_t o = (uint32_t)ly * kRow + L;
+        Flow2 v;
+        const bool x = two_flow<IEEE>(tp, S, o + M::X, o + M::Y, o + M::Z, o + M::F, o + M::H2, o + M::W2,
+                                      ld2(S, o + M::H), col >= 4 && col < iw + 8, v);
+        bad = bad || x;
+        st2(S, o + M::W, v.ux);
+        st2(S, o + M::V, v.uy);
+        st2(S, o + M::S, v.s1);
+        const bool row = (unsigned)(ly - 6) < (unsigned)ih, s0 = row && in0, s1 = row && in1;
+        const uint32_t g = B + (uint32_t)(ly - 6) * (uint32_t)W;
+        gst2<VEC>(q.h_out, g, v.hn, s0, s1);
+        gst2<VEC>(q.w_out, g, evaporate2(c, v.wn), s0, s1);
+    }
+    __syncthreads();
+    kernel_release();
+
+    // the second's transport
+    const f2 hx = pk((float)(x0 - 6 + col), (float)(x0 - 5 + col));
+    const uint32_t t = zero - ((uint32_t)(y0 - 6) << 8) - ((uint32_t)(x0 - 6) << 2);
+#pragma unroll 1
+    for (int ly = warp + 6; ly < ih + 6; ly += NW) {
+        const uint32_t o = (uint32_t)ly * kRow + L;
+        const f2 v = two_transport(c, S + M::S, M::A, ld2(S, o + M::W), ld2(S, o + M::V), hx, (float)(y0 - 6 + ly), t, t);
+        gst2<VEC>(q.s_out, B + (uint32_t)(ly - 6) * (uint32_t)W, v, in0, in1);
+    }
+    return bad;
+}
+
+template <int TY, int NW>
+__device__ __noinline__ void two_ieee(const TileParams &tp, const HydroWorld &q, char *S, int x0, int y0)
+{
+    two_body<TY, NW, false, true>(tp, q, S, x0, y0);
+}
+
+template <int TY, int NW, int MINB>
+__global__ __launch_bounds__(NW * 32, MINB) void k_hydro_two(const __grid_constant__ TileParams tp)
+{
+    extern __shared__ float4 tile_smem[];
+    __shared__ HydroWorld s_q;
+    __shared__ int s_xy[2];
+    char *S = reinterpret_cast<char *>(tile_smem);
+    if (threadIdx.x == 0) {
+        int wi, tx, ty;
+        tile_of(tp.p.tiles[blockIdx.x], &wi, &tx, &ty);
+        s_q = hydro_world(tp.p, tp.p.worlds[wi]);
+        s_xy[0] = tx * HTX2;
+        s_xy[1] = ty * TY;
+    }
+    __syncthreads();
+    kernel_wait();
+    const bool bad = s_q.W & 1 ? two_body<TY, NW, false, false>(tp, s_q, S, s_xy[0], s_xy[1])
+                               : two_body<TY, NW, true, false>(tp, s_q, S, s_xy[0], s_xy[1]);
+    // an operand outside the packed ranges: the tile once more in scalar form, from the same inputs
+    if (__syncthreads_or(bad)) two_ieee<TY, NW>(tp, s_q, S, s_xy[0], s_xy[1]);
+}
+
 // The step's rain increment (:2430-2437 with the seed of plate_tectonic_sim.cu:338), over the
 // hydraulic work list (tiles of 64 x ty cells).
 __global__ void k_rain(const WorldDev *worlds, const uint2 *tiles, int ty_cells, float dt, float rainfall)
@@ -316,15 +553,24 @@ struct HydroVariant {
     size_t smem;
     void (*fused)(TileParams);
     void (*split)(TileParams);
+    int ty2, nt2;  // two sub-iterations at once, 52 x ty2 cells (0: never)
+    size_t smem2;
+    void (*two)(TileParams);
 };
 #define TECTO_HYDRO_VARIANT(TY, NW, MINB) \
-    {TY, NW * 32, TileMem<TY>::bytes, k_hydro<TY, NW, MINB, true>, k_hydro<TY, NW, MINB, false>}
+    TY, NW * 32, TileMem<TY>::bytes, k_hydro<TY, NW, MINB, true>, k_hydro<TY, NW, MINB, false>
+#define TECTO_HYDRO_TWO(TY, NW, MINB) TY, NW * 32, TwoMem<TY>::bytes, k_hydro_two<TY, NW, MINB>
 const HydroVariant kHydroVariants[7] = {
-    TECTO_HYDRO_VARIANT(8, 16, 2), TECTO_HYDRO_VARIANT(8, 8, 4),  TECTO_HYDRO_VARIANT(16, 8, 4),
-    TECTO_HYDRO_VARIANT(24, 8, 3), TECTO_HYDRO_VARIANT(32, 10, 2), TECTO_HYDRO_VARIANT(16, 6, 4),
-    TECTO_HYDRO_VARIANT(4, 12, 2),
+    {TECTO_HYDRO_VARIANT(8, 16, 2), TECTO_HYDRO_TWO(9, 20, 1)},
+    {TECTO_HYDRO_VARIANT(8, 8, 4), TECTO_HYDRO_TWO(12, 8, 3)},
+    {TECTO_HYDRO_VARIANT(16, 8, 4), TECTO_HYDRO_TWO(24, 16, 2)},
+    {TECTO_HYDRO_VARIANT(24, 8, 3), TECTO_HYDRO_TWO(28, 12, 2)},
+    {TECTO_HYDRO_VARIANT(32, 10, 2), TECTO_HYDRO_TWO(20, 12, 2)},
+    {TECTO_HYDRO_VARIANT(16, 6, 4), 0, 0, 0, nullptr},
+    {TECTO_HYDRO_VARIANT(4, 12, 2), 0, 0, 0, nullptr},
 };
 #undef TECTO_HYDRO_VARIANT
+#undef TECTO_HYDRO_TWO
 // The rain field and the split path of the marching variants run on the tiles of variant 4.
 const HydroVariant &variant_of(int v) { return kHydroVariants[(v > 7 ? 4 : v) - 1]; }
 }  // namespace
@@ -334,14 +580,22 @@ int hydro_tile_attributes()
     for (const HydroVariant &v : kHydroVariants) {
         TECTO_CUDA(cudaFuncSetAttribute(v.fused, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)v.smem));
         TECTO_CUDA(cudaFuncSetAttribute(v.split, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)v.smem));
+        if (v.ty2) TECTO_CUDA(cudaFuncSetAttribute(v.two, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)v.smem2));
     }
     return TECTO_OK;
 }
 
-void hydro_tile_extent(int variant, int *tx, int *ty)
+void hydro_tile_extent(int variant, bool two, int *tx, int *ty)
 {
-    *tx = HTX;
-    *ty = variant_of(variant).ty;
+    const HydroVariant &v = variant_of(variant);
+    two = two && v.ty2;
+    *tx = two ? HTX2 : HTX;
+    *ty = two ? v.ty2 : v.ty;
+}
+
+bool hydro_tile_two(const Batch &b, const HydroParams &p)
+{
+    return b.hydro_variant < kHydroStripVariant && variant_of(b.hydro_variant).ty2 && hydro_march_two(p);
 }
 
 void launch_rain(const Batch &b, float dt, float rainfall, cudaStream_t st)
@@ -356,13 +610,18 @@ void launch_transport(const Batch &b, float dt, cudaStream_t st)
                    variant_of(b.hydro_variant).ty, b.cur_wsf, dt);
 }
 
-void launch_hydro_tile(const Batch &b, const HydroParams &p, bool fused, cudaStream_t st)
+void launch_hydro_tile(const Batch &b, const HydroParams &p, bool fused, bool two, cudaStream_t st)
 {
     const HydroVariant &v = variant_of(b.hydro_variant);
     TileParams tp{};
     tp.p = p;
     tp.c = pair_const(p);
     tp.ieee = p.fastL == 0 || !(p.dt >= 0.0f);
+    if (two) {
+        tp.p.tiles = b.d_tiles[TK_HYDRO_TWO];
+        launch_chained(v.two, (unsigned)b.ntiles[TK_HYDRO_TWO], v.nt2, v.smem2, st, tp);
+        return;
+    }
     const unsigned grid = (unsigned)b.ntiles[TK_HYDRO];
     launch_chained(fused ? v.fused : v.split, grid, v.nt, v.smem, st, tp);
 }

@@ -173,34 +173,70 @@ static int default_radix_bits(size_t cells)
 
 // The default thermal variant: one iteration with tiles (variant 4, two iterations a launch) against the
 // march (5), us: 512^2 5.3 / 6.5, 1024^2 11.6 / 11.0, 2048^2 37.4 / 23.0, 8192^2 570 / 230.
-// The default hydraulic variant follows the batch's cells, as whole steps measured it, us:
-//                256^2  512^2  724^2  1001x613  1024^2  1200x1000  2048^2  12 worlds (0.6 M)  60 worlds (1.6 M)
-//   1 (56x8)      167    313           567       838       942       3061        572
-//   3 (56x16)     168    279    367    461       617       700       2078        455              1051
-//   4 (56x24)     187    266    371    484       632       695       1948        475              1025
-//   9 (march)     253    283    390    432       547       583       1471        473               993
-// Small batches want many short tiles.  The march wants rows enough for every SM, and worlds that fill its
-// strips: the 12 worlds 200 to 300 wide and the 60 from 128 to 256 wide use 0.77 of theirs.  The line lies
-// at kMarchMinCells x (1 / use)^2 cells: 524 k x 0.75 at 724^2 and 0.6 M x 0.6 for the 12 are below it, 614 k x 0.86 at
-// 1001x613 and 1.04 M x 0.59 of 40 worlds 128 to 256 wide (752 against 766 us) above.
-static int default_hydro_variant(const Batch &b)
+// The default hydraulic variant: the one whose two sub-iterations a model of the measured shapes puts lowest.
+// Tiles run in waves of 152 SMs x the tiles an SM holds, and a wave's time depends on how many it holds; the
+// march's blocks take equal shares of the strips' rows (with what a strip's start costs, k_hydro_march.cu), at
+// 0.38 us a row, 0.42 counted as odd widths take longer.  Whole steps, us, the model's choice marked:
+//                    256^2  384^2  512^2  600^2  724^2  1001x613  900x800  1024^2  1200x1000  12 worlds  40 worlds
+//   1 (52x9)         129*   233    298    409    536     660       710     945      1098       625        1194
+//   2 (52x12)        143    178    225    290    379     447       479     640       721       451         780
+//   3 (52x24)        162    168*   237    251*   346*    428       484     572       648       428         754
+//   4 (52x28)        173    178    251    269    368     392*      453     545       621       396*        682*
+//   5 (52x20)        157    208    222*   307    379     457       461     593       656       454         766
+//   9 (march)        253           283    323    390     433       443*    533*      581*      474         750
+// (12 worlds 200 to 300 wide, 0.55 M cells; 40 of 128 to 256, 1.08 M.)  60 such worlds (1.6 M) take 986 with the march, which
+// it chooses, against 957; 100 (2.5 M) 1461 against 1471; 20 of 240x400 882 against 1039.
+static int default_hydro_variant(const Batch &b, bool split)
 {
-    double strips = 0.0;  // cells the march's strips hold
-    for (const tecto_world *w : b.members) strips += (double)((w->W + kMarchInner - 1) / kMarchInner * kMarchInner) * w->H;
-    const double cells = (double)b.total, use = strips > 0.0 ? cells / strips : 0.0;
-    const bool split = 50.0f * fabsf(b.settings.step.hydraulicDt) >= 1.5f;  // the march's transport reaches two cells
-    if (!split && cells * use * use >= (double)kMarchMinCells) return kHydroMarchVariant;
-    return b.total <= (size_t)1 << 17 ? 1 : b.total <= 450000 || b.total > (size_t)1 << 20 ? 4 : 3;
+    if (split)  // 50 dt >= 1.5: the march's transport reaches two cells; no two at once
+        return b.total <= (size_t)1 << 17 ? 1 : b.total <= (size_t)1 << 20 ? 3 : 4;
+    constexpr double kSms = 152.0;
+    struct Shape {
+        int ty, held;
+        double us[3];  // a wave of 1, 2, 3 tiles an SM
+    };
+    static const Shape shapes[5] = {
+        {9, 1, {5.6}}, {12, 3, {8.3, 11.5, 15.0}}, {24, 2, {10.2, 16.2}}, {28, 2, {11.3, 17.6}}, {20, 2, {9.7, 14.7}}};
+    int best = 1;
+    double best_us = INFINITY;
+    for (int v = 0; v < 5; ++v) {
+        double tiles = 0.0;
+        for (const tecto_world *w : b.members)
+            tiles += (double)((w->W + 51) / 52) * (double)((w->H + shapes[v].ty - 1) / shapes[v].ty);
+        const double wave = kSms * shapes[v].held, full = floor(tiles / wave), rest = ceil((tiles - full * wave) / kSms);
+        const double us = full * shapes[v].us[shapes[v].held - 1] + (rest > 0.0 ? shapes[v].us[(int)rest - 1] : 0.0);
+        if (us < best_us) {
+            best_us = us;
+            best = v + 1;
+        }
+    }
+    // strip-rows of two at once and of one, with the rows that starting a strip costs
+    double rows2 = 0.0, start2 = 0.0, rows1 = 0.0, start1 = 0.0;
+    for (const tecto_world *w : b.members) {
+        const double n2 = (w->W + kMarchTwoInner - 1) / kMarchTwoInner, n1 = (w->W + kMarchInner - 1) / kMarchInner;
+        rows2 += n2 * w->H;
+        start2 += n2 * 36.0;
+        rows1 += n1 * w->H;
+        start1 += n1 * 24.0;
+    }
+    const double march = 5.0 * rows2 <= 6.0 * rows1 ? 0.42 * ((rows2 + start2) / kSms + 36.0)
+                                                    : 2.0 * 0.46 * ((rows1 + start1) / (2.0 * kSms) + 24.0);
+    return march < best_us ? kHydroMarchVariant : best;
 }
 
-static void choose_tuning(const Batch &b, int *variant, int *rb, int *tvariant)
+static void choose_tuning(Batch &b, int *variant, int *rb, int *tvariant)
 {
     *tvariant = thermal_variant_for(b.settings);
     if (*tvariant == 0) *tvariant = b.tuned_thermal;
     if (*tvariant == 0) *tvariant = b.total >= kThermalMarchMinCells ? kThermalMarchVariant : kDefaultThermalVariant;
     *variant = hydro_variant_for(b.settings);
     if (*variant == 0) *variant = b.tuned_hydro;
-    if (*variant == 0) *variant = default_hydro_variant(b);
+    if (*variant == 0) {
+        const bool split = 50.0f * fabsf(b.settings.step.hydraulicDt) >= 1.5f;
+        int &d = b.hydro_default[split];
+        if (b.dirty || d == 0) d = default_hydro_variant(b, split);
+        *variant = d;
+    }
     *rb = b.settings.step.sortRadixBits;
     if (!valid_radix_bits(*rb)) *rb = valid_radix_bits(b.tuned_rb) ? b.tuned_rb : default_radix_bits(b.total);
 }

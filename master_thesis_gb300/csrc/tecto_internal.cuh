@@ -160,7 +160,7 @@ struct UpliftRefScratch {
 };
 
 // Phase work lists.
-enum TileKind { TK_RESOLVE = 0, TK_THERMAL, TK_HYDRO, TK_CCL, TK_STATS, TK_COUNT };
+enum TileKind { TK_RESOLVE = 0, TK_THERMAL, TK_HYDRO, TK_HYDRO_TWO, TK_CCL, TK_STATS, TK_COUNT };
 // CCL tiles: one warp per row of kCclTileX cells, kCclTileY rows per block
 constexpr int kCclTileX = 32, kCclTileY = 32;
 
@@ -183,6 +183,7 @@ struct Batch {
     int sort_final = 0;
     size_t total = 0;                        // sum of member cells
     int hydro_variant = 0;                   // tile variant the TK_HYDRO list was built for
+    int hydro_default[2] = {0, 0};           // untuned choice (split path: [1]), 0 until it is made
     int thermal_variant = 0;                 // tile variant the TK_THERMAL list was built for
     int tuned_thermal = 0;
     int tuned_hydro = 0, tuned_rb = 0;       // autotuner's choices (0 = none), used when the
@@ -391,7 +392,6 @@ constexpr int kHydroVariantCount = 9;
 constexpr int kDefaultHydroVariant = 4;          // 56 x 24 cells: where the autotuner starts from
 constexpr int kHydroStripVariant = 8;            // from here on: the march (8 is kept as another number for it)
 constexpr int kHydroMarchVariant = 9;            // marching row chunks in shared memory (fused path only)
-constexpr size_t kMarchMinCells = 500000;        // cells from which the hydraulic march is the default
 constexpr int kMarchTwoInner = 116;              // of a strip that takes two sub-iterations at once
 constexpr int kMarchInner = 120;                 // interior columns of one shared-memory strip (128 with it)
 constexpr int kThermalInner = 60;                // interior columns of one thermal strip (64 with the halo)

@@ -105,3 +105,23 @@ def test_two_sub_iterations_in_one_march(kind, W, H, iters):
         for name, f, v in zip(("height", "water", "sediment", "flux"),
                               (T.FIELD_HEIGHT, T.FIELD_WATER, T.FIELD_SEDIMENT, T.FIELD_FLUX), want):
             np.testing.assert_array_equal(w.download(f).view(np.uint32), v.view(np.uint32), err_msg=name)
+
+
+@pytest.mark.parametrize("W,H,iters", [(5, 3, 2), (3, 40, 3), (51, 9, 2), (52, 10, 2), (53, 25, 4), (105, 29, 2),
+                                       (104, 41, 3), (7, 130, 2)])
+@pytest.mark.parametrize("tile", [1, 2, 3, 4, 5])
+@pytest.mark.parametrize("kind", ["tiny", "clamp", "huge"])
+def test_two_sub_iterations_on_one_tile(kind, tile, W, H, iters):
+    """As above on tiles: one cell less and more than a tile, worlds that wrap within a halo, tiles that run
+    again in the scalar form, and an odd number left over."""
+    s = T.baseline_settings()
+    s.step.hydraulicTile = tile
+    h, water, sed, flux = fields(kind, W, H)
+    with T.World(s, W, H, seed=1000) as w:
+        for f, a in ((T.FIELD_HEIGHT, h), (T.FIELD_WATER, water), (T.FIELD_SEDIMENT, sed), (T.FIELD_FLUX, flux)):
+            w.upload(f, a)
+        w.hydraulic(iters, 0.02)
+        want = O.hydraulic(h, water, sed, flux, iters, 0.02, 1000, s)
+        for name, f, v in zip(("height", "water", "sediment", "flux"),
+                              (T.FIELD_HEIGHT, T.FIELD_WATER, T.FIELD_SEDIMENT, T.FIELD_FLUX), want):
+            np.testing.assert_array_equal(w.download(f).view(np.uint32), v.view(np.uint32), err_msg=name)
