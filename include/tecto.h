@@ -433,7 +433,7 @@ int tecto_batch_phase_thermal(tecto_batch *batch, int iterations, tecto_stream_t
  * The caller's worlds are not touched.  The choice is cached per device and batch shape class
  * (total cells and mean world cells, half-octave classes); batches whose settings leave
  * hydraulicTile / thermalTile / sortRadixBits at 0 use the choice cached for their class, else for
- * the nearest tuned class on their device, else the defaults (by the batch's
+ * the nearest tuned class on their device within an octave, else the defaults (by the batch's
  * cells, see hydraulicTile, thermalTile and sortRadixBits). */
 typedef struct tecto_tuning {
     int hydraulicTile;       /* chosen variant, 1..8 (8 is the march) */

@@ -3,7 +3,7 @@
 // Reference: rain/flux/flow/sediment/transport/evaporate,
 // src/cuda_compute/plate_tectonics_kernel.cu:2430-2593; driver plate_tectonic_sim.cu:331-373.
 //
-// The same sub-iteration as k_hydro (k_erosion.cu), with no row of the vertical halo computed twice.
+// The same sub-iteration as k_hydro (k_hydro_tile.cu), with no row of the vertical halo computed twice.
 // A block of 256 threads owns a column strip of a world (up to kMarchInner = 120 interior columns, 128
 // with the halo of 4 on each side) and marches down its rows, 4 rows per chunk; a thread owns two
 // adjacent cells of one row (64 pairs a row, a warp is half a row).  With r its first row, a chunk
@@ -18,9 +18,9 @@
 // Two cells a thread and packed arithmetic take 523 warp-instructions per 64 cells where one cell a
 // thread took 1036; two blocks of up to 128 registers per SM (three blocks of 80 wait on the shared-memory
 // pipe: 990 against 762 us).  One sub-iteration, before and after, us: 2048^2 93.9 -> 72, 4096^2
-// 303 -> 232, 8192^2 1120 -> 858 (4.8 TB/s of DRAM traffic), the 49.7 M cell batch 966 -> 762; with the
+// 303 -> 232, 8192^2 1120 -> 852 (4.8 TB/s of DRAM traffic), the 49.7 M cell batch 966 -> 759; with the
 // global accesses taken out 58 / 635 / 566 at 2048^2 / 8192^2 / the batch, so it is bound by issue and
-// shared-memory latency with DRAM close behind.
+// shared-memory latency with DRAM close behind.  Two at once: 54 / 731 / 648 (k_hydro_march_pair).
 // Rows live in rings of 16 rows indexed by the march's own row number (a chunk touches at most 15
 // consecutive rows of a ring).  A piece of a strip starts with three chunks of warm-up; every chunk
 // runs all three stages, and only the stores are limited to the piece's rows.  All strip-rows of the
@@ -421,11 +421,11 @@ __device__ __noinline__ void march_two_ieee(const PairParams &pp, const HydroWor
 // Two sub-iterations in one march.  The block's first 256 threads run the first on 128 columns, leaving what
 // it would store in shared memory; the other 256 run the second on the 116 columns inside, ten rows behind,
 // which is as close as the first's height and as far as the rings allow.
-// A sub-iteration moves 34 bytes a cell instead of 60 (DRAM 37% busy), and its instructions are as many as
+// A sub-iteration moves 35 bytes a cell instead of 60 (DRAM 37% busy), and its instructions are as many as
 // alone (530 a 64 cells, issue 56%, the shared-memory pipe 59%); one sub-iteration, alone and of two, us:
-// 2048^2 72 -> 54, 4096^2 232 -> 197, 8192^2 852 -> 749, the 49.7 M cell batch 759 -> 722.  Skipping the stages
-// that a piece's first and last chunks do not need costs more than it saves (8192^2 805: the branches
-// between the stages keep the compiler from overlapping them).
+// 2048^2 72 -> 54, 4096^2 232 -> 192, 8192^2 852 -> 731, the 49.7 M cell batch 759 -> 648.  Leaving out, by a
+// test a chunk, the stages that a piece's first and last chunks do not need gains where pieces are short (1024^2
+// 24.6 -> 22) and loses elsewhere (8192^2 747 -> 805: the branches keep the compiler from overlapping stages).
 __global__ __launch_bounds__(2 * kPairThreads, 1) void k_hydro_march_pair(const __grid_constant__ PairParams pp)
 {
     kernel_release();

@@ -19,8 +19,9 @@
 // more in scalar IEEE form.
 //
 // Before (one cell a thread, 64 columns, 1024 threads) and now, us per sub-iteration: 256^2 12.7 -> 5.7,
-// 1024^2 31.2 -> 23, 2048^2 103 -> 80, 8192^2 1444 -> 1154.  Bound by the latency of the three phases at
-// small sizes and by issue at large ones, where the march (k_hydro_march.cu) computes less halo.
+// 1024^2 31.2 -> 23, 2048^2 103 -> 78, 8192^2 1444 -> 1150.  Bound by the latency of the three phases at
+// small sizes, where k_hydro_two takes two sub-iterations at once (256^2 3.5), and by issue at large ones,
+// where the march (k_hydro_march.cu) computes less halo.
 #include "hydro_pair.cuh"
 #include "noise.cuh"
 

@@ -16,7 +16,7 @@
 //
 // 179 warp-instructions per 64 cells; the form before it (one cell a thread, flows in shared-memory rings,
 // two block barriers per 8 rows) took 390.  20 warps per SM (96 registers).  One iteration, before and
-// after, us: 2048^2 38.0 -> 23.0, 8192^2 416 -> 230, a 49.7 M cell batch 361 -> 191; the tiles of variant 4
+// after, us: 2048^2 38.0 -> 19.2, 8192^2 416 -> 224, a 49.7 M cell batch 361 -> 189; the tiles of variant 4
 // take 37.4, 570 and 463.  Bound by the floating-point and the compare-select pipes (48 % and 49 % busy)
 // and the dependent sums of 20 warps; DRAM is at 40 % of its rate at 8192^2.
 //

@@ -172,7 +172,8 @@ static int default_radix_bits(size_t cells)
 }
 
 // The default thermal variant: one iteration with tiles (variant 4, two iterations a launch) against the
-// march (5), us: 512^2 5.3 / 6.5, 1024^2 11.6 / 11.0, 2048^2 37.4 / 23.0, 8192^2 570 / 230.
+// march (5), us: 512^2 5.3 / 6.5, 1024^2 11.6 / 8.4, 2048^2 37.4 / 19.2, 8192^2 570 / 224; whole steps at 1001x613
+// 430 / 435, 900x800 444 / 443, 40 worlds of 1.1 M cells 783 / 746.
 // The default hydraulic variant: the one whose two sub-iterations a model of the measured shapes puts lowest.
 // Tiles run in waves of 152 SMs x the tiles an SM holds, and a wave's time depends on how many it holds; the
 // march's blocks take equal shares of the strips' rows (with what a strip's start costs, k_hydro_march.cu), at
@@ -247,11 +248,15 @@ int batch_prepare(Batch &b, cudaStream_t st)
         size_t cells = 0;
         for (const tecto_world *w : b.members) cells += w->N;
         b.total = cells;
-        int th = 0, tr = 0, tt = 0;
-        if (tune_lookup(b.device, cells, b.members.size(), &th, &tr, &tt)) {
-            b.tuned_hydro = th;
-            b.tuned_rb = tr;
-            b.tuned_thermal = tt;
+        // A choice of another size says less than the defaults' model: taken from an octave away at most in all.
+        // (2048^2 with the tiles that 1024^2 was tuned to 1980 us a step, with the default 1490.)
+        constexpr int kTunedSteps = 2;
+        int th = 0, tr = 0, tt = 0, steps = 0;
+        if (tune_lookup(b.device, cells, b.members.size(), &th, &tr, &tt, &steps)) {
+            const bool near = steps <= kTunedSteps;
+            b.tuned_hydro = near ? th : 0;
+            b.tuned_rb = near ? tr : 0;
+            b.tuned_thermal = near ? tt : 0;
         }
     }
     int variant = 0, rb = 0, tvariant = 0;

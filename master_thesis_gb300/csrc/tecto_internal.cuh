@@ -403,7 +403,8 @@ int thermal_variant_for(const tecto_settings &s);  // 0 when the settings leave 
 
 // Autotuner cache (tecto_tune.cu): best hydraulic tile variant and sort digit width for a batch
 // shape class on a device; false when nothing was tuned for that class.
-bool tune_lookup(int device, size_t total_cells, size_t worlds, int *hydro, int *rb, int *thermal);
+// steps: how many half-octave classes off the choice is (0: the class itself)
+bool tune_lookup(int device, size_t total_cells, size_t worlds, int *hydro, int *rb, int *thermal, int *steps = nullptr);
 int tune_batch(Batch &b, cudaStream_t st, tecto_tuning *out);  // tune on the members' shapes, apply
 
 // Radix sort core (k_sort.cu).  If worlds != nullptr the first pass generates the keys (the

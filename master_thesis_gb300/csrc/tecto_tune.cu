@@ -8,7 +8,7 @@
 // worlds of the same shapes with synthetic content, times the candidates, and frees them.
 // Choices are cached per device and batch shape class (total cells, mean world size, both in
 // half-octave steps); a batch whose settings leave hydraulicTile / thermalTile / sortRadixBits at
-// 0 uses the choice of its class, else of the nearest tuned class on its device.
+// 0 uses the choice of its class, else of the nearest tuned class on its device within kTunedSteps.
 #include <algorithm>
 #include <cmath>
 #include <map>
@@ -183,8 +183,9 @@ int tune_shapes(const tecto_settings &settings, const std::vector<int2> &shapes,
 
 }  // namespace
 
-bool tune_lookup(int device, size_t total, size_t worlds, int *hydro, int *rb, int *thermal)
+bool tune_lookup(int device, size_t total, size_t worlds, int *hydro, int *rb, int *thermal, int *steps)
 {
+    if (steps) *steps = 0;
     std::lock_guard<std::mutex> lock(g_tune_mu);
     const ClassKey k = class_of(device, total, worlds);
     auto it = g_tune.find(k);
@@ -200,6 +201,7 @@ bool tune_lookup(int device, size_t total, size_t worlds, int *hydro, int *rb, i
             }
         }
         if (best < 0) return false;
+        if (steps) *steps = best;
     }
     *hydro = it->second.hydro;
     *rb = it->second.rb;
