@@ -73,7 +73,7 @@ def measured_peak_hbm():
     return 6800.0, "fallback 6.8 TB/s"
 
 
-MARCH_VARIANT = 9  # hydraulic variant of k_hydro_march
+MARCH_VARIANT = 8  # hydraulic variants of the march: this one and above (one kernel, two numbers)
 
 
 def _profile_number(name, key):
@@ -85,18 +85,19 @@ def _profile_number(name, key):
 
 
 def profiled_traffic_per_cell(variant=MARCH_VARIANT):
-    """DRAM bytes per cell of one hydraulic launch from the committed ncu summaries: for the
-    marching kernel, captured on the mixed batch itself; for the tile kernels, a 2048^2 launch."""
-    if variant == MARCH_VARIANT:
+    """DRAM bytes per cell of one hydraulic launch (two sub-iterations) from the committed ncu
+    summaries: for the marching kernel, captured on the mixed batch itself; for the tile kernels, a
+    2048^2 launch."""
+    if variant >= MARCH_VARIANT:
         return _profile_number("k_hydro_march_traffic.md", "traffic_bytes_per_cell_batch")
     v = _profile_number("k_hydro_2048.md", "traffic_bytes_per_launch_2048")
     return None if v is None else v / (2048 * 2048)
 
 
 def profiled_instructions_per_cell(variant=MARCH_VARIANT):
-    """Warp-instructions per cell of one hydraulic launch at 2048^2, from the committed ncu summary
-    of the kernel that variant runs."""
-    name = "k_hydro_march_2048.md" if variant == MARCH_VARIANT else "k_hydro_2048.md"
+    """Warp-instructions per cell of one hydraulic launch (two sub-iterations) at 2048^2, from the
+    committed ncu summary of the kernel that variant runs."""
+    name = "k_hydro_march_2048.md" if variant >= MARCH_VARIANT else "k_hydro_2048.md"
     v = _profile_number(name, "warp_instructions_per_launch_2048")
     return None if v is None else v / (2048 * 2048)
 
@@ -459,16 +460,17 @@ def run_engine(args, ws, rank, local):
     total_all = reduce_sum(total, dist, "cuda")  # replicas hold different worlds
     value = job_rate(total_all, args.steps, ms)
 
-    # dominant kernel: the fused hydraulic sub-iteration over the whole batch, on the same stream
-    reps = 20
+    # dominant kernel: the hydraulic launch over the whole batch, two sub-iterations, on the same stream
+    reps, per_launch = 20, 2
     batch.hydraulic(2, s.step.hydraulicDt, stream)
-    hydro_ms = event_ms(torch, stream, lambda: batch.hydraulic(reps, s.step.hydraulicDt, stream)) / reps
+    hydro_ms = event_ms(torch, stream, lambda: batch.hydraulic(reps, s.step.hydraulicDt, stream)) / reps * per_launch
     peak, peak_src = measured_peak_hbm()
-    achieved = HYDRO_BYTES_PER_CELL * total / (hydro_ms / 1e3) / 1e9
+    hydro_bytes, hydro_engine_bytes = per_launch * HYDRO_BYTES_PER_CELL, per_launch * HYDRO_ENGINE_BYTES_PER_CELL
+    achieved = hydro_bytes * total / (hydro_ms / 1e3) / 1e9
     hv = tuning.hydraulicTile
     tpc = profiled_traffic_per_cell(hv)
     ipc = profiled_instructions_per_cell(hv)
-    hkernel = "k_hydro_march" if hv == MARCH_VARIANT else "k_hydro"
+    hkernel = "k_hydro_march_pair" if hv >= MARCH_VARIANT else "k_hydro_two"
     n_sms = torch.cuda.get_device_properties(local).multi_processor_count
 
     # e2e through the C ABI with host buffers: upload every world's state, step, download
@@ -551,19 +553,19 @@ def run_engine(args, ws, rank, local):
             "gpu_launches": int(launches),
             "e2e": {"value": e2e_value, "unit": "cell-updates/s", "h2d_bytes_per_step": int(h2d),
                     "d2h_bytes_per_step": int(d2h)},
-            "roofline": {"bound": "hbm", "kernel": f"{hkernel} (hydraulic variant {hv}: one fused sub-iteration, "
-                                                  "all worlds)",
+            "roofline": {"bound": "hbm", "kernel": f"{hkernel} (hydraulic variant {hv}: one launch of two "
+                                                  "sub-iterations, all worlds)",
                          "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                          "traffic": None if tpc is None else tpc * total,
                          "traffic_note": ("ncu dram bytes of one launch over this batch (profiles/k_hydro_march_traffic.md)"
-                                          if hv == MARCH_VARIANT else
+                                          if hv >= MARCH_VARIANT else
                                           "ncu dram bytes of a 2048^2 launch, scaled per cell"),
                          "peak_source": peak_src, "ms_per_launch": hydro_ms,
-                         "alg_bytes_per_launch": HYDRO_BYTES_PER_CELL * total,
-                         "engine_alg_bytes_per_launch": HYDRO_ENGINE_BYTES_PER_CELL * total,
-                         "engine_frac": HYDRO_ENGINE_BYTES_PER_CELL * total / (hydro_ms / 1e3) / 1e9 / peak,
-                         "bytes_note": "64 B/cell: read h, w, s, flux, write them and the velocity; the fused kernel "
-                                       "writes no velocity, so its own compulsory traffic is 56 B/cell (engine_*)"},
+                         "alg_bytes_per_launch": hydro_bytes * total,
+                         "engine_alg_bytes_per_launch": hydro_engine_bytes * total,
+                         "engine_frac": hydro_engine_bytes * total / (hydro_ms / 1e3) / 1e9 / peak,
+                         "bytes_note": "64 B/cell and sub-iteration: read h, w, s, flux, write them and the velocity; the fused kernels "
+                                       "write no velocity (56 B/cell, engine_*); two sub-iterations a launch move half"},
             "issue_roofline": issue_roofline(ipc, total, hydro_ms, clk.summary().get("sm_mhz"), n_sms, hkernel),
             "step_roofline": {"alg_bytes_per_cell": STEP_BYTES_PER_CELL,
                               "achieved_gbs": STEP_BYTES_PER_CELL * value / ws / 1e9,
@@ -746,8 +748,8 @@ def engine_extras(args, T, torch, stream, s, specs, total, batched_value):
 
 def run_case(args):
     """Small fixed workloads for ncu captures (no timing, no JSON line):
-    erosion2048  one 5-iteration thermal launch and one fused hydraulic launch (variant --hydro-tile,
-                 default 4) on a 2048^2 world;
+    erosion2048  5 thermal iterations and one hydraulic launch of two sub-iterations (variant
+                 --hydro-tile, default 4) on a 2048^2 world;
     erosion4096  the same on a 4096^2 world (each field 67 MB: a launch's working set is about
                  eight times the L2), one thermal launch of the default variant, two hydraulic
                  sub-iterations of the variant --hydro-tile (default 4);
@@ -774,7 +776,7 @@ def run_case(args):
         w.upload(T.FIELD_WATER, np.abs(rng.normal(0, 0.05, (2048, 2048))).astype(np.float32))
         w.upload(T.FIELD_SEDIMENT, np.abs(rng.normal(0, 0.01, (2048, 2048))).astype(np.float32))
         w.thermal(5, stream)
-        w.hydraulic(1, s.step.hydraulicDt, stream)
+        w.hydraulic(2, s.step.hydraulicDt, stream)
         w.check(stream)
     elif args.case == "erosion4096":
         s.step.hydraulicTile = args.hydro_tile
