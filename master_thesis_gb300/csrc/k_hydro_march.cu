@@ -20,7 +20,7 @@
 // pipe: 990 against 762 us).  One sub-iteration, before and after, us: 2048^2 93.9 -> 72, 4096^2
 // 303 -> 232, 8192^2 1120 -> 852 (4.8 TB/s of DRAM traffic), the 49.7 M cell batch 966 -> 759; with the
 // global accesses taken out 58 / 635 / 566 at 2048^2 / 8192^2 / the batch, so it is bound by issue and
-// shared-memory latency with DRAM close behind.  Two at once: 54 / 731 / 648 (k_hydro_march_pair).
+// shared-memory latency with DRAM close behind.  Two at once: 53 / 712 / 654 (k_hydro_march_pair).
 // Rows live in rings of 16 rows indexed by the march's own row number (a chunk touches at most 15
 // consecutive rows of a ring).  A piece of a strip starts with three chunks of warm-up; every chunk
 // runs all three stages, and only the stores are limited to the piece's rows.  All strip-rows of the
@@ -146,6 +146,10 @@ __device__ __forceinline__ void march_piece(const HydroParams &p, const PairCons
         const uint32_t v = g + W4;  // < 2N <= 2^31
         return min(v, v - N);
     };
+    // Whether a stage's operands are loaded before the stage ahead stores its results.  Of two at once: 8192^2
+    // 728 -> 712 us, 2048^2 54.1 -> 52.6, 1500x1100 25.5 -> 24.8; for odd widths it is the other way round (the
+    // batch, half of its worlds odd, 653 without and 664 with it).
+    constexpr bool EARLY = VEC && ROLE != kAlone;
     // Per chunk k (first row rk = r0 + 4k) this thread's base row is t = rk + rr and its items are rows
     // t + c: flux c = 7, flow c = 2, transport c = -4, and the loads c = 12 (height, water and rain),
     // c = 11 (old flux) and c = 6 (sediment).
@@ -201,6 +205,7 @@ __device__ __forceinline__ void march_piece(const HydroParams &p, const PairCons
         bool bad = false;  // an operand of this thread outside the packed path's ranges
         if (active && (ROLE != kSecondOfTwo || k >= 0)) {
             // ---- transport (:2572-2585): bilinear taps within two cells ----
+            f2 sn;
             {
                 const uint32_t pv = (P - 4 * kMRow) & kRMask;
                 const f2 px = sub2(fgx, mul2_z(ld2(S, pv + OVX), c.dt, Z));
@@ -221,7 +226,26 @@ __device__ __forceinline__ void march_piece(const HydroParams &p, const PairCons
                 const uint32_t u1 = (o1 & kRMask) + OS, d1 = ((o1 + kMRow) & kRMask) + OS;
                 const f2 I0 = add2(mul2_z(vx, pk(mld(S, u0), mld(S, u1)), Z), mul2_z(wx, pk(mld(S, u0 + 4), mld(S, u1 + 4)), Z));
                 const f2 I1 = add2(mul2_z(vx, pk(mld(S, d0), mld(S, d1)), Z), mul2_z(wx, pk(mld(S, d0 + 4), mld(S, d1 + 4)), Z));
-                const f2 sn = add2(mul2_z(vy, I0, Z), mul2_z(wy, I1, Z));
+                sn = add2(mul2_z(vy, I0, Z), mul2_z(wy, I1, Z));
+            }
+            // ---- flow, sediment exchange, evaporation ----
+            uint32_t fa0, fau, fad;
+            f2 sd;
+            Flux2 fc;
+            f2 fuw, fdy, fdw, fw, fh, fhu, fhd;
+            float flz, frx, fhl, fhr;
+            const auto load_flow = [&]() {
+                fa0 = (P + 2 * kMRow) & kRMask, fau = (P + 3 * kMRow) & kRMask, fad = (P + kMRow) & kRMask;
+                sd = ROLE == kSecondOfTwo ? ld2(S, fa0 + kOE + kSet) : ns;
+                fc = Flux2{ld2(S, fa0 + OX), ld2(S, fa0 + OY), ld2(S, fa0 + OZ), ld2(S, fa0 + OF)};
+                fuw = ld2(S, fau + OF), fdy = ld2(S, fad + OY), fdw = ld2(S, fad + OF);
+                fw = ld2(S, fa0 + OW), fh = ld2(S, fa0 + OH), fhu = ld2(S, fau + OH), fhd = ld2(S, fad + OH);
+                flz = mld(S, fa0 + OZ - 4), frx = mld(S, fa0 + OX + 8);
+                fhl = mld(S, fa0 + OH - 4), fhr = mld(S, fa0 + OH + 8);
+            };
+            if (EARLY) load_flow();
+            {
+                const uint32_t pv = (P - 4 * kMRow) & kRMask;
                 if (ROLE == kFirstOfTwo) {
                     st2(S, pv + kOE + kSet, sn);
                 } else {
@@ -229,23 +253,20 @@ __device__ __forceinline__ void march_piece(const HydroParams &p, const PairCons
                     gst2<VEC>(q.s_out, B - W4, sn, row && in0, row && in1);
                 }
             }
-            // ---- flow, sediment exchange, evaporation ----
+            if (!EARLY) load_flow();
+            f2 hn, wn, s_new, ux, uy;
             {
-                const uint32_t a0 = (P + 2 * kMRow) & kRMask, au = (P + 3 * kMRow) & kRMask, ad = (P + kMRow) & kRMask;
-                const uint32_t f0 = a0, fu = au, fd = ad;
-                const f2 sd = ROLE == kSecondOfTwo ? ld2(S, a0 + kOE + kSet) : ns;
-                f2 hn, wn, s_new, ux, uy;
                 if constexpr (IEEE) {
                     FlowOut v[2];
 #pragma unroll
                     for (uint32_t c4 = 0; c4 < 8; c4 += 4) {
-                        const float4 fC = make_float4(mld(S, f0 + c4 + OX), mld(S, f0 + c4 + OY), mld(S, f0 + c4 + OZ),
-                                                      mld(S, f0 + c4 + OF));
+                        const float4 fC = make_float4(mld(S, fa0 + c4 + OX), mld(S, fa0 + c4 + OY), mld(S, fa0 + c4 + OZ),
+                                                      mld(S, fa0 + c4 + OF));
                         v[c4 >> 2] = flow_cell_general(
-                            p, fC, mld(S, f0 + c4 + OZ - 4), mld(S, fu + c4 + OF), mld(S, f0 + c4 + OX + 4),
-                            mld(S, fd + c4 + OY), mld(S, fd + c4 + OF), mld(S, a0 + c4 + OW), mld(S, a0 + c4 + OH),
-                            c4 ? hi(sd) : lo(sd), mld(S, a0 + c4 + OH - 4), mld(S, a0 + c4 + OH + 4),
-                            mld(S, au + c4 + OH), mld(S, ad + c4 + OH));
+                            p, fC, mld(S, fa0 + c4 + OZ - 4), mld(S, fau + c4 + OF), mld(S, fa0 + c4 + OX + 4),
+                            mld(S, fad + c4 + OY), mld(S, fad + c4 + OF), mld(S, fa0 + c4 + OW), mld(S, fa0 + c4 + OH),
+                            c4 ? hi(sd) : lo(sd), mld(S, fa0 + c4 + OH - 4), mld(S, fa0 + c4 + OH + 4),
+                            mld(S, fau + c4 + OH), mld(S, fad + c4 + OH));
                     }
                     hn = pk(v[0].hn, v[1].hn);
                     wn = pk(v[0].wn, v[1].wn);
@@ -254,62 +275,70 @@ __device__ __forceinline__ void march_piece(const HydroParams &p, const PairCons
                     uy = pk(v[0].uy, v[1].uy);
                 } else {
                     Flow2 o;
-                    const Flux2 fc{ld2(S, f0 + OX), ld2(S, f0 + OY), ld2(S, f0 + OZ), ld2(S, f0 + OF)};
                     const bool mine = live_w && (uint32_t)(tr + 4 + MORE) < nrows + 4u + 2u * MORE;
-                    bad = flow_pair(c, fc, mld(S, f0 + OZ - 4), mld(S, f0 + OX + 8), ld2(S, fu + OF),
-                                    ld2(S, fd + OY), ld2(S, fd + OF), ld2(S, a0 + OW), ld2(S, a0 + OH),
-                                    mld(S, a0 + OH - 4), mld(S, a0 + OH + 8), ld2(S, au + OH), ld2(S, ad + OH), sd,
-                                    mine, o) || bad;
+                    bad = flow_pair(c, fc, flz, frx, fuw, fdy, fdw, fw, fh, fhl, fhr, fhu, fhd, sd, mine, o) || bad;
                     hn = o.hn, wn = o.wn, s_new = o.s1, ux = o.ux, uy = o.uy;
                 }
-                st2(S, a0 + OS, s_new);
-                st2(S, a0 + OVX, ux);
-                st2(S, a0 + OVY, uy);
+            }
+            // ---- flux (:2439-2485) ----
+            uint32_t xa0, xau, xad;
+            f2 xh, xw, xhu, xwu, xhd, xwd;
+            float xhl, xhr, xwl, xwr;
+            const auto load_flux = [&]() {
+                xa0 = (P + 7 * kMRow) & kRMask, xau = (P + 8 * kMRow) & kRMask, xad = (P + 6 * kMRow) & kRMask;
+                if (ROLE == kSecondOfTwo) {
+                    const f2 x = ld2(S, xa0 + kOX), y = ld2(S, xa0 + kOY), z = ld2(S, xa0 + kOZ), f = ld2(S, xa0 + kOF);
+                    fa = make_float4(lo(x), lo(y), lo(z), lo(f));
+                    fb = make_float4(hi(x), hi(y), hi(z), hi(f));
+                }
+                xh = ld2(S, xa0 + OH), xw = ld2(S, xa0 + OW), xhu = ld2(S, xau + OH), xwu = ld2(S, xau + OW);
+                xhd = ld2(S, xad + OH), xwd = ld2(S, xad + OW);
+                xhl = mld(S, xa0 + OH - 4), xhr = mld(S, xa0 + OH + 8);
+                xwl = mld(S, xa0 + OW - 4), xwr = mld(S, xa0 + OW + 8);
+            };
+            if (EARLY) load_flux();
+            {
+                st2(S, fa0 + OS, s_new);
+                st2(S, fa0 + OVX, ux);
+                st2(S, fa0 + OVY, uy);
                 // evaporate (:2587-2593)
                 const f2 wo = evaporate2(c, wn);
                 if (ROLE == kFirstOfTwo) {
-                    st2(S, a0 + kSet + kOH, hn);
-                    st2(S, a0 + kSet + kOW, add2(wo, ld2(S, a0 + kOE)));
+                    st2(S, fa0 + kSet + kOH, hn);
+                    st2(S, fa0 + kSet + kOW, add2(wo, ld2(S, fa0 + kOE)));
                 } else {
                     const bool row = (uint32_t)(tr + 2) < nrows, s0 = row && in0, s1 = row && in1;
                     gst2<VEC>(q.h_out, B + 2u * Wu, hn, s0, s1);
                     gst2<VEC>(q.w_out, B + 2u * Wu, wo, s0, s1);
                 }
             }
-            // ---- flux (:2439-2485) ----
+            if (!EARLY) load_flux();
+            f2 ox, oy, oz, ow;
             {
-                const uint32_t a0 = (P + 7 * kMRow) & kRMask, au = (P + 8 * kMRow) & kRMask, ad = (P + 6 * kMRow) & kRMask;
-                f2 ox, oy, oz, ow;
-                if (ROLE == kSecondOfTwo) {
-                    const f2 x = ld2(S, a0 + kOX), y = ld2(S, a0 + kOY), z = ld2(S, a0 + kOZ), f = ld2(S, a0 + kOF);
-                    fa = make_float4(lo(x), lo(y), lo(z), lo(f));
-                    fb = make_float4(hi(x), hi(y), hi(z), hi(f));
-                }
                 if constexpr (IEEE) {
                     float4 v[2];
 #pragma unroll
                     for (uint32_t c4 = 0; c4 < 8; c4 += 4)
-                        v[c4 >> 2] = flux_ieee(p, c4 ? fb : fa, mld(S, a0 + c4 + OH), mld(S, a0 + c4 + OW),
-                                               mld(S, a0 + c4 + OH - 4), mld(S, a0 + c4 + OW - 4),
-                                               mld(S, au + c4 + OH), mld(S, au + c4 + OW), mld(S, a0 + c4 + OH + 4),
-                                               mld(S, a0 + c4 + OW + 4), mld(S, ad + c4 + OH), mld(S, ad + c4 + OW));
+                        v[c4 >> 2] = flux_ieee(p, c4 ? fb : fa, mld(S, xa0 + c4 + OH), mld(S, xa0 + c4 + OW),
+                                               mld(S, xa0 + c4 + OH - 4), mld(S, xa0 + c4 + OW - 4),
+                                               mld(S, xau + c4 + OH), mld(S, xau + c4 + OW), mld(S, xa0 + c4 + OH + 4),
+                                               mld(S, xa0 + c4 + OW + 4), mld(S, xad + c4 + OH), mld(S, xad + c4 + OW));
                     ox = pk(v[0].x, v[1].x);
                     oy = pk(v[0].y, v[1].y);
                     oz = pk(v[0].z, v[1].z);
                     ow = pk(v[0].w, v[1].w);
                 } else {
-                    const f2 h = ld2(S, a0 + OH), w = ld2(S, a0 + OW);
                     Flux2 o;
                     const bool mine = live_f && (uint32_t)(tr + 10 + MORE) < nrows + 6u + 2u * MORE;
-                    bad = flux_pair(c, h, w, mld(S, a0 + OH - 4), mld(S, a0 + OH + 8), mld(S, a0 + OW - 4),
-                                    mld(S, a0 + OW + 8), ld2(S, au + OH), ld2(S, au + OW), ld2(S, ad + OH),
-                                    ld2(S, ad + OW), fa, fb, mine, o) || bad;
+                    bad = flux_pair(c, xh, xw, xhl, xhr, xwl, xwr, xhu, xwu, xhd, xwd, fa, fb, mine, o) || bad;
                     ox = o.x, oy = o.y, oz = o.z, ow = o.w;
                 }
-                st2(S, a0 + OX, ox);
-                st2(S, a0 + OY, oy);
-                st2(S, a0 + OZ, oz);
-                st2(S, a0 + OF, ow);
+            }
+            {
+                st2(S, xa0 + OX, ox);
+                st2(S, xa0 + OY, oy);
+                st2(S, xa0 + OZ, oz);
+                st2(S, xa0 + OF, ow);
                 if (ROLE != kFirstOfTwo) {
                     const bool row = (uint32_t)(tr + 7) < nrows, s0 = row && in0, s1 = row && in1;
                     gst_flux<VEC>(q.f_out, B + 7u * Wu, ox, oy, oz, ow, s0, s1);
@@ -423,7 +452,7 @@ __device__ __noinline__ void march_two_ieee(const PairParams &pp, const HydroWor
 // which is as close as the first's height and as far as the rings allow.
 // A sub-iteration moves 35 bytes a cell instead of 60 (DRAM 37% busy), and its instructions are as many as
 // alone (530 a 64 cells, issue 56%, the shared-memory pipe 59%); one sub-iteration, alone and of two, us:
-// 2048^2 72 -> 54, 4096^2 232 -> 192, 8192^2 852 -> 731, the 49.7 M cell batch 759 -> 648.  Leaving out, by a
+// 2048^2 72 -> 53, 4096^2 232 -> 187, 8192^2 852 -> 712, the 49.7 M cell batch 759 -> 654.  Leaving out, by a
 // test a chunk, the stages that a piece's first and last chunks do not need gains where pieces are short (1024^2
 // 24.6 -> 22) and loses elsewhere (8192^2 747 -> 805: the branches keep the compiler from overlapping stages).
 __global__ __launch_bounds__(2 * kPairThreads, 1) void k_hydro_march_pair(const __grid_constant__ PairParams pp)
