@@ -10,7 +10,8 @@
 // the evaporation on a halo of 2; the semi-Lagrangian sediment transport on the tile.  Transport's
 // back-trace reaches |v| dt <= 50 dt cells (velocity clamp at :2524-2528), inside the halo when 50 dt < 1.5;
 // larger steps take the split path (FUSED false: velocity and eroded sediment go to HBM and k_transport
-// gathers from there).
+// gathers from there), which needs a halo of 2 alone: 60 x TY cells of 64 x (TY + 4) instead of 56 x TY of
+// 64 x (TY + 8), the reference's 1024^2 step 25.5 -> 21.5 us a launch.
 //
 // All loads are asynchronous copies to where a phase reads them (the old flux of a pair to the pair's own
 // four flux slots), so that a tile's loads are in flight together without registers.  The velocity
@@ -30,14 +31,16 @@ namespace tecto {
 namespace {
 
 constexpr int HTX = 56;                   // interior columns of a tile
+constexpr int HTXS = 60;                  // on the split path
 constexpr uint32_t kRow = 64 * 4;         // bytes of a shared-memory row: 64 columns with the halo
 constexpr uint32_t kGuard = 16;           // an edge lane reads one cell past a row's end
 
 // Byte layout: guard, height, water (+ rain, then velocity x), sediment (then eroded), flux left, +y, right,
 // -y, velocity y (before: rain), guard.
-template <int TY>
+// HX: the halo, 4 cells where the transport follows, 2 on the split path.
+template <int TY, int HX>
 struct TileMem {
-    static constexpr uint32_t A = (TY + 8) * kRow;  // bytes of an array
+    static constexpr uint32_t A = (TY + 2 * HX) * kRow;  // bytes of an array
     static constexpr uint32_t H = kGuard, W = H + A, S = W + A, X = S + A, Y = X + A, Z = Y + A, F = Z + A, V = F + A;
     static constexpr uint32_t bytes = V + A + kGuard;
 };
@@ -68,15 +71,15 @@ __device__ __forceinline__ void cp_pair(uint32_t dst, const float *row, uint32_t
 }
 
 // The flux phase in scalar form (old fluxes from HBM).
-template <int TY, int NW>
+template <int TY, int NW, int HX>
 __device__ __noinline__ void flux_rows_ieee(const HydroParams &p, const HydroWorld &q, char *S, int x0, int y0)
 {
-    using M = TileMem<TY>;
+    using M = TileMem<TY, HX>;
     const int lane = (int)threadIdx.x & 31, warp = (int)threadIdx.x >> 5;
-    for (int ly = warp + 1; ly < TY + 7; ly += NW) {
+    for (int ly = warp + 1; ly < TY + 2 * HX - 1; ly += NW) {
 #pragma unroll 1
         for (int j = 0; j < 2; ++j) {
-            const int lx = 2 * lane + j, gx = x0 - 4 + lx, gy = y0 - 4 + ly;
+            const int lx = 2 * lane + j, gx = x0 - HX + lx, gy = y0 - HX + ly;
             const uint32_t o = (uint32_t)ly * kRow + (uint32_t)lx * 4u;
             const float4 f = q.f_in[cidx(gx, gy, q.W, q.H)];
             const float4 v = flux_ieee(p, f, mld(S, o + M::H), mld(S, o + M::W), mld(S, o + M::H - 4), mld(S, o + M::W - 4),
@@ -86,7 +89,7 @@ __device__ __noinline__ void flux_rows_ieee(const HydroParams &p, const HydroWor
             mst(S, o + M::Y, v.y);
             mst(S, o + M::Z, v.z);
             mst(S, o + M::F, v.w);
-            if (lx >= 4 && lx < HTX + 4 && ly >= 4 && ly < TY + 4 && gx < q.W && gy < q.H)
+            if (lx >= HX && lx < 64 - HX && ly >= HX && ly < TY + HX && gx < q.W && gy < q.H)
                 q.f_out[(uint32_t)gy * (uint32_t)q.W + (uint32_t)gx] = v;
         }
     }
@@ -96,12 +99,13 @@ __device__ __noinline__ void flux_rows_ieee(const HydroParams &p, const HydroWor
 template <int TY, int NW, bool FUSED>
 __device__ __noinline__ void flow_rows_ieee(const HydroParams &p, const HydroWorld &q, char *S, int x0, int y0)
 {
-    using M = TileMem<TY>;
+    constexpr int HX = FUSED ? 4 : 2;
+    using M = TileMem<TY, HX>;
     const int lane = (int)threadIdx.x & 31, warp = (int)threadIdx.x >> 5;
-    for (int ly = warp + 2; ly < TY + 6; ly += NW) {
+    for (int ly = warp + 2; ly < TY + 2 * HX - 2; ly += NW) {
 #pragma unroll 1
         for (int j = 0; j < 2; ++j) {
-            const int lx = 2 * lane + j, gx = x0 - 4 + lx, gy = y0 - 4 + ly;
+            const int lx = 2 * lane + j, gx = x0 - HX + lx, gy = y0 - HX + ly;
             const uint32_t o = (uint32_t)ly * kRow + (uint32_t)lx * 4u, i = cidx(gx, gy, q.W, q.H);
             const float4 fC = make_float4(mld(S, o + M::X), mld(S, o + M::Y), mld(S, o + M::Z), mld(S, o + M::F));
             const FlowOut v = flow_cell_general(
@@ -111,7 +115,7 @@ __device__ __noinline__ void flow_rows_ieee(const HydroParams &p, const HydroWor
             mst(S, o + M::W, v.ux);
             mst(S, o + M::V, v.uy);
             mst(S, o + M::S, v.s1);
-            if (lx >= 4 && lx < HTX + 4 && ly >= 4 && ly < TY + 4 && gx < q.W && gy < q.H) {
+            if (lx >= HX && lx < 64 - HX && ly >= HX && ly < TY + HX && gx < q.W && gy < q.H) {
                 const uint32_t g = (uint32_t)gy * (uint32_t)q.W + (uint32_t)gx;
                 q.h_out[g] = v.hn;
                 q.w_out[g] = fmaxf(0.0f, v.wn - (fminf(v.wn, 20.0f) * p.evap) * p.dt);
@@ -127,27 +131,28 @@ __device__ __noinline__ void flow_rows_ieee(const HydroParams &p, const HydroWor
 template <int TY, int NW, bool FUSED, bool VEC>
 __device__ __forceinline__ void tile_body(const TileParams &tp, const HydroWorld &q, char *S, int x0, int y0)
 {
-    using M = TileMem<TY>;
+    constexpr int HX = FUSED ? 4 : 2;
+    using M = TileMem<TY, HX>;
     const PairConst &c = tp.c;
     const int W = q.W, H = q.H;
     const int lane = (int)threadIdx.x & 31, warp = (int)threadIdx.x >> 5, col = 2 * lane;
     const uint32_t Sa = (uint32_t)__cvta_generic_to_shared(S);
-    const uint32_t c0 = (uint32_t)wrapc(x0 - 4 + col, W), c1 = VEC ? c0 + 1 : (uint32_t)wrapc(x0 - 3 + col, W);
-    const int iw = min(HTX, W - x0), ih = min(TY, H - y0);
-    const bool in0 = col >= 4 && col < iw + 4, in1 = col >= 4 && col + 1 < iw + 4;
-    const bool live_f = col < iw + 7, live_w = col >= 2 && col < iw + 6;
+    const uint32_t c0 = (uint32_t)wrapc(x0 - HX + col, W), c1 = VEC ? c0 + 1 : (uint32_t)wrapc(x0 - HX + 1 + col, W);
+    const int iw = min(64 - 2 * HX, W - x0), ih = min(TY, H - y0);
+    const bool in0 = col >= HX && col < iw + HX, in1 = col >= HX && col + 1 < iw + HX;
+    const bool live_f = col < iw + 2 * HX - 1, live_w = col >= 2 && col < iw + 2 * HX - 2;
     const uint32_t L = (uint32_t)lane * 8u;
-    const uint32_t B = (uint32_t)y0 * (uint32_t)W + (uint32_t)(x0 - 4 + col);  // global offset of row y0, this pair
+    const uint32_t B = (uint32_t)y0 * (uint32_t)W + (uint32_t)(x0 - HX + col);  // global offset of row y0, this pair
 
     // every load of the tile
 #pragma unroll 2
-    for (int ly = warp; ly < TY + 8; ly += NW) {
-        const uint32_t g = (uint32_t)wrapc(y0 - 4 + ly, H) * (uint32_t)W, d = Sa + (uint32_t)ly * kRow + L;
+    for (int ly = warp; ly < TY + 2 * HX; ly += NW) {
+        const uint32_t g = (uint32_t)wrapc(y0 - HX + ly, H) * (uint32_t)W, d = Sa + (uint32_t)ly * kRow + L;
         cp_pair<VEC>(d + M::H, q.h_in + g, c0, c1);
         cp_pair<VEC>(d + M::W, q.w_in + g, c0, c1);
         cp_pair<VEC>(d + M::V, q.rain + g, c0, c1);
-        if (ly >= 2 && ly < TY + 6) cp_pair<VEC>(d + M::S, q.s_in + g, c0, c1);
-        if (ly >= 1 && ly < TY + 7) {
+        if (ly >= 2 && ly < TY + 2 * HX - 2) cp_pair<VEC>(d + M::S, q.s_in + g, c0, c1);
+        if (ly >= 1 && ly < TY + 2 * HX - 1) {
             const char *f0 = reinterpret_cast<const char *>(q.f_in + g + c0), *f1 = reinterpret_cast<const char *>(q.f_in + g + c1);
             cp8(d + M::X, f0);
             cp8(d + M::Y, f0 + 8);
@@ -156,16 +161,16 @@ __device__ __forceinline__ void tile_body(const TileParams &tp, const HydroWorld
         }
     }
     asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
-    for (int ly = warp; ly < TY + 8; ly += NW) {
+    for (int ly = warp; ly < TY + 2 * HX; ly += NW) {
         const uint32_t o = (uint32_t)ly * kRow + L;
         st2(S, o + M::W, add2(ld2(S, o + M::W), ld2(S, o + M::V)));
     }
     __syncthreads();
 
-    // flux on rows 1 .. TY + 6
+    // flux on all rows but the first and the last
     bool bad = tp.ieee != 0;
 #pragma unroll 1
-    for (int ly = warp + 1; ly < TY + 7; ly += NW) {
+    for (int ly = warp + 1; ly < TY + 2 * HX - 1; ly += NW) {
         const uint32_t o = (uint32_t)ly * kRow + L;
         const f2 f0 = ld2(S, o + M::X), f1 = ld2(S, o + M::Y), f2_ = ld2(S, o + M::Z), f3 = ld2(S, o + M::F);
         Flux2 v;
@@ -179,18 +184,18 @@ __device__ __forceinline__ void tile_body(const TileParams &tp, const HydroWorld
         st2(S, o + M::Y, v.y);
         st2(S, o + M::Z, v.z);
         st2(S, o + M::F, v.w);
-        const bool row = (unsigned)(ly - 4) < (unsigned)ih;
-        gst_flux<VEC>(q.f_out, B + (uint32_t)(ly - 4) * (uint32_t)W, v.x, v.y, v.z, v.w, row && in0, row && in1);
+        const bool row = (unsigned)(ly - HX) < (unsigned)ih;
+        gst_flux<VEC>(q.f_out, B + (uint32_t)(ly - HX) * (uint32_t)W, v.x, v.y, v.z, v.w, row && in0, row && in1);
     }
     if (__syncthreads_or(bad)) {
-        flux_rows_ieee<TY, NW>(tp.p, q, S, x0, y0);
+        flux_rows_ieee<TY, NW, HX>(tp.p, q, S, x0, y0);
         __syncthreads();
     }
 
-    // flow, sediment exchange and evaporation on rows 2 .. TY + 5
+    // flow, sediment exchange and evaporation on all but two at either end
     bad = tp.ieee != 0;
 #pragma unroll 1
-    for (int ly = warp + 2; ly < TY + 6; ly += NW) {
+    for (int ly = warp + 2; ly < TY + 2 * HX - 2; ly += NW) {
         const uint32_t o = (uint32_t)ly * kRow + L;
         const Flux2 b{ld2(S, o + M::X), ld2(S, o + M::Y), ld2(S, o + M::Z), ld2(S, o + M::F)};
         Flow2 v;
@@ -204,8 +209,8 @@ __device__ __forceinline__ void tile_body(const TileParams &tp, const HydroWorld
             st2(S, o + M::V, v.uy);
             st2(S, o + M::S, v.s1);
         }
-        const bool row = (unsigned)(ly - 4) < (unsigned)ih, s0 = row && in0, s1 = row && in1;
-        const uint32_t g = B + (uint32_t)(ly - 4) * (uint32_t)W;
+        const bool row = (unsigned)(ly - HX) < (unsigned)ih, s0 = row && in0, s1 = row && in1;
+        const uint32_t g = B + (uint32_t)(ly - HX) * (uint32_t)W;
         gst2<VEC>(q.h_out, g, v.hn, s0, s1);
         gst2<VEC>(q.w_out, g, evaporate2(c, v.wn), s0, s1);
         if (!FUSED) {
@@ -242,7 +247,7 @@ __device__ __forceinline__ void tile_body(const TileParams &tp, const HydroWorld
         const f2 I0 = add2(mul2_z(vx, pk(mld(u, 0), mld(v, 0)), c.Z), mul2_z(wx, pk(mld(u, 4), mld(v, 4)), c.Z));
         const f2 I1 = add2(mul2_z(vx, pk(mld(u, kRow), mld(v, kRow)), c.Z),
                            mul2_z(wx, pk(mld(u, kRow + 4), mld(v, kRow + 4)), c.Z));
-        gst2<VEC>(q.s_out, B + (uint32_t)(ly - 4) * (uint32_t)W, add2(mul2_z(vy, I0, c.Z), mul2_z(wy, I1, c.Z)), in0, in1);
+        gst2<VEC>(q.s_out, B + (uint32_t)(ly - HX) * (uint32_t)W, add2(mul2_z(vy, I0, c.Z), mul2_z(wy, I1, c.Z)), in0, in1);
     }
 }
 
@@ -257,7 +262,7 @@ __global__ __launch_bounds__(NW * 32, MINB) void k_hydro(const __grid_constant__
         int wi, tx, ty;
         tile_of(tp.p.tiles[blockIdx.x], &wi, &tx, &ty);
         s_q = hydro_world(tp.p, tp.p.worlds[wi]);
-        s_xy[0] = tx * HTX;
+        s_xy[0] = tx * (FUSED ? HTX : HTXS);
         s_xy[1] = ty * TY;
     }
     __syncthreads();
@@ -551,7 +556,7 @@ __global__ __launch_bounds__(256) void k_transport(const WorldDev *worlds, const
 // Tile variants (tecto_step_settings::hydraulicTile 1 .. 7): 56 x TY cells, NW warps, MINB blocks per SM.
 struct HydroVariant {
     int ty, nt;
-    size_t smem;
+    size_t smem, smem_split;
     void (*fused)(TileParams);
     void (*split)(TileParams);
     int ty2, nt2;  // two sub-iterations at once, 52 x ty2 cells (0: never)
@@ -559,7 +564,7 @@ struct HydroVariant {
     void (*two)(TileParams);
 };
 #define TECTO_HYDRO_VARIANT(TY, NW, MINB) \
-    TY, NW * 32, TileMem<TY>::bytes, k_hydro<TY, NW, MINB, true>, k_hydro<TY, NW, MINB, false>
+    TY, NW * 32, TileMem<TY, 4>::bytes, TileMem<TY, 2>::bytes, k_hydro<TY, NW, MINB, true>, k_hydro<TY, NW, MINB, false>
 #define TECTO_HYDRO_TWO(TY, NW, MINB) TY, NW * 32, TwoMem<TY>::bytes, k_hydro_two<TY, NW, MINB>
 const HydroVariant kHydroVariants[7] = {
     {TECTO_HYDRO_VARIANT(8, 16, 2), TECTO_HYDRO_TWO(9, 20, 1)},
@@ -580,10 +585,16 @@ int hydro_tile_attributes()
 {
     for (const HydroVariant &v : kHydroVariants) {
         TECTO_CUDA(cudaFuncSetAttribute(v.fused, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)v.smem));
-        TECTO_CUDA(cudaFuncSetAttribute(v.split, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)v.smem));
+        TECTO_CUDA(cudaFuncSetAttribute(v.split, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)v.smem_split));
         if (v.ty2) TECTO_CUDA(cudaFuncSetAttribute(v.two, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)v.smem2));
     }
     return TECTO_OK;
+}
+
+void hydro_split_extent(int variant, int *tx, int *ty)
+{
+    *tx = HTXS;
+    *ty = variant_of(variant).ty;
 }
 
 void hydro_tile_extent(int variant, bool two, int *tx, int *ty)
@@ -623,8 +634,9 @@ void launch_hydro_tile(const Batch &b, const HydroParams &p, bool fused, bool tw
         launch_chained(v.two, (unsigned)b.ntiles[TK_HYDRO_TWO], v.nt2, v.smem2, st, tp);
         return;
     }
-    const unsigned grid = (unsigned)b.ntiles[TK_HYDRO];
-    launch_chained(fused ? v.fused : v.split, grid, v.nt, v.smem, st, tp);
+    if (!fused) tp.p.tiles = b.d_tiles[TK_HYDRO_SPLIT];
+    launch_chained(fused ? v.fused : v.split, (unsigned)b.ntiles[fused ? TK_HYDRO : TK_HYDRO_SPLIT], v.nt,
+                   fused ? v.smem : v.smem_split, st, tp);
 }
 
 }  // namespace tecto

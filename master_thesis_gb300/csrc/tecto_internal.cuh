@@ -160,7 +160,7 @@ struct UpliftRefScratch {
 };
 
 // Phase work lists.
-enum TileKind { TK_RESOLVE = 0, TK_THERMAL, TK_HYDRO, TK_HYDRO_TWO, TK_CCL, TK_STATS, TK_COUNT };
+enum TileKind { TK_RESOLVE = 0, TK_THERMAL, TK_HYDRO, TK_HYDRO_TWO, TK_HYDRO_SPLIT, TK_CCL, TK_STATS, TK_COUNT };
 // CCL tiles: one warp per row of kCclTileX cells, kCclTileY rows per block
 constexpr int kCclTileX = 32, kCclTileY = 32;
 
