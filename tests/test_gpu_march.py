@@ -125,3 +125,22 @@ def test_two_sub_iterations_on_one_tile(kind, tile, W, H, iters):
         for name, f, v in zip(("height", "water", "sediment", "flux"),
                               (T.FIELD_HEIGHT, T.FIELD_WATER, T.FIELD_SEDIMENT, T.FIELD_FLUX), want):
             np.testing.assert_array_equal(w.download(f).view(np.uint32), v.view(np.uint32), err_msg=name)
+
+
+@pytest.mark.parametrize("W,H", [(59, 8), (60, 17), (61, 25), (121, 33), (2, 5), (1, 40)])
+@pytest.mark.parametrize("tile", [1, 3, 4, 5, 7, 9])
+@pytest.mark.parametrize("kind", ["tiny", "clamp", "huge"])
+def test_split_path_tiles(kind, tile, W, H):
+    """The split path's narrower halo: one column and row less and more than its tiles, worlds that wrap within
+    it, and tiles that run again in the scalar form.  dt 0.5 lets the transport reach 25 cells."""
+    s = T.baseline_settings()
+    s.step.hydraulicTile = tile
+    h, water, sed, flux = fields(kind, W, H)
+    with T.World(s, W, H, seed=1000) as w:
+        for f, a in ((T.FIELD_HEIGHT, h), (T.FIELD_WATER, water), (T.FIELD_SEDIMENT, sed), (T.FIELD_FLUX, flux)):
+            w.upload(f, a)
+        w.hydraulic(3, 0.5)
+        want = O.hydraulic(h, water, sed, flux, 3, 0.5, 1000, s)
+        for name, f, v in zip(("height", "water", "sediment", "flux"),
+                              (T.FIELD_HEIGHT, T.FIELD_WATER, T.FIELD_SEDIMENT, T.FIELD_FLUX), want):
+            np.testing.assert_array_equal(w.download(f).view(np.uint32), v.view(np.uint32), err_msg=name)
