@@ -312,27 +312,20 @@ int batch_prepare(Batch &b, cudaStream_t st)
         TECTO_CUDA(cudaMalloc(&b.table_arena, need));
         b.table_bytes = need;
     }
-    char *p = (char *)b.table_arena;
-    b.d_worlds = (WorldDev *)p;
-    p += a256(n * sizeof(WorldDev));
-    b.d_vbase = (uint32_t *)p;
-    p += a256((n + 1) * 4);
-    for (int k = 0; k < TK_COUNT; ++k) {
-        b.d_tiles[k] = (uint2 *)p;
-        p += a256(tiles[k].size() * sizeof(uint2));
-    }
-    for (int k = 0; k < ST_COUNT; ++k) {
-        b.strips[k].d = (uint4 *)p;
-        p += a256(strips[k].size() * sizeof(uint4));
-    }
-    TECTO_CUDA(cudaMemcpyAsync(b.d_worlds, table.data(), n * sizeof(WorldDev), cudaMemcpyHostToDevice, st));
-    TECTO_CUDA(cudaMemcpyAsync(b.d_vbase, vbase.data(), (n + 1) * 4, cudaMemcpyHostToDevice, st));
-    for (int k = 0; k < TK_COUNT; ++k)
-        TECTO_CUDA(cudaMemcpyAsync(b.d_tiles[k], tiles[k].data(), tiles[k].size() * sizeof(uint2),
-                                   cudaMemcpyHostToDevice, st));
-    for (int k = 0; k < ST_COUNT; ++k)
-        TECTO_CUDA(cudaMemcpyAsync(b.strips[k].d, strips[k].data(), strips[k].size() * sizeof(uint4),
-                                   cudaMemcpyHostToDevice, st));
+    // the tables as one image and one copy: a first pass 210 -> 181 us against a copy a table
+    std::vector<char> image(need);
+    size_t at = 0;
+    const auto put = [&](const void *data, size_t bytes) {
+        memcpy(image.data() + at, data, bytes);
+        char *p = (char *)b.table_arena + at;
+        at += a256(bytes);
+        return (void *)p;
+    };
+    b.d_worlds = (WorldDev *)put(table.data(), n * sizeof(WorldDev));
+    b.d_vbase = (uint32_t *)put(vbase.data(), (n + 1) * 4);
+    for (int k = 0; k < TK_COUNT; ++k) b.d_tiles[k] = (uint2 *)put(tiles[k].data(), tiles[k].size() * sizeof(uint2));
+    for (int k = 0; k < ST_COUNT; ++k) b.strips[k].d = (uint4 *)put(strips[k].data(), strips[k].size() * sizeof(uint4));
+    TECTO_CUDA(cudaMemcpyAsync(b.table_arena, image.data(), need, cudaMemcpyHostToDevice, st));
     // batch-level buffers: key/value ping-pong for `capacity` cells, the control block, then the
     // sort scratch of the current size and digit width
     const int kb = key_bits_for(total);
