@@ -234,8 +234,9 @@ static void choose_tuning(Batch &b, int *variant, int *rb, int *tvariant)
     if (*variant == 0) *variant = b.tuned_hydro;
     if (*variant == 0) {
         const bool split = 50.0f * fabsf(b.settings.step.hydraulicDt) >= 1.5f;
+        if (b.dirty) b.hydro_default[0] = b.hydro_default[1] = 0;  // of other members
         int &d = b.hydro_default[split];
-        if (b.dirty || d == 0) d = default_hydro_variant(b, split);
+        if (d == 0) d = default_hydro_variant(b, split);
         *variant = d;
     }
     *rb = b.settings.step.sortRadixBits;
