@@ -144,7 +144,8 @@ typedef struct tecto_step_settings {
                                  sub-iterations in one march of 116-column strips by blocks of 512
                                  threads, a single one in 120-column strips by blocks of 256 (the split
                                  path, 50 dt >= 1.5, runs variant 4) */
-    int thermalTile;          /* 0 = autotuner's choice, else 5 from 2^20 cells and 4 below; 1: 64x32 tiles / 1024 threads, up to 5
+    int thermalTile;          /* 0 = autotuner's choice, else 3 up to 200 000 cells, 5 from 2^20
+                                 and 4 between; 1: 64x32 tiles / 1024 threads, up to 5
                                  iterations per launch; 2: 64x16 / 512, 2 blocks per SM, up to 4;
                                  3: 64x16 / 768, 2 blocks per SM, up to 3; 4: 64x16 / 512, 3 blocks
                                  per SM, up to 2; 5: column strips of up to 60 cells marched down by

@@ -173,7 +173,9 @@ static int default_radix_bits(size_t cells)
 
 // The default thermal variant: one iteration with tiles (variant 4, two iterations a launch) against the
 // march (5), us: 512^2 5.3 / 6.5, 1024^2 11.6 / 8.4, 2048^2 37.4 / 19.2, 8192^2 570 / 224; whole steps at 1001x613
-// 430 / 435, 900x800 444 / 443, 40 worlds of 1.1 M cells 783 / 746.
+// 430 / 435, 900x800 444 / 443, 40 worlds of 1.1 M cells 783 / 746.  Variant 3 (three iterations a launch, more
+// warps a tile) against 4 in whole steps: 64^2 112.6 / 115.9, 256^2 126.4 / 129.0, 384^2 162.2 / 165.0, 512^2
+// 220.3 / 220.2, 600^2 259 / 254.
 // The default hydraulic variant: the one whose two sub-iterations a model of the measured shapes puts lowest.
 // Tiles run in waves of 152 SMs x the tiles an SM holds, and a wave's time depends on how many it holds; the
 // march's blocks take equal shares of the strips' rows (with what a strip's start costs, k_hydro_march.cu), at
@@ -229,7 +231,10 @@ static void choose_tuning(Batch &b, int *variant, int *rb, int *tvariant)
 {
     *tvariant = thermal_variant_for(b.settings);
     if (*tvariant == 0) *tvariant = b.tuned_thermal;
-    if (*tvariant == 0) *tvariant = b.total >= kThermalMarchMinCells ? kThermalMarchVariant : kDefaultThermalVariant;
+    if (*tvariant == 0)
+        *tvariant = b.total >= kThermalMarchMinCells ? kThermalMarchVariant
+                    : b.total <= kThermalSmallCells  ? kThermalSmallVariant
+                                                     : kDefaultThermalVariant;
     *variant = hydro_variant_for(b.settings);
     if (*variant == 0) *variant = b.tuned_hydro;
     if (*variant == 0) {

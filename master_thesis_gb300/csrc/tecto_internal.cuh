@@ -397,6 +397,8 @@ constexpr int kMarchInner = 120;                 // interior columns of one shar
 constexpr int kThermalInner = 60;                // interior columns of one thermal strip (64 with the halo)
 constexpr int kThermalVariantCount = 5;
 constexpr int kDefaultThermalVariant = 4;        // 64 x 16 cells, 512 threads, 2 iterations per launch
+constexpr int kThermalSmallVariant = 3;           // 768 threads a tile, up to 3 iterations per launch
+constexpr size_t kThermalSmallCells = 200000;     // cells up to which that is the default
 constexpr size_t kThermalMarchMinCells = 1 << 20;  // cells from which the thermal march is the default
 constexpr int kThermalMarchVariant = 5;          // warps marching down column strips, one iteration per launch
 int thermal_variant_for(const tecto_settings &s);  // 0 when the settings leave the choice open
