@@ -640,6 +640,10 @@ int tecto_selftest_div_var(const float *a, const float *b, float *out, size_t n,
  * receives the mismatches per exponent field: bad[e] for the reciprocal, bad[256 + e] for the
  * square root. */
 int tecto_selftest_rcp_sqrt(unsigned long long *bad, tecto_stream_t stream);
+/* Self-test of a phase's work list (host only): the tiles of tile_x x tile_y cells of a width x height world
+ * that is member `world` of a batch, encoded and decoded as the kernels do; *bad receives how many are
+ * missing, repeated or decoded to another world or place. */
+int tecto_selftest_tiles(int width, int height, int world, int tile_x, int tile_y, unsigned long long *bad);
 const char *tecto_last_error_string(void);
 const char *tecto_version(void);
 

@@ -21,17 +21,21 @@ void drop_graphs(Batch &b)
     }
 }
 
+// the tiles of a W x H world, row by row
+void add_tiles(int world, int W, int H, int tx, int ty, std::vector<uint2> &out)
+{
+    const int nx = (W + tx - 1) / tx, ny = (H + ty - 1) / ty;
+    for (int y = 0; y < ny; ++y)
+        for (int x = 0; x < nx; ++x) out.push_back(tile_pack(world, x, y));
+}
+
 void build_tiles(const Batch &b, int kind, std::vector<uint2> &out)
 {
     int tx = 0, ty = 0;
     tile_extent(kind, kind == TK_THERMAL ? b.thermal_variant : b.hydro_variant, &tx, &ty);
     out.clear();
-    for (size_t wi = 0; wi < b.members.size(); ++wi) {
-        const tecto_world *w = b.members[wi];
-        const int nx = (w->W + tx - 1) / tx, ny = (w->H + ty - 1) / ty;
-        for (int y = 0; y < ny; ++y)
-            for (int x = 0; x < nx; ++x) out.push_back(make_uint2((unsigned)wi, ((unsigned)y << 16) | (unsigned)x));
-    }
+    for (size_t wi = 0; wi < b.members.size(); ++wi)
+        add_tiles((int)wi, b.members[wi]->W, b.members[wi]->H, tx, ty, out);
 }
 
 // every member's columns cut into strips of `inner`
@@ -462,6 +466,23 @@ int batch_step_graph(Batch &b, int nsteps, cudaStream_t st, bool use_graph)
 using namespace tecto;
 
 extern "C" {
+
+int tecto_selftest_tiles(int width, int height, int world, int tile_x, int tile_y, unsigned long long *bad)
+{
+    if (width < 1 || height < 1 || (long long)width * height > 1ll << 30 || world < 0 || world >= kMaxBatchWorlds ||
+        tile_x < 1 || tile_y < 1 || !bad)
+        return TECTO_ERR_INVALID;
+    std::vector<uint2> tiles;
+    add_tiles(world, width, height, tile_x, tile_y, tiles);
+    const size_t nx = (size_t)((width + tile_x - 1) / tile_x), ny = (size_t)((height + tile_y - 1) / tile_y);
+    *bad = tiles.size() > nx * ny ? tiles.size() - nx * ny : nx * ny - tiles.size();
+    for (size_t i = 0; i < tiles.size(); ++i) {
+        int w, x, y;
+        tile_of(tiles[i], &w, &x, &y);
+        if (w != world || (size_t)x != i % nx || (size_t)y != i / nx) *bad += 1;
+    }
+    return TECTO_OK;
+}
 
 int tecto_batch_create(tecto_batch **out)
 {

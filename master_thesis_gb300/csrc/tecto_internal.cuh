@@ -193,7 +193,7 @@ struct Batch {
     // device tables
     WorldDev *d_worlds = nullptr;
     uint32_t *d_vbase = nullptr;             // [n + 1] ascending virtual bases, last = total
-    uint2 *d_tiles[TK_COUNT] = {};           // (world, ty << 16 | tx)
+    uint2 *d_tiles[TK_COUNT] = {};           // tile_pack
     int ntiles[TK_COUNT] = {};
     StripTable strips[ST_COUNT];             // column strips of the marching kernels
     void *table_arena = nullptr;
@@ -345,11 +345,22 @@ __device__ __forceinline__ int find_world(const uint32_t *vbase, int n, uint32_t
     return lo;
 }
 
-__device__ __forceinline__ void tile_of(uint2 t, int *world, int *tx, int *ty)
+// An item of a work list: tile (tx, ty) of member `world`.  A world has up to 2^30 cells and any sides, so
+// that the smallest tiles (32 columns, 4 rows) come to 2^25 columns and 2^28 rows of tiles.
+static_assert(kMaxBatchWorlds <= 1 << 10, "tile_pack: ten bits for the world");
+__host__ __device__ __forceinline__ uint2 tile_pack(int world, int tx, int ty)
 {
-    *world = (int)t.x;
-    *tx = (int)(t.y & 0xffffu);
-    *ty = (int)(t.y >> 16);
+    uint2 t;
+    t.x = (unsigned)ty | (unsigned)(world & 15) << 28;
+    t.y = (unsigned)tx | (unsigned)(world >> 4) << 26;
+    return t;
+}
+
+__host__ __device__ __forceinline__ void tile_of(uint2 t, int *world, int *tx, int *ty)
+{
+    *world = (int)(t.x >> 28 | t.y >> 26 << 4);
+    *tx = (int)(t.y & 0x3ffffffu);
+    *ty = (int)(t.x & 0xfffffffu);
 }
 
 // ---- batch management (tecto_batch.cu) -----------------------------------------------------
