@@ -242,7 +242,7 @@ static void choose_tuning(Batch &b, int *variant, int *rb, int *tvariant)
     *variant = hydro_variant_for(b.settings);
     if (*variant == 0) *variant = b.tuned_hydro;
     if (*variant == 0) {
-        const bool split = 50.0f * fabsf(b.settings.step.hydraulicDt) >= 1.5f;
+        const bool split = !hydro_fused(b, b.settings.step.hydraulicDt);
         if (b.dirty) b.hydro_default[0] = b.hydro_default[1] = 0;  // of other members
         int &d = b.hydro_default[split];
         if (d == 0) d = default_hydro_variant(b, split);
@@ -256,7 +256,11 @@ int batch_prepare(Batch &b, cudaStream_t st)
 {
     if (b.dirty && !b.members.empty()) {  // membership changed: cached autotuner choice, if any
         size_t cells = 0;
-        for (const tecto_world *w : b.members) cells += w->N;
+        b.long_side = 0;
+        for (const tecto_world *w : b.members) {
+            cells += w->N;
+            b.long_side = std::max(b.long_side, std::max(w->W, w->H));
+        }
         b.total = cells;
         // A choice of another size says less than the defaults' model: taken from an octave away at most in all.
         // (2048^2 with the tiles that 1024^2 was tuned to 1980 us a step, with the default 1490.)

@@ -184,6 +184,7 @@ struct Batch {
     size_t total = 0;                        // sum of member cells
     int hydro_variant = 0;                   // tile variant the TK_HYDRO list was built for
     int hydro_default[2] = {0, 0};           // untuned choice (split path: [1]), 0 until it is made
+    int long_side = 0;                       // the longest side of a member
     int thermal_variant = 0;                 // tile variant the TK_THERMAL list was built for
     int tuned_thermal = 0;
     int tuned_hydro = 0, tuned_rb = 0;       // autotuner's choices (0 = none), used when the
@@ -398,6 +399,7 @@ void uplift_ref_release(Batch &b);
 void gaussian_weights(float sigma, int radius, float *out);
 int ensure_kernel_attributes();
 int hydro_variant_for(const tecto_settings &s);  // 0 when the settings leave the choice open
+bool hydro_fused(const Batch &b, float dt);      // whether a sub-iteration's transport is fused into it
 constexpr int kDefaultRadixBits = 8;
 constexpr int kHydroVariantCount = 9;
 constexpr int kDefaultHydroVariant = 4;          // 56 x 24 cells: where the autotuner starts from

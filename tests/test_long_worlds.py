@@ -59,3 +59,11 @@ def check(W, H, tile, thermal_tile, iters, dt):
                                                (3700000, 2, 9, 1, 0.02), (2, 1060000, 4, 1, 0.02)])
 def test_more_tiles_a_side_than_16_bits(W, H, tile, iters, dt):
     check(W, H, tile, 4, iters, dt)
+
+
+# positions above 2^22, where the fused kernels' floors would end: the tiles, the march, and two at once
+@pytest.mark.gpu
+@pytest.mark.parametrize("W,H,tile,iters", [(4250000, 2, 4, 2), (4250000, 2, 7, 1), (2, 4250000, 9, 2), (4194304, 4, 9, 1),
+                                            (4, 4194250, 0, 2)])
+def test_sides_above_two_to_the_22(W, H, tile, iters):
+    check(W, H, tile, 0, iters, 0.02)
