@@ -77,7 +77,7 @@ __device__ __forceinline__ int evidence_category(const uint8_t *bm, uint8_t A, u
     const float mnH = cond ? hA : hB, mxH = cond ? hB : hA;
     const uint32_t idx = tri_index(mn, mx);
     *pair = idx;
-    const uint32_t packed = __ldg(bm + idx);
+    const uint32_t packed = bm[idx];
     if ((packed & 1u) && ((packed >> 4) & (uint32_t)(0x0F < cooldown))) return -1;
     const bool minCont = mnH >= thr, maxCont = mxH >= thr;
     if (minCont && maxCont) return 4;

@@ -77,18 +77,20 @@ enum Role { kAlone = 0, kFirstOfTwo, kSecondOfTwo };
 static_assert(kPairThreads / 64 == kPairRows && kHydroMarchSmem % 16 == 0, "march: one pair per thread and phase");
 
 // Loads that stay where they are written (the march's prefetches): two cells of one row; VEC, adjacent
-// and 8-byte aligned (even world width), else `step` apart; and one cell's flux.
+// and 8-byte aligned (even world width), else `step` apart; and one cell's flux.  Not the read-only path: a march
+// is resident while the kernel ahead of it still writes these fields, and kernel_wait() makes them visible to
+// ordinary loads.
 template <bool VEC>
 __device__ __forceinline__ f2 gld2(const float *base, uint32_t i, uint32_t step)
 {
     if (VEC) {
         f2 v;
-        asm volatile("ld.global.nc.b64 %0, [%1];" : "=l"(v) : "l"(gaddr64(base, i)));
+        asm volatile("ld.global.b64 %0, [%1];" : "=l"(v) : "l"(gaddr64(base, i)));
         return v;
     }
     float x, y;
-    asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(x) : "l"(gaddr64(base, i)));
-    asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(y) : "l"(gaddr64(base, i + step)));
+    asm volatile("ld.global.f32 %0, [%1];" : "=f"(x) : "l"(gaddr64(base, i)));
+    asm volatile("ld.global.f32 %0, [%1];" : "=f"(y) : "l"(gaddr64(base, i + step)));
     return pk(x, y);
 }
 // the fluxes of two cells: VEC, one 32-byte access (a whole sector: two 16-byte halves of it, loaded or
@@ -97,15 +99,15 @@ template <bool VEC>
 __device__ __forceinline__ void gld_flux(const float4 *base, uint32_t i, uint32_t step, float4 &a, float4 &b)
 {
     if (VEC) {
-        asm volatile("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                      : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
                      : "l"(gaddr64(base, i)));
         return;
     }
-    asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];"
+    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];"
                  : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w)
                  : "l"(gaddr64(base, i)));
-    asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];"
+    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];"
                  : "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
                  : "l"(gaddr64(base, i + step)));
 }

@@ -56,7 +56,7 @@ __device__ __forceinline__ uint32_t pair_type(const uint8_t *bm, uint8_t A, uint
     const bool cond = A < B;
     const uint8_t mn = cond ? A : B, mx = cond ? B : A;
     const float mnH = cond ? hA : hB, mxH = cond ? hB : hA;
-    const uint32_t packed = __ldg(bm + tri_index(mn, mx));
+    const uint32_t packed = bm[tri_index(mn, mx)];
     const uint32_t hasType = packed & 1u, type = (packed >> 1) & 1u, pol = (packed >> 3) & 1u;
     uint32_t out = 0;
     if (hasType && type == 0) {
@@ -91,7 +91,7 @@ __device__ __forceinline__ float diverge_cell(const ResolveParams &p, const Reso
         const uint8_t mn = prev < oppId ? prev : oppId;
         const uint8_t mx = prev < oppId ? oppId : prev;
         const uint32_t bit = tri_index(mn, mx);
-        nid = (__ldg(w.div_bitmap + bit / 32u) & (1u << (bit % 32u))) ? mn : mx;
+        nid = (w.div_bitmap[bit / 32u] & (1u << (bit % 32u))) ? mn : mx;
         atomicOr(w.has_div + bit / 32u, 1u << (bit % 32u));
     }
     const float noise = simplex3((float)x, (float)y, (float)iteration, 0.01f, (int)seed);

@@ -78,9 +78,8 @@ __device__ __forceinline__ void copy_row(uint32_t dst, const float *row, uint32_
 // Rows [r0, r1) of the strip with interior columns [x0, x0 + iw).  S: the warp's ring, its guard before it.
 // Returns the lane's largest slope sum (MODE > 0).
 template <bool VEC, int MODE>
-__device__ __forceinline__ float tmarch_piece(const TMarchParams &tp, const float *__restrict__ hin,
-                                             float *__restrict__ hout, int W, int H, char *S, int x0, int iw, int r0,
-                                             int r1)
+__device__ __forceinline__ float tmarch_piece(const TMarchParams &tp, const float *hin, float *hout, int W, int H,
+                                             char *S, int x0, int iw, int r0, int r1)
 {
     const uint32_t Wu = (uint32_t)W, N = Wu * (uint32_t)H;
     const int lane = (int)threadIdx.x & 31, col = 2 * lane;

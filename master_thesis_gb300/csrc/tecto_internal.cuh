@@ -269,7 +269,9 @@ int cuda_fail(cudaError_t e, const char *what);
 // completed and is visible.  Every thread of such a kernel calls it before it touches memory that a kernel
 // writes, so completion is transitive along the stream; before it a kernel may read its parameters and the
 // batch's tables (worlds, tiles, strips, virtual bases), which batch_prepare has synchronised.  A launch
-// behind anything else (a copy, a kernel launched the ordinary way) waits for all of it.
+// behind anything else (a copy, a kernel launched the ordinary way) waits for all of it.  What the kernels of a
+// step write is read with ordinary loads, never through the read-only path (ld.global.nc, __ldg, const
+// __restrict__): that asks for memory that nobody writes while the kernel is resident.
 //
 // kernel_release() lets the next kernel's blocks be placed once every block of this one has called it (or
 // ended).  The tile kernels call it before their last phase: placed earlier, the next kernel's blocks fill
