@@ -24,7 +24,6 @@ namespace {
 
 constexpr int kWarps = kSortThreads / 32;
 constexpr int kLookAhead = 8;  // predecessor tiles read per look-back round
-constexpr int kDoneCounter = 8;  // word of SortScratch::counters that counts finished histogram blocks
 
 template <int RB>
 struct Digits {
@@ -435,12 +434,12 @@ int run_sort_rb(const SortArgs &a, const SortScratch &scr, cudaStream_t st, int 
     const uint32_t *kin = a.keys_in, *vin = a.vals_in;
     if (gen) {
         launch_chained(k_sort_hist<true, RB>, hist_blocks, 256, 0, st, g, nullptr, a.n, passes, scr.hist, a.keys[1],
-                       scr.counters + kDoneCounter);
+                       scr.counters + kSortDoneCounter);
         kin = a.keys[1];
         vin = nullptr;
     } else {
         launch_chained(k_sort_hist<false, RB>, hist_blocks, 256, 0, st, g, a.keys_in, a.n, passes, scr.hist, nullptr,
-                       scr.counters + kDoneCounter);
+                       scr.counters + kSortDoneCounter);
     }
     int half = 0;
     for (int p = 0; p < passes; ++p) {
@@ -487,7 +486,7 @@ size_t sort_scratch_bytes(size_t n, int key_bits, int rb)
     const size_t passes = (size_t)sort_passes_for(key_bits, rb);
     const size_t tiles = (n + kSortTile - 1) / kSortTile;
     const size_t R = (size_t)1 << rb;
-    return align256(passes * R * 4) + align256(passes * tiles * R * 4) + align256(kMaxSortPasses * 4) +
+    return align256(passes * R * 4) + align256(passes * tiles * R * 4) + align256(kSortCounters * 4) +
            align256(4);
 }
 
@@ -505,7 +504,7 @@ void sort_scratch_carve(void *base, size_t n, int key_bits, int rb, SortScratch 
     out->status = (uint32_t *)p;
     p += align256((size_t)passes * tiles * R * 4);
     out->counters = (uint32_t *)p;
-    p += align256(kMaxSortPasses * 4);
+    p += align256(kSortCounters * 4);
     out->error = (uint32_t *)p;
 }
 
@@ -514,7 +513,7 @@ size_t sort_clear_bytes(const SortScratch &scr, size_t n)
 {
     const size_t R = (size_t)1 << scr.radix_bits, tiles = (n + kSortTile - 1) / kSortTile;
     return align256((size_t)scr.passes * R * 4) + align256((size_t)scr.passes * tiles * R * 4) +
-           align256(kMaxSortPasses * 4);
+           align256(kSortCounters * 4);
 }
 
 int run_sort_clear(const SortScratch &scr, size_t n, cudaStream_t st)

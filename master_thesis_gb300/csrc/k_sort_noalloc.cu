@@ -18,7 +18,7 @@ constexpr size_t a256(size_t x) { return (x + 255) & ~(size_t)255; }
 // sort_scratch_bytes(kMaxPairs, 32, 8): histograms, look-back status (4 passes), counters, error word
 constexpr size_t kSortPart = a256((size_t)kMaxSortPasses * 256 * 4) +
                              a256((size_t)kMaxSortPasses * ((kMaxPairs + kSortTile - 1) / kSortTile) * 256 * 4) +
-                             a256((size_t)kMaxSortPasses * 4) + a256(4);
+                             a256((size_t)kSortCounters * 4) + a256(4);
 constexpr size_t kHalf = a256(kMaxPairs * sizeof(uint32_t));
 constexpr size_t kScratchBytes = kSortPart + 2 * kHalf;
 

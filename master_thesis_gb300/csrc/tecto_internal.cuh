@@ -25,6 +25,9 @@ constexpr int kSortThreads = 256;
 constexpr int kSortItems = kSortTile / kSortThreads;
 constexpr int kMaxSortPasses = 4;               // 32-bit keys, 8-bit digits
 constexpr int kMaxRadixBits = 11;              // widest sort digit
+constexpr int kSortDoneCounter = 8;             // sort counters: a tile counter a pass, and the finished histogram blocks
+constexpr int kSortCounters = kSortDoneCounter + 1;
+static_assert(kSortDoneCounter >= kMaxSortPasses, "sort counters: one word a pass before the last");
 constexpr int kMaxBatchWorlds = 1024;           // worlds per batch (world lookup table in smem)
 
 // Status word of the decoupled look-back: 2 flag bits + 30 value bits.
@@ -68,7 +71,7 @@ struct BatchCtl {
 struct SortScratch {
     uint32_t *hist;      // [passes][2^radix_bits] digit counts -> exclusive digit starts
     uint32_t *status;    // [passes][tiles][2^radix_bits] look-back words
-    uint32_t *counters;  // [passes] dynamic tile counters
+    uint32_t *counters;  // [kSortCounters]: dynamic tile counters by pass, finished histogram blocks
     uint32_t *error;     // error flag word
     int passes;
     int tiles;
