@@ -42,6 +42,7 @@ constexpr int kTAhead = 4;              // groups copied ahead of the march
 constexpr uint32_t kTMask = kTRows * kTRow - 1;
 constexpr uint32_t kTGuard = 16;        // an edge lane reads one cell past a row's end
 constexpr uint32_t kTWarpSmem = kTGuard + kTRows * kTRow + kTGuard;
+static_assert(kTWarpSmem % 16 == 0, "zeroed by 16 bytes");
 static_assert(kThermalInner == 64 - 4, "strips: interior plus a halo of 2 each side");
 static_assert(kTGroup * (kTAhead + 1) <= (int)kTRows, "no row is overwritten before its last reader is done");
 
@@ -222,6 +223,11 @@ __global__ __launch_bounds__(kTWarps * 32, 5) void k_thermal_march(const __grid_
     const int lane = (int)threadIdx.x & 31, wib = (int)threadIdx.x >> 5;
     const int gw = (int)blockIdx.x * kTWarps + wib;
     char *S = s_ring[wib] + kTGuard;
+    // Columns 0 and 63, which no stored height needs, read past their row: their sums count for the piece's largest
+    // and would send it through the scalar form by what an earlier kernel left there.
+    for (uint32_t i = lane; i < kTWarpSmem / 16; i += 32)
+        reinterpret_cast<float4 *>(s_ring[wib])[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    __syncwarp();
     // this warp's strip-rows [a, b); each strip counts kTWarmRows more before its first, which a warp that
     // starts another strip spends on it
     const unsigned long long all = tp.rows + (unsigned long long)tp.nstrips * kTWarmRows;
