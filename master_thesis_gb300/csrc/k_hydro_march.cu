@@ -47,7 +47,6 @@ namespace {
 struct PairParams {
     StripParams sp;
     PairConst c;
-    int ieee;  // the scalar form throughout: a pipe length outside [2^-32, 2^32] or dt < 0
 };
 
 constexpr int kPairThreads = 256;
@@ -416,7 +415,7 @@ __global__ __launch_bounds__(kPairThreads, 2) void k_hydro_march(const __grid_co
         if (b0 <= first) break;
         const int r0 = a > first ? (int)(a - first) : 0, r1 = (int)((b0 < last ? b0 : last) - first);
         const int x0 = (int)d.y, iw = (int)d.z;
-        if (pp.ieee || s_q.H < kPairRows) {
+        if (s_q.H < kPairRows) {
             march_ieee(pp, s_q, S, x0, iw, r0, r1);
         } else {
             if (s_q.W & 1) march_piece<false, false, kAlone>(sp.p, pp.c, s_q, S, x0, iw, r0, r1, s_flag);
@@ -524,7 +523,7 @@ int hydro_march_attributes()
     return TECTO_OK;
 }
 
-// `two`: two sub-iterations at once, which needs hydro_march_two's parameters and sp of ST_HYDRO_TWO.
+// Parameters that hydro_packed takes.  `two`: two sub-iterations at once, with the strips of ST_HYDRO_TWO.
 void launch_hydro_march(const Batch &b, StripParams sp, bool two, cudaStream_t st)
 {
     const void *kern = two ? (const void *)k_hydro_march_pair : (const void *)k_hydro_march;
@@ -533,11 +532,8 @@ void launch_hydro_march(const Batch &b, StripParams sp, bool two, cudaStream_t s
     sp.nwarps = march_blocks(b, sp.rows, kern, threads, smem, kHydroMarchMinRows);
     PairParams pp{};
     pp.sp = sp;
-    pp.ieee = !hydro_march_two(sp.p);
     pp.c = pair_const(sp.p);
     launch_chained(two ? k_hydro_march_pair : k_hydro_march, (unsigned)sp.nwarps, threads, smem, st, pp);
 }
-
-bool hydro_march_two(const HydroParams &p) { return p.fastL != 0 && p.dt >= 0.0f; }
 
 }  // namespace tecto

@@ -48,7 +48,7 @@ struct TileMem {
 struct TileParams {
     HydroParams p;
     PairConst c;
-    int ieee;  // the scalar form throughout: a pipe length outside [2^-32, 2^32] or dt < 0
+    int ieee;  // the flux phase in scalar form: a pipe length outside [2^-32, 2^32] or dt < 0
 };
 
 __device__ __forceinline__ void cp8(uint32_t dst, const void *src)
@@ -70,28 +70,38 @@ __device__ __forceinline__ void cp_pair(uint32_t dst, const float *row, uint32_t
     }
 }
 
-// The flux phase in scalar form (old fluxes from HBM).
-template <int TY, int NW, int HX>
+// The flux phase in scalar form.  FIRST: nothing has run on the tile, and the old fluxes lie where the loads put
+// them; else the packed run replaced them, and they come from HBM again.
+template <int TY, int NW, int HX, bool FIRST>
 __device__ __noinline__ void flux_rows_ieee(const HydroParams &p, const HydroWorld &q, char *S, int x0, int y0)
 {
     using M = TileMem<TY, HX>;
-    const int lane = (int)threadIdx.x & 31, warp = (int)threadIdx.x >> 5;
+    const int lane = (int)threadIdx.x & 31, warp = (int)threadIdx.x >> 5, lx = 2 * lane, gx = x0 - HX + lx;
     for (int ly = warp + 1; ly < TY + 2 * HX - 1; ly += NW) {
-#pragma unroll 1
-        for (int j = 0; j < 2; ++j) {
-            const int lx = 2 * lane + j, gx = x0 - HX + lx, gy = y0 - HX + ly;
-            const uint32_t o = (uint32_t)ly * kRow + (uint32_t)lx * 4u;
-            const float4 f = q.f_in[cidx(gx, gy, q.W, q.H)];
-            const float4 v = flux_ieee(p, f, mld(S, o + M::H), mld(S, o + M::W), mld(S, o + M::H - 4), mld(S, o + M::W - 4),
-                                       mld(S, o + M::H + kRow), mld(S, o + M::W + kRow), mld(S, o + M::H + 4),
-                                       mld(S, o + M::W + 4), mld(S, o + M::H - kRow), mld(S, o + M::W - kRow));
-            mst(S, o + M::X, v.x);
-            mst(S, o + M::Y, v.y);
-            mst(S, o + M::Z, v.z);
-            mst(S, o + M::F, v.w);
-            if (lx >= HX && lx < 64 - HX && ly >= HX && ly < TY + HX && gx < q.W && gy < q.H)
-                q.f_out[(uint32_t)gy * (uint32_t)q.W + (uint32_t)gx] = v;
+        const int gy = y0 - HX + ly;
+        const uint32_t o = (uint32_t)ly * kRow + (uint32_t)lx * 4u;
+        float4 f[2], v[2];
+        if (FIRST) {
+            const f2 a = ld2(S, o + M::X), b = ld2(S, o + M::Y), d = ld2(S, o + M::Z), e = ld2(S, o + M::F);
+            f[0] = make_float4(lo(a), hi(a), lo(b), hi(b));
+            f[1] = make_float4(lo(d), hi(d), lo(e), hi(e));
+        } else {
+            f[0] = q.f_in[cidx(gx, gy, q.W, q.H)];
+            f[1] = q.f_in[cidx(gx + 1, gy, q.W, q.H)];
         }
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const uint32_t c = o + 4u * j;
+            v[j] = flux_ieee(p, f[j], mld(S, c + M::H), mld(S, c + M::W), mld(S, c + M::H - 4), mld(S, c + M::W - 4),
+                             mld(S, c + M::H + kRow), mld(S, c + M::W + kRow), mld(S, c + M::H + 4),
+                             mld(S, c + M::W + 4), mld(S, c + M::H - kRow), mld(S, c + M::W - kRow));
+            if (lx + j >= HX && lx + j < 64 - HX && ly >= HX && ly < TY + HX && gx + j < q.W && gy < q.H)
+                q.f_out[(uint32_t)gy * (uint32_t)q.W + (uint32_t)(gx + j)] = v[j];
+        }
+        st2(S, o + M::X, pk(v[0].x, v[1].x));
+        st2(S, o + M::Y, pk(v[0].y, v[1].y));
+        st2(S, o + M::Z, pk(v[0].z, v[1].z));
+        st2(S, o + M::F, pk(v[0].w, v[1].w));
     }
 }
 
@@ -168,32 +178,37 @@ __device__ __forceinline__ void tile_body(const TileParams &tp, const HydroWorld
     __syncthreads();
 
     // flux on all rows but the first and the last
-    bool bad = tp.ieee != 0;
-#pragma unroll 1
-    for (int ly = warp + 1; ly < TY + 2 * HX - 1; ly += NW) {
-        const uint32_t o = (uint32_t)ly * kRow + L;
-        const f2 f0 = ld2(S, o + M::X), f1 = ld2(S, o + M::Y), f2_ = ld2(S, o + M::Z), f3 = ld2(S, o + M::F);
-        Flux2 v;
-        const bool b = flux_pair(c, ld2(S, o + M::H), ld2(S, o + M::W), mld(S, o + M::H - 4), mld(S, o + M::H + 8),
-                                 mld(S, o + M::W - 4), mld(S, o + M::W + 8), ld2(S, o + M::H + kRow),
-                                 ld2(S, o + M::W + kRow), ld2(S, o + M::H - kRow), ld2(S, o + M::W - kRow),
-                                 make_float4(lo(f0), hi(f0), lo(f1), hi(f1)), make_float4(lo(f2_), hi(f2_), lo(f3), hi(f3)),
-                                 live_f, v);
-        bad = bad || b;
-        st2(S, o + M::X, v.x);
-        st2(S, o + M::Y, v.y);
-        st2(S, o + M::Z, v.z);
-        st2(S, o + M::F, v.w);
-        const bool row = (unsigned)(ly - HX) < (unsigned)ih;
-        gst_flux<VEC>(q.f_out, B + (uint32_t)(ly - HX) * (uint32_t)W, v.x, v.y, v.z, v.w, row && in0, row && in1);
-    }
-    if (__syncthreads_or(bad)) {
-        flux_rows_ieee<TY, NW, HX>(tp.p, q, S, x0, y0);
+    bool bad = false;
+    if (tp.ieee) {
+        flux_rows_ieee<TY, NW, HX, true>(tp.p, q, S, x0, y0);
         __syncthreads();
+    } else {
+#pragma unroll 1
+        for (int ly = warp + 1; ly < TY + 2 * HX - 1; ly += NW) {
+            const uint32_t o = (uint32_t)ly * kRow + L;
+            const f2 f0 = ld2(S, o + M::X), f1 = ld2(S, o + M::Y), f2_ = ld2(S, o + M::Z), f3 = ld2(S, o + M::F);
+            Flux2 v;
+            const bool b = flux_pair(c, ld2(S, o + M::H), ld2(S, o + M::W), mld(S, o + M::H - 4), mld(S, o + M::H + 8),
+                                     mld(S, o + M::W - 4), mld(S, o + M::W + 8), ld2(S, o + M::H + kRow),
+                                     ld2(S, o + M::W + kRow), ld2(S, o + M::H - kRow), ld2(S, o + M::W - kRow),
+                                     make_float4(lo(f0), hi(f0), lo(f1), hi(f1)), make_float4(lo(f2_), hi(f2_), lo(f3), hi(f3)),
+                                     live_f, v);
+            bad = bad || b;
+            st2(S, o + M::X, v.x);
+            st2(S, o + M::Y, v.y);
+            st2(S, o + M::Z, v.z);
+            st2(S, o + M::F, v.w);
+            const bool row = (unsigned)(ly - HX) < (unsigned)ih;
+            gst_flux<VEC>(q.f_out, B + (uint32_t)(ly - HX) * (uint32_t)W, v.x, v.y, v.z, v.w, row && in0, row && in1);
+        }
+        if (__syncthreads_or(bad)) {
+            flux_rows_ieee<TY, NW, HX, false>(tp.p, q, S, x0, y0);
+            __syncthreads();
+        }
     }
 
     // flow, sediment exchange and evaporation on all but two at either end
-    bad = tp.ieee != 0;
+    bad = false;
 #pragma unroll 1
     for (int ly = warp + 2; ly < TY + 2 * HX - 2; ly += NW) {
         const uint32_t o = (uint32_t)ly * kRow + L;
@@ -607,7 +622,7 @@ void hydro_tile_extent(int variant, bool two, int *tx, int *ty)
 
 bool hydro_tile_two(const Batch &b, const HydroParams &p)
 {
-    return b.hydro_variant < kHydroStripVariant && variant_of(b.hydro_variant).ty2 && hydro_march_two(p);
+    return b.hydro_variant < kHydroStripVariant && variant_of(b.hydro_variant).ty2 && hydro_packed(p);
 }
 
 void launch_rain(const Batch &b, float dt, float rainfall, cudaStream_t st)
@@ -628,7 +643,7 @@ void launch_hydro_tile(const Batch &b, const HydroParams &p, bool fused, bool tw
     TileParams tp{};
     tp.p = p;
     tp.c = pair_const(p);
-    tp.ieee = p.fastL == 0 || !(p.dt >= 0.0f);
+    tp.ieee = !hydro_packed(p);
     if (two) {
         tp.p.tiles = b.d_tiles[TK_HYDRO_TWO];
         launch_chained(v.two, (unsigned)b.ntiles[TK_HYDRO_TWO], v.nt2, v.smem2, st, tp);
