@@ -293,7 +293,7 @@ void launch_thermal_march(const Batch &b, const ThermalParams &p, cudaStream_t s
     int e = 0;
     const bool pow2 = p.A > 0.0f && std::frexp(p.A, &e) == 0.5f && e >= -16 && e <= 16;
     tp.nrA = pk_host(pow2 ? -1.0f / p.A : 0.0f);
-    if (!(p.thr >= 0x1p-32f) || !p.pos_flows) launch_mode<0>(b, tp, st);
+    if (!p.packed) launch_mode<0>(b, tp, st);
     else if (pow2 && p.S == 1.0f) launch_mode<2>(b, tp, st);
     else launch_mode<1>(b, tp, st);
 }

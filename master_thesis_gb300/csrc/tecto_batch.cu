@@ -180,6 +180,9 @@ static int default_radix_bits(size_t cells)
 // 430 / 435, 900x800 444 / 443, 40 worlds of 1.1 M cells 783 / 746.  Variant 3 (three iterations a launch, more
 // warps a tile) against 4 in whole steps: 64^2 112.6 / 115.9, 256^2 126.4 / 129.0, 384^2 162.2 / 165.0, 512^2
 // 220.3 / 220.2, 600^2 259 / 254.
+// Parameters that the march's packed forms do not take (a threshold below 2^-32, a negative amplitude): ten
+// iterations with tiles / the march, threshold 0 and 1e-12, us: 1024^2 115 / 156 and 104 / 139, 1500x1100 174 / 194
+// and 157 / 171, 2048^2 407 / 402 and 363 / 348, 4096^2 1616 / 1347 and 1458 / 1162.
 // The default hydraulic variant: the one whose two sub-iterations a model of the measured shapes puts lowest.
 // Tiles run in waves of 152 SMs x the tiles an SM holds, and a wave's time depends on how many it holds; the
 // march's blocks take equal shares of the strips' rows (with what a strip's start costs, k_hydro_march.cu), at
@@ -235,10 +238,12 @@ static void choose_tuning(Batch &b, int *variant, int *rb, int *tvariant)
 {
     *tvariant = thermal_variant_for(b.settings);
     if (*tvariant == 0) *tvariant = b.tuned_thermal;
-    if (*tvariant == 0)
-        *tvariant = b.total >= kThermalMarchMinCells ? kThermalMarchVariant
-                    : b.total <= kThermalSmallCells  ? kThermalSmallVariant
-                                                     : kDefaultThermalVariant;
+    if (*tvariant == 0) {
+        const size_t march = thermal_packed(b.settings.kernel) ? kThermalMarchMinCells : kThermalScalarMarchMinCells;
+        *tvariant = b.total >= march                ? kThermalMarchVariant
+                    : b.total <= kThermalSmallCells ? kThermalSmallVariant
+                                                    : kDefaultThermalVariant;
+    }
     *variant = hydro_variant_for(b.settings);
     if (*variant == 0) *variant = b.tuned_hydro;
     if (*variant == 0) {

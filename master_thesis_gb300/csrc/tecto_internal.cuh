@@ -419,7 +419,9 @@ constexpr int kThermalSmallVariant = 3;           // 768 threads a tile, up to 3
 constexpr size_t kThermalSmallCells = 200000;     // cells up to which that is the default
 constexpr size_t kThermalMarchMinCells = 1 << 20;  // cells from which the thermal march is the default
 constexpr int kThermalMarchVariant = 5;          // warps marching down column strips, one iteration per launch
+constexpr size_t kThermalScalarMarchMinCells = 1 << 22;  // the same where the march runs its scalar form
 int thermal_variant_for(const tecto_settings &s);  // 0 when the settings leave the choice open
+bool thermal_packed(const tecto_kernel_settings &ks);  // whether the march runs a packed form
 
 // Autotuner cache (tecto_tune.cu): best hydraulic tile variant and sort digit width for a batch
 // shape class on a device; false when nothing was tuned for that class.
