@@ -139,12 +139,14 @@ typedef struct tecto_step_settings {
                                  worlds fill its strips.  Tiles of cells / warps, two cells a lane, for
                                  one sub-iteration and for two at once: 1: 56x8/16, 52x9/20; 2: 56x8/8,
                                  52x12/8; 3: 56x16/8, 52x24/16; 4: 56x24/8, 52x28/12; 5: 56x32/10,
-                                 52x20/12; 6: 56x16/6; 7: 56x4/12; 9 (and 8): column strips marched down
+                                 52x20/12; 6: 56x16/6; 7: 56x4/12 (1 and 7 up to 2^17 cells, 4 above);
+                                 9 (and 8): column strips marched down
                                  4 rows at a time, two cells a thread, rows kept in shared memory: two
                                  sub-iterations in one march of 116-column strips by blocks of 512
                                  threads, a single one in 120-column strips by blocks of 256 (the split
                                  path, 50 dt >= 1.5, runs variant 4) */
-    int thermalTile;          /* 0 = autotuner's choice, else 3 up to 200 000 cells, 5 from 2^20
+    int thermalTile;          /* 0 = autotuner's choice, else 3 up to 200 000 cells, 5 from 2^20 (2^22
+                                 for a threshold below 2^-32 or a negative amplitude or strength)
                                  and 4 between; 1: 64x32 tiles / 1024 threads, up to 5
                                  iterations per launch; 2: 64x16 / 512, 2 blocks per SM, up to 4;
                                  3: 64x16 / 768, 2 blocks per SM, up to 3; 4: 64x16 / 512, 3 blocks

@@ -24,3 +24,11 @@ def test_thermal_march_from_a_million_cells_in_its_packed_forms(thr, A, S, march
     s.kernel.thermalThresholdAngle, s.kernel.thermalCellSize = thr, 1.0
     s.kernel.thermalErosionAmplitude, s.kernel.thermalErosionStrength = A, S
     assert launches(1100, 1000, s, lambda w: w.thermal(10)) == (10 if march else 5)
+
+
+# rain, then two sub-iterations a launch (variant 4) or one (variant 7 has no form for two)
+@pytest.mark.parametrize("W,H,tile,count", [(400, 400, 7, 3), (362, 362, 7, 5), (400, 400, 4, 3)])
+def test_short_tiles_run_in_small_batches_only(W, H, tile, count):
+    s = T.baseline_settings()
+    s.step.hydraulicTile = tile
+    assert launches(W, H, s, lambda w: w.hydraulic(4, 0.02)) == count

@@ -51,10 +51,10 @@ def check(W, H, tile, thermal_tile, iters, dt):
                                       O.thermal(want[0], 2, s).reshape(H, W).view(np.uint32))
 
 
-# more tile rows than 16 bits hold: 56 x 4, 56 x 8 (one sub-iteration) and 52 x 9 (two) cells a tile; and more
+# more tile rows than 16 bits hold, for one sub-iteration (56 x 8) and for two (52 x 12); and more
 # tile columns (52 and 56 wide)
 @pytest.mark.gpu
-@pytest.mark.parametrize("W,H,tile,iters,dt", [(3, 270000, 7, 1, 0.02), (2, 530000, 1, 1, 0.02), (2, 530000, 2, 1, 0.5),
+@pytest.mark.parametrize("W,H,tile,iters,dt", [(3, 270000, 7, 1, 0.02), (2, 530000, 1, 1, 0.02), (2, 530000, 2, 1, 0.5), (2, 800000, 2, 2, 0.02),
                                                (2, 600000, 1, 2, 0.02), (2, 600000, 0, 3, 0.02), (3700000, 2, 4, 2, 0.02),
                                                (3700000, 2, 9, 1, 0.02), (2, 1060000, 4, 1, 0.02)])
 def test_more_tiles_a_side_than_16_bits(W, H, tile, iters, dt):
