@@ -32,7 +32,9 @@
 // quotients and roots.  A thread with an operand outside them flags its chunk, and when the piece is
 // done the block runs the rows that the flagged chunks reach once more in the scalar IEEE form, whose
 // results are the same bits wherever the packed form holds (inputs and outputs are different buffers,
-// so a second run of a row starts from the same inputs).
+// so a second run of a row starts from the same inputs).  A piece's chunks are flagged by up to 64 segments, so
+// that two far apart do not send the rows between them too.  A flag costs its block some 30 rows in scalar form and
+// a warm-up: FIGURES
 //
 // Addressing.  A thread keeps one running value P = row * 512 + column * 4 (unsigned, wrapping); the
 // byte offset of a ring cell is P & (ring bytes - 1) plus the ring's base and a constant column step.
@@ -110,13 +112,49 @@ __device__ __forceinline__ void gld_flux(const float4 *base, uint32_t i, uint32_
                  : "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
                  : "l"(gaddr64(base, i + step)));
 }
+// The chunks kFirst .. K of a piece of `nrows` rows, and their segments for flags: chunk k is in segment
+// (k - kFirst) >> shift, of 64 at most.
+struct Chunks {
+    int first, last, shift;
+};
+__device__ __forceinline__ Chunks chunks_of(int nrows, bool two)
+{
+    const int first = two ? -4 : -3, last = (nrows + (two ? kLag : 0) + kPairRows - 1) / kPairRows;
+    return Chunks{first, last, max(0, 26 - __clz(last - first))};
+}
+
+// Runs the rows that flagged segments reach once more: `run(lo, hi)` for each range of rows.  A cell of a chunk
+// whose first row is r reaches outputs r - back .. r + ahead - 1; ranges closer than a run's warm-up are one.
+template <typename F>
+__device__ __forceinline__ void rerun_flagged(const unsigned *flagged, const Chunks &c, int r0, int r1, int back,
+                                              int ahead, F &&run)
+{
+    unsigned long long m = (unsigned long long)flagged[1] << 32 | flagged[0];
+    int lo = 0, hi = 0;
+    while (m) {
+        const int s = __ffsll((long long)m) - 1;
+        m &= m - 1ull;
+        const int a = max(r0, r0 + kPairRows * ((s << c.shift) + c.first) - back);
+        const int b = min(r1, r0 + kPairRows * (((s + 1) << c.shift) - 1 + c.first) + ahead);
+        if (a >= b) continue;
+        if (hi > lo && a > hi + (int)kWarmRows) {
+            run(lo, hi);
+            lo = a;
+        } else if (hi == lo) {
+            lo = a;
+        }
+        hi = max(hi, b);
+    }
+    if (hi > lo) run(lo, hi);
+}
+
 // Rows [r0, r1) of the strip with interior columns [x0, x0 + iw) of world q.  VEC: the world's width is
 // even.  IEEE: the scalar form, for any operands; else the packed form, which needs p.fastL, dt >= 0 and
-// H >= 4, and leaves in flagged[0], flagged[1] the first and last chunk with an operand outside its
-// ranges.  ROLE: a sub-iteration by itself, or the first or the second of two (k_hydro_march_pair).
+// H >= 4, and sets in flagged[0], flagged[1] the segments (chunks_of) of chunks with an operand outside
+// its ranges.  ROLE: a sub-iteration by itself, or the first or the second of two (k_hydro_march_pair).
 template <bool VEC, bool IEEE, int ROLE>
 __device__ __forceinline__ void march_piece(const HydroParams &p, const PairConst &c, const HydroWorld &q, char *S,
-                                            int x0, int iw, int r0, int r1, int *flagged)
+                                            int x0, int iw, int r0, int r1, unsigned *flagged)
 {
     const int W = q.W, H = q.H;
     const uint32_t Wu = (uint32_t)W, N = Wu * (uint32_t)H, W4 = 4u * Wu;
@@ -154,7 +192,7 @@ __device__ __forceinline__ void march_piece(const HydroParams &p, const PairCons
     // Per chunk k (first row rk = r0 + 4k) this thread's base row is t = rk + rr and its items are rows
     // t + c: flux c = 7, flow c = 2, transport c = -4, and the loads c = 12 (height, water and rain),
     // c = 11 (old flux) and c = 6 (sediment).
-    constexpr int kFirst = ROLE ? -4 : -3;
+    constexpr int kFirst = ROLE ? -4 : -3;  // as in chunks_of
     uint32_t P = (uint32_t)(r0 + kFirst * kPairRows - LAG + rr) * kMRow + (uint32_t)col * 4u;  // ring value of row t
     int tr = rr + kFirst * kPairRows - LAG;                                                    // t - r0
     uint32_t B = (uint32_t)(r0 + kFirst * kPairRows - LAG + rr) * Wu + (uint32_t)gxi;          // global offset of row t
@@ -355,8 +393,8 @@ __device__ __forceinline__ void march_piece(const HydroParams &p, const PairCons
             }
         }
         if (!IEEE && bad) {
-            atomicMin(flagged, k);
-            atomicMax(flagged + 1, k);
+            const uint32_t seg = (uint32_t)(k - kFirst) >> chunks_of(r1 - r0, ROLE != kAlone).shift;
+            atomicOr(flagged + (seg >> 5), 1u << (seg & 31u));
         }
         barrier();
         P += kPairRows * kMRow;
@@ -384,7 +422,7 @@ __global__ __launch_bounds__(kPairThreads, 2) void k_hydro_march(const __grid_co
     extern __shared__ float4 march_smem[];
     char *S = reinterpret_cast<char *>(march_smem);
     __shared__ HydroWorld s_q;
-    __shared__ int s_flag[2];
+    __shared__ unsigned s_flag[2];
     // the edge lanes read ring cells before anything writes them: start from zeros
     for (uint32_t i = threadIdx.x; i < kHydroMarchSmem / 16; i += kPairThreads)
         march_smem[i] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -405,8 +443,7 @@ __global__ __launch_bounds__(kPairThreads, 2) void k_hydro_march(const __grid_co
         __syncthreads();  // the previous piece is done with s_q and the rings
         if (threadIdx.x == 0) {
             s_q = hydro_world(sp.p, sp.p.worlds[d.x]);
-            s_flag[0] = 0x7fffffff;
-            s_flag[1] = -0x7fffffff;
+            s_flag[0] = s_flag[1] = 0u;
         }
         __syncthreads();
         const unsigned long long first = d.w + (unsigned long long)(s + 1) * kWarmAlone,
@@ -420,14 +457,13 @@ __global__ __launch_bounds__(kPairThreads, 2) void k_hydro_march(const __grid_co
         } else {
             if (s_q.W & 1) march_piece<false, false, kAlone>(sp.p, pp.c, s_q, S, x0, iw, r0, r1, s_flag);
             else march_piece<true, false, kAlone>(sp.p, pp.c, s_q, S, x0, iw, r0, r1, s_flag);
-            // the piece's last barrier has passed since the last flag
-            const int k0 = s_flag[0], k1 = s_flag[1];
-            if (k1 >= k0) {
-                // a cell of chunk k (flux rows r+7 .. r+10, flow rows r+2 .. r+5) reaches outputs three rows away
-                __syncthreads();
-                march_ieee(pp, s_q, S, x0, iw, max(r0, r0 + kPairRows * k0),
-                           min(r1, r0 + kPairRows * k1 + 14));
-            }
+            // The piece's last barrier has passed since the last flag.  A cell of chunk k (flux rows r+7 .. r+10, flow
+            // rows r+2 .. r+5) reaches outputs three rows away.
+            if (s_flag[0] | s_flag[1])
+                rerun_flagged(s_flag, chunks_of(r1 - r0, false), r0, r1, 0, 14, [&](int lo, int hi) {
+                    __syncthreads();
+                    march_ieee(pp, s_q, S, x0, iw, lo, hi);
+                });
         }
         a = first + (unsigned long long)r1;
     }
@@ -436,7 +472,7 @@ __global__ __launch_bounds__(kPairThreads, 2) void k_hydro_march(const __grid_co
 // Both roles of two sub-iterations: the block's first half is the first of the two.
 template <bool VEC, bool IEEE>
 __device__ __forceinline__ void march_two(const HydroParams &p, const PairConst &c, const HydroWorld &q, char *S, int x0,
-                                          int iw, int r0, int r1, int *flagged)
+                                          int iw, int r0, int r1, unsigned *flagged)
 {
     if (threadIdx.x < kPairThreads) march_piece<VEC, IEEE, kFirstOfTwo>(p, c, q, S, x0, iw, r0, r1, flagged);
     else march_piece<VEC, IEEE, kSecondOfTwo>(p, c, q, S, x0, iw, r0, r1, flagged);
@@ -463,7 +499,7 @@ __global__ __launch_bounds__(2 * kPairThreads, 1) void k_hydro_march_pair(const 
     extern __shared__ float4 march_smem[];
     char *S = reinterpret_cast<char *>(march_smem);
     __shared__ HydroWorld s_q;
-    __shared__ int s_flag[2];
+    __shared__ unsigned s_flag[2];
     for (uint32_t i = threadIdx.x; i < kHydroPairSmem / 16; i += 2 * kPairThreads)
         march_smem[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     // Each strip counts kWarmRows more than it has, before its first: a block that starts another strip pays a
@@ -484,8 +520,7 @@ __global__ __launch_bounds__(2 * kPairThreads, 1) void k_hydro_march_pair(const 
         __syncthreads();  // the previous piece is done with s_q and the rings
         if (threadIdx.x == 0) {
             s_q = hydro_world(sp.p, sp.p.worlds[d.x]);
-            s_flag[0] = 0x7fffffff;
-            s_flag[1] = -0x7fffffff;
+            s_flag[0] = s_flag[1] = 0u;
         }
         __syncthreads();
         const unsigned long long first = d.w + (unsigned long long)(s + 1) * kWarmRows,
@@ -499,14 +534,13 @@ __global__ __launch_bounds__(2 * kPairThreads, 1) void k_hydro_march_pair(const 
         } else {
             if (s_q.W & 1) march_two<false, false>(sp.p, pp.c, s_q, S, x0, iw, r0, r1, s_flag);
             else march_two<true, false>(sp.p, pp.c, s_q, S, x0, iw, r0, r1, s_flag);
-            const int k0 = s_flag[0], k1 = s_flag[1];
-            if (k1 >= k0) {
-                // a cell of the first's chunk k (flux rows r+7 .. r+10, flow rows r+2 .. r+5) reaches outputs
-                // r-2 .. r+15, one of the second's, ten rows behind, outputs r-10 .. r+3
-                __syncthreads();
-                march_two_ieee(pp, s_q, S, x0, iw, max(r0, r0 + kPairRows * k0 - kLag),
-                               min(r1, r0 + kPairRows * k1 + 16));
-            }
+            // a cell of the first's chunk k (flux rows r+7 .. r+10, flow rows r+2 .. r+5) reaches outputs
+            // r-2 .. r+15, one of the second's, ten rows behind, outputs r-10 .. r+3
+            if (s_flag[0] | s_flag[1])
+                rerun_flagged(s_flag, chunks_of(r1 - r0, true), r0, r1, kLag, 16, [&](int lo, int hi) {
+                    __syncthreads();
+                    march_two_ieee(pp, s_q, S, x0, iw, lo, hi);
+                });
         }
         a = first + (unsigned long long)r1;
     }
