@@ -214,8 +214,9 @@ __global__ __launch_bounds__(256, 8) void k_resolve(ResolveParams p)
     __shared__ uint16_t s_list[RX * RY];  // divergent cells from the front, convergent ones from the back
     __shared__ int s_ndiv, s_nconv;
     __shared__ uint32_t s_seed, s_iteration;
-    __shared__ float s_vel[DYN ? kPlates : 1], s_mass[DYN ? kPlates : 1];
-    __shared__ unsigned long long s_fric[DYN ? kPlates : 1];
+    // one entry more than plates: an arrival from a cell without a plate (id 255) has no velocity, its friction is 0
+    __shared__ float s_vel[DYN ? kPlates + 1 : 1], s_mass[DYN ? kPlates + 1 : 1];
+    __shared__ unsigned long long s_fric[DYN ? kPlates + 1 : 1];
     int wi, tx, ty;
     tile_of(p.tiles[blockIdx.x], &wi, &tx, &ty);
     const WorldDev &wd = p.worlds[wi];
@@ -239,9 +240,9 @@ __global__ __launch_bounds__(256, 8) void k_resolve(ResolveParams p)
     const int x0 = tx * RX, y0 = ty * RY;
     for (int i = t; i < kPlates + 1; i += 256) s_off[i] = wd.off[i];
     if (DYN) {
-        for (int i = t; i < kPlates; i += 256) {
-            s_vel[i] = wd.plates[i].velocity;
-            s_mass[i] = wd.dyn[i].mass;
+        for (int i = t; i < kPlates + 1; i += 256) {
+            s_vel[i] = i < kPlates ? wd.plates[i].velocity : 0.0f;
+            s_mass[i] = i < kPlates ? wd.dyn[i].mass : 1.0f;
             s_fric[i] = 0ull;
         }
     }
