@@ -21,6 +21,8 @@ struct ResolveParams {
     float amount;
     float wts[2 * kMaxBlurRadius + 1];
     float tap0;        // what a tap without a convergent cell adds: +0, or NaN with weights that are NaN
+    int centre;        // Gaussian uplift of radius 0: the centre tap alone, centre_up[0] on a cell that is not
+    float centre_up[2];  // convergent and centre_up[1] on one that is
     float *upl_h;      // reference uplift: processConvergence's records by virtual cell, or null
     uint8_t *upl_t;
     float fricC, fricA, fricS;  // frictionCoefficientContinental / Accretion / Subduction
@@ -322,6 +324,7 @@ __global__ __launch_bounds__(256, 8) void k_resolve(ResolveParams p)
             const uint32_t d = (uint32_t)y * (uint32_t)w.W + (uint32_t)x;
             float hn = w.h_old[cidx(x - o.x, y - o.y, w.W, w.H)];
             if (R > 0) hn = hn + (raised ? uplift(lx, ly) : 0.0f);
+            else if (p.centre) hn = hn + p.centre_up[cv > 0xFFu];
             h_new[d] = hn;
             id_new[d] = id0;
         }
@@ -349,6 +352,7 @@ __global__ __launch_bounds__(256, 8) void k_resolve(ResolveParams p)
         float hn = e < ndiv ? diverge_cell(p, w, s_off, cellx, celly, d, s_seed, s_iteration, &nid)
                             : converge_cell<DYN>(p, w, s_off, cellx, celly, d, s_word[(cy + R) * SX + cx + R], &nid, dyn);
         if (R > 0) hn = hn + (blur ? uplift(cx, cy) : 0.0f);
+        else if (p.centre) hn = hn + p.centre_up[s_word[(cy + R) * SX + cx + R] > 0xFFu];
         h_new[d] = hn;
         id_new[d] = nid;
     }
@@ -449,6 +453,9 @@ int launch_resolve(Batch &b, bool flip, cudaStream_t st)
         }
         gaussian_weights(s.step.upliftSigma, R, p.wts);
         p.tap0 = p.wts[0] * 0.0f;  // the weights are finite or all NaN
+        p.centre = R == 0;
+        p.centre_up[0] = 0.0f + p.wts[0] * (0.0f + p.wts[0] * 0.0f);
+        p.centre_up[1] = 0.0f + p.wts[0] * (0.0f + p.wts[0] * p.amount);
     }
     static constexpr void (*kern[2][kMaxBlurRadius + 1])(ResolveParams) = {
         {k_resolve<0, false>, k_resolve<1, false>, k_resolve<2, false>, k_resolve<3, false>, k_resolve<4, false>,
