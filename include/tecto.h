@@ -637,6 +637,12 @@ int tecto_selftest_div(const float *a, const float *b, float *out, size_t n, tec
  * the quotient from a correctly rounded reciprocal (one Newton-Raphson step from the hardware's
  * approximation), with the IEEE division outside its safe range. */
 int tecto_selftest_div_var(const float *a, const float *b, float *out, size_t n, tecto_stream_t stream);
+/* The same for the packed forms, two cells at a time, that the marching and tile kernels run: quot[i] =
+ * amplitude * (a[i] / b[i]) with the amplitude, a power of two, folded into the quotient (1: the quotient), and
+ * root[i] = sqrt(a[i]), without a fallback.  Exact for dividends that are zero or in [2^-90, 2^64), divisors in
+ * [2^-32, 2^32] and roots of zero or of [2^-100, 2^64].  n is even. */
+int tecto_selftest_packed(const float *a, const float *b, float amplitude, float *quot, float *root, size_t n,
+                          tecto_stream_t stream);
 /* Exhaustive self-test of the erosion kernels' reciprocal and square root: for every positive
  * normal float, whether each equals the correctly rounded result.  bad (device, 512 counters)
  * receives the mismatches per exponent field: bad[e] for the reciprocal, bad[256 + e] for the

@@ -303,6 +303,7 @@ def _declare(L: C.CDLL) -> None:
         "tecto_server_live_stats": ([P, C.POINTER(ServerStats)], C.c_int),
         "tecto_selftest_div": ([P, P, P, C.c_size_t, P], C.c_int),
         "tecto_selftest_div_var": ([P, P, P, C.c_size_t, P], C.c_int),
+        "tecto_selftest_packed": ([P, P, C.c_float, P, P, C.c_size_t, P], C.c_int),
         "tecto_selftest_rcp_sqrt": ([P, P], C.c_int),
         "tecto_selftest_tiles": ([C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.POINTER(C.c_ulonglong)], C.c_int),
         "tecto_png_encode": ([P, C.c_int, C.c_int, C.c_int, P, C.c_size_t, C.POINTER(C.c_size_t)], C.c_int),
