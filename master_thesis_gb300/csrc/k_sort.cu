@@ -384,10 +384,11 @@ __device__ __forceinline__ void sort_tile(const uint32_t *keys_in, const uint32_
 // A sort of 3 M pairs 193 -> 103 us, of 43.6 M 1.91 -> 1.01 ms, against ranking by eight ballots a key with
 // the values held in registers at two and three blocks per SM.
 // Four blocks per SM (64 registers, some of the ranks spilled): a tile waits on its loads and its look-back
-// most of the time.  Tiles of 8192 keys by 512 threads were no faster (8192^2: 3.99 against 3.60 ms for a
+// most of the time.  Shared memory admits three of 10-bit digits (70 KB each) and two of 11 (106 KB), which take the
+// registers that leaves.  Tiles of 8192 keys by 512 threads were no faster (8192^2: 3.99 against 3.60 ms for a
 // step's phases other than erosion).
 template <int RB>
-__global__ __launch_bounds__(kSortThreads, 4) void k_sort_pass(
+__global__ __launch_bounds__(kSortThreads, RB <= 9 ? 4 : RB == 10 ? 3 : 2) void k_sort_pass(
     const uint32_t *keys_in, const uint32_t *vals_in, uint32_t *keys_out, uint32_t *vals_out, uint32_t n,
     int shift, const uint32_t *digit_start, uint32_t *status, uint32_t *tile_counter, uint32_t *error)
 {
