@@ -348,9 +348,8 @@ size_t tecto_sort_scratch_bytes_radix(size_t n, int key_bits, int radix_bits);
 int tecto_sort_pairs_radix(const uint32_t *keys_in, const uint32_t *vals_in, uint32_t *keys_out,
                            uint32_t *vals_out, size_t n, int key_bits, int radix_bits, void *scratch,
                            size_t scratch_bytes, tecto_stream_t stream);
-/* 1 when a sort of n pairs runs its passes in the form for large sorts (from 4096 tiles of 4096
- * keys, i.e. 16 777 216 pairs), 0 when it runs the form for smaller sorts; both are one form now.
- * The collision sort of a batch or world uses the same rule on its cell count. */
+/* 1 from 16 773 121 pairs (4096 tiles of 4096 keys) on, else 0.  Kept for callers: sorts of this size once ran a
+ * form of their own; all sizes run the same one now, and nothing in the library asks. */
 int tecto_sort_wide_pass(size_t n);
 
 /* The same stable sort for callers that cannot allocate device memory: it needs no scratch
@@ -430,7 +429,7 @@ int tecto_batch_phase_thermal(tecto_batch *batch, int iterations, tecto_stream_t
 /* ---- autotuner ---------------------------------------------------------------------------
  *
  * No counterpart in the reference (fixed launch shapes, plate_tectonic_sim.cu).  Times every
- * hydraulic tile variant (one sub-iteration), every thermal tile variant (ten iterations) and every
+ * hydraulic tile variant (two sub-iterations, as a step runs them), every thermal tile variant (ten iterations) and every
  * sort digit width (the collision sort) on scratch worlds of the given shapes with synthetic
  * content, and returns the fastest of each.
  * The caller's worlds are not touched.  The choice is cached per device and batch shape class
@@ -442,7 +441,7 @@ typedef struct tecto_tuning {
     int hydraulicTile;       /* chosen variant, 1..8 (8 is the march) */
     int sortRadixBits;       /* chosen digit width, 8..11 */
     int thermalTile;         /* chosen variant, 1..5 */
-    float hydraulic_ms[9];   /* one hydraulic sub-iteration with variant 1..9 */
+    float hydraulic_ms[9];   /* half of two hydraulic sub-iterations with variant 1..9 (8 and 9 are the march) */
     float sort_ms[4];        /* the collision sort with 8..11-bit digits */
     float thermal_ms[5];     /* ten thermal iterations with variant 1..5 */
 } tecto_tuning;

@@ -123,7 +123,7 @@ __device__ __forceinline__ const WorldDev *ccl_tile(const WorldDev *worlds, cons
 // component without looking at an edge.
 // 4096 x 3000 of 48 plates (61 MB of ids and labels, 9 us) 137 -> 50 us; a map of two ids at random, without
 // such tiles, 2048^2, all three kernels, 124 -> 120.
-// eight blocks per SM (32 registers, no spill): the pass waits on loads and shared atomics
+// eight blocks per SM (32 registers, some of the edges' state spilled): the pass waits on loads and shared atomics
 __global__ __launch_bounds__(256, 8) void k_ccl_local(const WorldDev *worlds, const uint2 *tiles, int cur_id,
                                                    int mode, int period)
 {

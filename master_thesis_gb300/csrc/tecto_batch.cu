@@ -183,7 +183,8 @@ static int default_radix_bits(size_t cells)
 // Parameters that the march's packed forms do not take (a threshold below 2^-32, a negative amplitude): ten
 // iterations with tiles / the march, threshold 0 and 1e-12, us: 1024^2 115 / 156 and 104 / 139, 1500x1100 174 / 194
 // and 157 / 171, 2048^2 407 / 402 and 363 / 348, 4096^2 1616 / 1347 and 1458 / 1162.
-// The default hydraulic variant: the one whose two sub-iterations a model of the measured shapes puts lowest.
+// The default hydraulic variant: the one whose two sub-iterations a model of the measured shapes puts lowest.  The
+// times are one chip's, and so is its number of SMs here, which belongs to them.
 // Tiles run in waves of 152 SMs x the tiles an SM holds, and a wave's time depends on how many it holds; the
 // march's blocks take equal shares of the strips' rows (with what a strip's start costs, k_hydro_march.cu), at
 // 0.38 us a row, 0.42 counted as odd widths take longer.  Whole steps, us, the model's choice marked:
@@ -198,7 +199,10 @@ static int default_radix_bits(size_t cells)
 // it chooses, against 957; 100 (2.5 M) 1461 against 1471; 20 of 240x400 882 against 1039.
 static int default_hydro_variant(const Batch &b, bool split)
 {
-    if (split)  // 50 dt >= 1.5: the march's transport reaches two cells; no two at once
+    // 50 dt >= 1.5: the march's transport reaches two cells; no two at once.  20 sub-iterations with 1 / 2 / 3 / 4, us:
+    // 256^2 138 / 142 / 176 / 221, 512^2 215 / 198 / 217 / 272, 701x503 276 / 254 / 267 / 288, 1024^2 643 / 546 / 504 /
+    // 538, 2048^2 2711 / 2067 / 1806 / 1840, 4096^2 10489 / 7869 / 6706 / 6671.
+    if (split)
         return b.total <= (size_t)1 << 17 ? 1 : b.total <= (size_t)1 << 20 ? 3 : 4;
     constexpr double kSms = 152.0;
     struct Shape {
