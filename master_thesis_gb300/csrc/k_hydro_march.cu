@@ -32,11 +32,12 @@
 // quotients and roots.  A thread with an operand outside them flags its chunk, and when the piece is
 // done the block runs the rows that the flagged chunks reach once more in the scalar IEEE form, whose
 // results are the same bits wherever the packed form holds (inputs and outputs are different buffers,
-// so a second run of a row starts from the same inputs).  A piece's chunks are flagged by up to 64 segments, so
-// that two far apart do not send the rows between them too.  A flag costs its block some 30 rows in scalar form and
-// a warm-up: two sub-iterations with no / 1 / 40 / 1000 such cells spread over the world, us: 2048^2 115 / 181 / 241 /
-// 342, 8192^2 1532 / 1587 / 1736 / 2760 (one range from the first flag to the last: 313 and 2417 with 40; the tiles of
-// variant 4, which repeat a tile: 165 / 165 / 186 / 300 and 2410 / 2410 / 2434 / 2598).
+// so a second run of a row starts from the same inputs).  Of two sub-iterations in a world of even width a piece's
+// chunks are flagged by up to 64 segments, so that two far apart do not send the rows between them too.  A flag costs
+// its block some 30 rows in scalar form and a warm-up: two sub-iterations with no / 1 / 40 / 1000 such cells spread over
+// the world, us: 2048^2 115 / 181 / 240 / 343, 8192^2 1525 / 1583 / 1732 / 2769 (one range from the first flag to the
+// last: 313 and 2417 with 40; the tiles of variant 4, which repeat a tile: 165 / 165 / 187 / 302 and 2413 / 2413 / 2437 /
+// 2603).
 //
 // Addressing.  A thread keeps one running value P = row * 512 + column * 4 (unsigned, wrapping); the
 // byte offset of a ring cell is P & (ring bytes - 1) plus the ring's base and a constant column step.
@@ -114,28 +115,42 @@ __device__ __forceinline__ void gld_flux(const float4 *base, uint32_t i, uint32_
                  : "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
                  : "l"(gaddr64(base, i + step)));
 }
-// The chunks kFirst .. K of a piece of `nrows` rows, and their segments for flags: chunk k is in segment
-// (k - kFirst) >> shift, of 64 at most.
+// The flags of a piece, two shared words.  Two sub-iterations of an even width: the segments of its chunks kFirst ..
+// K with an operand outside the packed ranges; chunk k is in segment (k - kFirst) >> shift, of 64 at most.  Odd widths,
+// and a single sub-iteration: the first and the last such chunk, as the segment's arithmetic, in a branch that is
+// hardly ever taken, changes how the loop compiles (20 sub-iterations, 2047x2048 1113 -> 1147 us, the 49.7 M cell batch
+// 13.1 -> 13.9 ms; even widths 1052 -> 1042; one sub-iteration at 8192^2 978 -> 986).
 struct Chunks {
     int first, last, shift;
 };
-__device__ __forceinline__ Chunks chunks_of(int nrows, bool two)
+__device__ __forceinline__ Chunks chunks_of(int nrows)
 {
-    const int first = two ? -4 : -3, last = (nrows + (two ? kLag : 0) + kPairRows - 1) / kPairRows;
+    const int first = -4, last = (nrows + kLag + kPairRows - 1) / kPairRows;
     return Chunks{first, last, max(0, 26 - __clz(last - first))};
 }
 
-// Runs the rows that flagged segments reach once more: `run(lo, hi)` for each range of rows.  A cell of a chunk
-// whose first row is r reaches outputs r - back .. r + ahead - 1; ranges closer than a run's warm-up are one.
-template <typename F>
-__device__ __forceinline__ void rerun_flagged(const unsigned *flagged, const Chunks &c, int r0, int r1, int back,
-                                              int ahead, F &&run)
+__device__ __forceinline__ void clear_flags(unsigned *flagged, bool range)
 {
-    unsigned long long m = (unsigned long long)flagged[1] << 32 | flagged[0];
+    flagged[0] = range ? 0x7fffffffu : 0u;
+    flagged[1] = range ? 0x80000000u : 0u;
+}
+
+// Runs the rows that the flagged chunks reach once more: `run(lo, hi)` for each range of rows.  A cell of a chunk
+// whose first row is r reaches outputs r - back .. r + ahead - 1.
+template <typename F>
+__device__ __forceinline__ void rerun_range(const unsigned *flagged, int r0, int r1, int back, int ahead, F &&run)
+{
+    const int k0 = (int)flagged[0], k1 = (int)flagged[1];
+    if (k1 >= k0) run(max(r0, r0 + kPairRows * k0 - back), min(r1, r0 + kPairRows * k1 + ahead));
+}
+// The same by segments; ranges closer than a run's warm-up are one.
+template <typename F>
+__device__ __forceinline__ void rerun_segments(const unsigned *flagged, int r0, int r1, int back, int ahead, F &&run)
+{
+    const Chunks c = chunks_of(r1 - r0);
     int lo = 0, hi = 0;
-    while (m) {
+    for (unsigned long long m = (unsigned long long)flagged[1] << 32 | flagged[0]; m; m &= m - 1ull) {
         const int s = __ffsll((long long)m) - 1;
-        m &= m - 1ull;
         const int a = max(r0, r0 + kPairRows * ((s << c.shift) + c.first) - back);
         const int b = min(r1, r0 + kPairRows * (((s + 1) << c.shift) - 1 + c.first) + ahead);
         if (a >= b) continue;
@@ -152,8 +167,7 @@ __device__ __forceinline__ void rerun_flagged(const unsigned *flagged, const Chu
 
 // Rows [r0, r1) of the strip with interior columns [x0, x0 + iw) of world q.  VEC: the world's width is
 // even.  IEEE: the scalar form, for any operands; else the packed form, which needs p.fastL, dt >= 0 and
-// H >= 4, and sets in flagged[0], flagged[1] the segments (chunks_of) of chunks with an operand outside
-// its ranges.  ROLE: a sub-iteration by itself, or the first or the second of two (k_hydro_march_pair).
+// H >= 4, and flags in flagged[0], flagged[1] the chunks with an operand outside its ranges.  ROLE: a sub-iteration by itself, or the first or the second of two (k_hydro_march_pair).
 template <bool VEC, bool IEEE, int ROLE>
 __device__ __forceinline__ void march_piece(const HydroParams &p, const PairConst &c, const HydroWorld &q, char *S,
                                             int x0, int iw, int r0, int r1, unsigned *flagged)
@@ -194,7 +208,7 @@ __device__ __forceinline__ void march_piece(const HydroParams &p, const PairCons
     // Per chunk k (first row rk = r0 + 4k) this thread's base row is t = rk + rr and its items are rows
     // t + c: flux c = 7, flow c = 2, transport c = -4, and the loads c = 12 (height, water and rain),
     // c = 11 (old flux) and c = 6 (sediment).
-    constexpr int kFirst = ROLE ? -4 : -3;  // as in chunks_of
+    constexpr int kFirst = ROLE ? -4 : -3;  // of two as in chunks_of
     uint32_t P = (uint32_t)(r0 + kFirst * kPairRows - LAG + rr) * kMRow + (uint32_t)col * 4u;  // ring value of row t
     int tr = rr + kFirst * kPairRows - LAG;                                                    // t - r0
     uint32_t B = (uint32_t)(r0 + kFirst * kPairRows - LAG + rr) * Wu + (uint32_t)gxi;          // global offset of row t
@@ -395,8 +409,13 @@ __device__ __forceinline__ void march_piece(const HydroParams &p, const PairCons
             }
         }
         if (!IEEE && bad) {
-            const uint32_t seg = (uint32_t)(k - kFirst) >> chunks_of(r1 - r0, ROLE != kAlone).shift;
-            atomicOr(flagged + (seg >> 5), 1u << (seg & 31u));
+            if constexpr (VEC && ROLE != kAlone) {
+                const uint32_t seg = (uint32_t)(k - kFirst) >> max(0, 26 - __clz(K - kFirst));
+                atomicOr(flagged + (seg >> 5), 1u << (seg & 31u));
+            } else {
+                atomicMin(reinterpret_cast<int *>(flagged), k);
+                atomicMax(reinterpret_cast<int *>(flagged) + 1, k);
+            }
         }
         barrier();
         P += kPairRows * kMRow;
@@ -445,7 +464,7 @@ __global__ __launch_bounds__(kPairThreads, 2) void k_hydro_march(const __grid_co
         __syncthreads();  // the previous piece is done with s_q and the rings
         if (threadIdx.x == 0) {
             s_q = hydro_world(sp.p, sp.p.worlds[d.x]);
-            s_flag[0] = s_flag[1] = 0u;
+            clear_flags(s_flag, true);
         }
         __syncthreads();
         const unsigned long long first = d.w + (unsigned long long)(s + 1) * kWarmAlone,
@@ -461,11 +480,10 @@ __global__ __launch_bounds__(kPairThreads, 2) void k_hydro_march(const __grid_co
             else march_piece<true, false, kAlone>(sp.p, pp.c, s_q, S, x0, iw, r0, r1, s_flag);
             // The piece's last barrier has passed since the last flag.  A cell of chunk k (flux rows r+7 .. r+10, flow
             // rows r+2 .. r+5) reaches outputs three rows away.
-            if (s_flag[0] | s_flag[1])
-                rerun_flagged(s_flag, chunks_of(r1 - r0, false), r0, r1, 0, 14, [&](int lo, int hi) {
-                    __syncthreads();
-                    march_ieee(pp, s_q, S, x0, iw, lo, hi);
-                });
+            rerun_range(s_flag, r0, r1, 0, 14, [&](int lo, int hi) {
+                __syncthreads();
+                march_ieee(pp, s_q, S, x0, iw, lo, hi);
+            });
         }
         a = first + (unsigned long long)r1;
     }
@@ -522,7 +540,7 @@ __global__ __launch_bounds__(2 * kPairThreads, 1) void k_hydro_march_pair(const 
         __syncthreads();  // the previous piece is done with s_q and the rings
         if (threadIdx.x == 0) {
             s_q = hydro_world(sp.p, sp.p.worlds[d.x]);
-            s_flag[0] = s_flag[1] = 0u;
+            clear_flags(s_flag, s_q.W & 1);
         }
         __syncthreads();
         const unsigned long long first = d.w + (unsigned long long)(s + 1) * kWarmRows,
@@ -538,11 +556,12 @@ __global__ __launch_bounds__(2 * kPairThreads, 1) void k_hydro_march_pair(const 
             else march_two<true, false>(sp.p, pp.c, s_q, S, x0, iw, r0, r1, s_flag);
             // a cell of the first's chunk k (flux rows r+7 .. r+10, flow rows r+2 .. r+5) reaches outputs
             // r-2 .. r+15, one of the second's, ten rows behind, outputs r-10 .. r+3
-            if (s_flag[0] | s_flag[1])
-                rerun_flagged(s_flag, chunks_of(r1 - r0, true), r0, r1, kLag, 16, [&](int lo, int hi) {
-                    __syncthreads();
-                    march_two_ieee(pp, s_q, S, x0, iw, lo, hi);
-                });
+            const auto run = [&](int lo, int hi) {
+                __syncthreads();
+                march_two_ieee(pp, s_q, S, x0, iw, lo, hi);
+            };
+            if (s_q.W & 1) rerun_range(s_flag, r0, r1, kLag, 16, run);
+            else rerun_segments(s_flag, r0, r1, kLag, 16, run);
         }
         a = first + (unsigned long long)r1;
     }
