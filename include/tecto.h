@@ -139,7 +139,8 @@ typedef struct tecto_step_settings {
                                  worlds fill its strips.  Tiles of cells / warps, two cells a lane, for
                                  one sub-iteration and for two at once: 1: 56x8/16, 52x9/20; 2: 56x8/8,
                                  52x12/8; 3: 56x16/8, 52x24/16; 4: 56x24/8, 52x28/12; 5: 56x32/10,
-                                 52x20/12; 6: 56x16/6; 7: 56x4/12 (1 and 7 up to 2^17 cells, 4 above);
+                                 52x20/12; 6: 56x16/6; 7: 56x4/12 (1 and 7 up to 2^17 cells, on
+                                 the split path up to 2^19, 4 above);
                                  9 (and 8): column strips marched down
                                  4 rows at a time, two cells a thread, rows kept in shared memory: two
                                  sub-iterations in one march of 116-column strips by blocks of 512

@@ -252,10 +252,11 @@ static void choose_tuning(Batch &b, int *variant, int *rb, int *tvariant)
     if (*variant == 0) *variant = b.tuned_hydro;
     // Variants 1 and 7, tiles of 8 and 4 rows, are shapes for batches that leave SMs idle; larger ones take 4.  20
     // sub-iterations with 1 / 7 / 4, us: 256^2 62 / 123 / 104, 512^2 216 / 304 / 168, 1024^2 785 / 1004 / 389, 4096^2
-    // 12833 / 16821 / 5839; the split path 138 / 143 / 221, 215 / 277 / 272, 643 / 909 / 538, 10489 / 16037 / 6671.
-    if ((*variant == 1 || *variant == 7) && b.total > kShortTileCells) *variant = 4;
+    // 12833 / 16821 / 5839; the split path 138 / 143 / 221, 215 / 277 / 272, 643 / 909 / 538, 10489 / 16037 / 6671, and
+    // 701x503 274 / 341 / 286.
+    const bool split = !hydro_fused(b, b.settings.step.hydraulicDt);
+    if ((*variant == 1 || *variant == 7) && b.total > (split ? kShortTileSplitCells : kShortTileCells)) *variant = 4;
     if (*variant == 0) {
-        const bool split = !hydro_fused(b, b.settings.step.hydraulicDt);
         if (b.dirty) b.hydro_default[0] = b.hydro_default[1] = 0;  // of other members
         int &d = b.hydro_default[split];
         if (d == 0) d = default_hydro_variant(b, split);

@@ -405,6 +405,7 @@ void gaussian_weights(float sigma, int radius, float *out);
 int ensure_kernel_attributes();
 int hydro_variant_for(const tecto_settings &s);  // 0 when the settings leave the choice open
 constexpr size_t kShortTileCells = 1 << 17;      // cells up to which a choice of variant 1 or 7 runs its own tiles
+constexpr size_t kShortTileSplitCells = 1 << 19;  // the same on the split path
 bool hydro_fused(const Batch &b, float dt);      // whether a sub-iteration's transport is fused into it
 constexpr int kDefaultRadixBits = 8;
 constexpr int kHydroVariantCount = 9;

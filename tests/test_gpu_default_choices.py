@@ -30,5 +30,5 @@ def test_thermal_march_from_a_million_cells_in_its_packed_forms(thr, A, S, march
 @pytest.mark.parametrize("W,H,tile,count", [(400, 400, 7, 3), (362, 362, 7, 5), (400, 400, 4, 3)])
 def test_short_tiles_run_in_small_batches_only(W, H, tile, count):
     s = T.baseline_settings()
-    s.step.hydraulicTile = tile
+    s.step.hydraulicTile = tile  # dt 0.02: not the split path
     assert launches(W, H, s, lambda w: w.hydraulic(4, 0.02)) == count
