@@ -20,7 +20,7 @@
 // pipe: 990 against 762 us).  One sub-iteration, before and after, us: 2048^2 93.9 -> 72, 4096^2
 // 303 -> 232, 8192^2 1120 -> 852 (4.8 TB/s of DRAM traffic), the 49.7 M cell batch 966 -> 759; with the
 // global accesses taken out 58 / 635 / 566 at 2048^2 / 8192^2 / the batch, so it is bound by issue and
-// shared-memory latency with DRAM close behind.  Two at once: 53 / 712 / 654 (k_hydro_march_pair).
+// shared-memory latency with DRAM close behind.  Two at once: 52 / 703 / 647 (k_hydro_march_pair).
 // Rows live in rings of 16 rows indexed by the march's own row number (a chunk touches at most 15
 // consecutive rows of a ring).  A piece of a strip starts with three chunks of warm-up; every chunk
 // runs all three stages, and only the stores are limited to the piece's rows.  All strip-rows of the
@@ -509,7 +509,7 @@ __device__ __noinline__ void march_two_ieee(const PairParams &pp, const HydroWor
 // which is as close as the first's height and as far as the rings allow.
 // A sub-iteration moves 35 bytes a cell instead of 60 (DRAM 37% busy), and its instructions are as many as
 // alone (530 a 64 cells, issue 56%, the shared-memory pipe 59%); one sub-iteration, alone and of two, us:
-// 2048^2 72 -> 53, 4096^2 232 -> 187, 8192^2 852 -> 712, the 49.7 M cell batch 759 -> 654.  Leaving out, by a
+// 2048^2 72 -> 52, 4096^2 232 -> 187, 8192^2 852 -> 703, the 49.7 M cell batch 759 -> 647.  Leaving out, by a
 // test a chunk, the stages that a piece's first and last chunks do not need gains where pieces are short (1024^2
 // 24.6 -> 22) and loses elsewhere (8192^2 747 -> 805: the branches keep the compiler from overlapping stages).
 __global__ __launch_bounds__(2 * kPairThreads, 1) void k_hydro_march_pair(const __grid_constant__ PairParams pp)
