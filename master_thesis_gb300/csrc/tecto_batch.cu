@@ -488,11 +488,12 @@ extern "C" {
 int tecto_selftest_tiles(int width, int height, int world, int tile_x, int tile_y, unsigned long long *bad)
 {
     if (width < 1 || height < 1 || (long long)width * height > 1ll << 30 || world < 0 || world >= kMaxBatchWorlds ||
-        tile_x < 1 || tile_y < 1 || !bad)
+        tile_x < 1 || tile_y < 1 || tile_x > 1 << 16 || tile_y > 1 << 16 || !bad)
         return TECTO_ERR_INVALID;
+    const size_t nx = ((size_t)width + tile_x - 1) / tile_x, ny = ((size_t)height + tile_y - 1) / tile_y;
+    if (nx > 1u << 26 || ny > 1u << 28 || nx * ny > 1u << 27) return TECTO_ERR_INVALID;  // no phase has that many
     std::vector<uint2> tiles;
     add_tiles(world, width, height, tile_x, tile_y, tiles);
-    const size_t nx = (size_t)((width + tile_x - 1) / tile_x), ny = (size_t)((height + tile_y - 1) / tile_y);
     *bad = tiles.size() > nx * ny ? tiles.size() - nx * ny : nx * ny - tiles.size();
     for (size_t i = 0; i < tiles.size(); ++i) {
         int w, x, y;

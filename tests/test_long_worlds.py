@@ -27,6 +27,7 @@ def test_work_list_arguments():
     bad = C.c_ulonglong()
     f = T.lib().tecto_selftest_tiles
     assert f(0, 1, 0, 56, 4, C.byref(bad)) == -1 and f(1 << 20, 1 << 20, 0, 56, 4, C.byref(bad)) == -1
+    assert f(1 << 15, 1 << 15, 0, 1, 1, C.byref(bad)) == -1 and f(4, 4, 0, 1 << 20, 4, C.byref(bad)) == -1
     assert f(4, 4, 1024, 56, 4, C.byref(bad)) == -1 and f(4, 4, 0, 0, 4, C.byref(bad)) == -1 and f(4, 4, 0, 56, 4, None) == -1
 
 
